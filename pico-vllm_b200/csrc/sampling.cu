@@ -9,39 +9,29 @@
 // first token, in vocabulary order, at which the running sum of kept probabilities passes
 // uniform * kept mass, so a row's result depends only on its logits, parameters and uniform.
 //
-// A vocabulary of 150 k entries is 600 KB per row, so every pass over a row is made by several
-// blocks (grid: parts x rows), and the block that arrives last at the row's counter finishes the
-// pass.  Masses are summed as 32.32 fixed-point integers (weight = exp((x - max) / T) <= 1), so that
-// sums do not depend on the order in which blocks and threads add: the choice is reproducible.
+// A row (600 KB for a vocabulary of 150 k entries) belongs to one cluster of eight blocks: each reads an eighth of it once, keeps
+// it in shared memory through all the passes, and what the blocks have to tell one another goes through distributed shared memory.
+// Masses are summed as 32.32 fixed-point integers (weight = exp((x - max) / T) <= 1), so that sums do not depend on the order in
+// which blocks and threads add: the choice is reproducible.
 //   1. maximum and its first index (greedy rows end here);
 //   2. the kept set without sorting: token i is kept iff the mass of tokens with a larger weight is
 //      < top_p * total.  The smallest kept weight is found by its bit pattern, 11 + 11 + 10 bits at a
 //      time: a histogram of mass per value of the next bits among the weights that share the bits
 //      found so far, then the lowest bin whose mass above is still below the limit (equal weights
 //      are kept or dropped together);
-//   3. kept mass per part, the part and then the token at which the running sum passes the target.
+//   3. kept mass per block, the block and then the token at which the running sum passes the target.
+// A pass that is a kernel of its own, over the row in L2, with the blocks' results in device memory, costs 10 to 25 us at 64 rows
+// of 152,064 whatever it computes; the whole choice with top-p took 200 us as five of them (162 without top-p) and SAMPLE_US.
+// Longer rows than shared memory holds (ROW_MAX entries) are read again in every pass.
 #include "common.cuh"
 
-#define SAMPLE_THREADS 1024
-#define SAMPLE_MAX_PARTS 64
-#define SAMPLE_ROWS 128          // rows per round of launches
+#define SAMPLE_THREADS 512
+#define SAMPLE_BLOCKS 8          // of a row
 #define SAMPLE_BINS 2048
+#define SAMPLE_FLUSH 65532       // elements whose masses' halves fit into 32-bit sums
+#define SAMPLE_KEEP 19456        // elements of a block's part that shared memory keeps (two blocks on a multiprocessor)
 
 typedef unsigned long long u64;
-
-struct SampleRow {
-    float mx, inv_t;
-    int arg, sampled;            // sampled: 0 = done (greedy), 1 = goes through steps 2 and 3
-    int resolved;                // the smallest kept weight is known (top_p >= 1, or all bits found)
-    unsigned prefix, thresh;     // bits of the smallest kept weight found so far; its whole pattern
-    u64 total, limit, above;     // sum of all weights; top_p * total; mass above the bits found so far
-    int arrived[5];              // blocks that have finished each pass
-};
-__device__ SampleRow g_sample_rows[SAMPLE_ROWS];
-__device__ float g_sample_part_max[SAMPLE_ROWS * SAMPLE_MAX_PARTS];
-__device__ int g_sample_part_arg[SAMPLE_ROWS * SAMPLE_MAX_PARTS];
-__device__ u64 g_sample_part_kept[SAMPLE_ROWS * SAMPLE_MAX_PARTS];
-__device__ u64 g_sample_hist[SAMPLE_ROWS * SAMPLE_BINS];
 
 __device__ __forceinline__ float sample_weight(float x, float mx, float inv_t) { return expf((x - mx) * inv_t); }
 __device__ __forceinline__ u64 sample_fixed(float w) { return __float2ull_rz(w * 4294967296.0f); }
@@ -90,230 +80,230 @@ __device__ __forceinline__ int block_min_int(int v, int* scratch) {       // scr
     __syncthreads();
     return scratch[32];
 }
-// true in every thread of the one block that arrives last at the counter (which it then resets)
-__device__ __forceinline__ bool sample_last_block(int* counter, int blocks, int* flag) {
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int last = atomicAdd(counter, 1) == blocks - 1;
-        if (last) *counter = 0;
-        *flag = last;
-    }
-    __syncthreads();
-    const bool last = *flag != 0;
-    if (last) __threadfence();
-    return last;
+
+// what every block of the cluster has written to another's shared memory is there afterwards
+__device__ __forceinline__ void sample_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ uint32_t sample_at(const void* mine, int block) {      // the same place in another block's shared memory
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(block));
+    return r;
+}
+__device__ __forceinline__ void sample_put(const u64* mine, int block, u64 v) {
+    asm volatile("st.shared::cluster.u64 [%0], %1;\n" ::"r"(sample_at(mine, block)), "l"(v) : "memory");
+}
+__device__ __forceinline__ u64 sample_get(const u64* mine, int block) {
+    u64 v;
+    asm volatile("ld.shared::cluster.u64 %0, [%1];\n" : "=l"(v) : "r"(sample_at(mine, block)) : "memory");
+    return v;
 }
 
-// Step 1.  grid (parts, rows): block (p, r) takes elements [p * per, (p + 1) * per) of row r.
+// Grid (8, rows) in clusters of 8.  Block b takes elements [b * per, (b + 1) * per) of the row, per a multiple of 4.  KEEP: they stay in
+// shared memory (as weights from pass 2 on); vec: the row starts on 16 bytes and V is a multiple of 4.
+template <bool KEEP>
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_max_kernel(const float* __restrict__ logits, int row_stride, int V, const float* __restrict__ temperature,
-                  int* __restrict__ out, int per) {
+sample_row_kernel(const float* __restrict__ logits, int row_stride, int V, const float* __restrict__ temperature,
+                  const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out, int per, bool vec) {
     pdl_launch_dependents();
-    pdl_wait();
+    extern __shared__ __align__(16) unsigned char sample_smem[];
+    u64* hist = reinterpret_cast<u64*>(sample_smem);                  // [BINS]: this block's masses
+    unsigned* halves = reinterpret_cast<unsigned*>(hist + SAMPLE_BINS);       // [BINS] lower 16 bits, [BINS] upper: while they are summed
+    u64* all = reinterpret_cast<u64*>(halves);                        // [BINS]: the row's masses, when `halves` is done with
+    float* kept = reinterpret_cast<float*>(all + SAMPLE_BINS);        // KEEP: [per]
     __shared__ float scratch[33];
     __shared__ int iscratch[33];
-    __shared__ int flag;
-    const int r = blockIdx.y, parts = gridDim.x, tid = threadIdx.x;
+    __shared__ u64 scratch64[33];
+    __shared__ u64 told[SAMPLE_BLOCKS], told_kept[SAMPLE_BLOCKS];     // what the blocks say: maximum and index; kept mass
+    __shared__ u64 s_above;
+    const int r = blockIdx.y, rank = blockIdx.x, tid = threadIdx.x;
+    sample_cluster_sync();              // every block of the cluster runs before another writes to it
+    pdl_wait();
     const float* x = logits + (size_t)r * row_stride;
+    const int p0 = min(V, rank * per), n = min(V, p0 + per) - p0;
+    x += p0;
+
+    // ---- 1: the maximum and its first index; the elements into shared memory
     float best = -INFINITY;
     int best_i = 0x7fffffff;
-    {
-        const int p0 = min(V, (int)blockIdx.x * per), p1 = min(V, p0 + per);
-        for (int i = p0 + tid; i < p1; i += blockDim.x) {
-            const float v = x[i];
-            if (v > best) { best = v; best_i = i; }
-        }
-    }
-    const float pm = block_max(best, scratch);
-    const int pc = block_min_int(best == pm ? best_i : 0x7fffffff, iscratch);
-    if (tid == 0) {
-        g_sample_part_max[r * SAMPLE_MAX_PARTS + blockIdx.x] = pm;
-        g_sample_part_arg[r * SAMPLE_MAX_PARTS + blockIdx.x] = pc;
-    }
-    SampleRow& row = g_sample_rows[r];
-    if (!sample_last_block(&row.arrived[0], parts, &flag)) return;
-    // the parts in their order: the first index of the maximum stays the first
-    best = -INFINITY;
-    best_i = 0x7fffffff;
-    if (tid < parts) {
-        best = __ldcg(&g_sample_part_max[r * SAMPLE_MAX_PARTS + tid]);
-        best_i = __ldcg(&g_sample_part_arg[r * SAMPLE_MAX_PARTS + tid]);
-    }
-    const float mx = block_max(best, scratch);
-    const int arg = block_min_int(best == mx ? best_i : 0x7fffffff, iscratch);
-    const float temp = temperature ? temperature[r] : 0.f;
-    const bool greedy = !(temp > 0.f) || arg == 0x7fffffff;       // or a row without a finite maximum
-    for (int b = tid; b < SAMPLE_BINS; b += blockDim.x) g_sample_hist[r * SAMPLE_BINS + b] = 0ull;
-    if (tid == 0) {
-        if (greedy) out[r] = arg == 0x7fffffff ? 0 : arg;
-        row.mx = mx;
-        row.arg = arg == 0x7fffffff ? 0 : arg;
-        row.inv_t = greedy ? 0.f : 1.0f / temp;
-        row.sampled = greedy ? 0 : 1;
-        row.resolved = 0;
-        row.prefix = 0u;
-        row.thresh = 0u;
-        row.total = row.limit = row.above = 0ull;
-    }
-}
-
-// Step 2, LEVEL 0, 1, 2: mass per value of the next 11, 11, 10 bits of the weight's pattern.
-template <int LEVEL>
-__global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_hist_kernel(const float* __restrict__ logits, int row_stride, int V, const float* __restrict__ top_p, int per) {
-    pdl_launch_dependents();
-    pdl_wait();
-    __shared__ u64 sh[SAMPLE_BINS];
-    __shared__ u64 scratch[33];
-    __shared__ int iscratch[33];
-    __shared__ int flag;
-    const int r = blockIdx.y, parts = gridDim.x, tid = threadIdx.x;
-    SampleRow& row = g_sample_rows[r];
-    if (!row.sampled || row.resolved) return;          // written by an earlier kernel: the same for every block of the row
-    constexpr int NB = LEVEL == 2 ? 1024 : SAMPLE_BINS;
-    const float* x = logits + (size_t)r * row_stride;
-    const float mx = row.mx, inv_t = row.inv_t;
-    const unsigned prefix = row.prefix;
-    for (int b = tid; b < NB; b += blockDim.x) sh[b] = 0ull;
-    __syncthreads();
-    u64 zsum = 0ull;
-    {
-        const int p0 = min(V, (int)blockIdx.x * per), p1 = min(V, p0 + per);
-        for (int i = p0 + tid; i < p1; i += blockDim.x) {
-            const float w = sample_weight(x[i], mx, inv_t);
-            const unsigned pat = __float_as_uint(w);
-            const u64 fx = sample_fixed(w);
-            if (LEVEL == 0) {
-                zsum += fx;
-                atomicAdd(&sh[pat >> 21], fx);
-            } else if (LEVEL == 1) {
-                if ((pat >> 21) == prefix) atomicAdd(&sh[(pat >> 10) & 0x7ffu], fx);
-            } else {
-                if ((pat >> 10) == prefix) atomicAdd(&sh[pat & 0x3ffu], fx);
+    auto see = [&](float v, int i) {
+        if (v > best) { best = v; best_i = i; }
+    };
+    if (vec) {
+        constexpr int STEP = SAMPLE_THREADS * 4;
+        for (int i0 = tid * 4; i0 < n; i0 += 4 * STEP) {              // four loads of 16 bytes under way
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u * STEP < n) v[u] = *reinterpret_cast<const float4*>(x + i0 + u * STEP);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * STEP;
+                if (i < n) {
+                    if (KEEP) *reinterpret_cast<float4*>(kept + i) = v[u];
+                    see(v[u].x, p0 + i);
+                    see(v[u].y, p0 + i + 1);
+                    see(v[u].z, p0 + i + 2);
+                    see(v[u].w, p0 + i + 3);
+                }
             }
         }
-    }
-    __syncthreads();
-    for (int b = tid; b < NB; b += blockDim.x)
-        if (sh[b]) atomicAdd(&g_sample_hist[r * SAMPLE_BINS + b], sh[b]);
-    if (LEVEL == 0) {
-        u64 tot;
-        block_excl_scan_u64(zsum, scratch, &tot);
-        if (tid == 0) atomicAdd(&row.total, tot);
-    }
-    if (!sample_last_block(&row.arrived[1 + LEVEL], parts, &flag)) return;
-    // the lowest bin whose mass above (in higher bins, and above the bits found before) is below the limit
-    u64 limit = row.limit, base = row.above;
-    bool all = false;
-    if (LEVEL == 0) {
-        const u64 total = __ldcg(&row.total);
-        const float tp = top_p ? top_p[r] : 1.f;
-        all = !(tp < 1.f);
-        limit = (u64)((double)tp * (double)total);
-    }
-    // thread t takes bins NB - 1 - 2t and NB - 2 - 2t: descending, so that a prefix sum is the mass above
-    const int hi_bin = NB - 1 - 2 * tid, lo_bin = hi_bin - 1;
-    const u64 h_hi = hi_bin >= 0 ? __ldcg(&g_sample_hist[r * SAMPLE_BINS + hi_bin]) : 0ull;
-    const u64 h_lo = lo_bin >= 0 ? __ldcg(&g_sample_hist[r * SAMPLE_BINS + lo_bin]) : 0ull;
-    u64 tot;
-    const u64 before = base + block_excl_scan_u64(h_hi + h_lo, scratch, &tot);
-    int cand = 0x7fffffff;
-    if (hi_bin >= 0 && before < limit) cand = hi_bin;
-    if (lo_bin >= 0 && before + h_hi < limit) cand = lo_bin;
-    const int bin = block_min_int(cand, iscratch);
-    for (int b = tid; b < SAMPLE_BINS; b += blockDim.x) g_sample_hist[r * SAMPLE_BINS + b] = 0ull;      // for the next pass
-    if (all) {
-        if (tid == 0) { row.limit = limit; row.thresh = 0u; row.resolved = 1; }
-        return;
-    }
-    if (bin == 0x7fffffff) {          // a limit of zero: only the largest weight (1.0) is kept
-        if (tid == 0) { row.limit = limit; row.thresh = __float_as_uint(1.0f); row.resolved = 1; }
-        return;
-    }
-    // the mass above the chosen bin: this thread knows it if the bin is one of its two
-    if (bin == hi_bin || bin == lo_bin) {
-        row.limit = limit;
-        row.above = bin == hi_bin ? before : before + h_hi;
-        if (LEVEL == 0) row.prefix = (unsigned)bin;
-        else if (LEVEL == 1) row.prefix = (prefix << 11) | (unsigned)bin;
-        else {
-            row.thresh = (prefix << 10) | (unsigned)bin;
-            row.resolved = 1;
+    } else {
+#pragma unroll 4
+        for (int i = tid; i < n; i += SAMPLE_THREADS) {
+            const float v = x[i];
+            if (KEEP) kept[i] = v;
+            see(v, p0 + i);
         }
     }
-}
-
-// Step 3.  Kept mass per part; the last block finds the part and the token where the running sum passes the target.
-__global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_pick_kernel(const float* __restrict__ logits, int row_stride, int V, const float* __restrict__ uniform,
-                   int* __restrict__ out, int per) {
-    pdl_launch_dependents();
-    pdl_wait();
-    __shared__ u64 scratch[33];
-    __shared__ int iscratch[33];
-    __shared__ int flag;
-    __shared__ u64 sh_before;
-    const int r = blockIdx.y, parts = gridDim.x, tid = threadIdx.x;
-    SampleRow& row = g_sample_rows[r];
-    if (!row.sampled) return;
-    const float* x = logits + (size_t)r * row_stride;
-    const float mx = row.mx, inv_t = row.inv_t;
-    const unsigned thresh = row.thresh;
-    u64 mine = 0ull;
     {
-        const int p0 = min(V, (int)blockIdx.x * per), p1 = min(V, p0 + per);
-        for (int i = p0 + tid; i < p1; i += blockDim.x) {
-            const float w = sample_weight(x[i], mx, inv_t);
-            if (__float_as_uint(w) >= thresh) mine += sample_fixed(w);
+        const float pm = block_max(best, scratch);
+        const int pc = block_min_int(best == pm ? best_i : 0x7fffffff, iscratch);
+        if (tid < SAMPLE_BLOCKS) sample_put(told + rank, tid, ((u64)__float_as_uint(pm) << 32) | (unsigned)pc);
+    }
+    sample_cluster_sync();
+    float mx = -INFINITY;
+    int arg = 0x7fffffff;
+#pragma unroll
+    for (int b = 0; b < SAMPLE_BLOCKS; ++b) {                         // in the row's order: the first index of the maximum stays the first
+        const float m = __uint_as_float((unsigned)(told[b] >> 32));
+        const int i = (int)(unsigned)told[b];
+        if (m > mx || (m == mx && i < arg)) { mx = m; arg = i; }
+    }
+    const float temp = temperature ? temperature[r] : 0.f;
+    if (!(temp > 0.f) || arg == 0x7fffffff) {                         // greedy, or a row without a finite maximum
+        if (rank == 0 && tid == 0) out[r] = arg == 0x7fffffff ? 0 : arg;
+        return;
+    }
+    const float inv_t = 1.0f / temp;
+    const float tp = top_p ? top_p[r] : 1.f;
+
+    // ---- 2: the smallest kept weight
+    unsigned thresh = 0u, prefix = 0u;
+    bool weights = false;                                             // `kept` holds weights
+    if (tp < 1.f) {
+        u64 limit = 0ull, above = 0ull;
+        for (int level = 0; level < 3; ++level) {
+            const int bins = level == 2 ? 1024 : SAMPLE_BINS;
+            for (int f0 = 0; f0 < n || f0 == 0; f0 += SAMPLE_FLUSH) {
+                for (int b = tid; b < 2 * SAMPLE_BINS; b += SAMPLE_THREADS) halves[b] = 0u;
+                __syncthreads();
+                const int f1 = min(n, f0 + SAMPLE_FLUSH);
+#pragma unroll 4
+                for (int i = f0 + tid; i < f1; i += SAMPLE_THREADS) {
+                    float w;
+                    if (KEEP && level > 0) w = kept[i];
+                    else {
+                        w = sample_weight(KEEP ? kept[i] : x[i], mx, inv_t);
+                        if (KEEP) kept[i] = w;
+                    }
+                    const unsigned pat = __float_as_uint(w);
+                    const u64 fx = sample_fixed(w);
+                    if (fx == 0ull || (level == 1 && (pat >> 21) != prefix) || (level == 2 && (pat >> 10) != prefix)) continue;
+                    const unsigned bin = level == 0 ? pat >> 21 : level == 1 ? (pat >> 10) & 0x7ffu : pat & 0x3ffu;
+                    // (32-bit adds: 64-bit ones in shared memory are loops)
+                    atomicAdd(halves + bin, (unsigned)fx & 0xffffu);
+                    atomicAdd(halves + SAMPLE_BINS + bin, (unsigned)(fx >> 16));
+                }
+                __syncthreads();
+                for (int b = tid; b < SAMPLE_BINS; b += SAMPLE_THREADS) {
+                    const u64 m = (u64)halves[b] + ((u64)halves[SAMPLE_BINS + b] << 16);
+                    hist[b] = f0 == 0 ? m : hist[b] + m;
+                }
+                __syncthreads();
+            }
+            weights = KEEP;
+            sample_cluster_sync();                                    // every block's masses are there, every block's `halves` free
+            if (tid < SAMPLE_BINS / SAMPLE_BLOCKS) {                  // a block adds up its share of the bins and tells all
+                const int b = rank * (SAMPLE_BINS / SAMPLE_BLOCKS) + tid;
+                u64 sum = 0ull;
+#pragma unroll
+                for (int o = 0; o < SAMPLE_BLOCKS; ++o) sum += sample_get(hist + b, o);
+#pragma unroll
+                for (int o = 0; o < SAMPLE_BLOCKS; ++o) sample_put(all + b, o, sum);
+            }
+            sample_cluster_sync();
+            // the lowest bin whose mass above (in higher bins, and above the bits found before) is below the limit: thread t has
+            // four bins, descending, so that a prefix sum is the mass above
+            const int top = bins - 1 - 4 * tid;
+            u64 h[4], mine = 0ull, total;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                h[e] = top - e >= 0 ? all[top - e] : 0ull;
+                mine += h[e];
+            }
+            u64 before = above + block_excl_scan_u64(mine, scratch64, &total);
+            if (level == 0) limit = (u64)((double)tp * (double)total);
+            int cand = 0x7fffffff;
+            u64 cand_above = 0ull;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (top - e >= 0 && before < limit) {
+                    cand = top - e;
+                    cand_above = before;
+                }
+                before += h[e];
+            }
+            const int bin = block_min_int(cand, iscratch);
+            if (bin == 0x7fffffff) {                                  // a limit of zero: only the largest weight (1.0) is kept
+                thresh = __float_as_uint(1.0f);
+                break;
+            }
+            if (cand == bin) s_above = cand_above;
+            __syncthreads();
+            above = s_above;
+            prefix = level == 0 ? (unsigned)bin : level == 1 ? (prefix << 11) | (unsigned)bin : (prefix << 10) | (unsigned)bin;
+            thresh = prefix;
+            __syncthreads();                                          // `all` has been read, as has s_above
         }
     }
-    u64 part_kept;
-    block_excl_scan_u64(mine, scratch, &part_kept);
-    if (tid == 0) g_sample_part_kept[r * SAMPLE_MAX_PARTS + blockIdx.x] = part_kept;
-    if (!sample_last_block(&row.arrived[4], parts, &flag)) return;
-    // the parts in vocabulary order: the last part that is not empty and starts at or below the target
-    const u64 pk = tid < parts ? __ldcg(&g_sample_part_kept[r * SAMPLE_MAX_PARTS + tid]) : 0ull;
-    u64 kept;
-    const u64 pbefore = block_excl_scan_u64(pk, scratch, &kept);
-    const u64 target = (u64)((double)uniform[r] * (double)kept);
-    const int winner = -block_min_int((tid < parts && pk > 0ull && pbefore <= target) ? -tid : 1, iscratch);
-    if (winner < 0) {                 // nothing was kept (cannot happen with a finite maximum)
-        if (tid == 0) out[r] = row.arg;
-        return;
-    }
-    if (tid == winner) sh_before = pbefore;
-    __syncthreads();
-    // the winning part, a contiguous chunk per thread so that the scan runs in vocabulary order
-    const int p0 = min(V, winner * per), p1 = min(V, p0 + per);
-    const int chunk = (p1 - p0 + (int)blockDim.x - 1) / (int)blockDim.x;
-    const int c0 = min(p1, p0 + tid * chunk), c1 = min(p1, c0 + chunk);
-    u64 cmine = 0ull;
+
+    // ---- 3: kept mass, a run of neighbours a thread (an odd number: distinct banks), so that the scan is in the row's order
+    const int run = ((n + SAMPLE_THREADS - 1) / SAMPLE_THREADS) | 1;
+    const int c0 = min(n, tid * run), c1 = min(n, c0 + run);
+    auto weight = [&](int i) { return weights ? kept[i] : sample_weight(KEEP ? kept[i] : x[i], mx, inv_t); };
+    u64 mine = 0ull, part;
     for (int i = c0; i < c1; ++i) {
-        const float w = sample_weight(x[i], mx, inv_t);
-        if (__float_as_uint(w) >= thresh) cmine += sample_fixed(w);
+        const float w = weight(i);
+        if (__float_as_uint(w) >= thresh) mine += sample_fixed(w);
     }
-    u64 unused;
-    const u64 cbefore = sh_before + block_excl_scan_u64(cmine, scratch, &unused);
-    const int who = -block_min_int((cmine > 0ull && cbefore <= target) ? -tid : 1, iscratch);
-    if (who < 0) {
-        if (tid == 0) out[r] = row.arg;
+    u64 before = block_excl_scan_u64(mine, scratch64, &part);
+    if (tid < SAMPLE_BLOCKS) sample_put(told_kept + rank, tid, part);
+    sample_cluster_sync();
+    u64 mass = 0ull, start = 0ull;
+#pragma unroll
+    for (int b = 0; b < SAMPLE_BLOCKS; ++b) {
+        if (b < rank) start += told_kept[b];
+        mass += told_kept[b];
+    }
+    const u64 target = (u64)((double)uniform[r] * (double)mass);
+    int winner = -1;                    // the last block that is not empty and starts at or below the target
+    u64 at = 0ull;
+#pragma unroll
+    for (int b = 0; b < SAMPLE_BLOCKS; ++b) {
+        if (told_kept[b] > 0ull && at <= target) winner = b;
+        at += told_kept[b];
+    }
+    if (winner < 0) {                   // nothing was kept (cannot happen with a finite maximum)
+        if (rank == 0 && tid == 0) out[r] = arg;
         return;
     }
+    if (rank != winner) return;
+    before += start;
+    const int who = -block_min_int((mine > 0ull && before <= target) ? -tid : 1, iscratch);
     if (tid == who) {
-        u64 acc = cbefore;
         int pick = -1, last = -1;
         for (int i = c0; i < c1; ++i) {
-            const float w = sample_weight(x[i], mx, inv_t);
+            const float w = weight(i);
             if (__float_as_uint(w) >= thresh) {
                 const u64 fx = sample_fixed(w);
                 if (fx == 0ull) continue;
-                acc += fx;
-                last = i;
-                if (acc > target) { pick = i; break; }
+                before += fx;
+                last = p0 + i;
+                if (before > target) { pick = p0 + i; break; }
             }
         }
-        out[r] = pick >= 0 ? pick : (last >= 0 ? last : row.arg);
+        out[r] = pick >= 0 ? pick : (last >= 0 ? last : arg);
     }
 }
 
@@ -324,26 +314,22 @@ PICO_API int pico_sample(const float* logits, int row_stride, int R, int V, cons
     if (R <= 0) return 0;
     if (V <= 0) return PICO_ERR_SIZE;
     if (temperature && !uniform) return PICO_ERR_SIZE;
-    const int wave = 2 * pico_num_sms();
-    for (int r0 = 0; r0 < R; r0 += SAMPLE_ROWS) {
-        const int rows = R - r0 < SAMPLE_ROWS ? R - r0 : SAMPLE_ROWS;
-        // parts of at least 2048 entries, as many as give every SM a block or two
-        int parts = 1;
-        while (parts < SAMPLE_MAX_PARTS && parts * 2 * 2048 <= V && parts * rows < wave) parts *= 2;
-        const int per = (V + parts - 1) / parts;
+    const int per = ((V + SAMPLE_BLOCKS - 1) / SAMPLE_BLOCKS + 3) / 4 * 4;
+    const bool keep = per <= SAMPLE_KEEP;
+    const size_t smem = 2 * SAMPLE_BINS * sizeof(u64) + (keep ? (size_t)per * sizeof(float) : 0);
+    const bool vec = V % 4 == 0 && row_stride % 4 == 0 && ((uintptr_t)logits & 15) == 0;
+    for (int r0 = 0; r0 < R; r0 += 65535) {
+        const int rows = R - r0 < 65535 ? R - r0 : 65535;
         const float* lg = logits + (size_t)r0 * row_stride;
-        const dim3 grid(parts, rows), block(SAMPLE_THREADS);
-        pico_launch(sample_max_kernel, grid, block, 0, stream, lg, row_stride, V, temperature ? temperature + r0 : nullptr,
-                    out + r0, per);
-        if (temperature) {
-            const float* tp = top_p ? top_p + r0 : nullptr;
-            pico_launch(sample_hist_kernel<0>, grid, block, 0, stream, lg, row_stride, V, tp, per);
-            if (top_p) {
-                pico_launch(sample_hist_kernel<1>, grid, block, 0, stream, lg, row_stride, V, tp, per);
-                pico_launch(sample_hist_kernel<2>, grid, block, 0, stream, lg, row_stride, V, tp, per);
-            }
-            pico_launch(sample_pick_kernel, grid, block, 0, stream, lg, row_stride, V, uniform + r0, out + r0, per);
-        }
+        const float *t = temperature ? temperature + r0 : nullptr, *tp = top_p ? top_p + r0 : nullptr, *u = uniform ? uniform + r0 : nullptr;
+#define SAMPLE_LAUNCH(K)                                                                                                         \
+    do {                                                                                                                         \
+        cudaFuncSetAttribute(sample_row_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                      \
+        pico_launch_cluster((sample_row_kernel<K>), dim3(SAMPLE_BLOCKS, rows), dim3(SAMPLE_THREADS), smem, stream, SAMPLE_BLOCKS, \
+                            lg, row_stride, V, t, tp, u, out + r0, per, vec);                                                    \
+    } while (0)
+        if (keep) SAMPLE_LAUNCH(true); else SAMPLE_LAUNCH(false);
+#undef SAMPLE_LAUNCH
     }
     return pico_launch_status();
 }
