@@ -9,7 +9,7 @@ code path serves portions of prompts and single decoded tokens; the reference ha
 """
 from __future__ import annotations
 
-from dataclasses import dataclass
+from dataclasses import dataclass, replace
 from typing import List, Optional
 
 import torch
@@ -25,6 +25,9 @@ class AttentionPlan(MixerPlan):
     splits: int = 1            # parts each single token's key range is cut into
     pair_min_keys: int = 0     # > 0: prompt attention gives every query tile two blocks, which share a tile
                                # that sees at least this many keys (two partial results per token and head in scratch)
+
+
+MAX_MIXED_SCRATCH = 32 << 20       # float32 numbers (128 MB) that splitting the single tokens of a mixed step may ask for
 
 
 def decode_splits(shape: StepShape, n_kv_heads: int, window: Optional[int] = None) -> int:
@@ -80,7 +83,21 @@ class GQAAttention(Part):
         return AttentionPlan(key=(splits, pair), scratch_floats=scratch, splits=splits, pair_min_keys=pair)
 
     def _splits(self, shape: StepShape) -> int:
-        return decode_splits(shape, self.n_kv_heads)
+        """As :func:`decode_splits`, but where single tokens run in a kernel of their own beside the portions only they are
+        counted: 37 of them with 3,001 tokens at most beside two portions (2,013 tokens, 28 / 4 heads) make 148 blocks unsplit,
+        and the longest sets the time (MIXED_US).  Scratch is laid out for every token of the step: no more parts than
+        MAX_MIXED_SCRATCH holds."""
+        portions = sum(n for n in shape.q_lens if n > 1)
+        dtype = getattr(torch, getattr(shape.engine, "dtype", "") or "float32")
+        if not portions or not ops.mma_attention_takes(dtype, self.n_heads, self.n_kv_heads, self.head_dim):
+            return decode_splits(shape, self.n_kv_heads)
+        if portions == shape.num_tokens:
+            return 1
+        longest = max([st + n for n, st in zip(shape.q_lens, shape.starts) if n == 1], default=1)
+        splits = decode_splits(replace(shape, num_tokens=shape.num_tokens - portions, max_kv=longest), self.n_kv_heads)
+        while splits > 1 and ops.attention_scratch_floats(shape.num_tokens, self.n_heads, self.head_dim, splits) > MAX_MIXED_SCRATCH:
+            splits //= 2
+        return splits
 
     def _pair_min_keys(self, shape: StepShape) -> int:
         """Whether prompt attention should give every query tile two blocks (the threshold in keys, or 0):

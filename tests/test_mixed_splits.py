@@ -1,0 +1,33 @@
+"""Parts of the key range in steps that hold portions of prompts beside single tokens."""
+from pico_vllm_b200.config import EngineConfig
+from pico_vllm_b200.parts import GQAAttention, Rotary
+from pico_vllm_b200.parts import attention
+from pico_vllm_b200.parts.base import StepShape
+
+
+def _plan(q_lens, starts, dtype="bfloat16", heads=28, kv=4, sms=148, pad=0):
+    part = GQAAttention(512, heads, kv, 128, position=Rotary(128, 1e6))
+    T = sum(q_lens) + pad
+    return part.plan(StepShape(num_tokens=T, num_segments=len(q_lens) + pad, q_lens=q_lens, starts=starts,
+                               max_kv=max(n + s for n, s in zip(q_lens, starts)), decode_only=max(q_lens) == 1, num_sms=sms,
+                               engine=EngineConfig(dtype=dtype)))
+
+
+def test_only_single_tokens_are_counted_beside_portions():
+    alone = _plan([1] * 8, [3000] * 8)
+    assert alone.splits == 8
+    assert _plan([1] * 8 + [500], [3000] * 8 + [0]).splits == alone.splits
+    assert _plan([500, 1], [0, 3000]).splits == 16                   # few blocks: as a batch of one
+    assert _plan([500, 1], [4000, 100]).splits == 1                  # a long portion does not split a short single token
+    assert _plan([500], [3000]).splits == 1
+    assert _plan([500], [3000], pad=1).splits == 1                   # a padding row holds no keys
+
+
+def test_scratch_for_every_token_bounds_the_parts():
+    plan = _plan([1] * 8 + [2040], [3000] * 8 + [0])
+    assert plan.splits == 2 or plan.scratch_floats <= attention.MAX_MIXED_SCRATCH
+    assert 1 < plan.splits < 8 and plan.scratch_floats == 2048 * 28 * plan.splits * 130
+
+
+def test_the_32_bit_path_still_counts_every_token():
+    assert _plan([1] * 8 + [500], [3000] * 8 + [0], dtype="float32").splits == 1
