@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(128)
 delta_prepare_kernel(const float* __restrict__ xc, int xc_stride, int q_off, int k_off, const TA* __restrict__ proj,
                      int proj_stride, int b_off, const TA* __restrict__ dt, int dt_stride, const float* __restrict__ dt_bias,
                      const float* __restrict__ a_log, float* __restrict__ prep, int P, int H, int G, int d, float q_scale,
-                     float unit_eps, int back) {
+                     float unit_eps, int back, int vec) {
     pdl_launch_dependents();
     pdl_wait();
     const size_t t = blockIdx.x;
@@ -59,6 +59,50 @@ delta_prepare_kernel(const float* __restrict__ xc, int xc_stride, int q_off, int
         return;
     }
     const float* row = xc + t * xc_stride;
+    if (PER_HEAD && vec) {
+        // four numbers a lane, each read once (2,048 tokens of 6 heads of 128: PREP_US, 18 in two passes a number a load)
+        for (int g = warp; g < G; g += nw) {
+            const int i = lane * 4;
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 a = zero, b = zero, c[3] = {zero, zero, zero};
+            if (i < d) {
+                a = *reinterpret_cast<const float4*>(row + q_off + g * d + i);
+                b = *reinterpret_cast<const float4*>(row + k_off + g * d + i);
+                if (back) {
+#pragma unroll
+                    for (int j = 0; j < 3; ++j)
+                        if (t > j) c[j] = *reinterpret_cast<const float4*>(row - (size_t)(j + 1) * xc_stride + k_off + g * d + i);
+                }
+            }
+            auto dot = [](float4 x, float4 y) { return fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, x.x * y.x))); };
+            float s[12] = {dot(a, a), dot(b, b), dot(a, b), dot(c[0], c[0]), dot(c[1], c[1]), dot(c[2], c[2]),
+                           dot(a, c[0]), dot(a, c[1]), dot(a, c[2]), dot(b, c[0]), dot(b, c[1]), dot(b, c[2])};
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+                for (int x = 0; x < 12; ++x)
+                    if (x < 3 || back) s[x] += __shfl_xor_sync(0xffffffffu, s[x], o);
+            }
+            const float iq = q_scale / sqrtf(s[0] + unit_eps), ik = 1.0f / sqrtf(s[1] + unit_eps);
+            if (i < d) {
+                *reinterpret_cast<float4*>(out + g * d + i) = make_float4(a.x * iq, a.y * iq, a.z * iq, a.w * iq);
+                *reinterpret_cast<float4*>(out + G * d + g * d + i) = make_float4(b.x * ik, b.y * ik, b.z * ik, b.w * ik);
+            }
+            if (lane == 0) {
+                float* dots = out + 2 * G * d + 4 * H + 8 * g;
+                dots[0] = s[2] * iq * ik;
+                if (back) {
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        const float in = 1.0f / sqrtf(s[3 + j] + unit_eps);
+                        dots[1 + j] = s[6 + j] * iq * in;
+                        dots[4 + j] = s[9 + j] * ik * in;
+                    }
+                }
+            }
+        }
+        return;
+    }
     for (int g = warp; g < G; g += nw) {
         float sq = 0.f, sk = 0.f;
         for (int i = lane; i < d; i += 32) {
@@ -118,9 +162,10 @@ PICO_API int pico_delta_prepare(const float* xc, int xc_stride, int q_off, int k
     if (H < 1 || G < 1 || H % G || d < 1 || H + 1 > 65535) return PICO_ERR_SIZE;
     const int P = 2 * G * d + (per_head ? 4 * H + 8 * G : H * d + H + G);
     const dim3 grid(T, per_head ? 1 : 1 + H);
+    const int vec = d % 4 == 0 && d <= 128 && xc_stride % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && (((uintptr_t)xc | (uintptr_t)prep) & 15) == 0;
 #define DP_LAUNCH(TA, PH)                                                                                                   \
     pico_launch((delta_prepare_kernel<TA, PH>), grid, dim3(128), 0, stream, xc, xc_stride, q_off, k_off, (const TA*)proj,   \
-                proj_stride, b_off, (const TA*)dt, dt_stride, dt_bias, a_log, prep, P, H, G, d, q_scale, unit_eps, back)
+                proj_stride, b_off, (const TA*)dt, dt_stride, dt_bias, a_log, prep, P, H, G, d, q_scale, unit_eps, back, vec)
     if (dtype == PICO_F32) { if (per_head) DP_LAUNCH(float, true); else DP_LAUNCH(float, false); }
     else if (dtype == PICO_BF16) { if (per_head) DP_LAUNCH(bf16, true); else DP_LAUNCH(bf16, false); }
     else
@@ -532,6 +577,482 @@ gated_delta_block_kernel(const float* __restrict__ prep, int P, const float* __r
             if (col < dv && i + 1 < d) st[(size_t)col * d + i + 1] = f.y;
         }
     }
+}
+
+// ------------------------------------------------------------------------------------------ thirty-two tokens at a time
+// The same recurrence for a whole chunk of C = 32 tokens, as products of small matrices (the chunked form of the delta rule:
+// Yang, Wang, Zhang, Shen, Kim, "Parallelizing Linear Transformers with the Delta Rule over Sequence Length", with the decays of
+// Yang, Kautz, Hatamizadeh, "Gated Delta Networks").  With D_ij = g_(j+1) ... g_i, G_i = g_1 ... g_i, rows k_i, q_i, v_i:
+//
+//   L_ij = beta_i D_ij (k_i . k_j) for j < i        M = (I + L)^-1 diag(beta)        E_ij = D_ij (q_i . k_j) for j <= i
+//   U = M V - (M diag(G) K) S        S' = G_C S + K^T diag(D_Cj) U        O = diag(G) Q S + E U
+//
+// Only U and S' depend on the chunk before, so the work is in three kernels: M V, M diag(G) K and E for all chunks side by side;
+// the chain from chunk to chunk, two products, which leaves U and every chunk's S behind; O for all chunks side by side.  All
+// float32; decays are products of decays (none is above one, nothing is divided), the inverse comes from forward substitution.
+// Tokens beyond a segment's end are blanks (k = q = v = 0, beta = 0, g = 1).
+// The chain is bound by what a block reads from shared memory (K, M diag(G) K and S once a chunk for every four columns), over
+// len / 32 dependent steps of the longest segment: hence the two products only (with all four in the chain 170 us for the
+// tokens below), four warps a block (eight, with half the columns each: 225) and 16 columns.
+// 2,048 tokens of twelve heads with d = dv = 128 in segments of 341, 682 and 1,025: CHUNK_US (four tokens at a time: 248).
+#define DC_C 32
+#define DC_D 128                               // rows of S, keys padded with zeros
+#define DC_LD (DC_D + 4)                       // rows that lanes read side by side, 16 bytes each
+#define DC_LDK (DC_D + 16)                     // rows that four lanes read 64 bytes of
+#define DC_NC 16                               // columns of S a block of the chain
+#define DC_OC 128                              // columns of O a block
+#define DC_COEF (DC_C * DC_D + DC_C * DC_C + 2 * DC_C)      // floats a chunk and head: M diag(G) K, E by columns, G, D_Cj
+
+// Which chunk of which segment number c is; false when there are not that many, or it is padding.
+__device__ __forceinline__ bool dc_find(const int* __restrict__ cu_q, const int* __restrict__ positions, int S, int c, int& t0, int& n) {
+    for (int seg = 0; seg < S; ++seg) {
+        const int begin = cu_q[seg], len = cu_q[seg + 1] - begin, k = (len + DC_C - 1) / DC_C;
+        if (c < k) {
+            t0 = begin + c * DC_C;
+            n = min(DC_C, len - c * DC_C);
+            return positions[begin] >= 0;
+        }
+        c -= k;
+    }
+    return false;
+}
+
+// Grid (chunks at most, G): block (c, g) takes the heads of query/key head g.  u0 float32 [T, H * dv]: M V.
+__global__ void __launch_bounds__(256)
+delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* __restrict__ v, int v_stride, const int* __restrict__ cu_q,
+                           const int* __restrict__ positions, int S, float* __restrict__ coef, float* __restrict__ u0, int H, int G,
+                           int d, int dv) {
+    pdl_launch_dependents();
+    pdl_wait();
+    int t0, n;
+    if (!dc_find(cu_q, positions, S, blockIdx.x, t0, n)) return;
+    extern __shared__ __align__(16) float dsm[];
+    float* k_s = dsm;                          // [C][LD]
+    float* q_s = k_s + DC_C * DC_LD;
+    float* kk = q_s + DC_C * DC_LD;            // [C][C + 1]: k_i . k_j
+    float* qk = kk + DC_C * (DC_C + 1);        // q_i . k_j
+    float* l_s = qk + DC_C * (DC_C + 1);       // a head's L [C][C], then M by columns; one for each of the warps that take heads
+    float* g_s = l_s + 8 * DC_C * DC_C;        // [8][C]: G
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = blockIdx.y;
+    for (int idx = threadIdx.x; idx < DC_C * (DC_D / 4); idx += 256) {
+        const int i = idx / (DC_D / 4), c = idx % (DC_D / 4) * 4;
+        float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), q4 = k4;
+        if (i < n && c < d) {
+            const float* row = prep + (size_t)(t0 + i) * P + g * d + c;
+            q4 = *reinterpret_cast<const float4*>(row);
+            k4 = *reinterpret_cast<const float4*>(row + G * d);
+        }
+        *reinterpret_cast<float4*>(k_s + i * DC_LD + c) = k4;
+        *reinterpret_cast<float4*>(q_s + i * DC_LD + c) = q4;
+    }
+    __syncthreads();
+    {   // lane: token j; a warp: tokens i = 4 warp .. + 3 of both products, over even and odd places
+        f32x2 sk[4], sq[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sk[i] = sq[i] = db_pair(0.f, 0.f);
+#pragma unroll 4
+        for (int c = 0; c < DC_D; c += 4) {
+            const ulonglong2 kj = *reinterpret_cast<const ulonglong2*>(k_s + lane * DC_LD + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const ulonglong2 ki = *reinterpret_cast<const ulonglong2*>(k_s + (4 * warp + i) * DC_LD + c);
+                const ulonglong2 qi = *reinterpret_cast<const ulonglong2*>(q_s + (4 * warp + i) * DC_LD + c);
+                sk[i] = db_fma2(ki.y, kj.y, db_fma2(ki.x, kj.x, sk[i]));
+                sq[i] = db_fma2(qi.y, kj.y, db_fma2(qi.x, kj.x, sq[i]));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 a = db_split(sk[i]), b = db_split(sq[i]);
+            kk[(4 * warp + i) * (DC_C + 1) + lane] = a.x + a.y;
+            qk[(4 * warp + i) * (DC_C + 1) + lane] = b.x + b.y;
+        }
+    }
+    __syncthreads();
+    const int heads = H / G;
+    for (int h0 = 0; h0 < heads; h0 += 8) {    // eight heads at a time, a warp each
+        if (h0 + warp < heads) {
+            const int h = g * heads + h0 + warp;
+            float* L = l_s + warp * DC_C * DC_C;
+            // lane i: decay and beta of token i
+            float a = 1.f, beta = 0.f;
+            if (lane < n) {
+                const float2 ab = *reinterpret_cast<const float2*>(prep + (size_t)(t0 + lane) * P + 2 * G * d + 4 * h);
+                a = ab.x;
+                beta = ab.y;
+            }
+            float* out = coef + ((size_t)blockIdx.x * H + h) * DC_COEF + DC_C * DC_D;
+            // lane j: column j of L (to shared memory) and of E
+            float D = 1.f, Gi = 1.f, E[DC_C];
+#pragma unroll
+            for (int i = 0; i < DC_C; ++i) {
+                const float ai = __shfl_sync(0xffffffffu, a, i), bi = __shfl_sync(0xffffffffu, beta, i);
+                if (i > lane) D *= ai;
+                if (i <= lane) Gi *= ai;
+                L[i * DC_C + lane] = i > lane ? bi * D * kk[i * (DC_C + 1) + lane] : 0.f;
+                E[i] = i >= lane ? D * qk[i * (DC_C + 1) + lane] : 0.f;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < DC_C; i += 4)
+                *reinterpret_cast<float4*>(out + lane * DC_C + i) = make_float4(E[i], E[i + 1], E[i + 2], E[i + 3]);
+            out[DC_C * DC_C + lane] = Gi;
+            out[DC_C * DC_C + DC_C + lane] = D;
+            g_s[warp * DC_C + lane] = Gi;
+            // lane j: column j of (I + L)^-1, row after row
+            float X[DC_C];
+#pragma unroll
+            for (int i = 0; i < DC_C; ++i) X[i] = 0.f;
+#pragma unroll
+            for (int i = 0; i < DC_C; ++i) {
+                float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+                for (int l = 0; l < i; l += 4) {           // (a row of L is nought from its own place on)
+                    const float4 m = *reinterpret_cast<const float4*>(L + i * DC_C + l);
+                    s0 = fmaf(m.x, X[l], s0);
+                    s1 = fmaf(m.y, X[l + 1], s1);
+                    s2 = fmaf(m.z, X[l + 2], s2);
+                    s3 = fmaf(m.w, X[l + 3], s3);
+                }
+                X[i] = (i == lane ? 1.f : 0.f) - ((s0 + s1) + (s2 + s3));
+            }
+            __syncwarp();                                  // L has been read: M by columns takes its place
+#pragma unroll
+            for (int i = 0; i < DC_C; i += 4)
+                *reinterpret_cast<float4*>(L + lane * DC_C + i) = make_float4(X[i] * beta, X[i + 1] * beta, X[i + 2] * beta, X[i + 3] * beta);
+        }
+        __syncthreads();
+        // M diag(G) K and M V, the heads one after the other: a thread has four columns and eight tokens i
+        const int cg = DC_D / 4 + (dv + 3) / 4;
+        for (int hh = 0; hh < 8 && h0 + hh < heads; ++hh) {
+            const int h = g * heads + h0 + hh;
+            const float* M = l_s + hh * DC_C * DC_C;
+            float* mgk = coef + ((size_t)blockIdx.x * H + h) * DC_COEF;
+            for (int idx = threadIdx.x; idx < 4 * cg; idx += 256) {
+                const int c = idx % cg * 4, i0 = idx / cg * 8;
+                const bool of_k = c < DC_D;
+                float acc[8][4];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+                const float* vc = v + (size_t)t0 * v_stride + (size_t)h * dv + (of_k ? 0 : c - DC_D);
+#pragma unroll 4
+                for (int j = 0; j < DC_C; ++j) {
+                    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (of_k) {
+                        b = *reinterpret_cast<const float4*>(k_s + j * DC_LD + c);
+                        const float gj = g_s[hh * DC_C + j];
+                        b = make_float4(gj * b.x, gj * b.y, gj * b.z, gj * b.w);
+                    } else if (j < n) {
+                        b = *reinterpret_cast<const float4*>(vc + (size_t)j * v_stride);
+                    }
+                    float m[8];
+                    *reinterpret_cast<float4*>(m) = *reinterpret_cast<const float4*>(M + j * DC_C + i0);
+                    *reinterpret_cast<float4*>(m + 4) = *reinterpret_cast<const float4*>(M + j * DC_C + i0 + 4);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        acc[i][0] = fmaf(m[i], b.x, acc[i][0]);
+                        acc[i][1] = fmaf(m[i], b.y, acc[i][1]);
+                        acc[i][2] = fmaf(m[i], b.z, acc[i][2]);
+                        acc[i][3] = fmaf(m[i], b.w, acc[i][3]);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float4 r = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+                    if (of_k) *reinterpret_cast<float4*>(mgk + (i0 + i) * DC_D + c) = r;
+                    else if (i0 + i < n) *reinterpret_cast<float4*>(u0 + (size_t)(t0 + i0 + i) * H * dv + (size_t)h * dv + c - DC_D) = r;
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// The chain.  Grid (column tiles, H, segments), four warps.  S is kept by the threads (lane: rows 4 lane .. + 3, warp: columns 4 warp ..
+// + 3) and, by columns, in shared memory for the product with it.  u: M V on the way in, U on the way out; s0 float32 [chunks, H,
+// dv rounded up to 4, 128]: S before each chunk, by columns.
+__global__ void __launch_bounds__(128)
+delta_chunk_kernel(const float* __restrict__ prep, int P, float* __restrict__ state, const int* __restrict__ seg_slots,
+                   const int* __restrict__ cu_q, const int* __restrict__ positions, const float* __restrict__ coef, float* __restrict__ u,
+                   float* __restrict__ s0, int H, int G, int d, int dv) {
+    pdl_wait();                         // the kernel that follows is released at the end (see above)
+    extern __shared__ __align__(16) float dsm[];
+    constexpr int MG = DC_C * DC_LDK, BUF = 2 * MG + 2 * DC_C + DC_C * DC_NC;      // a chunk: K, M diag(G) K, G, D_Cj, M V [C][NC]
+    const int seg = blockIdx.z, h = blockIdx.y, col_base = blockIdx.x * DC_NC;
+    const int t_begin = cu_q[seg], t_end = cu_q[seg + 1];
+    if (t_end <= t_begin || positions[t_begin] < 0) return;      // an empty or a padding segment
+    float* s_s = dsm + 2 * BUF;                // S by columns [NC][LDK]
+    float* w_s = s_s + DC_NC * DC_LDK;         // diag(D_Cj) U [C][NC]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hq = h / (H / G);
+    int chunk = 0;
+    for (int s = 0; s < seg; ++s) chunk += (cu_q[s + 1] - cu_q[s] + DC_C - 1) / DC_C;
+    auto fetch = [&](int t0, int ch, float* buf) {
+        const int n = min(DC_C, t_end - t0);
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* cf = coef + ((size_t)ch * H + h) * DC_COEF;
+        for (int idx = threadIdx.x; idx < DC_C * (DC_D / 4); idx += 128) {
+            const int i = idx / (DC_D / 4), c = idx % (DC_D / 4) * 4;
+            float* dst = buf + i * DC_LDK + c;
+            if (i < n && c < d) dr_cp16(dst, prep + (size_t)(t0 + i) * P + G * d + hq * d + c);
+            else *reinterpret_cast<float4*>(dst) = zero;
+            dr_cp16(dst + MG, cf + i * DC_D + c);
+        }
+        if (threadIdx.x < 2 * DC_C / 4) dr_cp16(buf + 2 * MG + 4 * threadIdx.x, cf + DC_C * DC_D + DC_C * DC_C + 4 * threadIdx.x);
+        {
+            const int i = threadIdx.x / (DC_NC / 4), c = threadIdx.x % (DC_NC / 4) * 4;
+            float* dst = buf + 2 * MG + 2 * DC_C + i * DC_NC + c;
+            if (i < n && col_base + c < dv) dr_cp16(dst, u + (size_t)(t0 + i) * H * dv + (size_t)h * dv + col_base + c);
+            else *reinterpret_cast<float4*>(dst) = zero;
+        }
+        dr_commit();
+    };
+    fetch(t_begin, chunk, dsm);
+    float* st = state + ((size_t)seg_slots[seg] * H + h) * (size_t)dv * d;
+    f32x2 S[4][2];                             // [column][row pair]
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int col = col_base + 4 * warp + c;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (col < dv && 4 * lane < d) x = *reinterpret_cast<const float4*>(st + (size_t)col * d + 4 * lane);
+        S[c][0] = db_pair(x.x, x.y);
+        S[c][1] = db_pair(x.z, x.w);
+        *reinterpret_cast<float4*>(s_s + (4 * warp + c) * DC_LDK + 4 * lane) = x;
+    }
+    // the product with S: a lane has rows rt, rt + 8, .. of M diag(G) K, columns 4 warp .. + 3, and of the sums over the rows of S
+    // every fourth four (kg)
+    const int kg = lane & 3, rt = lane >> 2;
+    int turn = 0;
+    for (int t0 = t_begin; t0 < t_end; t0 += DC_C, turn ^= 1, ++chunk) {
+        dr_wait_all();
+        __syncthreads();                       // the chunk is in, S is written, everyone is done with the other buffer
+        if (t0 + DC_C < t_end) fetch(t0 + DC_C, chunk + 1, dsm + (turn ? 0 : BUF));
+        const float* buf = dsm + (turn ? BUF : 0);
+        const float *k_s = buf, *Gd = buf + 2 * MG, *Wd = Gd + DC_C, *u_s = Wd + DC_C;
+        {
+            f32x2 acc[4][4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[r][e] = db_pair(0.f, 0.f);
+            const float* row = buf + MG + rt * DC_LDK + 4 * kg;
+            const float* c0 = s_s + 4 * warp * DC_LDK + 4 * kg;
+#pragma unroll 4
+            for (int c = 0; c < DC_D; c += 16) {
+                ulonglong2 b[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) b[e] = *reinterpret_cast<const ulonglong2*>(c0 + e * DC_LDK + c);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(row + r * 8 * DC_LDK + c);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[r][e] = db_fma2(a.y, b[e].y, db_fma2(a.x, b[e].x, acc[r][e]));
+                }
+            }
+            // S before this chunk, for the outputs
+            float* s_out = s0 + (((size_t)chunk * H + h) * ((dv + 3) / 4 * 4) + col_base + 4 * warp) * DC_D + 4 * lane;
+            if (col_base + 4 * warp < dv) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float2 a = db_split(S[c][0]), b = db_split(S[c][1]);
+                    *reinterpret_cast<float4*>(s_out + c * DC_D) = make_float4(a.x, a.y, b.x, b.y);
+                }
+            }
+            // the four lanes' sums: each lane ends with one row
+            float s[4][4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 f = db_split(acc[r][e]);
+                    s[r][e] = f.x + f.y;
+                }
+            const bool hi = kg & 1, second = kg & 2;
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float send = hi ? s[r][e] : s[r + 2][e], keep = hi ? s[r + 2][e] : s[r][e];
+                    s[r][e] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+                }
+            float x[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float send = second ? s[0][e] : s[1][e], keep = second ? s[1][e] : s[0][e];
+                x[e] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+            }
+            const int i = rt + 8 * ((hi ? 2 : 0) + (second ? 1 : 0));
+            const float4 mv = *reinterpret_cast<const float4*>(u_s + i * DC_NC + 4 * warp);
+            const float4 uu = make_float4(mv.x - x[0], mv.y - x[1], mv.z - x[2], mv.w - x[3]);
+            const float wj = Wd[i];
+            *reinterpret_cast<float4*>(w_s + i * DC_NC + 4 * warp) = make_float4(wj * uu.x, wj * uu.y, wj * uu.z, wj * uu.w);
+            if (t0 + i < t_end && col_base + 4 * warp < dv)
+                *reinterpret_cast<float4*>(u + (size_t)(t0 + i) * H * dv + (size_t)h * dv + col_base + 4 * warp) = uu;
+        }
+        __syncthreads();                       // everyone has read S
+        {
+            const float gc = Gd[DC_C - 1];
+            const f32x2 g2 = db_pair(gc, gc);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                S[c][0] = db_mul2(S[c][0], g2);
+                S[c][1] = db_mul2(S[c][1], g2);
+            }
+#pragma unroll 8
+            for (int j = 0; j < DC_C; ++j) {
+                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(k_s + j * DC_LDK + 4 * lane);
+                const float4 w = *reinterpret_cast<const float4*>(w_s + j * DC_NC + 4 * warp);
+                const float wc[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const f32x2 w2 = db_pair(wc[c], wc[c]);
+                    S[c][0] = db_fma2(k.x, w2, S[c][0]);
+                    S[c][1] = db_fma2(k.y, w2, S[c][1]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                ulonglong2 x;
+                x.x = S[c][0];
+                x.y = S[c][1];
+                *reinterpret_cast<ulonglong2*>(s_s + (4 * warp + c) * DC_LDK + 4 * lane) = x;
+            }
+        }
+    }
+    pdl_launch_dependents();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int col = col_base + 4 * warp + c;
+        const float2 a = db_split(S[c][0]), b = db_split(S[c][1]);
+        if (col < dv && 4 * lane < d) *reinterpret_cast<float4*>(st + (size_t)col * d + 4 * lane) = make_float4(a.x, a.y, b.x, b.y);
+    }
+}
+
+// The outputs.  Grid (chunks at most, H, tiles of 128 columns): O = diag(G) Q S + E U; a thread has tokens 8 ty .. + 7 and columns tx, tx +
+// 32, ..
+__global__ void __launch_bounds__(128)
+delta_chunk_out_kernel(const float* __restrict__ prep, int P, const int* __restrict__ cu_q, const int* __restrict__ positions, int S,
+                       const float* __restrict__ coef, const float* __restrict__ u, const float* __restrict__ s0, float* __restrict__ out,
+                       int out_stride, int H, int G, int d, int dv) {
+    pdl_launch_dependents();
+    pdl_wait();
+    int t0, n;
+    if (!dc_find(cu_q, positions, S, blockIdx.x, t0, n)) return;
+    extern __shared__ __align__(16) float dsm[];
+    float* s_s = dsm;                          // [OC][LD]: S by columns
+    float* q_s = s_s + DC_OC * DC_LD;          // [C][LD]: Q
+    float* u_s = q_s + DC_C * DC_LD;           // [C][OC]
+    float* e_s = u_s + DC_C * DC_OC;           // [C][C]: E by columns, then G
+    const int h = blockIdx.y, hq = h / (H / G), col_base = blockIdx.z * DC_OC, cols = min(DC_OC, dv - col_base);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float* sc = s0 + (((size_t)blockIdx.x * H + h) * ((dv + 3) / 4 * 4) + col_base) * DC_D;
+    const float* cf = coef + ((size_t)blockIdx.x * H + h) * DC_COEF + DC_C * DC_D;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int idx = threadIdx.x; idx < DC_OC * (DC_D / 4); idx += 128) {
+        const int c = idx / (DC_D / 4), i = idx % (DC_D / 4) * 4;
+        float* dst = s_s + c * DC_LD + i;
+        if (c < cols) dr_cp16(dst, sc + (size_t)c * DC_D + i);
+        else *reinterpret_cast<float4*>(dst) = zero;
+    }
+    for (int idx = threadIdx.x; idx < DC_C * (DC_D / 4); idx += 128) {
+        const int i = idx / (DC_D / 4), c = idx % (DC_D / 4) * 4;
+        float* dst = q_s + i * DC_LD + c;
+        if (i < n && c < d) dr_cp16(dst, prep + (size_t)(t0 + i) * P + hq * d + c);
+        else *reinterpret_cast<float4*>(dst) = zero;
+        dst = u_s + i * DC_OC + c;
+        if (i < n && c < cols) dr_cp16(dst, u + (size_t)(t0 + i) * H * dv + (size_t)h * dv + col_base + c);
+        else *reinterpret_cast<float4*>(dst) = zero;
+    }
+    for (int idx = threadIdx.x; idx < (DC_C * DC_C + DC_C) / 4; idx += 128) dr_cp16(e_s + 4 * idx, cf + 4 * idx);
+    dr_commit();
+    dr_wait_all();
+    __syncthreads();
+    // warp: tokens 8 warp .. + 7, lane: columns lane, lane + 32, ..
+    f32x2 acc[8][4];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[r][e] = db_pair(0.f, 0.f);
+    const float* row = q_s + 8 * warp * DC_LD;
+    const float* col = s_s + lane * DC_LD;
+#pragma unroll 2
+    for (int c = 0; c < DC_D; c += 4) {
+        ulonglong2 b[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) b[e] = *reinterpret_cast<const ulonglong2*>(col + 32 * e * DC_LD + c);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(row + r * DC_LD + c);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[r][e] = db_fma2(a.y, b[e].y, db_fma2(a.x, b[e].x, acc[r][e]));
+        }
+    }
+    float o[8][4];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const float gi = e_s[DC_C * DC_C + 8 * warp + r];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = db_split(acc[r][e]);
+            o[r][e] = gi * (f.x + f.y);
+        }
+    }
+    for (int j = 0; j < 8 * warp + 8; ++j) {           // (E is nought beyond a token's own place)
+        float ev[8], uv[4];
+        *reinterpret_cast<float4*>(ev) = *reinterpret_cast<const float4*>(e_s + j * DC_C + 8 * warp);
+        *reinterpret_cast<float4*>(ev + 4) = *reinterpret_cast<const float4*>(e_s + j * DC_C + 8 * warp + 4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) uv[e] = u_s[j * DC_OC + lane + 32 * e];
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[r][e] = fmaf(ev[r], uv[e], o[r][e]);
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int i = 8 * warp + r;
+        if (i >= n) break;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int c = lane + 32 * e;
+            if (c < cols) out[(size_t)(t0 + i) * out_stride + (size_t)h * dv + col_base + c] = o[r][e];
+        }
+    }
+}
+
+// Floats of scratch that pico_gated_delta_chunks needs for T tokens in S segments: coefficients, U, S before every chunk.
+static long long dc_chunks(int T, int S) { return (long long)T / DC_C + S; }
+PICO_API long long pico_gated_delta_chunk_floats(int T, int S, int H, int dv) {
+    return dc_chunks(T, S) * H * (DC_COEF + (long long)((dv + 3) / 4 * 4) * DC_D) + (long long)T * H * dv;
+}
+
+// The recurrence with one decay a head in chunks; T: tokens of all segments.  d up to 128; d, dv, the strides multiples of 4, all
+// addresses of 16 bytes: anything else is refused.
+PICO_API int pico_gated_delta_chunks(const float* prep, const float* v, int v_stride, float* state, const int* seg_slots,
+                                     const int* cu_q, const int* positions, float* out, int out_stride, int T, int S, int H, int G,
+                                     int d, int dv, float* scratch, cudaStream_t stream) {
+    if (S <= 0 || T <= 0) return 0;
+    if (H < 1 || G < 1 || H % G || d < 4 || d > DC_D || dv < 4) return PICO_ERR_SIZE;
+    if (d % 4 || dv % 4 || v_stride % 4 || out_stride % 4 || (((uintptr_t)prep | (uintptr_t)v | (uintptr_t)state | (uintptr_t)out | (uintptr_t)scratch) & 15))
+        return PICO_ERR_ALIGN;
+    if (S > 65535 || H > 65535 || (dv + DC_OC - 1) / DC_OC > 65535 || dc_chunks(T, S) > 0x7fffffffLL) return PICO_ERR_SIZE;
+    const int P = 2 * G * d + 4 * H + 8 * G, chunks = (int)dc_chunks(T, S);
+    float* coef = scratch;
+    float* s0 = coef + (size_t)chunks * H * DC_COEF;
+    float* u = s0 + (size_t)chunks * H * ((dv + 3) / 4 * 4) * DC_D;
+    const size_t sm1 = (size_t)(2 * DC_C * DC_LD + 2 * DC_C * (DC_C + 1) + 8 * DC_C * DC_C + 8 * DC_C) * sizeof(float);
+    cudaFuncSetAttribute(delta_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
+    pico_launch(delta_chunk_prepare_kernel, dim3(chunks, G), dim3(256), sm1, stream, prep, P, v, v_stride, cu_q, positions, S, coef, u, H, G, d, dv);
+    const dim3 grid((dv + DC_NC - 1) / DC_NC, H, S);
+    size_t sm2 = (size_t)(2 * (2 * DC_C * DC_LDK + 2 * DC_C + DC_C * DC_NC) + DC_NC * DC_LDK + DC_C * DC_NC) * sizeof(float);
+    // (one block a multiprocessor where there are enough of them: see pico_gated_delta_rule)
+    if ((long long)grid.x * grid.y * grid.z <= pico_num_sms() && sm2 < 116 * 1024) sm2 = 116 * 1024;
+    cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);
+    pico_launch(delta_chunk_kernel, grid, dim3(128), sm2, stream, prep, P, state, seg_slots, cu_q, positions, (const float*)coef, u, s0, H, G, d, dv);
+    const size_t sm3 = (size_t)(DC_OC * DC_LD + DC_C * DC_LD + DC_C * DC_OC + DC_C * DC_C + DC_C) * sizeof(float);
+    cudaFuncSetAttribute(delta_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3);
+    pico_launch(delta_chunk_out_kernel, dim3(chunks, H, (dv + DC_OC - 1) / DC_OC), dim3(128), sm3, stream, prep, P, cu_q, positions, S,
+                (const float*)coef, (const float*)u, (const float*)s0, out, out_stride, H, G, d, dv);
+    return pico_launch_status();
 }
 
 PICO_API int pico_gated_delta_rule(const float* prep, const float* v, int v_stride, float* state, const int* seg_slots,

@@ -111,6 +111,11 @@ struct TpArgs {
     float* resid;             // RESIDUAL: [M, N]
     float limit;              // CAPPED: as SWIGLU with g' sigmoid(1.702 g') (u' + 1), g' = min(g, limit), u' = clamp(u, -limit, limit)
     const float* bias;        // GELU: as SWIGLU with gelu_tanh(g + bias[i]) * (u + bias[I + i]); float32 [N], or null
+    // GROUPED: x holds the rows of group e at offsets[e] .. offsets[e + 1] - 1, w is [E, N, K]; tile_start[e]: tiles of 256 MB rows
+    // of the groups before (both [E + 1], on the device: the host never sees them)
+    const int* offsets;
+    const int* tile_start;
+    int E;
 };
 
 __device__ __forceinline__ void tp_st32(void* p, const uint32_t (&r)[8]) {      // one 32-byte store (a whole sector)
@@ -156,8 +161,12 @@ __device__ __forceinline__ uint32_t tp_pack(float a, float b) {
 // double-buffered in tensor memory (the epilogue of a tile runs beside the products of the next).
 // MB = 2: a block holds 256 rows (two products per k step share its half of the w tile, which cuts
 // the bytes that come from L2 per product by a quarter - at these sizes the copies, not the tensor
-// cores, set the pace), the two accumulators fill tensor memory, and eight epilogue warps drain them.
-template <int BN, int EPI, int STAGES, int MB>
+// cores, set the pace), the two accumulators fill tensor memory, and eight epilogue warps drain them.  Accumulator j of a tall tile holds its rows 256 j .. + 255, so a last
+// tile of no more than 256 rows leaves out the second one's copies and products (2,111 rows are five tall tiles, the last with
+// 63 rows: TAIL_US).
+// GROUPED: one product per group of neighbouring rows, each with a matrix of its own (the experts of a routed feed-forward); a
+// tile lies inside one group.  MOE_US
+template <int BN, int EPI, int STAGES, int MB, bool GROUPED>
 __global__ void __launch_bounds__(64 + 128 * MB)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const TpArgs p,
                          int m_tiles, int n_tiles) {
@@ -180,7 +189,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
     asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int nkb = (p.K + TP_BK - 1) / TP_BK;
-    const int total_tiles = m_tiles * n_tiles;
+    int* group_at = reinterpret_cast<int*>(const_cast<int*>(abort_s) + 1);      // GROUPED: offsets [E + 1], tile_start [E + 1]
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -204,13 +213,35 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();                 // x comes from the kernel before
+    if (GROUPED) {
+        for (int i = threadIdx.x; i < 2 * (p.E + 1); i += blockDim.x) group_at[i] = i <= p.E ? p.offsets[i] : p.tile_start[i - p.E - 1];
+        __syncthreads();
+        m_tiles = group_at[2 * p.E + 1];
+    }
+    const int total_tiles = m_tiles * n_tiles;
+    // rows m0 .. m_end - 1 of tile t (this block has 128 of every 256), and the row of w its group starts at
+    struct Place { int m0, m_end, w0; };
+    auto place = [&](int t) {
+        const int mt = t % m_tiles;
+        if (!GROUPED) return Place{mt * 2 * ROWS, p.M, 0};
+        const int* first = group_at + p.E + 1;
+        int lo = 0, hi = p.E;                 // the largest e with first[e] <= mt
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (first[mid] <= mt) lo = mid; else hi = mid;
+        }
+        return Place{group_at[lo] + (mt - first[lo]) * 2 * ROWS, group_at[lo + 1], lo * p.N};
+    };
+    // accumulators that tile has rows for
+    auto accumulators = [&](const Place& at) { return MB == 2 && at.m_end - at.m0 <= 2 * TP_BM ? 1 : MB; };
 
     if (warp == 0) {
         if (lane == 0) {
             int step = 0;
             for (int t = pair; t < total_tiles && !*abort_s; t += n_pairs) {
-                const int m0 = (t % m_tiles) * 2 * ROWS + (int)rank * ROWS, n0 = (t / m_tiles) * COLS;
-                const int w_row = tp_is_glu(EPI) ? (rank ? p.N / 2 + n0 : n0) : n0 + (int)rank * (BN / 2);
+                const Place at = place(t);
+                const int jn = accumulators(at), m0 = at.m0 + (int)rank * TP_BM, n0 = (t / m_tiles) * COLS;
+                const int w_row = at.w0 + (tp_is_glu(EPI) ? (rank ? p.N / 2 + n0 : n0) : n0 + (int)rank * (BN / 2));
                 for (int kb = 0; kb < nkb; ++kb, ++step) {
                     const int s = step % STAGES;
                     if (step >= STAGES && !tp_wait(empty + s, ((step / STAGES) - 1) & 1)) {
@@ -219,8 +250,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
                     }
                     if (*abort_s) break;
                     unsigned char* a = smem + s * STAGE_BYTES;
-                    if (rank == 0) tp_expect_tx(full + s, 2 * STAGE_BYTES);
-                    tp_tma_2d(a, &x_map, kb * TP_BK, m0, full + s);
+                    if (rank == 0) tp_expect_tx(full + s, 2 * (jn * A_BLOCK + B_BYTES));
+                    for (int j = 0; j < jn; ++j) tp_tma_2d(a + j * A_BLOCK, &x_map, kb * TP_BK, m0 + j * 2 * TP_BM, full + s);
                     tp_tma_2d(a + A_BYTES, &w_map, kb * TP_BK, w_row, full + s);
                 }
             }
@@ -239,6 +270,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const uint32_t acc = tmem_base + buf * MB * BN;
+                const int jn = accumulators(place(t));
                 for (int kb = 0; kb < nkb; ++kb, ++step) {
                     const int s = step % STAGES;
                     if (!tp_wait(full + s, (step / STAGES) & 1)) {
@@ -253,7 +285,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
                         const uint64_t bd = tp_desc(b, k16);
 #pragma unroll
                         for (int j = 0; j < MB; ++j)
-                            tp_mma(acc + j * BN, tp_desc(a + j * A_BLOCK, k16), bd, idesc, (kb > 0 || k16 > 0) ? 1u : 0u);
+                            if (j < jn) tp_mma(acc + j * BN, tp_desc(a + j * A_BLOCK, k16), bd, idesc, (kb > 0 || k16 > 0) ? 1u : 0u);
                     }
                     tp_commit_both(empty + s);     // the stage is free in both blocks when these products have read it
                 }
@@ -267,8 +299,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
         int it = 0;
         for (int t = pair; t < total_tiles; t += n_pairs, ++it) {
             const int buf = it % NBUF, use = it / NBUF;
-            const int m0 = (t % m_tiles) * 2 * ROWS + (int)rank * ROWS + j * TP_BM, n0 = (t / m_tiles) * COLS;
-            const int row = m0 + q * 32 + lane;
+            const Place at = place(t);
+            const int n0 = (t / m_tiles) * COLS, row = at.m0 + j * 2 * TP_BM + (int)rank * TP_BM + q * 32 + lane;
+            const bool empty_part = j >= accumulators(at);       // nothing was computed for this warp's rows
             bool ok = tp_wait(acc_full + buf, use & 1);
             if (!ok) {
                 g_tp_status = 1;
@@ -277,7 +310,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
             if (__any_sync(0xffffffffu, !ok || *abort_s != 0)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t taddr = tmem_base + (buf * MB + j) * BN + ((uint32_t)(q * 32) << 16);
-            if (tp_is_glu(EPI)) {
+            if (empty_part) {
+            } else if (tp_is_glu(EPI)) {
                 const int I = p.N / 2;
                 const bool wide = (I & 15) == 0;               // rows of out start on 32 bytes
 #pragma unroll 1
@@ -301,7 +335,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
                             }
                         }
                     }
-                    if (row < p.M) {
+                    if (row < at.m_end) {
                         bf16* dst = p.out + (size_t)row * I + n0 + c;
 #pragma unroll
                         for (int i = 0; i < 32; i += 16) {
@@ -326,7 +360,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
                     uint32_t v[32];
                     tp_ld32(taddr + c, v);
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                    if (row < p.M) {
+                    if (row < at.m_end) {
                         float* dst = p.resid + (size_t)row * p.N + n0 + c;
                         if (wide && n0 + c + 32 <= p.N) {
                             uint32_t r[4][8];
@@ -361,7 +395,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
                     tp_ld32(taddr + c, *reinterpret_cast<uint32_t(*)[32]>(v));
                     tp_ld32(taddr + c + 32, *reinterpret_cast<uint32_t(*)[32]>(v + 32));
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                    if (row < p.M) {
+                    if (row < at.m_end) {
                         bf16* dst = p.out + (size_t)row * p.N + n0 + c;
 #pragma unroll
                         for (int i = 0; i < 64; i += 16) {
@@ -427,23 +461,26 @@ static int tp_make_map(CUtensorMap* map, const void* base, long long rows, int K
 
 static int tp_num_sms() { return pico_num_sms(); }
 
-template <int BN, int EPI, int MB>
+#define TP_MAX_GROUPS 512
+
+template <int BN, int EPI, int MB, bool GROUPED>
 static int tp_launch(const void* x, int ldx, const void* w, const TpArgs& a, cudaStream_t stream) {
     constexpr int STAGE_BYTES = (MB * TP_BM + BN / 2) * TP_BK * 2;
     constexpr int STAGES = (200 * 1024) / STAGE_BYTES > 8 ? 8 : (200 * 1024) / STAGE_BYTES;
     CUtensorMap xm, wm;
-    int rc = tp_make_map(&xm, x, a.M, a.K, ldx, MB * TP_BM);
+    int rc = tp_make_map(&xm, x, a.M, a.K, ldx, TP_BM);
     if (rc) return rc;
-    rc = tp_make_map(&wm, w, a.N, a.K, a.K, BN / 2);
+    rc = tp_make_map(&wm, w, GROUPED ? (long long)a.E * a.N : a.N, a.K, a.K, BN / 2);
     if (rc) return rc;
-    const size_t smem = (size_t)STAGES * STAGE_BYTES + (2 * STAGES + 4) * 8 + 16 + 1024;
-    cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<BN, EPI, STAGES, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = (size_t)STAGES * STAGE_BYTES + (2 * STAGES + 4) * 8 + 16 + 1024 + (GROUPED ? 2 * (a.E + 1) * sizeof(int) : 0);
+    cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<BN, EPI, STAGES, MB, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int n_out = tp_is_glu(EPI) ? a.N / 2 : a.N;
     const int cols = tp_is_glu(EPI) ? BN / 2 : BN;
-    const int n_tiles = (n_out + cols - 1) / cols, m_tiles = (a.M + 2 * MB * TP_BM - 1) / (2 * MB * TP_BM);
+    // (the groups' tiles: at most so many; the kernel reads how many there are)
+    const int n_tiles = (n_out + cols - 1) / cols, m_tiles = GROUPED ? a.M / (2 * MB * TP_BM) + (a.E < a.M ? a.E : a.M) : (a.M + 2 * MB * TP_BM - 1) / (2 * MB * TP_BM);
     const int max_pairs = tp_num_sms() / 2;
     const int pairs = n_tiles * m_tiles < max_pairs ? n_tiles * m_tiles : max_pairs;
-    pico_launch_cluster((gemm_tcgen05_pair_kernel<BN, EPI, STAGES, MB>), dim3(2 * pairs), dim3(64 + 128 * MB), smem, stream, 2,
+    pico_launch_cluster((gemm_tcgen05_pair_kernel<BN, EPI, STAGES, MB, GROUPED>), dim3(2 * pairs), dim3(64 + 128 * MB), smem, stream, 2,
                         xm, wm, a, m_tiles, n_tiles);
     return pico_launch_status();
 }
@@ -484,22 +521,44 @@ PICO_API int pico_gemm_tcgen05_pair(const void* x, int ldx, const void* w, void*
     if (tp_is_glu(epi) && (N % 2 != 0 || (N / 2) % 8 != 0)) return PICO_ERR_SIZE;
     if (!tp_is_glu(epi) && N % 8 != 0) return PICO_ERR_SIZE;
     if (rows_per_pair != 0 && rows_per_pair != 256 && rows_per_pair != 512) return PICO_ERR_SIZE;
-    TpArgs a;
+    TpArgs a = {};
     a.M = M; a.N = N; a.K = K; a.out = (bf16*)out; a.resid = resid; a.limit = limit; a.bias = bias;
     int bn = 256, mb = 1;
     tp_pick(M, tp_is_glu(epi) ? N / 2 : N, tp_is_glu(epi), rows_per_pair / 256, bn, mb);
 #define TP_CASE(BN, MB)                                                                       \
     if (bn == BN && mb == MB) {                                                               \
-        if (epi == TP_STORE) return tp_launch<BN, TP_STORE, MB>(x, ldx, w, a, stream);        \
-        if (epi == TP_RESIDUAL) return tp_launch<BN, TP_RESIDUAL, MB>(x, ldx, w, a, stream);  \
-        if (epi == TP_SWIGLU) return tp_launch<BN, TP_SWIGLU, MB>(x, ldx, w, a, stream);      \
-        if (epi == TP_CAPPED) return tp_launch<BN, TP_CAPPED, MB>(x, ldx, w, a, stream);      \
-        if (epi == TP_GELU) return tp_launch<BN, TP_GELU, MB>(x, ldx, w, a, stream);          \
+        if (epi == TP_STORE) return tp_launch<BN, TP_STORE, MB, false>(x, ldx, w, a, stream);        \
+        if (epi == TP_RESIDUAL) return tp_launch<BN, TP_RESIDUAL, MB, false>(x, ldx, w, a, stream);  \
+        if (epi == TP_SWIGLU) return tp_launch<BN, TP_SWIGLU, MB, false>(x, ldx, w, a, stream);      \
+        if (epi == TP_CAPPED) return tp_launch<BN, TP_CAPPED, MB, false>(x, ldx, w, a, stream);      \
+        if (epi == TP_GELU) return tp_launch<BN, TP_GELU, MB, false>(x, ldx, w, a, stream);          \
     }
     TP_CASE(256, 2)
     TP_CASE(256, 1)
     TP_CASE(192, 1)
     TP_CASE(128, 1)
 #undef TP_CASE
+    return PICO_ERR_SIZE;
+}
+
+// Rows of a group's tile in pico_gemm_tcgen05_grouped for n rows in E groups: 512, or 256 where the groups are short (with 512 rows a
+// product reads a quarter less from L2, with 256 less of a tile lies beyond its group's end).
+PICO_API int pico_gemm_tcgen05_group_rows(int n, int E) { return n >= 384LL * E ? 512 : 256; }
+
+// One product per group: out[r] = x[r] w[e]^T for the rows r = offsets[e] .. offsets[e + 1] - 1; w [E, N, K], x [n, K] contiguous.  epi 0 (out
+// [n, N]), 2 or 3 (out [n, N / 2]) as above.  tile_start: tiles of `rows` rows (pico_gemm_tcgen05_group_rows) of the groups before.
+PICO_API int pico_gemm_tcgen05_grouped(const void* x, const void* w, void* out, const int* offsets, const int* tile_start, int n, int E, int N,
+                                       int K, int epi, int rows, float limit, cudaStream_t stream) {
+    if (n <= 0) return 0;
+    if (E < 1 || E > TP_MAX_GROUPS || N < 16 || K < 64 || K % 8 != 0 || (rows != 256 && rows != 512)) return PICO_ERR_SIZE;
+    if (epi == TP_STORE ? N % 8 != 0 : (N % 2 != 0 || (N / 2) % 8 != 0)) return PICO_ERR_SIZE;
+    if (epi == TP_CAPPED && !(limit > 0.f)) return PICO_ERR_SIZE;
+    TpArgs a = {};
+    a.M = n; a.N = N; a.K = K; a.out = (bf16*)out; a.limit = limit; a.offsets = offsets; a.tile_start = tile_start; a.E = E;
+#define TP_GROUPED(EPI) return rows == 512 ? tp_launch<256, EPI, 2, true>(x, K, w, a, stream) : tp_launch<256, EPI, 1, true>(x, K, w, a, stream)
+    if (epi == TP_STORE) TP_GROUPED(TP_STORE);
+    if (epi == TP_SWIGLU) TP_GROUPED(TP_SWIGLU);
+    if (epi == TP_CAPPED) TP_GROUPED(TP_CAPPED);
+#undef TP_GROUPED
     return PICO_ERR_SIZE;
 }

@@ -29,7 +29,9 @@ enum { MOE_SCORE_SOFTMAX_CHOSEN = 0, MOE_SCORE_SIGMOID = 1, MOE_SCORE_SOFTMAX_AL
 
 // TOK tokens per block (their rows of h in shared memory as float32, so that a warp reads an expert's router row once
 // for all of them); 8 warps take the experts in turn; warp w < TOK then chooses for token w.
-template <typename TA, int TOK>
+// VEC: rows of h are read 16 bytes a thread (their length and place allow it).  2,048 tokens of 1,536 to 16 experts:
+// 16 us (21 element by element, with two divisions and a 2-byte load for each number).
+template <typename TA, int TOK, bool VEC>
 __global__ void __launch_bounds__(256) moe_route_kernel(const TA* __restrict__ h, const float* __restrict__ wr,
                                                         const float* __restrict__ br, int T, int D, int E, int top,
                                                         int mode, int* __restrict__ idx, float* __restrict__ wgt,
@@ -43,10 +45,26 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const TA* __restrict__ h
     float* z = rsm + TOK * Dp;
     const int t0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int nt = min(TOK, T - t0);
+    if (VEC) {
+        constexpr int W = 16 / (int)sizeof(TA);
+#pragma unroll
+        for (int k = 0; k < TOK; ++k) {
+#pragma unroll 2
+            for (int d = threadIdx.x * W; d < D; d += blockDim.x * W) {
+                uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+                if (k < nt) raw = *reinterpret_cast<const uint4*>(h + (size_t)(t0 + k) * D + d);
+                const TA* v = reinterpret_cast<const TA*>(&raw);
+#pragma unroll
+                for (int i = 0; i < W; i += 4)
+                    *reinterpret_cast<float4*>(hs + k * Dp + d + i) = make_float4(to_f32(v[i]), to_f32(v[i + 1]), to_f32(v[i + 2]), to_f32(v[i + 3]));
+            }
+        }
+    } else {
 #pragma unroll 4
-    for (int i = threadIdx.x; i < TOK * D; i += blockDim.x) {
-        const int k = i / D, d = i - k * D;
-        hs[k * Dp + d] = k < nt ? to_f32(h[(size_t)(t0 + k) * D + d]) : 0.f;
+        for (int i = threadIdx.x; i < TOK * D; i += blockDim.x) {
+            const int k = i / D, d = i - k * D;
+            hs[k * Dp + d] = k < nt ? to_f32(h[(size_t)(t0 + k) * D + d]) : 0.f;
+        }
     }
     __syncthreads();
     const bool vec = (D & 3) == 0;
@@ -440,21 +458,24 @@ PICO_API int pico_moe_route(const void* h, const float* wr, const float* br, int
     if (groups < 1 || E % groups || groups_keep < 1 || groups_keep > groups) return PICO_ERR_SIZE;
     if ((groups > 1 || renorm) && mode != MOE_SCORE_SOFTMAX_ALL) return PICO_ERR_SIZE;
     if (renorm && !(weight_scale != 0.f)) return PICO_ERR_SIZE;
-    // four tokens a block when there are many (the router matrix is read once per block), one otherwise
+    // four tokens a block when there are many (the router matrix is read once per block; eight were slower), one otherwise
     const int tok = T >= 512 ? 4 : 1;
     const size_t smem = ((size_t)tok * ((D + 3) & ~3) + (size_t)3 * tok * E) * sizeof(float);
     if (smem > 200 * 1024) return PICO_ERR_SIZE;
     const dim3 grid((T + tok - 1) / tok);
-#define LAUNCH_ROUTE(TA, TOK)                                                                                             \
+#define LAUNCH_ROUTE(TA, TOK, VEC)                                                                                        \
     do {                                                                                                                  \
         if (smem > 48 * 1024)                                                                                             \
-            cudaFuncSetAttribute(moe_route_kernel<TA, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
-        pico_launch((moe_route_kernel<TA, TOK>), grid, dim3(256), smem, stream, (const TA*)h, wr, br, T, D, E, top, mode, idx, wgt, choice_bias, weight_scale, groups, groups_keep, renorm); \
+            cudaFuncSetAttribute(moe_route_kernel<TA, TOK, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        pico_launch((moe_route_kernel<TA, TOK, VEC>), grid, dim3(256), smem, stream, (const TA*)h, wr, br, T, D, E, top, mode, idx, wgt, choice_bias, weight_scale, groups, groups_keep, renorm); \
     } while (0)
+    const bool vec = D % (dtype == PICO_F32 ? 4 : 8) == 0 && ((uintptr_t)h & 15) == 0;
     if (dtype == PICO_F32) {
-        if (tok == 4) LAUNCH_ROUTE(float, 4); else LAUNCH_ROUTE(float, 1);
+        if (tok == 4) { if (vec) LAUNCH_ROUTE(float, 4, true); else LAUNCH_ROUTE(float, 4, false); }
+        else { if (vec) LAUNCH_ROUTE(float, 1, true); else LAUNCH_ROUTE(float, 1, false); }
     } else if (dtype == PICO_BF16) {
-        if (tok == 4) LAUNCH_ROUTE(bf16, 4); else LAUNCH_ROUTE(bf16, 1);
+        if (tok == 4) { if (vec) LAUNCH_ROUTE(bf16, 4, true); else LAUNCH_ROUTE(bf16, 4, false); }
+        else { if (vec) LAUNCH_ROUTE(bf16, 1, true); else LAUNCH_ROUTE(bf16, 1, false); }
     } else
         return PICO_ERR_DTYPE;
 #undef LAUNCH_ROUTE
@@ -474,13 +495,13 @@ PICO_API int pico_moe_tile_rows(int n, int E, int dtype, int K1, int K2) {
 PICO_API int pico_moe_group(const int* idx, int n, int E, int bm, int* offsets, int* tile_start, int* perm, int* place,
                             cudaStream_t stream) {
     if (n <= 0) return 0;
-    if (E < 1 || E > 4096 || (bm != 16 && bm != MOE_BM)) return PICO_ERR_SIZE;
+    if (E < 1 || E > 4096 || (bm != 16 && bm != MOE_BM && bm != 256 && bm != 512)) return PICO_ERR_SIZE;
     pico_launch(moe_group_kernel, dim3(1), dim3(n >= 4096 ? 1024 : 256), (size_t)2 * E * sizeof(int), stream, idx, n, E, bm,
                 offsets, tile_start, perm, place);
     return pico_launch_status();
 }
 
-// The library path for many tokens: rows gathered into expert order, a library grouped product on them, and the
+// For many tokens: rows gathered into expert order, the grouped tcgen05 product (gemm_tcgen05_pair.cu) on them, and the
 // weighted sum read back through ``place``.
 // xs[p, :] = x[perm[p] / top, :], 16 bytes per thread and access (D * sizeof a multiple of 16).
 __global__ void moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ perm, int top, int row16,

@@ -539,6 +539,90 @@ causal_conv_silu_kernel(const TA* __restrict__ proj, int row_stride, int c_off, 
     }
 }
 
+// The same with four channels a thread (rows start on four elements) and CV_TOK tokens a block, whose inputs are all asked for
+// before the first is used: one thread's loads came one after the other before (2,048 tokens of 3,072 channels, bfloat16: CONV_US,
+// 25 one channel a thread).
+template <typename TA> struct Four;
+template <> struct Four<float> {
+    float4 v;
+    __device__ __forceinline__ float4 get() const { return v; }
+};
+template <> struct Four<bf16> {
+    uint2 v;
+    __device__ __forceinline__ float4 get() const {
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+        return make_float4(a.x, a.y, b.x, b.y);
+    }
+};
+template <typename TA>
+__global__ void __launch_bounds__(256)
+causal_conv_silu4_kernel(const TA* __restrict__ proj, int row_stride, int c_off, const float* __restrict__ w, const float* __restrict__ b,
+                         const float* __restrict__ conv_state, const int* __restrict__ tok_seg, const int* __restrict__ seg_slots,
+                         const int* __restrict__ cu_q, const int* __restrict__ positions, int C, int taps, int T,
+                         float* __restrict__ out, int act) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int M = 4;                       // taps in registers
+    const int tb = blockIdx.x * CV_TOK, te = min(T, tb + CV_TOK), c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    if (c >= C) return;
+    Four<TA> x[CV_TOK];
+    int pos[CV_TOK], seg[CV_TOK];
+#pragma unroll
+    for (int i = 0; i < CV_TOK; ++i) {
+        const int t = min(tb + i, te - 1);
+        x[i] = *reinterpret_cast<const Four<TA>*>(proj + (size_t)t * row_stride + c_off + c);
+        pos[i] = positions[t];
+        seg[i] = tok_seg[t];
+    }
+    float4 wt[M], win[M];
+#pragma unroll
+    for (int k = 0; k < M; ++k) {
+        float wk[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) wk[e] = k < taps ? w[(size_t)(c + e) * taps + taps - 1 - k] : 0.f;
+        wt[M - 1 - k] = make_float4(wk[0], wk[1], wk[2], wk[3]);
+        win[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float4 bias = b ? *reinterpret_cast<const float4*>(b + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    bool have = false;
+#pragma unroll
+    for (int i = 0; i < CV_TOK; ++i) {
+        const int t = tb + i;
+        if (t >= te) break;
+        float4* dst = reinterpret_cast<float4*>(out + (size_t)t * C + c);
+        if (pos[i] < 0) {
+            *dst = make_float4(0.f, 0.f, 0.f, 0.f);
+            have = false;
+            continue;
+        }
+        // the inputs before this token: of this step, or kept by the request
+        if (!have || seg[i] != seg[i > 0 ? i - 1 : 0]) {
+            const int begin = cu_q[seg[i]];
+            const float* st = conv_state + (size_t)seg_slots[seg[i]] * (taps - 1) * C;
+#pragma unroll
+            for (int k = 1; k < M; ++k)
+                if (k < taps) {
+                    const int src = t - k;
+                    win[M - 1 - k] = src >= begin ? reinterpret_cast<const Four<TA>*>(proj + (size_t)src * row_stride + c_off + c)->get()
+                                                  : *reinterpret_cast<const float4*>(st + (size_t)(taps - 1 + src - begin) * C + c);
+                }
+            have = true;
+        }
+        win[M - 1] = x[i].get();
+        float4 acc = bias;
+#pragma unroll
+        for (int k = 0; k < M; ++k) {          // oldest first; unused taps weigh zero
+            acc.x = fmaf(wt[k].x, win[k].x, acc.x);
+            acc.y = fmaf(wt[k].y, win[k].y, acc.y);
+            acc.z = fmaf(wt[k].z, win[k].z, acc.z);
+            acc.w = fmaf(wt[k].w, win[k].w, acc.w);
+        }
+        *dst = act ? make_float4(rc_silu(acc.x), rc_silu(acc.y), rc_silu(acc.z), rc_silu(acc.w)) : acc;
+#pragma unroll
+        for (int k = 0; k < M - 1; ++k) win[k] = win[k + 1];
+    }
+}
+
 template <typename TA>
 __global__ void conv_state_kernel(const TA* __restrict__ proj, int row_stride, int c_off, float* __restrict__ conv_state,
                                   const int* __restrict__ seg_slots, const int* __restrict__ cu_q,
@@ -568,9 +652,16 @@ PICO_API int pico_causal_conv_silu(const void* proj, int row_stride, int c_off, 
     if (C < 1 || taps < 1 || taps > CONV_MAX_TAPS || S > 65535 || (C + 255) / 256 > 65535) return PICO_ERR_SIZE;
     const int tpb = T >= 32 * CV_TOK ? CV_TOK : 1;
     const int blocks = (T + tpb - 1) / tpb;
+    // four channels a thread from the sizes on where tokens share a block, if every row and table starts on four elements
+    const bool four = tpb == CV_TOK && taps <= 4 && C % 4 == 0 && c_off % 4 == 0 && row_stride % 4 == 0 &&
+                      ((uintptr_t)proj & (dtype == PICO_F32 ? 15 : 7)) == 0 &&
+                      (((uintptr_t)b | (uintptr_t)conv_state | (uintptr_t)out) & 15) == 0;
 #define CV_LAUNCH(TA)                                                                                                    \
     do {                                                                                                                 \
-        if (taps <= 4)                                                                                                   \
+        if (four)                                                                                                        \
+            pico_launch((causal_conv_silu4_kernel<TA>), dim3(blocks, (C / 4 + 255) / 256), dim3(256), 0, stream, (const TA*)proj, \
+                        row_stride, c_off, w, b, (const float*)conv_state, tok_seg, seg_slots, cu_q, positions, C, taps, T, out, act); \
+        else if (taps <= 4)                                                                                                   \
             pico_launch((causal_conv_silu_kernel<TA, 4>), dim3(blocks, (C + 255) / 256), dim3(256), 0, stream, (const TA*)proj,  \
                         row_stride, c_off, w, b, (const float*)conv_state, tok_seg, seg_slots, cu_q, positions, C, taps, T, tpb, out, act); \
         else                                                                                                             \
@@ -683,6 +774,54 @@ group_rms_norm_kernel(const float* __restrict__ x, int x_stride, int group_strid
     }
 }
 
+// The plain form (no normaliser, skip or gate before the norm) of groups of up to 512 columns whose rows start on four numbers: a lane
+// reads its columns once, four at a time, and keeps them (2,048 rows of 12 groups of 128 with a gate: NORM_US, 15 with a pass for
+// the sum and a pass for the result, a number a load).
+template <typename TA>
+__global__ void __launch_bounds__(128)
+group_rms_norm4_kernel(const float* __restrict__ x, int x_stride, int group_stride, int groups, int n, const float* __restrict__ w,
+                       float eps, const TA* __restrict__ post_gate, int post_stride, int post_act, TA* __restrict__ y) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t t = blockIdx.x;
+    const int g = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (g >= groups) return;
+    const float* xg = x + t * x_stride + (size_t)g * group_stride;
+    float4 v[4];
+    Four<TA> gate[4];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int j = lane * 4 + 128 * i;
+        if (j < n) {
+            v[i] = *reinterpret_cast<const float4*>(xg + j);
+            if (post_gate) gate[i] = *reinterpret_cast<const Four<TA>*>(post_gate + t * post_stride + g * n + j);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (lane * 4 + 128 * i < n) ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+    const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)n + eps);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int j = lane * 4 + 128 * i, col = g * n + j;
+        if (j >= n) break;
+        const float4 wv = w ? *reinterpret_cast<const float4*>(w + col) : make_float4(1.f, 1.f, 1.f, 1.f);
+        float o[4] = {v[i].x * inv * wv.x, v[i].y * inv * wv.y, v[i].z * inv * wv.z, v[i].w * inv * wv.w};
+        if (post_gate) {
+            const float4 z = gate[i].get();
+            o[0] *= post_act ? rc_silu(z.x) : rc_sigmoid(z.x);
+            o[1] *= post_act ? rc_silu(z.y) : rc_sigmoid(z.y);
+            o[2] *= post_act ? rc_silu(z.z) : rc_sigmoid(z.z);
+            o[3] *= post_act ? rc_silu(z.w) : rc_sigmoid(z.w);
+        }
+        __align__(16) TA r[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[e] = from_f32<TA>(o[e]);
+        *reinterpret_cast<Four<TA>*>(y + t * ((size_t)groups * n) + col) = *reinterpret_cast<const Four<TA>*>(r);
+    }
+}
+
 PICO_API int pico_group_rms_norm(const float* x, int x_stride, int group_stride, int groups, int n, const float* w, float eps,
                                  const float* den_floor, const float* skip, int skip_stride, const float* skip_w, int skip_head,
                                  const void* pre_gate, int pre_stride, const void* post_gate, int post_stride, int post_act, void* y,
@@ -692,6 +831,19 @@ PICO_API int pico_group_rms_norm(const float* x, int x_stride, int group_stride,
     if (groups > 65535 * 4) return PICO_ERR_SIZE;
     const bool wide = n >= 512;
     const dim3 grid(T, wide ? groups : (groups + 3) / 4), block(wide ? 256 : 128);
+    const int at = dtype == PICO_F32 ? 15 : 7;             // where four of the activation type start
+    if (!wide && !den_floor && !skip && !pre_gate && n % 4 == 0 && x_stride % 4 == 0 && group_stride % 4 == 0 && post_stride % 4 == 0 &&
+        (((uintptr_t)x | (uintptr_t)w) & 15) == 0 && (((uintptr_t)post_gate | (uintptr_t)y) & at) == 0) {
+        if (dtype == PICO_F32)
+            pico_launch((group_rms_norm4_kernel<float>), grid, block, 0, stream, x, x_stride, group_stride, groups, n, w, eps,
+                        (const float*)post_gate, post_stride, post_act, (float*)y);
+        else if (dtype == PICO_BF16)
+            pico_launch((group_rms_norm4_kernel<bf16>), grid, block, 0, stream, x, x_stride, group_stride, groups, n, w, eps,
+                        (const bf16*)post_gate, post_stride, post_act, (bf16*)y);
+        else
+            return PICO_ERR_DTYPE;
+        return pico_launch_status();
+    }
 #define GN_LAUNCH(TA, W)                                                                                                 \
     pico_launch((group_rms_norm_kernel<TA, W>), grid, block, 0, stream, x, x_stride, group_stride, groups, n, w, eps,     \
                 den_floor, skip, skip_stride, skip_w, skip_head, (const TA*)pre_gate, pre_stride, (const TA*)post_gate,  \

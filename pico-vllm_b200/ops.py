@@ -94,6 +94,8 @@ def library():
         "pico_moe_gather": [vp, vp, i32, i32, i32, vp, vp],
         "pico_moe_combine_placed": [vp, vp, vp, i32, i32, i32, vp, vp, i32, vp, i32, vp, vp],
         "pico_moe_gemm": [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp, i32, f32, i32, vp],
+        "pico_gemm_tcgen05_grouped": [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp],
+        "pico_gemm_tcgen05_group_rows": [i32, i32],
         "pico_moe_combine": [vp, vp, i32, i32, i32, vp, vp, i32, vp, i32, vp, vp],
         "pico_moe_scaled_act": [vp, vp, vp, i32, i32, i32, vp, i32, vp],
         "pico_qk_norm_rope_store": [vp, i32, vp, vp, vp, f32, vp, vp, f32, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32,
@@ -115,6 +117,7 @@ def library():
         "pico_mamba2_prepare": [vp, i32, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, vp],
         "pico_group_rms_norm": [vp, i32, i32, i32, i32, vp, f32, vp, vp, i32, vp, i32, vp, i32, vp, i32, i32, vp, i32, i32, vp],
         "pico_delta_prepare": [vp, i32, i32, i32, vp, i32, i32, vp, i32, vp, vp, vp, i32, i32, i32, i32, f32, f32, i32, i32, i32, vp],
+        "pico_gated_delta_chunks": [vp, vp, i32, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp],
         "pico_gated_delta_rule": [vp, vp, i32, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp],
         "pico_pair_rope_norm_store": [vp, i32, i32, i32, i32, vp, vp, i32, i32, vp, vp, f32, vp, vp, vp, vp, i32, i32, i32, i32,
                                       i32, i32, i32, i32, vp],
@@ -129,6 +132,8 @@ def library():
         fn = getattr(lib, name)
         fn.argtypes = args
         fn.restype = ctypes.c_int
+    lib.pico_gated_delta_chunk_floats.argtypes = [i32, i32, i32, i32]
+    lib.pico_gated_delta_chunk_floats.restype = i64
     _lib = lib
     return lib
 
@@ -1110,14 +1115,15 @@ def moe_experts(h: torch.Tensor, idx: torch.Tensor, wgt: torch.Tensor, gate_up_w
         raise KernelError("moe_experts: experts that pass their input on are built with the weight on the output only")
     n = T * top
     lib, code, st = library(), _dtype_code(h), _stream()
-    grouped = moe_library_takes(h, n, D, ff)
+    grouped = moe_tc_takes(h, gate_up_weight, down_weight, n)
     # entries are listed for the E real experts and, after them, for the ones that pass their input on: the products
     # below see the first E lists only (offsets[E] and tile_start[E] end the real entries), the sum reads h for the rest
     Et = E + identity
     meta = torch.empty(2 * (Et + 1) + 2 * n, dtype=torch.int32, device=h.device)
     offsets, tile_start = meta[:Et + 1], meta[Et + 1:2 * (Et + 1)]
     perm, place = meta[2 * (Et + 1):2 * (Et + 1) + n], meta[2 * (Et + 1) + n:]
-    bm = lib.pico_moe_tile_rows(n, E, code, D, ff)      # rows per tile of this package's grouped kernels
+    # rows per tile of the grouped products
+    bm = lib.pico_gemm_tcgen05_group_rows(n, E) if grouped else lib.pico_moe_tile_rows(n, E, code, D, ff)
     _check(lib.pico_moe_group(_ptr(idx), n, Et, bm, _ptr(offsets), _ptr(tile_start), _ptr(perm),
                               _ptr(place) if grouped else None, st), "moe_group")
     eidx, hsrc = (idx, h) if identity else (None, None)
@@ -1125,31 +1131,22 @@ def moe_experts(h: torch.Tensor, idx: torch.Tensor, wgt: torch.Tensor, gate_up_w
     in_w = wgt if (not gated and weight_on_input) else None         # the weight inside the activation ...
     out_w = None if (not gated and weight_on_input) else wgt        # ... or on the expert's output
     if grouped:
-        # many tokens: rows in expert order, the library's grouped products (their group ends are read on the device),
-        # the activation kernel between them.  A shape the library refuses goes to this package's kernels below.
-        try:
-            xs = torch.empty((n, D), dtype=h.dtype, device=h.device)
-            _check(lib.pico_moe_gather(_ptr(h), _ptr(perm), n, top, D * h.element_size(), _ptr(xs), st), "moe_gather")
-            ends = offsets[1:E + 1]
-            gu = torch._grouped_mm(xs, gate_up_weight.transpose(1, 2), offs=ends)
-            if gated:
-                if act == MOE_ACT_CAPPED:
-                    a = capped_glu(gu, ff, limit)
-                else:
-                    a = torch.empty((n, ff), dtype=h.dtype, device=h.device)
-                    swiglu(gu, a)
-            else:
-                a = gu
-                _check(lib.pico_moe_scaled_act(_ptr(gu), _ptr(perm), _ptr(in_w), n, ff, int(act), _ptr(a), code, st),
-                       "moe_scaled_act")
-            ys = torch._grouped_mm(a, down_weight.transpose(1, 2), offs=ends)
-            _check(lib.pico_moe_combine_placed(_ptr(ys), _ptr(place), _ptr(out_w), T, top, D, _ptr(y), _ptr(base), code, _ptr(eidx), E,
-                                               _ptr(hsrc), st), "moe_combine_placed")
-            _count(3)
-            return y
-        except (RuntimeError, NotImplementedError):
-            if torch.cuda.is_current_stream_capturing():
-                raise
+        # many tokens: rows in expert order and the tcgen05 products over them, a gated activation in the first one's epilogue
+        xs = torch.empty((n, D), dtype=h.dtype, device=h.device)
+        _check(lib.pico_moe_gather(_ptr(h), _ptr(perm), n, top, D * h.element_size(), _ptr(xs), st), "moe_gather")
+        a = torch.empty((n, ff), dtype=h.dtype, device=h.device)
+        up_epi = 0 if not gated else 3 if act == MOE_ACT_CAPPED else 2
+        _check(lib.pico_gemm_tcgen05_grouped(_ptr(xs), _ptr(gate_up_weight), _ptr(a), _ptr(offsets), _ptr(tile_start), n, E, ff_rows, D, up_epi, bm,
+                                             float(limit), st), "gemm_tcgen05_grouped (up)")
+        if not gated:
+            _check(lib.pico_moe_scaled_act(_ptr(a), _ptr(perm), _ptr(in_w), n, ff, int(act), _ptr(a), code, st), "moe_scaled_act")
+        ys = torch.empty((n, D), dtype=h.dtype, device=h.device)
+        _check(lib.pico_gemm_tcgen05_grouped(_ptr(a), _ptr(down_weight), _ptr(ys), _ptr(offsets), _ptr(tile_start), n, E, D, ff, 0, bm, 0.0, st),
+               "gemm_tcgen05_grouped (down)")
+        _check(lib.pico_moe_combine_placed(_ptr(ys), _ptr(place), _ptr(out_w), T, top, D, _ptr(y), _ptr(base), code, _ptr(eidx), E,
+                                           _ptr(hsrc), st), "moe_combine_placed")
+        _count(5 if gated else 6)
+        return y
     a = torch.empty((n, ff), dtype=h.dtype, device=h.device)
     _check(lib.pico_moe_gemm(_ptr(h), _ptr(gate_up_weight), _ptr(offsets), _ptr(tile_start), _ptr(perm), n, E, top, ff, D,
                              0 if gated else 2, bm, _ptr(a), None, _ptr(in_w), int(act), float(limit), code, st), "moe_gemm (up)")
@@ -1291,14 +1288,17 @@ def gated_rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor], gate_logits:
     return y
 
 
-MOE_LIBRARY_MIN_ROWS = 1024       # (token, expert) pairs from which the library's grouped product is used
+# (token, expert) pairs from which the experts' products run on the tcgen05 tensor cores over rows in expert order: MOE_RULE
+MOE_TC_MIN_ROWS = 1024
+MOE_TC_MAX_EXPERTS = 512
 
 
-def moe_library_takes(h: torch.Tensor, n: int, D: int, ff: int) -> bool:
-    """Whether the experts' products go to the library's grouped matrix product (bfloat16, many rows, row sizes
-    that are multiples of 16 bytes) instead of this package's grouped kernels."""
-    return (h.dtype == torch.bfloat16 and n >= MOE_LIBRARY_MIN_ROWS and D % 8 == 0 and ff % 8 == 0
-            and hasattr(torch, "_grouped_mm"))
+def moe_tc_takes(h: torch.Tensor, gate_up_weight: torch.Tensor, down_weight: torch.Tensor, n: int) -> bool:
+    """Whether the experts' products run on the tcgen05 tensor cores (bfloat16, many rows, row sizes that are multiples of 16
+    bytes) instead of the grouped kernels that need no rows in order."""
+    (E, _, D), ff = gate_up_weight.shape, down_weight.shape[2]
+    return (h.dtype == torch.bfloat16 and n >= MOE_TC_MIN_ROWS and E <= MOE_TC_MAX_EXPERTS and D % 8 == 0 and ff % 8 == 0 and D >= 64 and ff >= 64
+            and (h.data_ptr() | gate_up_weight.data_ptr() | down_weight.data_ptr()) % 16 == 0)
 
 
 # ------------------------------------------------------------------------------------------ several residual streams
@@ -1612,6 +1612,17 @@ def delta_prepare(xc: torch.Tensor, q_off: int, k_off: int, proj: torch.Tensor, 
     return prep
 
 
+# longest segment from which the recurrence with a decay per head runs in chunks of 32 tokens: CHUNK_RULE
+DELTA_CHUNK_MIN_TOKENS = 64
+
+
+def delta_chunks_take(v: torch.Tensor, state: torch.Tensor, d: int, dv: int, max_q_len: int) -> bool:
+    """Long segments, keys of 65 to 128 numbers, and everything the kernel reads 16 bytes at a time lies on 16 bytes.  What is prepared
+    for such a step needs no dot products with earlier rows (:func:`delta_prepare` with ``max_q_len`` 1)."""
+    return (max_q_len >= DELTA_CHUNK_MIN_TOKENS and 64 < d <= 128 and d % 4 == 0 and dv % 4 == 0 and v.stride(0) % 4 == 0
+            and (v.data_ptr() | state.data_ptr()) % 16 == 0)
+
+
 def gated_delta_rule(prep: torch.Tensor, v: torch.Tensor, state: torch.Tensor, seg_slots: torch.Tensor, cu_q: torch.Tensor,
                      positions: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int, per_head: bool = False,
                      max_q_len: int = 1) -> torch.Tensor:
@@ -1638,6 +1649,16 @@ def gated_delta_rule(prep: torch.Tensor, v: torch.Tensor, state: torch.Tensor, s
     if cu_q.shape[0] != S + 1 or positions.shape[0] != T:
         raise KernelError("gated_delta_rule: cu_q must have one more entry than seg_slots, positions one per token")
     out = torch.empty((T, H * vdim), dtype=torch.float32, device=prep.device)
+    if per_head and delta_chunks_take(v, state, d, vdim, max_q_len):
+        if prep.data_ptr() % 16:
+            raise KernelError("gated_delta_rule: prep must start on 16 bytes")
+        lib = library()
+        scratch = torch.empty(lib.pico_gated_delta_chunk_floats(T, S, H, vdim), dtype=torch.float32, device=prep.device)
+        _check(lib.pico_gated_delta_chunks(_ptr(prep), _ptr(v), v.stride(0), _ptr(state), _ptr(seg_slots), _ptr(cu_q), _ptr(positions),
+                                           _ptr(out), out.stride(0), T, S, H, G, d, vdim, _ptr(scratch), _stream()),
+               f"gated_delta_chunks (dim {d})")
+        _count(3)
+        return out
     _check(library().pico_gated_delta_rule(_ptr(prep), _ptr(v), v.stride(0), _ptr(state), _ptr(seg_slots), _ptr(cu_q),
                                            _ptr(positions), _ptr(out), out.stride(0), S, H, G, d, vdim, 1 if per_head else 0,
                                            1 if max_q_len >= DELTA_BLOCK_MIN_TOKENS else 0, _stream()),

@@ -1,0 +1,66 @@
+"""The delta rule with a decay per head in chunks of 32 tokens against the recurrence token by token in float64: the edges of
+chunks, single tokens and padding beside them, key sizes that are padded, column tiles that are not full, decays of nought and one."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _segments(lens, pad_at=None):
+    cu, pos = [0], []
+    for s, n in enumerate(lens):
+        cu.append(cu[-1] + n)
+        pos += [-1] * n if s == pad_at else list(range(5 * s, 5 * s + n))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32)
+    return i32(cu), i32(pos), i32(list(range(len(lens) - 1, -1, -1)))
+
+
+def _oracle(q, k, v, a, beta, state, slots, cu, pos):
+    T, H, dv = v.shape
+    G = q.shape[1]
+    out, state = torch.zeros(T, H, dv, dtype=torch.float64), state.double().clone()
+    q, k = (x.double().repeat_interleave(H // G, 1) for x in (q, k))
+    for s in range(slots.shape[0]):
+        a0, a1 = int(cu[s]), int(cu[s + 1])
+        if a1 <= a0 or int(pos[a0]) < 0:
+            continue
+        S = state[int(slots[s])]                                  # [H, dv, d]
+        for t in range(a0, a1):
+            S = S * a[t].double()[:, None, None]
+            u = beta[t].double()[:, None] * (v[t].double() - torch.einsum("hvd,hd->hv", S, k[t]))
+            S = S + u[:, :, None] * k[t][:, None, :]
+            out[t] = torch.einsum("hvd,hd->hv", S, q[t])
+        state[int(slots[s])] = S
+    return out, state
+
+
+@pytest.mark.parametrize("H,G,d,dv", [(2, 1, 128, 128), (3, 3, 68, 20), (10, 2, 100, 36), (1, 1, 128, 4)])
+@pytest.mark.parametrize("lens,pad_at", [([64], None), ([1, 31, 32, 33, 70, 1], None), ([97, 5, 2, 64], 1), ([0, 128, 0, 65], None)])
+@pytest.mark.parametrize("decays", ["middling", "nought and one"])
+def test_chunks(H, G, d, dv, lens, pad_at, decays):
+    from pico_vllm_b200 import ops
+    assert max(lens) >= ops.DELTA_CHUNK_MIN_TOKENS
+    g = torch.Generator().manual_seed(d + dv + len(lens))
+    cu, pos, slots = _segments(lens, pad_at)
+    T, S = int(cu[-1]), len(lens)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, d, generator=g), dim=-1) for _ in range(2))
+    q = q * d ** -0.5
+    k[1::3] = k[0::3][:k[1::3].shape[0]]                          # keys that repeat: what is held under them is taken off
+    v = torch.randn(T, H, dv, generator=g)
+    a = torch.rand(T, H, generator=g) * 0.2 + 0.8 if decays == "middling" else (torch.rand(T, H, generator=g) > 0.1).float()
+    beta = torch.rand(T, H, generator=g)
+    state = torch.randn(S + 1, H, dv, d, generator=g) * 0.3
+    prep = torch.cat([q.reshape(T, -1), k.reshape(T, -1), torch.stack([a, beta, a * float("nan"), beta], -1).reshape(T, -1),
+                      torch.full((T, 8 * G), float("nan"))], 1).contiguous()
+    want_o, want_s = _oracle(q, k, v, a, beta, state, slots, cu, pos)
+    wide = torch.cat([torch.zeros(T, 4), v.reshape(T, -1)], 1).to(DEV)
+    got_s, p = state.to(DEV), prep.to(DEV)
+    assert ops.delta_chunks_take(wide[:, 4:], got_s, d, dv, max(lens))
+    got_o = ops.gated_delta_rule(p, wide[:, 4:], got_s, slots.to(DEV), cu.to(DEV), pos.to(DEV), H, G, d, dv, per_head=True,
+                                 max_q_len=max(lens))
+    live = pos >= 0
+    # float32 sums of up to d + 32 products of order one, through a forward substitution of 32 rows
+    for got, want in ((got_o.cpu().view(T, H, dv)[live], want_o[live]), (got_s.cpu(), want_s)):
+        off = float((got.double() - want).abs().max())
+        assert off <= 2e-5 * max(1.0, float(want.abs().max())), off

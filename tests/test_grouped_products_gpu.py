@@ -1,0 +1,62 @@
+"""One product per group of rows on the tcgen05 tensor cores: groups that are empty, of one row, of whole tiles and one more; widths that
+end inside a tile; and dense products whose last tile is short."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _silu_mul(y, limit):
+    g, u = y.chunk(2, -1)
+    if limit:
+        g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+        return g * torch.sigmoid(1.702 * g) * (u + 1)
+    return g * torch.sigmoid(g) * u
+
+
+@pytest.mark.parametrize("counts", [[1], [0, 256, 0, 1, 257, 0], [512, 513, 128, 0, 300], [0, 0, 5], [40] * 40, [1030, 129]])
+@pytest.mark.parametrize("N,K", [(256, 64), (272, 200), (1552, 136)])
+@pytest.mark.parametrize("epi,limit", [(0, 0.0), (2, 0.0), (3, 1.5)])
+@pytest.mark.parametrize("rows", [256, 512])
+def test_groups(counts, N, K, epi, limit, rows):
+    from pico_vllm_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(sum(counts) + N)
+    E, n = len(counts), sum(counts)
+    x = torch.randn(n + 3, K, generator=g, device=DEV).bfloat16()[:n]
+    w = (torch.randn(E, N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    c = torch.tensor(counts)
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), c.cumsum(0)]).to(torch.int32).to(DEV)
+    tiles = torch.cat([torch.zeros(1, dtype=torch.long), (-(-c // rows)).cumsum(0)]).to(torch.int32).to(DEV)
+    cols = N if epi == 0 else N // 2
+    out = torch.full((n + 2, cols), float("nan"), dtype=torch.bfloat16, device=DEV)
+    lib = ops.library()
+    assert lib.pico_gemm_tcgen05_grouped(x.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), tiles.data_ptr(), n, E, N, K, epi, rows,
+                                         limit, ops._stream()) == 0
+    at = 0
+    for e, k in enumerate(counts):
+        y = x[at:at + k].float() @ w[e].float().t()
+        want = y if epi == 0 else _silu_mul(y, limit)
+        got = out[at:at + k].float()
+        # one rounding to 16 bits of a float32 sum of K products of order K^-1/2
+        assert torch.allclose(got, want, atol=2e-2, rtol=1e-2), (e, float((got - want).abs().max()))
+        at += k
+    assert torch.isnan(out[n:].float()).all()
+    assert ops.tc_status() == 0
+
+
+@pytest.mark.parametrize("M", [512, 513, 640, 768, 769, 1025, 2111])
+def test_a_short_last_tile_of_a_dense_product(M):
+    from pico_vllm_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(M)
+    K, I = 328, 1000
+    x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(2 * I, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    y = x.float() @ w.float().t()
+    for rows in (256, 512):
+        assert torch.allclose(ops.tc_linear(x, w, rows=rows).float(), y, atol=2e-2, rtol=1e-2)
+        assert torch.allclose(ops.tc_gate_up_swiglu(x, w, rows=rows).float(), _silu_mul(y, 0.0), atol=2e-2, rtol=1e-2)
+        res = torch.ones(M, 2 * I, device=DEV)
+        ops.tc_linear_residual(x, w, res, rows=rows)
+        assert torch.allclose(res, y + 1, atol=1e-3, rtol=1e-3)
+    assert ops.tc_status() == 0
