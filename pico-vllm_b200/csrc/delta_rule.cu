@@ -621,7 +621,7 @@ __device__ __forceinline__ bool dc_find(const int* __restrict__ cu_q, const int*
 __global__ void __launch_bounds__(256)
 delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* __restrict__ v, int v_stride, const int* __restrict__ cu_q,
                            const int* __restrict__ positions, int S, float* __restrict__ coef, float* __restrict__ u0, int H, int G,
-                           int d, int dv) {
+                           int d, int dv, bool keep_v) {
     pdl_launch_dependents();
     pdl_wait();
     int t0, n;
@@ -631,9 +631,19 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* _
     float* q_s = k_s + DC_C * DC_LD;
     float* kk = q_s + DC_C * DC_LD;            // [C][C + 1]: k_i . k_j
     float* qk = kk + DC_C * (DC_C + 1);        // q_i . k_j
+    const int heads = H / G, slots = min(heads, 8);
     float* l_s = qk + DC_C * (DC_C + 1);       // a head's L [C][C], then M by columns; one for each of the warps that take heads
-    float* g_s = l_s + 8 * DC_C * DC_C;        // [8][C]: G
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = blockIdx.y;
+    float* g_s = l_s + slots * DC_C * DC_C;    // [slots][C]: G
+    float* v_s = g_s + slots * DC_C;           // keep_v: [C][heads * dv]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = blockIdx.y, vw = heads * dv;
+    if (keep_v) {                              // the heads' values, side by side in a row, on their way while M is made
+        for (int idx = threadIdx.x; idx < DC_C * (vw / 4); idx += 256) {
+            const int j = idx / (vw / 4), c = idx % (vw / 4) * 4;
+            if (j < n) dr_cp16(v_s + j * vw + c, v + (size_t)(t0 + j) * v_stride + (size_t)g * vw + c);
+            else *reinterpret_cast<float4*>(v_s + j * vw + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        dr_commit();
+    }
     for (int idx = threadIdx.x; idx < DC_C * (DC_D / 4); idx += 256) {
         const int i = idx / (DC_D / 4), c = idx % (DC_D / 4) * 4;
         float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), q4 = k4;
@@ -669,7 +679,6 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* _
         }
     }
     __syncthreads();
-    const int heads = H / G;
     for (int h0 = 0; h0 < heads; h0 += 8) {    // eight heads at a time, a warp each
         if (h0 + warp < heads) {
             const int h = g * heads + h0 + warp;
@@ -721,6 +730,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* _
             for (int i = 0; i < DC_C; i += 4)
                 *reinterpret_cast<float4*>(L + lane * DC_C + i) = make_float4(X[i] * beta, X[i + 1] * beta, X[i + 2] * beta, X[i + 3] * beta);
         }
+        dr_wait_all();
         __syncthreads();
         // M diag(G) K and M V, the heads one after the other: a thread has four columns and eight tokens i
         const int cg = DC_D / 4 + (dv + 3) / 4;
@@ -742,6 +752,8 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* _
                         b = *reinterpret_cast<const float4*>(k_s + j * DC_LD + c);
                         const float gj = g_s[hh * DC_C + j];
                         b = make_float4(gj * b.x, gj * b.y, gj * b.z, gj * b.w);
+                    } else if (keep_v) {
+                        b = *reinterpret_cast<const float4*>(v_s + j * vw + (h0 + hh) * dv + c - DC_D);
                     } else if (j < n) {
                         b = *reinterpret_cast<const float4*>(vc + (size_t)j * v_stride);
                     }
@@ -782,7 +794,7 @@ delta_chunk_kernel(const float* __restrict__ prep, int P, float* __restrict__ st
     const int t_begin = cu_q[seg], t_end = cu_q[seg + 1];
     if (t_end <= t_begin || positions[t_begin] < 0) return;      // an empty or a padding segment
     float* s_s = dsm + 2 * BUF;                // S by columns [NC][LDK]
-    float* w_s = s_s + DC_NC * DC_LDK;         // diag(D_Cj) U [C][NC]
+    float* w_s = s_s + DC_NC * DC_LDK;         // diag(D_Cj) U [C][NC], every number twice (the pairs that two rows at a time want)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hq = h / (H / G);
     int chunk = 0;
     for (int s = 0; s < seg; ++s) chunk += (cu_q[s + 1] - cu_q[s] + DC_C - 1) / DC_C;
@@ -884,7 +896,9 @@ delta_chunk_kernel(const float* __restrict__ prep, int P, float* __restrict__ st
             const float4 mv = *reinterpret_cast<const float4*>(u_s + i * DC_NC + 4 * warp);
             const float4 uu = make_float4(mv.x - x[0], mv.y - x[1], mv.z - x[2], mv.w - x[3]);
             const float wj = Wd[i];
-            *reinterpret_cast<float4*>(w_s + i * DC_NC + 4 * warp) = make_float4(wj * uu.x, wj * uu.y, wj * uu.z, wj * uu.w);
+            const float4 w4 = make_float4(wj * uu.x, wj * uu.y, wj * uu.z, wj * uu.w);
+            *reinterpret_cast<float4*>(w_s + 2 * (i * DC_NC + 4 * warp)) = make_float4(w4.x, w4.x, w4.y, w4.y);
+            *reinterpret_cast<float4*>(w_s + 2 * (i * DC_NC + 4 * warp) + 4) = make_float4(w4.z, w4.z, w4.w, w4.w);
             if (t0 + i < t_end && col_base + 4 * warp < dv)
                 *reinterpret_cast<float4*>(u + (size_t)(t0 + i) * H * dv + (size_t)h * dv + col_base + 4 * warp) = uu;
         }
@@ -900,14 +914,16 @@ delta_chunk_kernel(const float* __restrict__ prep, int P, float* __restrict__ st
 #pragma unroll 8
             for (int j = 0; j < DC_C; ++j) {
                 const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(k_s + j * DC_LDK + 4 * lane);
-                const float4 w = *reinterpret_cast<const float4*>(w_s + j * DC_NC + 4 * warp);
-                const float wc[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const f32x2 w2 = db_pair(wc[c], wc[c]);
-                    S[c][0] = db_fma2(k.x, w2, S[c][0]);
-                    S[c][1] = db_fma2(k.y, w2, S[c][1]);
-                }
+                const ulonglong2 wa = *reinterpret_cast<const ulonglong2*>(w_s + 2 * (j * DC_NC + 4 * warp));
+                const ulonglong2 wb = *reinterpret_cast<const ulonglong2*>(w_s + 2 * (j * DC_NC + 4 * warp) + 4);
+                S[0][0] = db_fma2(k.x, wa.x, S[0][0]);
+                S[0][1] = db_fma2(k.y, wa.x, S[0][1]);
+                S[1][0] = db_fma2(k.x, wa.y, S[1][0]);
+                S[1][1] = db_fma2(k.y, wa.y, S[1][1]);
+                S[2][0] = db_fma2(k.x, wb.x, S[2][0]);
+                S[2][1] = db_fma2(k.y, wb.x, S[2][1]);
+                S[3][0] = db_fma2(k.x, wb.y, S[3][0]);
+                S[3][1] = db_fma2(k.y, wb.y, S[3][1]);
             }
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -1039,11 +1055,14 @@ PICO_API int pico_gated_delta_chunks(const float* prep, const float* v, int v_st
     float* coef = scratch;
     float* s0 = coef + (size_t)chunks * H * DC_COEF;
     float* u = s0 + (size_t)chunks * H * ((dv + 3) / 4 * 4) * DC_D;
-    const size_t sm1 = (size_t)(2 * DC_C * DC_LD + 2 * DC_C * (DC_C + 1) + 8 * DC_C * DC_C + 8 * DC_C) * sizeof(float);
+    const int slots = H / G < 8 ? H / G : 8;
+    size_t sm1 = (size_t)(2 * DC_C * DC_LD + 2 * DC_C * (DC_C + 1) + slots * (DC_C * DC_C + DC_C)) * sizeof(float);
+    const bool keep_v = (size_t)DC_C * (H / G) * dv * sizeof(float) <= 32 * 1024;
+    if (keep_v) sm1 += (size_t)DC_C * (H / G) * dv * sizeof(float);
     cudaFuncSetAttribute(delta_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
-    pico_launch(delta_chunk_prepare_kernel, dim3(chunks, G), dim3(256), sm1, stream, prep, P, v, v_stride, cu_q, positions, S, coef, u, H, G, d, dv);
+    pico_launch(delta_chunk_prepare_kernel, dim3(chunks, G), dim3(256), sm1, stream, prep, P, v, v_stride, cu_q, positions, S, coef, u, H, G, d, dv, keep_v);
     const dim3 grid((dv + DC_NC - 1) / DC_NC, H, S);
-    size_t sm2 = (size_t)(2 * (2 * DC_C * DC_LDK + 2 * DC_C + DC_C * DC_NC) + DC_NC * DC_LDK + DC_C * DC_NC) * sizeof(float);
+    size_t sm2 = (size_t)(2 * (2 * DC_C * DC_LDK + 2 * DC_C + DC_C * DC_NC) + DC_NC * DC_LDK + 2 * DC_C * DC_NC) * sizeof(float);
     // (one block a multiprocessor where there are enough of them: see pico_gated_delta_rule)
     if ((long long)grid.x * grid.y * grid.z <= pico_num_sms() && sm2 < 116 * 1024) sm2 = 116 * 1024;
     cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);

@@ -111,10 +111,9 @@ struct TpArgs {
     float* resid;             // RESIDUAL: [M, N]
     float limit;              // CAPPED: as SWIGLU with g' sigmoid(1.702 g') (u' + 1), g' = min(g, limit), u' = clamp(u, -limit, limit)
     const float* bias;        // GELU: as SWIGLU with gelu_tanh(g + bias[i]) * (u + bias[I + i]); float32 [N], or null
-    // GROUPED: x holds the rows of group e at offsets[e] .. offsets[e + 1] - 1, w is [E, N, K]; tile_start[e]: tiles of 256 MB rows
-    // of the groups before (both [E + 1], on the device: the host never sees them)
+    // GROUPED: x holds the rows of group e at offsets[e] .. offsets[e + 1] - 1 ([E + 1], on the device: the host never sees them),
+    // w is [E, N, K]
     const int* offsets;
-    const int* tile_start;
     int E;
 };
 
@@ -189,7 +188,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
     asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int nkb = (p.K + TP_BK - 1) / TP_BK;
-    int* group_at = reinterpret_cast<int*>(const_cast<int*>(abort_s) + 1);      // GROUPED: offsets [E + 1], tile_start [E + 1]
+    int* group_at = reinterpret_cast<int*>(const_cast<int*>(abort_s) + 1);      // GROUPED: offsets [E + 1], then two more [E + 1]
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -213,24 +212,57 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();                 // x comes from the kernel before
+    // GROUPED: tiles with more than half their rows come first (all columns of them), then the short last ones of the groups, so that
+    // the pairs, which take tiles in turn, end together
+    int* tall_at = group_at + p.E + 1;        // [E + 1]: running number of such tiles of the groups
+    int* short_at = tall_at + p.E + 1;
+    int n_tall = 0, n_short = 0;
     if (GROUPED) {
-        for (int i = threadIdx.x; i < 2 * (p.E + 1); i += blockDim.x) group_at[i] = i <= p.E ? p.offsets[i] : p.tile_start[i - p.E - 1];
+        for (int i = threadIdx.x; i <= p.E; i += blockDim.x) group_at[i] = p.offsets[i];
         __syncthreads();
-        m_tiles = group_at[2 * p.E + 1];
+        if (warp == 0) {
+            int tall = 0, shorts = 0;
+            for (int e0 = 0; e0 < p.E; e0 += 32) {
+                const int e = e0 + lane, c = e < p.E ? group_at[e + 1] - group_at[e] : 0, rest = c % (2 * ROWS);
+                int a = c / (2 * ROWS) + (rest > ROWS ? 1 : 0), b = rest > 0 && rest <= ROWS ? 1 : 0;
+                const int a0 = a, b0 = b;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int au = __shfl_up_sync(0xffffffffu, a, o), bu = __shfl_up_sync(0xffffffffu, b, o);
+                    if (lane >= o) { a += au; b += bu; }
+                }
+                if (e < p.E) {
+                    tall_at[e] = tall + a - a0;
+                    short_at[e] = shorts + b - b0;
+                }
+                tall += __shfl_sync(0xffffffffu, a, 31);
+                shorts += __shfl_sync(0xffffffffu, b, 31);
+            }
+            if (lane == 0) {
+                tall_at[p.E] = tall;
+                short_at[p.E] = shorts;
+            }
+        }
+        __syncthreads();
+        n_tall = tall_at[p.E];
+        n_short = short_at[p.E];
     }
-    const int total_tiles = m_tiles * n_tiles;
+    const int total_tiles = (GROUPED ? n_tall + n_short : m_tiles) * n_tiles;
     // rows m0 .. m_end - 1 of tile t (this block has 128 of every 256), and the row of w its group starts at
-    struct Place { int m0, m_end, w0; };
+    struct Place { int m0, m_end, w0, nt; };
     auto place = [&](int t) {
-        const int mt = t % m_tiles;
-        if (!GROUPED) return Place{mt * 2 * ROWS, p.M, 0};
-        const int* first = group_at + p.E + 1;
+        if (!GROUPED) return Place{t % m_tiles * 2 * ROWS, p.M, 0, t / m_tiles};
+        const bool tall = t < n_tall * n_tiles;
+        if (!tall) t -= n_tall * n_tiles;
+        const int per = tall ? n_tall : n_short, mt = t % per;
+        const int* first = tall ? tall_at : short_at;
         int lo = 0, hi = p.E;                 // the largest e with first[e] <= mt
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
             if (first[mid] <= mt) lo = mid; else hi = mid;
         }
-        return Place{group_at[lo] + (mt - first[lo]) * 2 * ROWS, group_at[lo + 1], lo * p.N};
+        const int tile = tall ? mt - first[lo] : (group_at[lo + 1] - group_at[lo]) / (2 * ROWS);
+        return Place{group_at[lo] + tile * 2 * ROWS, group_at[lo + 1], lo * p.N, t / per};
     };
     // accumulators that tile has rows for
     auto accumulators = [&](const Place& at) { return MB == 2 && at.m_end - at.m0 <= 2 * TP_BM ? 1 : MB; };
@@ -240,7 +272,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
             int step = 0;
             for (int t = pair; t < total_tiles && !*abort_s; t += n_pairs) {
                 const Place at = place(t);
-                const int jn = accumulators(at), m0 = at.m0 + (int)rank * TP_BM, n0 = (t / m_tiles) * COLS;
+                const int jn = accumulators(at), m0 = at.m0 + (int)rank * TP_BM, n0 = at.nt * COLS;
                 const int w_row = at.w0 + (tp_is_glu(EPI) ? (rank ? p.N / 2 + n0 : n0) : n0 + (int)rank * (BN / 2));
                 for (int kb = 0; kb < nkb; ++kb, ++step) {
                     const int s = step % STAGES;
@@ -300,7 +332,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
         for (int t = pair; t < total_tiles; t += n_pairs, ++it) {
             const int buf = it % NBUF, use = it / NBUF;
             const Place at = place(t);
-            const int n0 = (t / m_tiles) * COLS, row = at.m0 + j * 2 * TP_BM + (int)rank * TP_BM + q * 32 + lane;
+            const int n0 = at.nt * COLS, row = at.m0 + j * 2 * TP_BM + (int)rank * TP_BM + q * 32 + lane;
             const bool empty_part = j >= accumulators(at);       // nothing was computed for this warp's rows
             bool ok = tp_wait(acc_full + buf, use & 1);
             if (!ok) {
@@ -472,7 +504,7 @@ static int tp_launch(const void* x, int ldx, const void* w, const TpArgs& a, cud
     if (rc) return rc;
     rc = tp_make_map(&wm, w, GROUPED ? (long long)a.E * a.N : a.N, a.K, a.K, BN / 2);
     if (rc) return rc;
-    const size_t smem = (size_t)STAGES * STAGE_BYTES + (2 * STAGES + 4) * 8 + 16 + 1024 + (GROUPED ? 2 * (a.E + 1) * sizeof(int) : 0);
+    const size_t smem = (size_t)STAGES * STAGE_BYTES + (2 * STAGES + 4) * 8 + 16 + 1024 + (GROUPED ? 3 * (a.E + 1) * sizeof(int) : 0);
     cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<BN, EPI, STAGES, MB, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int n_out = tp_is_glu(EPI) ? a.N / 2 : a.N;
     const int cols = tp_is_glu(EPI) ? BN / 2 : BN;
@@ -543,18 +575,19 @@ PICO_API int pico_gemm_tcgen05_pair(const void* x, int ldx, const void* w, void*
 
 // Rows of a group's tile in pico_gemm_tcgen05_grouped for n rows in E groups: 512, or 256 where the groups are short (with 512 rows a
 // product reads a quarter less from L2, with 256 less of a tile lies beyond its group's end).
-PICO_API int pico_gemm_tcgen05_group_rows(int n, int E) { return n >= 384LL * E ? 512 : 256; }
+PICO_API int pico_gemm_tcgen05_group_rows(int n, int E) { return n >= 352LL * E ? 512 : 256; }
 
 // One product per group: out[r] = x[r] w[e]^T for the rows r = offsets[e] .. offsets[e + 1] - 1; w [E, N, K], x [n, K] contiguous.  epi 0 (out
-// [n, N]), 2 or 3 (out [n, N / 2]) as above.  tile_start: tiles of `rows` rows (pico_gemm_tcgen05_group_rows) of the groups before.
-PICO_API int pico_gemm_tcgen05_grouped(const void* x, const void* w, void* out, const int* offsets, const int* tile_start, int n, int E, int N,
-                                       int K, int epi, int rows, float limit, cudaStream_t stream) {
+// [n, N]), 2 or 3 (out [n, N / 2]) as above.  rows: of a tile, 0 = pico_gemm_tcgen05_group_rows.
+PICO_API int pico_gemm_tcgen05_grouped(const void* x, const void* w, void* out, const int* offsets, int n, int E, int N, int K, int epi,
+                                       int rows, float limit, cudaStream_t stream) {
+    if (rows == 0) rows = pico_gemm_tcgen05_group_rows(n, E);
     if (n <= 0) return 0;
     if (E < 1 || E > TP_MAX_GROUPS || N < 16 || K < 64 || K % 8 != 0 || (rows != 256 && rows != 512)) return PICO_ERR_SIZE;
     if (epi == TP_STORE ? N % 8 != 0 : (N % 2 != 0 || (N / 2) % 8 != 0)) return PICO_ERR_SIZE;
     if (epi == TP_CAPPED && !(limit > 0.f)) return PICO_ERR_SIZE;
     TpArgs a = {};
-    a.M = n; a.N = N; a.K = K; a.out = (bf16*)out; a.limit = limit; a.offsets = offsets; a.tile_start = tile_start; a.E = E;
+    a.M = n; a.N = N; a.K = K; a.out = (bf16*)out; a.limit = limit; a.offsets = offsets; a.E = E;
 #define TP_GROUPED(EPI) return rows == 512 ? tp_launch<256, EPI, 2, true>(x, K, w, a, stream) : tp_launch<256, EPI, 1, true>(x, K, w, a, stream)
     if (epi == TP_STORE) TP_GROUPED(TP_STORE);
     if (epi == TP_SWIGLU) TP_GROUPED(TP_SWIGLU);

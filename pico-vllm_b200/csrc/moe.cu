@@ -495,7 +495,7 @@ PICO_API int pico_moe_tile_rows(int n, int E, int dtype, int K1, int K2) {
 PICO_API int pico_moe_group(const int* idx, int n, int E, int bm, int* offsets, int* tile_start, int* perm, int* place,
                             cudaStream_t stream) {
     if (n <= 0) return 0;
-    if (E < 1 || E > 4096 || (bm != 16 && bm != MOE_BM && bm != 256 && bm != 512)) return PICO_ERR_SIZE;
+    if (E < 1 || E > 4096 || (bm != 16 && bm != MOE_BM)) return PICO_ERR_SIZE;
     pico_launch(moe_group_kernel, dim3(1), dim3(n >= 4096 ? 1024 : 256), (size_t)2 * E * sizeof(int), stream, idx, n, E, bm,
                 offsets, tile_start, perm, place);
     return pico_launch_status();

@@ -34,7 +34,8 @@
 typedef unsigned long long u64;
 
 __device__ __forceinline__ float sample_weight(float x, float mx, float inv_t) { return expf((x - mx) * inv_t); }
-__device__ __forceinline__ u64 sample_fixed(float w) { return __float2ull_rz(w * 4294967296.0f); }
+// (a 32-bit conversion: the 64-bit one takes several times as long, once per entry and pass)
+__device__ __forceinline__ u64 sample_fixed(float w) { return w < 1.0f ? (u64)__float2uint_rz(w * 4294967296.0f) : 1ull << 32; }
 
 // sums and exclusive prefix sums of 64-bit integers over the block, in thread order; scratch: 33 entries
 __device__ __forceinline__ u64 block_excl_scan_u64(u64 v, u64* scratch, u64* total) {

@@ -94,8 +94,7 @@ def library():
         "pico_moe_gather": [vp, vp, i32, i32, i32, vp, vp],
         "pico_moe_combine_placed": [vp, vp, vp, i32, i32, i32, vp, vp, i32, vp, i32, vp, vp],
         "pico_moe_gemm": [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp, i32, f32, i32, vp],
-        "pico_gemm_tcgen05_grouped": [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp],
-        "pico_gemm_tcgen05_group_rows": [i32, i32],
+        "pico_gemm_tcgen05_grouped": [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp],
         "pico_moe_combine": [vp, vp, i32, i32, i32, vp, vp, i32, vp, i32, vp, vp],
         "pico_moe_scaled_act": [vp, vp, vp, i32, i32, i32, vp, i32, vp],
         "pico_qk_norm_rope_store": [vp, i32, vp, vp, vp, f32, vp, vp, f32, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32,
@@ -1122,8 +1121,7 @@ def moe_experts(h: torch.Tensor, idx: torch.Tensor, wgt: torch.Tensor, gate_up_w
     meta = torch.empty(2 * (Et + 1) + 2 * n, dtype=torch.int32, device=h.device)
     offsets, tile_start = meta[:Et + 1], meta[Et + 1:2 * (Et + 1)]
     perm, place = meta[2 * (Et + 1):2 * (Et + 1) + n], meta[2 * (Et + 1) + n:]
-    # rows per tile of the grouped products
-    bm = lib.pico_gemm_tcgen05_group_rows(n, E) if grouped else lib.pico_moe_tile_rows(n, E, code, D, ff)
+    bm = lib.pico_moe_tile_rows(n, E, code, D, ff)      # rows per tile of the grouped kernels that need no rows in order
     _check(lib.pico_moe_group(_ptr(idx), n, Et, bm, _ptr(offsets), _ptr(tile_start), _ptr(perm),
                               _ptr(place) if grouped else None, st), "moe_group")
     eidx, hsrc = (idx, h) if identity else (None, None)
@@ -1136,12 +1134,12 @@ def moe_experts(h: torch.Tensor, idx: torch.Tensor, wgt: torch.Tensor, gate_up_w
         _check(lib.pico_moe_gather(_ptr(h), _ptr(perm), n, top, D * h.element_size(), _ptr(xs), st), "moe_gather")
         a = torch.empty((n, ff), dtype=h.dtype, device=h.device)
         up_epi = 0 if not gated else 3 if act == MOE_ACT_CAPPED else 2
-        _check(lib.pico_gemm_tcgen05_grouped(_ptr(xs), _ptr(gate_up_weight), _ptr(a), _ptr(offsets), _ptr(tile_start), n, E, ff_rows, D, up_epi, bm,
+        _check(lib.pico_gemm_tcgen05_grouped(_ptr(xs), _ptr(gate_up_weight), _ptr(a), _ptr(offsets), n, E, ff_rows, D, up_epi, 0,
                                              float(limit), st), "gemm_tcgen05_grouped (up)")
         if not gated:
             _check(lib.pico_moe_scaled_act(_ptr(a), _ptr(perm), _ptr(in_w), n, ff, int(act), _ptr(a), code, st), "moe_scaled_act")
         ys = torch.empty((n, D), dtype=h.dtype, device=h.device)
-        _check(lib.pico_gemm_tcgen05_grouped(_ptr(a), _ptr(down_weight), _ptr(ys), _ptr(offsets), _ptr(tile_start), n, E, D, ff, 0, bm, 0.0, st),
+        _check(lib.pico_gemm_tcgen05_grouped(_ptr(a), _ptr(down_weight), _ptr(ys), _ptr(offsets), n, E, D, ff, 0, 0, 0.0, st),
                "gemm_tcgen05_grouped (down)")
         _check(lib.pico_moe_combine_placed(_ptr(ys), _ptr(place), _ptr(out_w), T, top, D, _ptr(y), _ptr(base), code, _ptr(eidx), E,
                                            _ptr(hsrc), st), "moe_combine_placed")
@@ -1288,8 +1286,11 @@ def gated_rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor], gate_logits:
     return y
 
 
-# (token, expert) pairs from which the experts' products run on the tcgen05 tensor cores over rows in expert order: MOE_RULE
-MOE_TC_MIN_ROWS = 1024
+# the experts' products run on the tcgen05 tensor cores, over rows in expert order, from this many (token, expert) pairs per expert on
+# (below, the experts' lists fit into tiles of 16 rows of the grouped mma.sync kernels, a stream of the weights; a layer of 16
+# experts, top 4, width 1,536, in us: 256 pairs 97 here and 98 there, 512 98 and 198, 8,192 208 and 763; 32 experts, width
+# 2,048: 256 pairs 255 and 231, 512 265 and 266, 800 269 and 360)
+MOE_TC_MIN_ROWS = 16
 MOE_TC_MAX_EXPERTS = 512
 
 
@@ -1297,7 +1298,7 @@ def moe_tc_takes(h: torch.Tensor, gate_up_weight: torch.Tensor, down_weight: tor
     """Whether the experts' products run on the tcgen05 tensor cores (bfloat16, many rows, row sizes that are multiples of 16
     bytes) instead of the grouped kernels that need no rows in order."""
     (E, _, D), ff = gate_up_weight.shape, down_weight.shape[2]
-    return (h.dtype == torch.bfloat16 and n >= MOE_TC_MIN_ROWS and E <= MOE_TC_MAX_EXPERTS and D % 8 == 0 and ff % 8 == 0 and D >= 64 and ff >= 64
+    return (h.dtype == torch.bfloat16 and n > MOE_TC_MIN_ROWS * E and E <= MOE_TC_MAX_EXPERTS and D % 8 == 0 and ff % 8 == 0 and D >= 64 and ff >= 64
             and (h.data_ptr() | gate_up_weight.data_ptr() | down_weight.data_ptr()) % 16 == 0)
 
 

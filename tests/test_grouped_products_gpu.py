@@ -15,7 +15,7 @@ def _silu_mul(y, limit):
     return g * torch.sigmoid(g) * u
 
 
-@pytest.mark.parametrize("counts", [[1], [0, 256, 0, 1, 257, 0], [512, 513, 128, 0, 300], [0, 0, 5], [40] * 40, [1030, 129]])
+@pytest.mark.parametrize("counts", [[1], [0, 256, 0, 1, 257, 0], [512, 513, 128, 0, 300], [0, 0, 5], [40] * 40, [1030, 129], [3] * 70 + [600]])
 @pytest.mark.parametrize("N,K", [(256, 64), (272, 200), (1552, 136)])
 @pytest.mark.parametrize("epi,limit", [(0, 0.0), (2, 0.0), (3, 1.5)])
 @pytest.mark.parametrize("rows", [256, 512])
@@ -27,11 +27,10 @@ def test_groups(counts, N, K, epi, limit, rows):
     w = (torch.randn(E, N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
     c = torch.tensor(counts)
     offsets = torch.cat([torch.zeros(1, dtype=torch.long), c.cumsum(0)]).to(torch.int32).to(DEV)
-    tiles = torch.cat([torch.zeros(1, dtype=torch.long), (-(-c // rows)).cumsum(0)]).to(torch.int32).to(DEV)
     cols = N if epi == 0 else N // 2
     out = torch.full((n + 2, cols), float("nan"), dtype=torch.bfloat16, device=DEV)
     lib = ops.library()
-    assert lib.pico_gemm_tcgen05_grouped(x.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), tiles.data_ptr(), n, E, N, K, epi, rows,
+    assert lib.pico_gemm_tcgen05_grouped(x.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), n, E, N, K, epi, rows,
                                          limit, ops._stream()) == 0
     at = 0
     for e, k in enumerate(counts):
