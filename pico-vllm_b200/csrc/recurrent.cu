@@ -540,8 +540,8 @@ causal_conv_silu_kernel(const TA* __restrict__ proj, int row_stride, int c_off, 
 }
 
 // The same with four channels a thread (rows start on four elements) and CV_TOK tokens a block, whose inputs are all asked for
-// before the first is used: one thread's loads came one after the other before (2,048 tokens of 3,072 channels, bfloat16: CONV_US,
-// 25 one channel a thread).
+// before the first is used: one thread's loads came one after the other before (2,048 tokens of 3,072 channels, bfloat16: 16 us,
+// 25 one channel a thread; 22 with the weights of four taps read one by one).
 template <typename TA> struct Four;
 template <> struct Four<float> {
     float4 v;
@@ -575,14 +575,24 @@ causal_conv_silu4_kernel(const TA* __restrict__ proj, int row_stride, int c_off,
         seg[i] = tok_seg[t];
     }
     float4 wt[M], win[M];
+    if (taps == M) {       // a channel's four weights in one load (one by one, 64 bytes apart from lane to lane, they bound the kernel)
+        const float4* w4 = reinterpret_cast<const float4*>(w) + c;
+        const float4 a = w4[0], b1 = w4[1], c1 = w4[2], d1 = w4[3];
+        wt[0] = make_float4(a.x, b1.x, c1.x, d1.x);
+        wt[1] = make_float4(a.y, b1.y, c1.y, d1.y);
+        wt[2] = make_float4(a.z, b1.z, c1.z, d1.z);
+        wt[3] = make_float4(a.w, b1.w, c1.w, d1.w);
+    } else {
 #pragma unroll
-    for (int k = 0; k < M; ++k) {
-        float wk[4];
+        for (int k = 0; k < M; ++k) {
+            float wk[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) wk[e] = k < taps ? w[(size_t)(c + e) * taps + taps - 1 - k] : 0.f;
-        wt[M - 1 - k] = make_float4(wk[0], wk[1], wk[2], wk[3]);
-        win[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int e = 0; e < 4; ++e) wk[e] = k < taps ? w[(size_t)(c + e) * taps + taps - 1 - k] : 0.f;
+            wt[M - 1 - k] = make_float4(wk[0], wk[1], wk[2], wk[3]);
+        }
     }
+#pragma unroll
+    for (int k = 0; k < M; ++k) win[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 bias = b ? *reinterpret_cast<const float4*>(b + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     bool have = false;
 #pragma unroll
@@ -655,7 +665,7 @@ PICO_API int pico_causal_conv_silu(const void* proj, int row_stride, int c_off, 
     // four channels a thread from the sizes on where tokens share a block, if every row and table starts on four elements
     const bool four = tpb == CV_TOK && taps <= 4 && C % 4 == 0 && c_off % 4 == 0 && row_stride % 4 == 0 &&
                       ((uintptr_t)proj & (dtype == PICO_F32 ? 15 : 7)) == 0 &&
-                      (((uintptr_t)b | (uintptr_t)conv_state | (uintptr_t)out) & 15) == 0;
+                      (((uintptr_t)w | (uintptr_t)b | (uintptr_t)conv_state | (uintptr_t)out) & 15) == 0;
 #define CV_LAUNCH(TA)                                                                                                    \
     do {                                                                                                                 \
         if (four)                                                                                                        \
