@@ -785,7 +785,7 @@ group_rms_norm_kernel(const float* __restrict__ x, int x_stride, int group_strid
 }
 
 // The plain form (no normaliser, skip or gate before the norm) of groups of up to 512 columns whose rows start on four numbers: a lane
-// reads its columns once, four at a time, and keeps them (2,048 rows of 12 groups of 128 with a gate: NORM_US, 15 with a pass for
+// reads its columns once, four at a time, and keeps them (2,048 rows of 12 groups of 128 with a gate: 11 us, 15 with a pass for
 // the sum and a pass for the result, a number a load).
 template <typename TA>
 __global__ void __launch_bounds__(128)

@@ -21,8 +21,8 @@
 //      are kept or dropped together);
 //   3. kept mass per block, the block and then the token at which the running sum passes the target.
 // A pass that is a kernel of its own, over the row in L2, with the blocks' results in device memory, costs 10 to 25 us at 64 rows
-// of 152,064 whatever it computes; the whole choice with top-p took 200 us as five of them (162 without top-p) and SAMPLE_US.
-// Longer rows than shared memory holds (ROW_MAX entries) are read again in every pass.
+// of 152,064 whatever it computes; the whole choice with top-p took 200 us as five of them (162 without top-p) and 80 (34) as this one; 37 rows run at a time.
+// Longer rows than shared memory holds (155,648 entries) are read again in every pass.
 #include "common.cuh"
 
 #define SAMPLE_THREADS 512
@@ -34,8 +34,7 @@
 typedef unsigned long long u64;
 
 __device__ __forceinline__ float sample_weight(float x, float mx, float inv_t) { return expf((x - mx) * inv_t); }
-// (a 32-bit conversion: the 64-bit one takes several times as long, once per entry and pass)
-__device__ __forceinline__ u64 sample_fixed(float w) { return w < 1.0f ? (u64)__float2uint_rz(w * 4294967296.0f) : 1ull << 32; }
+__device__ __forceinline__ u64 sample_fixed(float w) { return __float2ull_rz(w * 4294967296.0f); }
 
 // sums and exclusive prefix sums of 64-bit integers over the block, in thread order; scratch: 33 entries
 __device__ __forceinline__ u64 block_excl_scan_u64(u64 v, u64* scratch, u64* total) {
