@@ -30,18 +30,33 @@ class AttentionPlan(MixerPlan):
 MAX_MIXED_SCRATCH = 32 << 20       # float32 numbers (128 MB) that splitting the single tokens of a mixed step may ask for
 
 
+DECODE_RAGGED_KEYS = 4096          # longest context from which the parts of a ragged batch need not all run at once
+
+
 def decode_splits(shape: StepShape, n_kv_heads: int, window: Optional[int] = None) -> int:
     """How many parts to cut each single token's key range into: a power of two (the parts of one
     token and kv head run as one thread-block cluster): up to 16 while that is at most one block
     per SM, else up to 8 while the blocks make no more than one wave of two per SM; each part at
-    least two tiles of 64 keys of the context, or of the ``window`` a token sees of it."""
+    least two tiles of 64 keys of the context, or of the ``window`` a token sees of it.
+
+    bfloat16: up to eight parts of one tile, but no two parts of fewer than 512 keys (attention of the 1.5B / 7B shape with its
+    projections, 512 keys each: batch 4 in 8 parts 22 / 36 us, in 2 or 4 24 / 38; 200 keys, batch 8 / 16: 24 / 42 us whole, 24 / 42
+    or more in two parts).  Contexts of all ages, the longest DECODE_RAGGED_KEYS and more: four parts also where that
+    makes more than a wave, since unsplit the longest sets the time (up to 8,000 keys, 4 kv heads: batch 40 / 64 / 48 in 139 / 158 /
+    145 us, now 108 / 133 / 119; up to 4,096, batch 40 / 64: 88 / 100, now 80 / 96; at 3,000 some gain and some lose).  Of
+    one length they stay whole (8,000 keys, batch 40: 150 us, 156 in four parts)."""
     groups = max(1, shape.num_tokens * n_kv_heads)
+    keys = shape.max_kv if window is None else min(shape.max_kv, window)
     want = 16 if groups * 16 <= shape.num_sms else min(2 * shape.num_sms // groups, 8)
-    want = min(want, (shape.max_kv if window is None else min(shape.max_kv, window)) // 128)
+    short = getattr(shape.engine, "dtype", "") == "bfloat16"
+    if short and want < 4 and keys >= DECODE_RAGGED_KEYS:
+        seen = [min(st + 1, keys) for n, st in zip(shape.q_lens, shape.starts) if n == 1]
+        want = 4 if seen and 4 * sum(seen) <= 3 * keys * len(seen) else want
+    want = min(want, max(keys // 128, min(keys // 64, 8) if short else 0))
     splits = 1
     while splits * 2 <= want:
         splits *= 2
-    return splits
+    return 1 if short and splits == 2 and keys < 1024 else splits
 
 
 @register("mixer", "gqa_attention")
@@ -85,7 +100,7 @@ class GQAAttention(Part):
     def _splits(self, shape: StepShape) -> int:
         """As :func:`decode_splits`, but where single tokens run in a kernel of their own beside the portions only they are
         counted: 37 of them with 3,001 tokens at most beside two portions (2,013 tokens, 28 / 4 heads) make 148 blocks unsplit,
-        and the longest sets the time (MIXED_US).  Scratch is laid out for every token of the step: no more parts than
+        and the longest sets the time (68 us; 58 in two parts).  Scratch is laid out for every token of the step: no more parts than
         MAX_MIXED_SCRATCH holds."""
         portions = sum(n for n in shape.q_lens if n > 1)
         dtype = getattr(torch, getattr(shape.engine, "dtype", "") or "float32")

@@ -1,0 +1,29 @@
+"""How many parts a single token's keys are cut into: by the contexts' lengths and by how even they are."""
+import pytest
+
+from pico_vllm_b200.config import EngineConfig
+from pico_vllm_b200.parts.attention import decode_splits
+from pico_vllm_b200.parts.base import StepShape
+
+
+def _splits(contexts, kv_heads, dtype="bfloat16", window=None):
+    n = len(contexts)
+    shape = StepShape(num_tokens=n, num_segments=n, q_lens=[1] * n, starts=[c - 1 for c in contexts], max_kv=max(contexts),
+                      decode_only=True, num_sms=148, engine=EngineConfig(dtype=dtype))
+    return decode_splits(shape, kv_heads, window)
+
+
+@pytest.mark.parametrize("contexts,kv_heads,parts,before", [
+    ([200], 2, 1, 1), ([255], 2, 1, 1), ([256], 2, 4, 2), ([512], 2, 8, 4), ([1500], 2, 8, 8), ([2048], 2, 16, 16),
+    ([500] * 32, 4, 1, 2), ([1023] * 32, 4, 1, 2), ([1024] * 32, 4, 2, 2),                                      # two parts at most
+    ([8000] * 40, 4, 1, 1), ([8000] + [3000] * 39, 4, 4, 1), ([4095] + [1000] * 39, 4, 1, 1), ([4096] + [1000] * 39, 4, 4, 1),
+])
+def test_parts(contexts, kv_heads, parts, before):
+    assert _splits(contexts, kv_heads) == parts
+    assert _splits(contexts, kv_heads, "float32") == before
+
+
+def test_a_window_bounds_the_keys():
+    assert _splits([8000] + [3000] * 39, 4, window=4000) == 1
+    assert _splits([8000] + [100] * 39, 4, window=5000) == 4
+    assert _splits([8000], 2, window=300) == 4
