@@ -60,7 +60,7 @@ delta_prepare_kernel(const float* __restrict__ xc, int xc_stride, int q_off, int
     }
     const float* row = xc + t * xc_stride;
     if (PER_HEAD && vec) {
-        // four numbers a lane, each read once (2,048 tokens of 6 heads of 128: PREP_US, 18 in two passes a number a load)
+        // four numbers a lane, each read once (2,048 tokens of 6 heads of 128: 14 us, 18 in two passes a number a load)
         for (int g = warp; g < G; g += nw) {
             const int i = lane * 4;
             const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(16 * LPC / CPL)
 gated_delta_block_kernel(const float* __restrict__ prep, int P, const float* __restrict__ v, int v_stride,
                          float* __restrict__ state, const int* __restrict__ seg_slots, const int* __restrict__ cu_q,
                          const int* __restrict__ positions, float* __restrict__ out, int out_stride, int H, int G, int d,
-                         int dv, int vec) {
+                         int dv, int vec, int below) {
     pdl_wait();                         // the kernel that follows is released at the end (see above)
     extern __shared__ __align__(16) float dsm[];
     constexpr int dp = RPL * LPC, NC = 16, NTH = NC / CPL * LPC, NV = 8 * CPL, VL = LPC / NV;      // VL: lanes that share a sum
@@ -366,7 +366,7 @@ gated_delta_block_kernel(const float* __restrict__ prep, int P, const float* __r
     constexpr int VAT = 2 * dp, SAT = VAT + NC, tok_floats = SAT + 12;      // q [dp], k [dp], v [NC], a, beta, -, -, eight dot products
     const int seg = blockIdx.z, h = blockIdx.y, col_base = blockIdx.x * NC;
     const int t_begin = cu_q[seg], t_end = cu_q[seg + 1];
-    if (t_end <= t_begin || positions[t_begin] < 0) return;      // an empty or a padding segment
+    if (t_end <= t_begin || t_end - t_begin >= below || positions[t_begin] < 0) return;      // an empty, a long or a padding segment
     const int sub = threadIdx.x % LPC, lcol = threadIdx.x / LPC * CPL, lane0 = (threadIdx.x & 31) - sub;
     const int hq = h / (H / G);
     float* st = state + ((size_t)seg_slots[seg] * H + h) * (size_t)dv * d;
@@ -594,7 +594,7 @@ gated_delta_block_kernel(const float* __restrict__ prep, int P, const float* __r
 // The chain is bound by what a block reads from shared memory (K, M diag(G) K and S once a chunk for every four columns), over
 // len / 32 dependent steps of the longest segment: hence the two products only (with all four in the chain 170 us for the
 // tokens below), four warps a block (eight, with half the columns each: 225) and 16 columns.
-// 2,048 tokens of twelve heads with d = dv = 128 in segments of 341, 682 and 1,025: CHUNK_US (four tokens at a time: 248).
+// 2,048 tokens of twelve heads with d = dv = 128 in segments of 341, 682 and 1,025: 195 us, of which the chain 118 (four tokens at a time: 248).
 #define DC_C 32
 #define DC_D 128                               // rows of S, keys padded with zeros
 #define DC_LD (DC_D + 4)                       // rows that lanes read side by side, 16 bytes each
@@ -603,16 +603,31 @@ gated_delta_block_kernel(const float* __restrict__ prep, int P, const float* __r
 #define DC_OC 128                              // columns of O a block
 #define DC_COEF (DC_C * DC_D + DC_C * DC_C + 2 * DC_C)      // floats a chunk and head: M diag(G) K, E by columns, G, D_Cj
 
-// Which chunk of which segment number c is; false when there are not that many, or it is padding.
+#define DC_LEAST 64                            // tokens of a segment that goes in chunks; shorter ones are pico_gated_delta_rule's
+
+__device__ __forceinline__ int dc_chunks_of(const int* __restrict__ cu_q, int S, int seg) {
+    const int len = seg < S ? cu_q[seg + 1] - cu_q[seg] : 0;
+    return len >= DC_LEAST ? (len + DC_C - 1) / DC_C : 0;
+}
+// Which chunk of which segment number c is, found by every warp for itself; false when there are not that many, or it is padding.
 __device__ __forceinline__ bool dc_find(const int* __restrict__ cu_q, const int* __restrict__ positions, int S, int c, int& t0, int& n) {
-    for (int seg = 0; seg < S; ++seg) {
-        const int begin = cu_q[seg], len = cu_q[seg + 1] - begin, k = (len + DC_C - 1) / DC_C;
-        if (c < k) {
-            t0 = begin + c * DC_C;
-            n = min(DC_C, len - c * DC_C);
+    const int lane = threadIdx.x & 31;
+    for (int first = 0; first < S; first += 32) {
+        const int mine = dc_chunks_of(cu_q, S, first + lane);
+        int upto = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += up;
+        }
+        const unsigned after = __ballot_sync(0xffffffffu, c < upto);
+        if (after) {
+            const int l = __ffs(after) - 1, at = c - __shfl_sync(0xffffffffu, upto - mine, l), begin = cu_q[first + l];
+            t0 = begin + at * DC_C;
+            n = min(DC_C, cu_q[first + l + 1] - t0);
             return positions[begin] >= 0;
         }
-        c -= k;
+        c -= __shfl_sync(0xffffffffu, upto, 31);
     }
     return false;
 }
@@ -792,12 +807,14 @@ delta_chunk_kernel(const float* __restrict__ prep, int P, float* __restrict__ st
     constexpr int MG = DC_C * DC_LDK, BUF = 2 * MG + 2 * DC_C + DC_C * DC_NC;      // a chunk: K, M diag(G) K, G, D_Cj, M V [C][NC]
     const int seg = blockIdx.z, h = blockIdx.y, col_base = blockIdx.x * DC_NC;
     const int t_begin = cu_q[seg], t_end = cu_q[seg + 1];
-    if (t_end <= t_begin || positions[t_begin] < 0) return;      // an empty or a padding segment
+    if (t_end - t_begin < DC_LEAST || positions[t_begin] < 0) return;      // a short or a padding segment
     float* s_s = dsm + 2 * BUF;                // S by columns [NC][LDK]
     float* w_s = s_s + DC_NC * DC_LDK;         // diag(D_Cj) U [C][NC], every number twice (the pairs that two rows at a time want)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hq = h / (H / G);
     int chunk = 0;
-    for (int s = 0; s < seg; ++s) chunk += (cu_q[s + 1] - cu_q[s] + DC_C - 1) / DC_C;
+    for (int s = lane; s < seg; s += 32) chunk += dc_chunks_of(cu_q, seg, s);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) chunk += __shfl_xor_sync(0xffffffffu, chunk, o);
     auto fetch = [&](int t0, int ch, float* buf) {
         const int n = min(DC_C, t_end - t0);
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1036,12 +1053,12 @@ delta_chunk_out_kernel(const float* __restrict__ prep, int P, const int* __restr
 }
 
 // Floats of scratch that pico_gated_delta_chunks needs for T tokens in S segments: coefficients, U, S before every chunk.
-static long long dc_chunks(int T, int S) { return (long long)T / DC_C + S; }
+static long long dc_chunks(int T, int S) { return (long long)T / DC_C + (S < T / DC_LEAST ? S : T / DC_LEAST) + 1; }
 PICO_API long long pico_gated_delta_chunk_floats(int T, int S, int H, int dv) {
     return dc_chunks(T, S) * H * (DC_COEF + (long long)((dv + 3) / 4 * 4) * DC_D) + (long long)T * H * dv;
 }
 
-// The recurrence with one decay a head in chunks; T: tokens of all segments.  d up to 128; d, dv, the strides multiples of 4, all
+// The recurrence with one decay a head in chunks for the segments of DC_LEAST tokens and more; T: tokens of all segments.  d up to 128; d, dv, the strides multiples of 4, all
 // addresses of 16 bytes: anything else is refused.
 PICO_API int pico_gated_delta_chunks(const float* prep, const float* v, int v_stride, float* state, const int* seg_slots,
                                      const int* cu_q, const int* positions, float* out, int out_stride, int T, int S, int H, int G,
@@ -1074,11 +1091,12 @@ PICO_API int pico_gated_delta_chunks(const float* prep, const float* v, int v_st
     return pico_launch_status();
 }
 
+// below > 0 (with blocked): only the segments of fewer tokens.
 PICO_API int pico_gated_delta_rule(const float* prep, const float* v, int v_stride, float* state, const int* seg_slots,
                                    const int* cu_q, const int* positions, float* out, int out_stride, int S, int H, int G,
-                                   int d, int dv, int per_head, int blocked, cudaStream_t stream) {
+                                   int d, int dv, int per_head, int blocked, int below, cudaStream_t stream) {
     if (S <= 0) return 0;
-    if (H < 1 || G < 1 || H % G || d < 1 || d > 256 || dv < 1) return PICO_ERR_SIZE;
+    if (H < 1 || G < 1 || H % G || d < 1 || d > 256 || dv < 1 || (below > 0 && !(per_head && blocked))) return PICO_ERR_SIZE;
     const int P = 2 * G * d + (per_head ? 4 * H + 8 * G : H * d + H + G);
     const dim3 grid((dv + 15) / 16, H, S);
     if (grid.z > 65535 || grid.y > 65535) return PICO_ERR_SIZE;
@@ -1107,7 +1125,7 @@ PICO_API int pico_gated_delta_rule(const float* prep, const float* v, int v_stri
         if (smem > 48 * 1024)                                                                                               \
             cudaFuncSetAttribute(gated_delta_block_kernel<N, L, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         pico_launch((gated_delta_block_kernel<N, L, C>), grid, dim3(16 * L / C), smem, stream, prep, P, v, v_stride, state, \
-                    seg_slots, cu_q, positions, out, out_stride, H, G, d, dv, vec);                                         \
+                    seg_slots, cu_q, positions, out, out_stride, H, G, d, dv, vec, below > 0 ? below : 0x7fffffff);                                         \
     } while (0)
     if (per_head && blocked) {
         const int vec = d % 4 == 0 && dv % 4 == 0 && v_stride % 4 == 0 && (((uintptr_t)prep | (uintptr_t)v) & 15) == 0;

@@ -117,7 +117,7 @@ def library():
         "pico_group_rms_norm": [vp, i32, i32, i32, i32, vp, f32, vp, vp, i32, vp, i32, vp, i32, vp, i32, i32, vp, i32, i32, vp],
         "pico_delta_prepare": [vp, i32, i32, i32, vp, i32, i32, vp, i32, vp, vp, vp, i32, i32, i32, i32, f32, f32, i32, i32, i32, vp],
         "pico_gated_delta_chunks": [vp, vp, i32, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp],
-        "pico_gated_delta_rule": [vp, vp, i32, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp],
+        "pico_gated_delta_rule": [vp, vp, i32, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp],
         "pico_pair_rope_norm_store": [vp, i32, i32, i32, i32, vp, vp, i32, i32, vp, vp, f32, vp, vp, vp, vp, i32, i32, i32, i32,
                                       i32, i32, i32, i32, vp],
         "pico_sum_add_norm": [vp, vp, vp, i32, f32, f32, vp, vp, i32, f32, f32, vp, vp, i32, f32, f32, vp, i32, f32, vp, vp, i32,
@@ -1613,14 +1613,30 @@ def delta_prepare(xc: torch.Tensor, q_off: int, k_off: int, proj: torch.Tensor, 
     return prep
 
 
-# longest segment from which the recurrence with a decay per head runs in chunks of 32 tokens: CHUNK_RULE
-DELTA_CHUNK_MIN_TOKENS = 64
+# Longest segment from which the recurrence with a decay per head runs in chunks of 32 tokens, and what every further segment adds to it.
+# In chunks a step costs more work and fewer dependent steps, so it pays while the longest segment sets the time (us in chunks / four
+# tokens at a time, 12 heads of 128): 256 tokens 48 / 46, 512 71 / 87, 2,048 232 / 333; two of 1,024 199 / 271, but four of 512 180 / 142.
+# The short ones are a launch of their own, and blocks that find nothing to do: 60 single tokens beside 512 122 / 137 (16 heads 161 / 138),
+# beside 1,024 208 / 267; 250 beside 700 304 / 217.
+DELTA_CHUNK_MIN_TOKENS = 512
+DELTA_CHUNK_PER_SEGMENT = 8
 
 
-def delta_chunks_take(v: torch.Tensor, state: torch.Tensor, d: int, dv: int, max_q_len: int) -> bool:
-    """Long segments, keys of 65 to 128 numbers, and everything the kernel reads 16 bytes at a time lies on 16 bytes.  What is prepared
-    for such a step needs no dot products with earlier rows (:func:`delta_prepare` with ``max_q_len`` 1)."""
-    return (max_q_len >= DELTA_CHUNK_MIN_TOKENS and 64 < d <= 128 and d % 4 == 0 and dv % 4 == 0 and v.stride(0) % 4 == 0
+DELTA_CHUNK_LEAST = 64             # (as in delta_rule.cu)
+# float32 numbers (512 MB) that a step in chunks may ask for: 86 KB a chunk and head of 128 and the values once more
+DELTA_CHUNK_MAX_SCRATCH = 128 << 20
+
+
+def delta_chunks_take(v: torch.Tensor, state: torch.Tensor, d: int, dv: int, max_q_len: int, segments: int) -> bool:
+    """A long segment that holds half of the tokens, keys of 65 to 128 numbers, scratch within its bound, and everything the kernels read 16 bytes at a time lies on 16
+    bytes.  The segments of DELTA_CHUNK_LEAST tokens and more then go in chunks, the others as in any step; where there is only one,
+    its rows need no dot products with earlier ones (:func:`delta_prepare` with ``max_q_len`` 1)."""
+    T, H = v.shape[0], state.shape[1]
+    if (T // 32 + min(segments, T // DELTA_CHUNK_LEAST) + 1) * H * (5184 + 128 * dv) + T * H * dv > DELTA_CHUNK_MAX_SCRATCH:
+        return False
+    if max_q_len < DELTA_CHUNK_MIN_TOKENS + DELTA_CHUNK_PER_SEGMENT * (segments - 1) or 2 * max_q_len < T:
+        return False
+    return (64 < d <= 128 and d % 4 == 0 and dv % 4 == 0 and v.stride(0) % 4 == 0
             and (v.data_ptr() | state.data_ptr()) % 16 == 0)
 
 
@@ -1650,10 +1666,14 @@ def gated_delta_rule(prep: torch.Tensor, v: torch.Tensor, state: torch.Tensor, s
     if cu_q.shape[0] != S + 1 or positions.shape[0] != T:
         raise KernelError("gated_delta_rule: cu_q must have one more entry than seg_slots, positions one per token")
     out = torch.empty((T, H * vdim), dtype=torch.float32, device=prep.device)
-    if per_head and delta_chunks_take(v, state, d, vdim, max_q_len):
-        if prep.data_ptr() % 16:
-            raise KernelError("gated_delta_rule: prep must start on 16 bytes")
+    chunks = per_head and delta_chunks_take(v, state, d, vdim, max_q_len, S)
+    if chunks and prep.data_ptr() % 16 == 0:
         lib = library()
+        if S > 1:
+            _check(lib.pico_gated_delta_rule(_ptr(prep), _ptr(v), v.stride(0), _ptr(state), _ptr(seg_slots), _ptr(cu_q), _ptr(positions),
+                                             _ptr(out), out.stride(0), S, H, G, d, vdim, 1, 1, DELTA_CHUNK_LEAST, _stream()),
+                   f"gated_delta_rule (dim {d})")
+            _count()
         scratch = torch.empty(lib.pico_gated_delta_chunk_floats(T, S, H, vdim), dtype=torch.float32, device=prep.device)
         _check(lib.pico_gated_delta_chunks(_ptr(prep), _ptr(v), v.stride(0), _ptr(state), _ptr(seg_slots), _ptr(cu_q), _ptr(positions),
                                            _ptr(out), out.stride(0), T, S, H, G, d, vdim, _ptr(scratch), _stream()),
@@ -1662,7 +1682,7 @@ def gated_delta_rule(prep: torch.Tensor, v: torch.Tensor, state: torch.Tensor, s
         return out
     _check(library().pico_gated_delta_rule(_ptr(prep), _ptr(v), v.stride(0), _ptr(state), _ptr(seg_slots), _ptr(cu_q),
                                            _ptr(positions), _ptr(out), out.stride(0), S, H, G, d, vdim, 1 if per_head else 0,
-                                           1 if max_q_len >= DELTA_BLOCK_MIN_TOKENS else 0, _stream()),
+                                           1 if max_q_len >= DELTA_BLOCK_MIN_TOKENS and not (chunks and S == 1) else 0, 0, _stream()),
            f"gated_delta_rule (dim {d})")
     _count()
     return out

@@ -123,10 +123,10 @@ class GatedDeltaRule(Part):
         if self.head_decay:
             g0 = self.channels
             b0, a0 = g0 + H * dv, g0 + H * dv + H
-            # (a step that runs in chunks needs no dot products between neighbouring rows)
-            chunks = ops.delta_chunks_take(xc[:, 2 * G * d:], memory.state, d, dv, batch.max_prefill_q)
+            # (one segment that goes in chunks needs no dot products between neighbouring rows)
+            alone = batch.seg_slots.shape[0] == 1 and ops.delta_chunks_take(xc[:, 2 * G * d:], memory.state, d, dv, batch.max_prefill_q, 1)
             prep = ops.delta_prepare(xc, 0, G * d, proj, b0, proj[:, a0:a0 + H], self.dt_bias, self.a_log, H, G, d, per_head=True,
-                                     max_q_len=1 if chunks else batch.max_prefill_q)
+                                     max_q_len=1 if alone else batch.max_prefill_q)
             o = ops.gated_delta_rule(prep, xc[:, 2 * G * d:], memory.state, batch.seg_slots, batch.cu_q, batch.positions,
                                      H, G, d, dv, per_head=True, max_q_len=batch.max_prefill_q)
             y = ops.group_rms_norm(o, H, dv, dv, self.out_norm, self.eps, h.dtype, post_gate=proj[:, g0:g0 + H * dv],

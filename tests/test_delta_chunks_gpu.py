@@ -37,10 +37,10 @@ def _oracle(q, k, v, a, beta, state, slots, cu, pos):
 
 @pytest.mark.parametrize("H,G,d,dv", [(2, 1, 128, 128), (3, 3, 68, 20), (10, 2, 100, 36), (1, 1, 128, 4)])
 @pytest.mark.parametrize("lens,pad_at", [([64], None), ([1, 31, 32, 33, 70, 1], None), ([97, 5, 2, 64], 1), ([0, 128, 0, 65], None)])
-@pytest.mark.parametrize("decays", ["middling", "nought and one"])
-def test_chunks(H, G, d, dv, lens, pad_at, decays):
+@pytest.mark.parametrize("decays,off", [("middling", 0), ("nought and one", 0), ("middling", 1)])
+def test_chunks(H, G, d, dv, lens, pad_at, decays, off, monkeypatch):
     from pico_vllm_b200 import ops
-    assert max(lens) >= ops.DELTA_CHUNK_MIN_TOKENS
+    monkeypatch.setattr(ops, "delta_chunks_take", lambda *a: True)
     g = torch.Generator().manual_seed(d + dv + len(lens))
     cu, pos, slots = _segments(lens, pad_at)
     T, S = int(cu[-1]), len(lens)
@@ -51,16 +51,33 @@ def test_chunks(H, G, d, dv, lens, pad_at, decays):
     a = torch.rand(T, H, generator=g) * 0.2 + 0.8 if decays == "middling" else (torch.rand(T, H, generator=g) > 0.1).float()
     beta = torch.rand(T, H, generator=g)
     state = torch.randn(S + 1, H, dv, d, generator=g) * 0.3
+    dots = torch.full((T, G, 8), float("nan"))                    # with the same row's key and the three before, for short segments
+    dots[:, :, 0] = (q * k).sum(-1)
+    for j in range(3):
+        dots[j + 1:, :, 1 + j] = (q[j + 1:] * k[:T - j - 1]).sum(-1)
+        dots[j + 1:, :, 4 + j] = (k[j + 1:] * k[:T - j - 1]).sum(-1)
     prep = torch.cat([q.reshape(T, -1), k.reshape(T, -1), torch.stack([a, beta, a * float("nan"), beta], -1).reshape(T, -1),
-                      torch.full((T, 8 * G), float("nan"))], 1).contiguous()
+                      dots.reshape(T, -1)], 1).contiguous()
     want_o, want_s = _oracle(q, k, v, a, beta, state, slots, cu, pos)
     wide = torch.cat([torch.zeros(T, 4), v.reshape(T, -1)], 1).to(DEV)
     got_s, p = state.to(DEV), prep.to(DEV)
-    assert ops.delta_chunks_take(wide[:, 4:], got_s, d, dv, max(lens))
+    if off:                                                       # rows off 16 bytes: nothing in chunks
+        p = torch.cat([torch.zeros(off, device=DEV), p.flatten()])[off:].view(p.shape)
     got_o = ops.gated_delta_rule(p, wide[:, 4:], got_s, slots.to(DEV), cu.to(DEV), pos.to(DEV), H, G, d, dv, per_head=True,
                                  max_q_len=max(lens))
     live = pos >= 0
     # float32 sums of up to d + 32 products of order one, through a forward substitution of 32 rows
     for got, want in ((got_o.cpu().view(T, H, dv)[live], want_o[live]), (got_s.cpu(), want_s)):
-        off = float((got.double() - want).abs().max())
-        assert off <= 2e-5 * max(1.0, float(want.abs().max())), off
+        worst = float((got.double() - want).abs().max())
+        assert worst <= 2e-5 * max(1.0, float(want.abs().max())), worst
+
+
+@pytest.mark.parametrize("lens,d,take", [([511], 128, False), ([512], 128, True), ([2048], 64, False), ([2048], 130, False), ([512, 500], 68, False),
+                                         ([520, 500], 68, True), ([1024, 600, 500], 128, False), ([991] + [1] * 60, 128, False),
+                                         ([992] + [1] * 60, 128, True), ([300000], 128, False)])
+def test_which_steps_go_in_chunks(lens, d, take):
+    from pico_vllm_b200 import ops
+    T, S = sum(lens), len(lens)
+    v, state = torch.empty(T, 2 * 128, device=DEV), torch.empty(S, 2, 128, d, device=DEV)
+    assert ops.delta_chunks_take(v, state, d, 128, max(lens), S) == take
+    assert not ops.delta_chunks_take(v[:, 1:], state, d, 128, max(lens), S)
