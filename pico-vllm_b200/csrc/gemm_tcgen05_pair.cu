@@ -66,6 +66,12 @@ __device__ __forceinline__ void tp_tma_2d(void* dst, const CUtensorMap* map, int
         ::"r"(tp_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(tp_u32(bar) & 0xFEFFFFFFu)
         : "memory");
 }
+__device__ __forceinline__ void tp_tma_5d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];\n"
+        ::"r"(tp_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(tp_u32(bar) & 0xFEFFFFFFu)
+        : "memory");
+}
 __device__ __forceinline__ uint64_t tp_desc(uint32_t tile_addr, int k16) {
     const uint32_t addr = tile_addr + k16 * 32;
     return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
@@ -162,9 +168,9 @@ __device__ __forceinline__ uint32_t tp_pack(float a, float b) {
 // the bytes that come from L2 per product by a quarter - at these sizes the copies, not the tensor
 // cores, set the pace), the two accumulators fill tensor memory, and eight epilogue warps drain them.  Accumulator j of a tall tile holds its rows 256 j .. + 255, so a last
 // tile of no more than 256 rows leaves out the second one's copies and products (2,111 rows are five tall tiles, the last with
-// 63 rows: TAIL_US).
+// 63 rows: gate_up and down of 3,584 x 18,944 took 713 us with them, 690 without).
 // GROUPED: one product per group of neighbouring rows, each with a matrix of its own (the experts of a routed feed-forward); a
-// tile lies inside one group.  MOE_US
+// tile lies inside one group.  The form for short groups, where the weights are a stream: see pico_gemm_tcgen05_grouped.
 template <int BN, int EPI, int STAGES, int MB, bool GROUPED>
 __global__ void __launch_bounds__(64 + 128 * MB)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const TpArgs p,
@@ -493,8 +499,6 @@ static int tp_make_map(CUtensorMap* map, const void* base, long long rows, int K
 
 static int tp_num_sms() { return pico_num_sms(); }
 
-#define TP_MAX_GROUPS 512
-
 template <int BN, int EPI, int MB, bool GROUPED>
 static int tp_launch(const void* x, int ldx, const void* w, const TpArgs& a, cudaStream_t stream) {
     constexpr int STAGE_BYTES = (MB * TP_BM + BN / 2) * TP_BK * 2;
@@ -573,25 +577,355 @@ PICO_API int pico_gemm_tcgen05_pair(const void* x, int ldx, const void* w, void*
     return PICO_ERR_SIZE;
 }
 
-// Rows of a group's tile in pico_gemm_tcgen05_grouped for n rows in E groups: 512, or 256 where the groups are short (with 512 rows a
-// product reads a quarter less from L2, with 256 less of a tile lies beyond its group's end).
-PICO_API int pico_gemm_tcgen05_group_rows(int n, int E) { return n >= 352LL * E ? 512 : 256; }
+// ------------------------------------------------------------------------------------------ products of groups
+// One product per group of neighbouring rows of x, each with a matrix of its own (the experts of a routed feed-forward):
+// out[r] = x[r] w[e]^T for the rows r = offsets[e] .. offsets[e + 1] - 1; offsets [E + 1] on the device, the host never sees them;
+// w [E, N, K].  Groups are short and of any length, so here the ROWS OF x are the instruction's N (any multiple of 32 to 256) and
+// the rows of w its M: a tile of a group of 260 rows costs 288 rows, where 256-row tiles cost 512 and read w twice.
+//
+// A pair of blocks computes 256 rows of w (GLU: 128 gate rows and the up rows beside them) x the group's rows of a tile, 512 at most
+// in two accumulators of tensor memory.  Roles as above.  GLU: the 128 rows of a block are 16 gate rows, the 16 up rows beside
+// them, the next 16 gate rows and so on - one copy of a map with the dimensions (k, row of 16, gate or up, sixteens, group) - so that
+// lanes l and l + 16 of an epilogue warp hold the gate and the up number of one feature.  The epilogue has a
+// feature a lane and a row of x a register; lanes exchange until each stores four neighbouring features of a row.
+// A group's rows are dealt out evenly to as few tiles as the longest tile allows (64 .. 512 rows); which length, each block
+// works out from the offsets: rounds of the pairs times the mean time of a tile, which the tensor cores
+// bound (2 clocks a row of x and k-block and SM) or the copies from L2 (1.6 a row of x or w).  A stage is as long as the
+// longest tile needs, and there are as many as fit (at most TG_STAGES).
+// (2,048 tokens, four of 16 experts of 1,536 x 2,240 each: 201 us both products where tiles are 256 or 512 rows of x, 190 here; of 32
+// experts of 2,048 x 2,752: 423 / 361.  With a copy per 16 rows of w and per 32 rows of x from one lane 220, with a lane each 207.)
+#define TG_MAX_GROUPS 512
+#define TG_STAGES 8
+#define TG_RING (200 * 1024)
+#define TG_THREADS 320
+#define TG_A_BYTES (TP_BM * TP_BK * 2)         // rows of w of a block and k-block
+#define TG_BOX 32                              // rows of x in a copy
+struct TgArgs {
+    int n, E, N, K;
+    bf16* out;                // STORE: [n, N]; GLU: [n, N / 2]
+    const int* offsets;
+    float limit;              // CAPPED
+    int rows;                 // most rows of x in a tile (a multiple of 64 to 512); 0: chosen from the offsets
+    int sixteens;             // GLU with N / 2 no multiple of 16: the rows of w in boxes of 16, a lane each
+};
+// a tile with m rows of x: rows of its first and second accumulator's product (one product where it holds them: an instruction takes its
+// issuing thread about 100 clocks however few its rows)
+__device__ __forceinline__ int2 tg_split(int m) {
+    if (m <= 256) return make_int2((m + 31) / 32 * 32, 0);
+    const int a = ((m + 1) / 2 + 31) / 32 * 32;
+    return make_int2(a, (m - a + 31) / 32 * 32);
+}
+__device__ __forceinline__ int tg_boxes(int n) { return (n / 2 + TG_BOX - 1) / TG_BOX; }      // copies of a block for its half of n rows
 
-// One product per group: out[r] = x[r] w[e]^T for the rows r = offsets[e] .. offsets[e + 1] - 1; w [E, N, K], x [n, K] contiguous.  epi 0 (out
-// [n, N]), 2 or 3 (out [n, N / 2]) as above.  rows: of a tile, 0 = pico_gemm_tcgen05_group_rows.
+template <int EPI>
+__global__ void __launch_bounds__(TG_THREADS, 1)
+gemm_tcgen05_group_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const TgArgs p, int n_tiles) {
+    pdl_launch_dependents();
+    extern __shared__ unsigned char tp_dyn[];
+    unsigned char* smem = tp_dyn + ((1024u - (tp_u32(tp_dyn) & 1023u)) & 1023u);
+    constexpr bool GLU = tp_is_glu(EPI);
+    constexpr int FEATURES = GLU ? 128 : 256;                  // of a tile
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + TG_RING);
+    uint64_t* empty = full + TG_STAGES;
+    uint64_t* acc_full = empty + TG_STAGES;
+    uint64_t* acc_empty = acc_full + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
+    volatile int* abort_s = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    float* cost = reinterpret_cast<float*>(tmem_slot + 2);     // [8]: of the lengths 64, 128 .. 512
+    int* group_at = reinterpret_cast<int*>(cost + 8);          // [E + 1]: offsets
+    int* first_tile = group_at + p.E + 1;                      // [E + 1]: running number of tiles of the groups, then their longest tile
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+    const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    const int nkb = (p.K + TP_BK - 1) / TP_BK;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < TG_STAGES; ++s) {
+            tp_mbar_init(full + s, 1);
+            tp_mbar_init(empty + s, 1);
+        }
+        tp_mbar_init(acc_full, 1);
+        tp_mbar_init(acc_empty, 16);               // one arrival per epilogue warp of both blocks
+        *abort_s = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tp_u32(tmem_slot)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    tp_cluster_sync();          // both blocks' barriers are initialised before anything arrives on them
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();                 // x and the offsets come from the kernels before
+    for (int i = threadIdx.x; i <= p.E; i += TG_THREADS) group_at[i] = p.offsets[i];
+    __syncthreads();
+    if (warp < 8 && p.rows == 0) {
+        const int w = 64 * (warp + 1);
+        int tiles = 0;
+        float work = 0.f;
+        for (int e = lane; e < p.E; e += 32) {
+            const int c = group_at[e + 1] - group_at[e], nt = (c + w - 1) / w;
+            if (nt > 0) {
+                const int2 n = tg_split((c + nt - 1) / nt);
+                const float m = (float)(n.x + n.y);
+                tiles += nt;
+                work += (float)nt * fmaxf(2.f * m, 1.6f * (m + 256.f));
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            tiles += __shfl_xor_sync(0xffffffffu, tiles, o);
+            work += __shfl_xor_sync(0xffffffffu, work, o);
+        }
+        if (lane == 0) cost[warp] = tiles ? (float)((tiles * n_tiles + n_pairs - 1) / n_pairs) * (work / (float)tiles) : 0.f;
+    }
+    __syncthreads();
+    int most = p.rows;
+    if (most == 0) {
+        most = 512;
+        float best = cost[7];
+        for (int i = 6; i >= 0; --i)
+            if (cost[i] < best) {
+                best = cost[i];
+                most = 64 * (i + 1);
+            }
+    }
+    if (warp == 0) {
+        int running = 0, longest = 1;
+        for (int e0 = 0; e0 < p.E; e0 += 32) {
+            const int e = e0 + lane, c = e < p.E ? group_at[e + 1] - group_at[e] : 0, mine = (c + most - 1) / most;
+            int upto = mine;
+            if (mine > 0) longest = max(longest, (c + mine - 1) / mine);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += up;
+            }
+            if (e < p.E) first_tile[e] = running + upto - mine;
+            running += __shfl_sync(0xffffffffu, upto, 31);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+        if (lane == 0) {
+            first_tile[p.E] = running;
+            first_tile[p.E + 1] = longest;
+        }
+    }
+    __syncthreads();
+    const int m_tiles = first_tile[p.E], total_tiles = m_tiles * n_tiles;
+    const int2 longest = tg_split(first_tile[p.E + 1]);
+    const int stage_bytes = TG_A_BYTES + (tg_boxes(longest.x) + tg_boxes(longest.y)) * TG_BOX * TP_BK * 2;
+    const int stages = min(TG_STAGES, TG_RING / stage_bytes);
+    // rows t0 .. t0 + m - 1 of x, group, first feature
+    struct Place { int t0, m, e, f0; };
+    auto place = [&](int t) {
+        const int mt = t % m_tiles;
+        int lo = 0, hi = p.E;                 // the largest e with first_tile[e] <= mt
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (first_tile[mid] <= mt) lo = mid; else hi = mid;
+        }
+        const int c = group_at[lo + 1] - group_at[lo], nt = first_tile[lo + 1] - first_tile[lo], each = (c + nt - 1) / nt;
+        const int from = (mt - first_tile[lo]) * each;
+        return Place{group_at[lo] + from, min(each, c - from), lo, t / m_tiles * FEATURES};
+    };
+
+    if (warp == 0) {
+        // lane 0 copies the rows of w, lanes 1 .. 8 a box of rows of x each (one lane gets only about two copies under way)
+        int s = 0, round = 0;
+        bool stop = false;                        // the same in all lanes
+        for (int t = pair; t < total_tiles && !stop; t += n_pairs) {
+            const Place at = place(t);
+            const int2 n = tg_split(at.m);
+            const int boxes0 = tg_boxes(n.x), boxes = boxes0 + tg_boxes(n.y), i = lane - 1;
+            const int row = at.t0 + (i < boxes0 ? (int)rank * (n.x / 2) + i * TG_BOX : n.x + (int)rank * (n.y / 2) + (i - boxes0) * TG_BOX);
+            for (int kb = 0; kb < nkb; ++kb) {
+                if (round > 0 && !tp_wait(empty + s, (round - 1) & 1)) {
+                    g_tp_status = 1;
+                    *abort_s = 1;
+                }
+                stop = __any_sync(0xffffffffu, *abort_s != 0);
+                if (stop) break;
+                if (rank == 0 && lane == 0) tp_expect_tx(full + s, 2 * (TG_A_BYTES + boxes * TG_BOX * TP_BK * 2));
+                unsigned char* a = smem + s * stage_bytes;
+                if (lane == 0) {
+                    if (GLU && !p.sixteens) tp_tma_5d(a, &w_map, kb * TP_BK, 0, 0, at.f0 / 16 + (int)rank * 4, at.e, full + s);
+                    if (!GLU) tp_tma_2d(a, &w_map, kb * TP_BK, at.e * p.N + at.f0 + (int)rank * TP_BM, full + s);
+                } else if (i < boxes) {
+                    tp_tma_2d(a + TG_A_BYTES + i * TG_BOX * TP_BK * 2, &x_map, kb * TP_BK, row, full + s);
+                } else if (GLU && p.sixteens && lane >= 16 && lane < 24) {
+                    tp_tma_2d(a + (lane - 16) * 16 * TP_BK * 2, &w_map, kb * TP_BK,
+                              at.e * p.N + at.f0 + (int)rank * 64 + (lane - 16) / 2 * 16 + (lane & 1) * (p.N / 2), full + s);
+                }
+                if (++s == stages) {
+                    s = 0;
+                    ++round;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            // instruction descriptor as above: N rows of x, M = 256 rows of w (the pair)
+            const uint32_t base = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 4) << 24);
+            int s = 0, round = 0, it = 0;
+            for (int t = pair; t < total_tiles && !*abort_s; t += n_pairs, ++it) {
+                if (it > 0 && !tp_wait(acc_empty, (it - 1) & 1)) {      // both epilogues have read the accumulators
+                    g_tp_status = 1;
+                    *abort_s = 1;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const int2 n = tg_split(place(t).m);
+                const uint32_t id0 = base | ((uint32_t)(n.x >> 3) << 17), id1 = base | ((uint32_t)(n.y >> 3) << 17);
+                const uint32_t second = tg_boxes(n.x) * TG_BOX * TP_BK * 2;
+                for (int kb = 0; kb < nkb; ++kb) {
+                    if (!tp_wait(full + s, round & 1)) {
+                        g_tp_status = 1;
+                        *abort_s = 1;
+                    }
+                    if (*abort_s) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    const uint32_t a = tp_u32(smem + s * stage_bytes), b = a + TG_A_BYTES;
+#pragma unroll
+                    for (int k16 = 0; k16 < TP_BK / 16; ++k16) {
+                        const uint32_t acc = (kb > 0 || k16 > 0) ? 1u : 0u;
+                        tp_mma(tmem_base, tp_desc(a, k16), tp_desc(b, k16), id0, acc);
+                        if (n.y) tp_mma(tmem_base + 256, tp_desc(a, k16), tp_desc(b + second, k16), id1, acc);
+                    }
+                    tp_commit_both(empty + s);
+                    if (++s == stages) {
+                        s = 0;
+                        ++round;
+                    }
+                }
+                tp_commit_both(acc_full);
+            }
+        }
+    } else {
+        // epilogue warps 2 .. 9: warp w drains lanes 32 (w % 4) .., the first or second half of the rows of x
+        const int q = warp & 3, j = (warp - 2) >> 2, n_out = GLU ? p.N / 2 : p.N;
+        const bool odd = lane & 1, two = lane & 2;
+        int it = 0;
+        for (int t = pair; t < total_tiles; t += n_pairs, ++it) {
+            const Place at = place(t);
+            const int2 n = tg_split(at.m);
+            // this warp's rows of x (none if <= 0) and columns of tensor memory: an accumulator, or half of the only one
+            const int half = n.y ? n.x : (n.x / 2 + 31) / 32 * 32, row = at.t0 + (j ? half : 0), rows = j ? at.m - half : min(at.m, half);
+            // the four features that this lane stores
+            const int f = GLU ? at.f0 + (int)rank * 64 + q * 16 + (lane & 12) : at.f0 + (int)rank * TP_BM + q * 32 + (lane & 28);
+            bool ok = tp_wait(acc_full, it & 1);
+            if (!ok) {
+                g_tp_status = 1;
+                *abort_s = 1;
+            }
+            if (__any_sync(0xffffffffu, !ok || *abort_s != 0)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t taddr = tmem_base + (j ? (n.y ? 256 : half) : 0) + ((uint32_t)(q * 32) << 16);
+            bf16* dst = p.out + (size_t)row * n_out + f;
+#pragma unroll 1
+            for (int c = 0; c < rows; c += 32) {
+                uint32_t v[32];
+                tp_ld32(taddr + c, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                constexpr int R = GLU ? 16 : 32;               // numbers of the lane's feature after the gate: rows of x
+                if (GLU) {                                     // rows 2 i + (lane >> 4), feature lane & 15
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const bool up = lane & 16;
+                        const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? v[2 * i] : v[2 * i + 1], 16);
+                        const float g = __uint_as_float(up ? got : v[2 * i]), u = __uint_as_float(up ? v[2 * i + 1] : got);
+                        v[i] = __float_as_uint(tp_glu<EPI>(g, u, p.limit));
+                    }
+                }
+                uint32_t h[R / 2];                             // two features of number 2 i + odd
+#pragma unroll
+                for (int i = 0; i < R / 2; ++i) {
+                    const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? v[2 * i] : v[2 * i + 1], 1);
+                    const float a = __uint_as_float(odd ? got : v[2 * i]), b = __uint_as_float(odd ? v[2 * i + 1] : got);
+                    h[i] = tp_pack(a, b);
+                }
+#pragma unroll
+                for (int i = 0; i < R / 4; ++i) {              // four features of number 4 i + (lane & 3)
+                    const uint32_t got = __shfl_xor_sync(0xffffffffu, two ? h[2 * i] : h[2 * i + 1], 2);
+                    const uint2 four = two ? make_uint2(got, h[2 * i + 1]) : make_uint2(h[2 * i], got);
+                    const int number = 4 * i + (lane & 3), r = c + (GLU ? 2 * number + (lane >> 4) : number);
+                    if (r < rows && f < n_out) *reinterpret_cast<uint2*>(dst + (size_t)r * n_out) = four;
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tp_arrive_rank0(acc_empty);
+        }
+    }
+    // nobody leaves while its partner may still signal its barriers or read its shared memory
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    tp_cluster_sync();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512));
+    }
+}
+
+// gate and up rows of w [E, 2 I, K], sixteen of each in turn, 64 of each in a box
+static int tg_make_glu_map(CUtensorMap* map, const void* w, const TgArgs& a) {
+    TpEncodeFn fn = tp_encode_fn();
+    if (!fn) return -7;
+    if (((uintptr_t)w & 15) != 0) return PICO_ERR_ALIGN;
+    const cuuint64_t row = (cuuint64_t)a.K * 2, I = a.N / 2;
+    const cuuint64_t dims[5] = {(cuuint64_t)a.K, 16, 2, I / 16, (cuuint64_t)a.E}, strides[4] = {row, I * row, 16 * row, 2 * I * row};
+    const cuuint32_t box[5] = {TP_BK, 16, 2, 4, 1}, estr[5] = {1, 1, 1, 1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : -7;
+}
+
+template <int EPI>
+static int tg_launch(const void* x, const void* w, const TgArgs& a, cudaStream_t stream) {
+    constexpr bool GLU = tp_is_glu(EPI);
+    CUtensorMap xm, wm;
+    int rc = tp_make_map(&xm, x, a.n, a.K, a.K, TG_BOX);
+    if (rc) return rc;
+    rc = GLU && !a.sixteens ? tg_make_glu_map(&wm, w, a) : tp_make_map(&wm, w, (long long)a.E * a.N, a.K, a.K, GLU ? 16 : TP_BM);
+    if (rc) return rc;
+    const size_t smem = TG_RING + (2 * TG_STAGES + 2) * 8 + 8 + 8 * sizeof(float) + (2 * (a.E + 1) + 1) * sizeof(int) + 1024;
+    cudaFuncSetAttribute(gemm_tcgen05_group_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int n_out = GLU ? a.N / 2 : a.N, n_tiles = (n_out + (GLU ? 128 : 256) - 1) / (GLU ? 128 : 256);
+    const long long most = ((long long)a.n / 64 + (a.E < a.n ? a.E : a.n)) * n_tiles;      // (the kernel reads how many tiles there are)
+    const int max_pairs = tp_num_sms() / 2, pairs = most < max_pairs ? (int)most : max_pairs;
+    pico_launch_cluster(gemm_tcgen05_group_kernel<EPI>, dim3(2 * pairs), dim3(TG_THREADS), smem, stream, 2, xm, wm, a, n_tiles);
+    return pico_launch_status();
+}
+
+// Rows a group from which its rows are the instruction's N; below, tiles of 256 rows of x stand beside 256 of w (gemm_tcgen05_pair_kernel,
+// GROUPED): shorter groups leave a tile partly empty either way, what counts is the stream of weights, and there two blocks that
+// copy 128 rows of each operand a k-block do better.  The two products of a gated feed-forward, that form / this, us: 16 experts of
+// 1,536 x 2,240, 100 rows a group 55 + 36 / 63 + 44, 175 55 + 38 / 67 + 46, 256 91 + 53 / 71 + 48, 512 135 + 73 / 128 + 71; 32 of
+// 2,048 x 2,752, 128 rows 175 + 92 / 195 + 102, 231 185 + 101 / 228 + 119, 256 276 + 147 / 238 + 121, 288 344 + 180 / 250 + 128.
+#define TG_MIN_ROWS 240
+
+// x [n, K] and w [E, N, K] contiguous; epi 0 (out [n, N]), 2 or 3 (out [n, N / 2]) as above.  rows: 0 = chosen here, < 0: the form for
+// short groups, else of x in a tile at most (a multiple of 64 to 512).
 PICO_API int pico_gemm_tcgen05_grouped(const void* x, const void* w, void* out, const int* offsets, int n, int E, int N, int K, int epi,
                                        int rows, float limit, cudaStream_t stream) {
-    if (rows == 0) rows = pico_gemm_tcgen05_group_rows(n, E);
     if (n <= 0) return 0;
-    if (E < 1 || E > TP_MAX_GROUPS || N < 16 || K < 64 || K % 8 != 0 || (rows != 256 && rows != 512)) return PICO_ERR_SIZE;
+    if (E < 1 || E > TG_MAX_GROUPS || N < 16 || K < 64 || K % 8 != 0 || rows > 512 || (rows > 0 && rows % 64 != 0)) return PICO_ERR_SIZE;
     if (epi == TP_STORE ? N % 8 != 0 : (N % 2 != 0 || (N / 2) % 8 != 0)) return PICO_ERR_SIZE;
     if (epi == TP_CAPPED && !(limit > 0.f)) return PICO_ERR_SIZE;
-    TpArgs a = {};
-    a.M = n; a.N = N; a.K = K; a.out = (bf16*)out; a.limit = limit; a.offsets = offsets; a.E = E;
-#define TP_GROUPED(EPI) return rows == 512 ? tp_launch<256, EPI, 2, true>(x, K, w, a, stream) : tp_launch<256, EPI, 1, true>(x, K, w, a, stream)
-    if (epi == TP_STORE) TP_GROUPED(TP_STORE);
-    if (epi == TP_SWIGLU) TP_GROUPED(TP_SWIGLU);
-    if (epi == TP_CAPPED) TP_GROUPED(TP_CAPPED);
-#undef TP_GROUPED
+    if (rows < 0 || (rows == 0 && n < (long long)TG_MIN_ROWS * E)) {
+        TpArgs b = {};
+        b.M = n; b.N = N; b.K = K; b.out = (bf16*)out; b.limit = limit; b.offsets = offsets; b.E = E;
+        if (epi == TP_STORE) return tp_launch<256, TP_STORE, 1, true>(x, K, w, b, stream);
+        if (epi == TP_SWIGLU) return tp_launch<256, TP_SWIGLU, 1, true>(x, K, w, b, stream);
+        if (epi == TP_CAPPED) return tp_launch<256, TP_CAPPED, 1, true>(x, K, w, b, stream);
+        return PICO_ERR_SIZE;
+    }
+    TgArgs a = {};
+    a.n = n; a.E = E; a.N = N; a.K = K; a.out = (bf16*)out; a.offsets = offsets; a.limit = limit; a.rows = rows; a.sixteens = N % 32 != 0;
+    if (epi == TP_STORE) return tg_launch<TP_STORE>(x, w, a, stream);
+    if (epi == TP_SWIGLU) return tg_launch<TP_SWIGLU>(x, w, a, stream);
+    if (epi == TP_CAPPED) return tg_launch<TP_CAPPED>(x, w, a, stream);
     return PICO_ERR_SIZE;
 }

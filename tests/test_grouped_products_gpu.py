@@ -18,7 +18,7 @@ def _silu_mul(y, limit):
 @pytest.mark.parametrize("counts", [[1], [0, 256, 0, 1, 257, 0], [512, 513, 128, 0, 300], [0, 0, 5], [40] * 40, [1030, 129], [3] * 70 + [600]])
 @pytest.mark.parametrize("N,K", [(256, 64), (272, 200), (1552, 136)])
 @pytest.mark.parametrize("epi,limit", [(0, 0.0), (2, 0.0), (3, 1.5)])
-@pytest.mark.parametrize("rows", [256, 512])
+@pytest.mark.parametrize("rows", [0, -1, 64, 320, 512])
 def test_groups(counts, N, K, epi, limit, rows):
     from pico_vllm_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(sum(counts) + N)
