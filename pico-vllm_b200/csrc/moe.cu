@@ -649,7 +649,7 @@ PICO_API int pico_moe_combine(const float* out2, const float* wgt, int T, int to
     return pico_launch_status();
 }
 
-// out[p, :] = act(wgt[perm[p]] * u[p, :]) in float32: the activation of experts without a gate between the library's
+// out[p, :] = act(wgt[perm[p]] * u[p, :]) in float32: the activation of experts without a gate between the
 // two grouped products (rows in expert order), with the entry's router weight acting on the expert's input.  perm and
 // wgt nullptr: a plain activation over [n, ff] (a dense layer of the same form, such as a shared expert).  In place
 // when out == u.
