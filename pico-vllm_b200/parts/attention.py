@@ -51,7 +51,10 @@ def decode_splits(shape: StepShape, n_kv_heads: int, window: Optional[int] = Non
     short = getattr(shape.engine, "dtype", "") == "bfloat16"
     if short and want < 4 and keys >= DECODE_RAGGED_KEYS:
         seen = [min(st + 1, keys) for n, st in zip(shape.q_lens, shape.starts) if n == 1]
-        want = 4 if seen and 4 * sum(seen) <= 3 * keys * len(seen) else want
+        portions = sum(n for n in shape.q_lens if n > 1)
+        counted = portions == 0 or shape.num_tokens < len(seen) + portions      # (scratch is for all tokens: not beside portions
+        if counted and seen and 4 * sum(seen) <= 3 * keys * len(seen):          # that the mixer has not taken off)
+            want = 4
     want = min(want, max(keys // 128, min(keys // 64, 8) if short else 0))
     splits = 1
     while splits * 2 <= want:

@@ -1,4 +1,6 @@
 """How many parts a single token's keys are cut into: by the contexts' lengths and by how even they are."""
+from dataclasses import replace
+
 import pytest
 
 from pico_vllm_b200.config import EngineConfig
@@ -21,6 +23,13 @@ def _splits(contexts, kv_heads, dtype="bfloat16", window=None):
 def test_parts(contexts, kv_heads, parts, before):
     assert _splits(contexts, kv_heads) == parts
     assert _splits(contexts, kv_heads, "float32") == before
+
+
+def test_portions_that_are_counted_keep_ragged_batches_whole():
+    shape = StepShape(num_tokens=2040, num_segments=41, q_lens=[2000] + [1] * 40, starts=[0, 7999] + [2999] * 39, max_kv=8000,
+                      decode_only=False, num_sms=148, engine=EngineConfig(dtype="bfloat16"))
+    assert decode_splits(shape, 4) == 1
+    assert decode_splits(replace(shape, num_tokens=40), 4) == 4
 
 
 def test_a_window_bounds_the_keys():
