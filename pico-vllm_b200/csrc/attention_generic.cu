@@ -52,6 +52,11 @@ __device__ __forceinline__ void fma2(float2& d, float2 a, float2 b) {
         : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
 }
 
+// What the sums of a part (its maximum m and denominator l) are multiplied with when parts are put together under the maximum M.
+// A part without keys has m = -inf and l = 0 and counts for nothing; with scores that are all no numbers m is -inf too (a
+// maximum passes them over), but l is none, and so is the row that the part belongs to.
+__device__ __forceinline__ float part_factor(float m, float l, float M) { return m == -INFINITY ? l : expf(m - M); }
+
 struct TileArgs {
     int q_row_stride, table_stride, T, nh, nkv, hd, page_size, window, n_splits, chunk, bq, row_chunks;
     float scale, softcap;
@@ -300,16 +305,15 @@ __global__ void __launch_bounds__(128) paged_attention_tiled_kernel(const T* __r
 #pragma unroll
         for (int w = 0; w < PARTS; ++w) {
             const float2 ml = ml_s[w * RT + r];
-            f[w] = ml.x == -INFINITY ? 0.f : expf(ml.x - M);
+            f[w] = part_factor(ml.x, ml.y, M);
             L += ml.y * f[w];
         }
-        const float inv = a.n_splits == 1 ? (L > 0.f ? 1.0f / L : 0.f) : 1.0f;
+        const float inv = a.n_splits == 1 ? (L == 0.f ? 0.f : 1.0f / L) : 1.0f;
         const size_t slot = ((size_t)tok * a.nh + h) * a.n_splits + sp;
         for (int d = lane; d < hd; d += 32) {
             float v = 0.f;
 #pragma unroll
-            for (int w = 0; w < PARTS; ++w)
-                if (f[w] != 0.f) v = fmaf(po_s[(size_t)(w * RT + r) * ld + d], f[w], v);
+            for (int w = 0; w < PARTS; ++w) v = fmaf(po_s[(size_t)(w * RT + r) * ld + d], f[w], v);
             if (a.n_splits == 1) out[((size_t)tok * a.nh + h) * hd + d] = from_f32<T>(v * inv);
             else a.part_o[slot * hd + d] = v;
         }
@@ -363,17 +367,11 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_o, const
     float M = sinks ? sinks[th % nh] : -INFINITY;
     for (int i = 0; i < n_splits; ++i) M = fmaxf(M, ml[2 * i]);
     float L = sinks ? expf(sinks[th % nh] - M) : 0.f;
-    for (int i = 0; i < n_splits; ++i) {
-        const float mi = ml[2 * i];
-        if (mi != -INFINITY) L += ml[2 * i + 1] * expf(mi - M);
-    }
-    const float inv = L > 0.f ? 1.0f / L : 0.f;
+    for (int i = 0; i < n_splits; ++i) L += ml[2 * i + 1] * part_factor(ml[2 * i], ml[2 * i + 1], M);
+    const float inv = L == 0.f ? 0.f : 1.0f / L;
     for (int d = threadIdx.x; d < hd; d += blockDim.x) {
         float acc = 0.f;
-        for (int i = 0; i < n_splits; ++i) {
-            const float mi = ml[2 * i];
-            if (mi != -INFINITY) acc += part_o[(th * n_splits + i) * hd + d] * expf(mi - M);
-        }
+        for (int i = 0; i < n_splits; ++i) acc += part_o[(th * n_splits + i) * hd + d] * part_factor(ml[2 * i], ml[2 * i + 1], M);
         out[th * hd + d] = from_f32<T>(acc * inv);
     }
 }

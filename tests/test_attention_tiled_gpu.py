@@ -84,3 +84,24 @@ def test_a_value_that_is_no_number_stays_with_the_rows_that_see_it(T):
     ops.paged_attention(q.to(DEV), k.to(DEV), v.to(DEV), out, seg.to(DEV), pos.to(DEV), table.to(DEV), H, G, hd, ps, None, 0.2)
     finite = torch.isfinite(out).all(1).cpu()
     assert finite[:bad].all() and not finite[bad:].any()
+
+
+@pytest.mark.parametrize("what", ["query", "key"])
+@pytest.mark.parametrize("T,start,splits", [(1, 48, 1), (1, 48, 2), (1, 200, 1), (40, 0, 1), (40, 0, 3), (320, 0, 1)])
+def test_a_score_that_is_no_number_makes_its_row_none(what, T, start, splits):
+    """A query that is no number (none of its row's scores is one), or a key (one score of each row that sees it is none; with 49
+    keys it is the only one a warp, or the second part, has): those rows of the output are no numbers, all others are."""
+    from pico_vllm_b200 import ops
+    H, G, hd, ps = 32, 8, 32, 8
+    g, k, v, seg, pos, table = _batch(6, [T], [start], G, hd, ps, torch.float32)
+    q = torch.randn(T, H * hd, generator=g)
+    row = max(0, T - 3)
+    if what == "query":
+        q[row] = float("nan")
+    else:
+        k[table[0, (start + row) // ps], :, (start + row) % ps] = float("nan")
+    out = torch.zeros(T, H * hd, device=DEV)
+    scratch = torch.zeros(max(1, ops.attention_scratch_floats(T, H, hd, splits)), device=DEV)
+    ops.paged_attention(q.to(DEV), k.to(DEV), v.to(DEV), out, seg.to(DEV), pos.to(DEV), table.to(DEV), H, G, hd, ps, None, 0.2, splits, scratch)
+    want = torch.arange(T) == row if what == "query" else torch.arange(T) >= row
+    assert torch.equal(out.isnan().all(1).cpu(), want) and torch.equal(out.isnan().any(1).cpu(), want)
