@@ -760,18 +760,20 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* _
 #pragma unroll
                 for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
                 const float* vc = v + (size_t)t0 * v_stride + (size_t)h * dv + (of_k ? 0 : c - DC_D);
-#pragma unroll 4
-                for (int j = 0; j < DC_C; ++j) {
-                    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+                auto row_of = [&](int j) {
                     if (of_k) {
-                        b = *reinterpret_cast<const float4*>(k_s + j * DC_LD + c);
+                        const float4 k4 = *reinterpret_cast<const float4*>(k_s + j * DC_LD + c);
                         const float gj = g_s[hh * DC_C + j];
-                        b = make_float4(gj * b.x, gj * b.y, gj * b.z, gj * b.w);
-                    } else if (keep_v) {
-                        b = *reinterpret_cast<const float4*>(v_s + j * vw + (h0 + hh) * dv + c - DC_D);
-                    } else if (j < n) {
-                        b = *reinterpret_cast<const float4*>(vc + (size_t)j * v_stride);
+                        return make_float4(gj * k4.x, gj * k4.y, gj * k4.z, gj * k4.w);
                     }
+                    if (keep_v) return *reinterpret_cast<const float4*>(v_s + j * vw + (h0 + hh) * dv + c - DC_D);
+                    return j < n ? *reinterpret_cast<const float4*>(vc + (size_t)j * v_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+                };
+                // M is nought above its diagonal, and those places are left out, not multiplied with: a token that holds no
+                // number must not reach the tokens before it (0 * inf)
+#pragma unroll 4
+                for (int j = 0; j < i0; ++j) {
+                    const float4 b = row_of(j);
                     float m[8];
                     *reinterpret_cast<float4*>(m) = *reinterpret_cast<const float4*>(M + j * DC_C + i0);
                     *reinterpret_cast<float4*>(m + 4) = *reinterpret_cast<const float4*>(M + j * DC_C + i0 + 4);
@@ -781,6 +783,18 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* _
                         acc[i][1] = fmaf(m[i], b.y, acc[i][1]);
                         acc[i][2] = fmaf(m[i], b.z, acc[i][2]);
                         acc[i][3] = fmaf(m[i], b.w, acc[i][3]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float4 b = row_of(i0 + j);
+#pragma unroll
+                    for (int i = j; i < 8; ++i) {
+                        const float m = M[(i0 + j) * DC_C + i0 + i];
+                        acc[i][0] = fmaf(m, b.x, acc[i][0]);
+                        acc[i][1] = fmaf(m, b.y, acc[i][1]);
+                        acc[i][2] = fmaf(m, b.z, acc[i][2]);
+                        acc[i][3] = fmaf(m, b.w, acc[i][3]);
                     }
                 }
 #pragma unroll
@@ -1029,7 +1043,8 @@ delta_chunk_out_kernel(const float* __restrict__ prep, int P, const int* __restr
             o[r][e] = gi * (f.x + f.y);
         }
     }
-    for (int j = 0; j < 8 * warp + 8; ++j) {           // (E is nought beyond a token's own place)
+    // E is nought beyond a token's own place, and those places are left out (as above)
+    auto add_u = [&](int j, auto from) {
         float ev[8], uv[4];
         *reinterpret_cast<float4*>(ev) = *reinterpret_cast<const float4*>(e_s + j * DC_C + 8 * warp);
         *reinterpret_cast<float4*>(ev + 4) = *reinterpret_cast<const float4*>(e_s + j * DC_C + 8 * warp + 4);
@@ -1037,9 +1052,13 @@ delta_chunk_out_kernel(const float* __restrict__ prep, int P, const int* __restr
         for (int e = 0; e < 4; ++e) uv[e] = u_s[j * DC_OC + lane + 32 * e];
 #pragma unroll
         for (int r = 0; r < 8; ++r)
+            if (r >= from)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) o[r][e] = fmaf(ev[r], uv[e], o[r][e]);
-    }
+                for (int e = 0; e < 4; ++e) o[r][e] = fmaf(ev[r], uv[e], o[r][e]);
+    };
+    for (int j = 0; j < 8 * warp; ++j) add_u(j, 0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) add_u(8 * warp + j, j);
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const int i = 8 * warp + r;

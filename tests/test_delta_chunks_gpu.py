@@ -81,3 +81,34 @@ def test_which_steps_go_in_chunks(lens, d, take):
     v, state = torch.empty(T, 2 * 128, device=DEV), torch.empty(S, 2, 128, d, device=DEV)
     assert ops.delta_chunks_take(v, state, d, 128, max(lens), S) == take
     assert not ops.delta_chunks_take(v[:, 1:], state, d, 128, max(lens), S)
+
+
+@pytest.mark.parametrize("bad", [0, 5, 31, 32, 45, 69])
+@pytest.mark.parametrize("where", ["v", "k", "q", "beta", "decay"])
+def test_what_is_no_number_does_not_reach_the_tokens_before_it(where, bad, monkeypatch):
+    """A value, key, query, write strength or decay of one head that is no number: the outputs of the tokens before it and of the
+    heads that have no part in it stay what they are, bit for bit (a query's also of the tokens after it)."""
+    from pico_vllm_b200 import ops
+    monkeypatch.setattr(ops, "delta_chunks_take", lambda *a: True)
+    H, G, d, dv, T = 4, 2, 128, 36, 70
+    g = torch.Generator().manual_seed(bad)
+    cu, pos, slots = _segments([T])
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, d, generator=g), dim=-1) for _ in range(2))
+    v = torch.randn(T, H, dv, generator=g)
+    ab = torch.rand(T, H, 4, generator=g)
+    state = torch.randn(1, H, dv, d, generator=g) * 0.3
+    outs = []
+    for spoil in (False, True):
+        if spoil:
+            {"v": v[bad, 1], "k": k[bad, 0], "q": q[bad, 0], "beta": ab[bad, 1, 1:2], "decay": ab[bad, 1, :1]}[where].fill_(float("inf") if where in "vq" else float("nan"))
+        prep = torch.cat([q.reshape(T, -1), k.reshape(T, -1), ab.reshape(T, -1), torch.zeros(T, 8 * G)], 1).to(DEV)
+        outs.append(ops.gated_delta_rule(prep, v.reshape(T, -1).to(DEV), state.to(DEV), slots.to(DEV), cu.to(DEV), pos.to(DEV), H, G, d, dv,
+                                         per_head=True, max_q_len=T).cpu().view(T, H, dv))
+    clean, got = outs
+    reached = [0, 1] if where in "kq" else [1]
+    others = [h for h in range(H) if h not in reached]
+    assert clean.isfinite().all() and torch.equal(got[:, others], clean[:, others])
+    assert torch.equal(got[:bad], clean[:bad])
+    assert not got[bad][reached].isfinite().any()
+    if where == "q":
+        assert torch.equal(got[bad + 1:], clean[bad + 1:])
