@@ -1613,13 +1613,21 @@ def delta_prepare(xc: torch.Tensor, q_off: int, k_off: int, proj: torch.Tensor, 
     return prep
 
 
-# Longest segment from which the recurrence with a decay per head runs in chunks of 32 tokens, and what every further segment adds to it.
-# In chunks a step costs more work and fewer dependent steps, so it pays while the longest segment sets the time (us in chunks / four
-# tokens at a time, 12 heads of 128): 256 tokens 48 / 46, 512 71 / 87, 2,048 232 / 333; two of 1,024 199 / 271, but four of 512 180 / 142.
-# The short ones are a launch of their own, and blocks that find nothing to do: 60 single tokens beside 512 122 / 137 (16 heads 161 / 138),
-# beside 1,024 208 / 267; 250 beside 700 304 / 217.
+# Longest segment from which the recurrence with a decay per head runs in chunks of 32 tokens.  In chunks a step costs more work and
+# fewer dependent steps, so it pays while the longest segment sets the time, not the number of blocks: on average over a step
+# heads x column tiles x tokens / longest blocks are at work, and two a multiprocessor run side by side.  us in chunks / four tokens at
+# a time, keys and values of 128, with their preparation:
+#   one segment of 384, 512, 2,048: 12 heads 64 / 66, 74 / 87, 237 / 333; 32 heads 93 / 107, 114 / 140, 416 / 541; 48 heads (384 blocks)
+#   131 / 109, 182 / 142, 651 / 550; 64 heads 176 / 166, 218 / 219, 800 / 849
+#   512 x 4: 4 heads 76 / 88, 8 heads (256 blocks) 117 / 139, 12 (384) 186 / 142, 16 219 / 216, 24 324 / 278; 683 x 3, 12 heads (288) 172 / 186
+#   of 2,048 tokens 1,025, 682 and 341: 12 heads 210 / 273, 16 (256 blocks on average) 225 / 275, 24 (384) 310 / 280, 32 421 / 344
+#   a longest of 1,024 with a share of 0.4, 0.3 beside sixteen: 8 heads 194 / 271, 213 / 273; 12 heads (240, 321 blocks) 217 / 274, 285 / 279;
+#   16 heads (320, 428) 274 / 277, 370 / 284
+# The short ones are a launch of their own, and blocks that find nothing to do, some 0.065 us a segment and head, while every token of the longest
+# gains about 0.1: 60 single tokens beside 512, 1,024, 2,048: 8 heads 100 / 135, 148 / 266, 311 / 526; 12 heads 120 / 137, 210 / 268, 361 / 532;
+# 16 heads 161 / 138, 231 / 270, 389 / 533; 24 heads 198 / 147, 295 / 273, 467 / 538; 32 heads 236 / 194, 338 / 277, 539 / 542.
 DELTA_CHUNK_MIN_TOKENS = 512
-DELTA_CHUNK_PER_SEGMENT = 8
+DELTA_CHUNK_BLOCKS = 296           # two on each of 148 multiprocessors
 
 
 DELTA_CHUNK_LEAST = 64             # (as in delta_rule.cu)
@@ -1628,13 +1636,16 @@ DELTA_CHUNK_MAX_SCRATCH = 128 << 20
 
 
 def delta_chunks_take(v: torch.Tensor, state: torch.Tensor, d: int, dv: int, max_q_len: int, segments: int) -> bool:
-    """A long segment that holds half of the tokens, keys of 65 to 128 numbers, scratch within its bound, and everything the kernels read 16 bytes at a time lies on 16
+    """A segment long enough for the heads and segments beside it, no more blocks on average than run side by side, keys of 65 to 128
+    numbers, scratch within its bound, and everything the kernels read 16 bytes at a time lies on 16
     bytes.  The segments of DELTA_CHUNK_LEAST tokens and more then go in chunks, the others as in any step; where there is only one,
     its rows need no dot products with earlier ones (:func:`delta_prepare` with ``max_q_len`` 1)."""
-    T, H = v.shape[0], state.shape[1]
-    if (T // 32 + min(segments, T // DELTA_CHUNK_LEAST) + 1) * H * (5184 + 128 * dv) + T * H * dv > DELTA_CHUNK_MAX_SCRATCH:
+    if max_q_len < DELTA_CHUNK_MIN_TOKENS:                         # (nearly every step: nothing else is looked at)
         return False
-    if max_q_len < DELTA_CHUNK_MIN_TOKENS + DELTA_CHUNK_PER_SEGMENT * (segments - 1) or 2 * max_q_len < T:
+    T, H = v.shape[0], state.shape[1]
+    if max_q_len < DELTA_CHUNK_MIN_TOKENS + 2 * H * (segments - 1) // 3 or H * -(-dv // 16) * T > DELTA_CHUNK_BLOCKS * max_q_len:
+        return False
+    if (T // 32 + min(segments, T // DELTA_CHUNK_LEAST) + 1) * H * (5184 + 128 * dv) + T * H * dv > DELTA_CHUNK_MAX_SCRATCH:
         return False
     return (64 < d <= 128 and d % 4 == 0 and dv % 4 == 0 and v.stride(0) % 4 == 0
             and (v.data_ptr() | state.data_ptr()) % 16 == 0)
