@@ -1653,13 +1653,13 @@ def delta_chunks_take(v: torch.Tensor, state: torch.Tensor, d: int, dv: int, max
 
 def gated_delta_rule(prep: torch.Tensor, v: torch.Tensor, state: torch.Tensor, seg_slots: torch.Tensor, cu_q: torch.Tensor,
                      positions: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int, per_head: bool = False,
-                     max_q_len: int = 1) -> torch.Tensor:
+                     max_q_len: int = 1, min_q_len: int = 1) -> torch.Tensor:
     """Per head h, token by token in the order of each segment, from and into ``state`` float32 [slots, heads, vdim, dim] (S
     transposed; row ``seg_slots[s]``):  S <- diag(a) S;  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q.  ``prep``: the rows
     :func:`delta_prepare` made with the same ``per_head`` and ``max_q_len`` (with a decay
     per head and segments of DELTA_BLOCK_MIN_TOKENS and more, four tokens share one pass over the memory; head h reads query and key head h // (heads / kv_heads)); ``v`` float32 rows with head h's values
-    at h * vdim (a column slice is fine).  A segment whose first position is negative is padding.  Returns o float32
-    [T, heads * vdim]."""
+    at h * vdim (a column slice is fine).  A segment whose first position is negative is padding.  ``min_q_len``: no segment that is
+    not padding has fewer tokens.  Returns o float32 [T, heads * vdim]."""
     _cuda(prep, v, state, seg_slots, cu_q, positions)
     _f32_rows(v, "gated_delta_rule: v")
     T, S = prep.shape[0], seg_slots.shape[0]
@@ -1680,7 +1680,7 @@ def gated_delta_rule(prep: torch.Tensor, v: torch.Tensor, state: torch.Tensor, s
     chunks = per_head and delta_chunks_take(v, state, d, vdim, max_q_len, S)
     if chunks and prep.data_ptr() % 16 == 0:
         lib = library()
-        if S > 1:
+        if S > 1 and min_q_len < DELTA_CHUNK_LEAST:
             _check(lib.pico_gated_delta_rule(_ptr(prep), _ptr(v), v.stride(0), _ptr(state), _ptr(seg_slots), _ptr(cu_q), _ptr(positions),
                                              _ptr(out), out.stride(0), S, H, G, d, vdim, 1, 1, DELTA_CHUNK_LEAST, _stream()),
                    f"gated_delta_rule (dim {d})")
