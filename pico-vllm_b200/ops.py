@@ -1651,6 +1651,14 @@ def delta_chunks_take(v: torch.Tensor, state: torch.Tensor, d: int, dv: int, max
             and (v.data_ptr() | state.data_ptr()) % 16 == 0)
 
 
+def _chunk_scratch(floats: int, device: torch.device) -> Optional[torch.Tensor]:
+    """Scratch for a step in chunks, or None when the device has no room for it: such a step then goes as it does without chunks."""
+    try:
+        return torch.empty(floats, dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def gated_delta_rule(prep: torch.Tensor, v: torch.Tensor, state: torch.Tensor, seg_slots: torch.Tensor, cu_q: torch.Tensor,
                      positions: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int, per_head: bool = False,
                      max_q_len: int = 1, min_q_len: int = 1) -> torch.Tensor:
@@ -1678,14 +1686,16 @@ def gated_delta_rule(prep: torch.Tensor, v: torch.Tensor, state: torch.Tensor, s
         raise KernelError("gated_delta_rule: cu_q must have one more entry than seg_slots, positions one per token")
     out = torch.empty((T, H * vdim), dtype=torch.float32, device=prep.device)
     chunks = per_head and delta_chunks_take(v, state, d, vdim, max_q_len, S)
+    scratch = None
     if chunks and prep.data_ptr() % 16 == 0:
+        scratch = _chunk_scratch(library().pico_gated_delta_chunk_floats(T, S, H, vdim), prep.device)
+    if scratch is not None:
         lib = library()
         if S > 1 and min_q_len < DELTA_CHUNK_LEAST:
             _check(lib.pico_gated_delta_rule(_ptr(prep), _ptr(v), v.stride(0), _ptr(state), _ptr(seg_slots), _ptr(cu_q), _ptr(positions),
                                              _ptr(out), out.stride(0), S, H, G, d, vdim, 1, 1, DELTA_CHUNK_LEAST, _stream()),
                    f"gated_delta_rule (dim {d})")
             _count()
-        scratch = torch.empty(lib.pico_gated_delta_chunk_floats(T, S, H, vdim), dtype=torch.float32, device=prep.device)
         _check(lib.pico_gated_delta_chunks(_ptr(prep), _ptr(v), v.stride(0), _ptr(state), _ptr(seg_slots), _ptr(cu_q), _ptr(positions),
                                            _ptr(out), out.stride(0), T, S, H, G, d, vdim, _ptr(scratch), _stream()),
                f"gated_delta_chunks (dim {d})")

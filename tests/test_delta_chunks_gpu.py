@@ -93,6 +93,34 @@ def test_no_launch_for_short_segments_that_are_not_there(lens, launches):
     assert ops.launches - before == launches and not out.any()
 
 
+@pytest.mark.parametrize("lens", [[520], [600, 70, 3]])
+def test_without_room_for_its_scratch_a_step_goes_without_chunks(lens, monkeypatch):
+    """The same outputs and memory, from the allocator's own error on; one segment's rows come without the dot products of neighbours."""
+    from pico_vllm_b200 import ops
+    H, d, dv, T, S = 2, 68, 8, sum(lens), len(lens)
+    g = torch.Generator().manual_seed(T)
+    cu, pos, slots = (t.to(DEV) for t in _segments(lens))
+    xc, proj = torch.randn(T, H * (2 * d + dv), generator=g).to(DEV), torch.randn(T, 2 * H, generator=g).to(DEV)
+    bias, state = torch.zeros(H, device=DEV), torch.randn(S, H, dv, d, generator=g).to(DEV)
+    prep = ops.delta_prepare(xc, 0, H * d, proj, 0, proj[:, H:], bias, bias, H, H, d, per_head=True, max_q_len=1 if S == 1 else max(lens))
+    real, asked, got = torch.empty, [], []
+
+    def empty(*size, **how):
+        if size and isinstance(size[0], int):
+            asked.append(size[0])
+            raise torch.OutOfMemoryError("no room")
+        return real(*size, **how)
+    for full in (False, True):
+        if full:
+            monkeypatch.setattr(torch, "empty", empty)
+        after = state.clone()
+        out = ops.gated_delta_rule(prep, xc[:, 2 * H * d:], after, slots, cu, pos, H, H, d, dv, per_head=True, max_q_len=max(lens))
+        got.append((out, after))
+    assert len(asked) == 1
+    for a, b in zip(*got):
+        assert torch.allclose(a, b, atol=2e-5 * max(1.0, float(a.abs().max())), rtol=0)
+
+
 @pytest.mark.parametrize("bad", [0, 5, 31, 32, 45, 69])
 @pytest.mark.parametrize("where", ["v", "k", "q", "beta", "decay"])
 def test_what_is_no_number_does_not_reach_the_tokens_before_it(where, bad, monkeypatch):
