@@ -340,6 +340,12 @@ def mma_attention_takes(dtype: torch.dtype, n_heads: int, n_kv_heads: int, head_
             and n_heads % n_kv_heads == 0 and n_heads // n_kv_heads <= 16)
 
 
+def decode_tma_takes(head_dim: int, page_size: int) -> bool:
+    """True when the single tokens' kernel that brings pages in by TMA takes these sizes (the parts of a token's keys are then one cluster,
+    which adds them up; in the other kernels a second launch does)."""
+    return head_dim in (64, 128) and page_size in (8, 16, 32, 64)
+
+
 def make_kv_tensor_map(pages: torch.Tensor):
     """A TMA tensor map over the cache pages of one layer ([pages, kv_heads, page_size, head_dim]
     bfloat16, contiguous), for the TMA-fed decode kernel; None when the sizes are not taken (head_dim
@@ -347,7 +353,7 @@ def make_kv_tensor_map(pages: torch.Tensor):
     if not pages.is_cuda or pages.dtype != torch.bfloat16 or not pages.is_contiguous() or pages.dim() != 4:
         return None
     n_pages, nkv, ps, hd = pages.shape
-    if hd not in (64, 128) or ps not in (8, 16, 32, 64):
+    if not decode_tma_takes(hd, ps):
         return None
     buf = (ctypes.c_ubyte * 192)()
     addr = ctypes.addressof(buf)

@@ -33,13 +33,21 @@ MAX_MIXED_SCRATCH = 32 << 20       # float32 numbers (128 MB) that splitting the
 DECODE_RAGGED_KEYS = 4096          # longest context from which the parts of a ragged batch need not all run at once
 
 
-def decode_splits(shape: StepShape, n_kv_heads: int, window: Optional[int] = None) -> int:
+def adds_in_cluster(shape: StepShape, n_heads: int, n_kv_heads: int, head_dim: int) -> bool:
+    """Whether single tokens run in the kernel that adds the parts of a token's keys up in a cluster (see :func:`decode_splits`)."""
+    engine = shape.engine
+    dtype = getattr(torch, getattr(engine, "dtype", "") or "float32")
+    return ops.mma_attention_takes(dtype, n_heads, n_kv_heads, head_dim) and ops.decode_tma_takes(head_dim, getattr(engine, "page_size", 0))
+
+
+def decode_splits(shape: StepShape, n_kv_heads: int, window: Optional[int] = None, cluster: bool = True) -> int:
     """How many parts to cut each single token's key range into: a power of two (the parts of one
     token and kv head run as one thread-block cluster): up to 16 while that is at most one block
     per SM, else up to 8 while the blocks make no more than one wave of two per SM; each part at
     least two tiles of 64 keys of the context, or of the ``window`` a token sees of it.
 
-    bfloat16: up to eight parts of one tile, but no two parts of fewer than 512 keys (attention of the 1.5B / 7B shape with its
+    bfloat16, in the kernel that adds a token's parts up in a ``cluster`` (in the others a second launch does, and a part costs more: 16
+    tokens of 2 kv heads with 512 keys in 1 / 2 / 4 parts 29 / 19 / 14 us, here 8.9 / 8.0 / 6.6): up to eight parts of one tile, but no two parts of fewer than 512 keys (attention of the 1.5B / 7B shape with its
     projections, 512 keys each: batch 4 in 8 parts 22 / 36 us, in 2 or 4 24 / 38; 200 keys, batch 8 / 16: 24 / 42 us whole, 24 / 42
     or more in two parts).  Contexts of all ages, the longest DECODE_RAGGED_KEYS and more: four parts also where that
     makes more than a wave, since unsplit the longest sets the time (up to 8,000 keys, 4 kv heads: batch 40 / 64 / 48 in 139 / 158 /
@@ -48,7 +56,7 @@ def decode_splits(shape: StepShape, n_kv_heads: int, window: Optional[int] = Non
     groups = max(1, shape.num_tokens * n_kv_heads)
     keys = shape.max_kv if window is None else min(shape.max_kv, window)
     want = 16 if groups * 16 <= shape.num_sms else min(2 * shape.num_sms // groups, 8)
-    short = getattr(shape.engine, "dtype", "") == "bfloat16"
+    short = cluster and getattr(shape.engine, "dtype", "") == "bfloat16"
     if short and want < 4 and keys >= DECODE_RAGGED_KEYS:
         seen = [min(st + 1, keys) for n, st in zip(shape.q_lens, shape.starts) if n == 1]
         portions = sum(n for n in shape.q_lens if n > 1)
@@ -108,12 +116,13 @@ class GQAAttention(Part):
         MAX_MIXED_SCRATCH holds."""
         portions = sum(n for n in shape.q_lens if n > 1)
         dtype = getattr(torch, getattr(shape.engine, "dtype", "") or "float32")
+        cluster = adds_in_cluster(shape, self.n_heads, self.n_kv_heads, self.head_dim)
         if not portions or not ops.mma_attention_takes(dtype, self.n_heads, self.n_kv_heads, self.head_dim):
-            return decode_splits(shape, self.n_kv_heads)
+            return decode_splits(shape, self.n_kv_heads, cluster=cluster)
         if portions == shape.num_tokens:
             return 1
         longest = max([st + n for n, st in zip(shape.q_lens, shape.starts) if n == 1], default=1)
-        splits = decode_splits(replace(shape, num_tokens=shape.num_tokens - portions, max_kv=longest), self.n_kv_heads)
+        splits = decode_splits(replace(shape, num_tokens=shape.num_tokens - portions, max_kv=longest), self.n_kv_heads, cluster=cluster)
         while splits > 1 and ops.attention_scratch_floats(shape.num_tokens, self.n_heads, self.head_dim, splits) > MAX_MIXED_SCRATCH:
             splits //= 2
         return splits
@@ -256,7 +265,7 @@ class QKNormAttention(Part):
         return ("qk_norm_attention", self.n_heads, self.n_kv_heads, self.row, self.window)
 
     def plan(self, shape: StepShape) -> AttentionPlan:
-        splits = decode_splits(shape, self.n_kv_heads)
+        splits = decode_splits(shape, self.n_kv_heads, cluster=adds_in_cluster(shape, self.n_heads, self.n_kv_heads, self.row))
         scratch = ops.attention_scratch_floats(shape.num_tokens, self.n_heads, self.row, splits)
         return AttentionPlan(key=(splits, 0), scratch_floats=scratch, splits=splits, pair_min_keys=0)
 

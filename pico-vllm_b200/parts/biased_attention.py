@@ -34,7 +34,7 @@ import torch
 
 from .. import ops
 from ..errors import ConfigError
-from .attention import AttentionPlan, _linear, decode_splits
+from .attention import AttentionPlan, _linear, adds_in_cluster, decode_splits
 from .base import CacheView, MixerPlan, PagedKV, Param, Part, Piece, StepShape
 from .registry import register
 
@@ -97,7 +97,8 @@ class DistanceBiasAttention(Part):
         return ("distance_bias_attention", self.n_heads, self.n_kv_heads, self.row, self.window, self.chunk)
 
     def plan(self, shape: StepShape) -> AttentionPlan:
-        splits = decode_splits(shape, self.n_kv_heads, self.window)
+        splits = decode_splits(shape, self.n_kv_heads, self.window,
+                               cluster=not self.chunk and adds_in_cluster(shape, self.n_heads, self.n_kv_heads, self.row))
         if self.chunk:                                           # no token reads more keys than a chunk holds: parts of
             while splits > 1 and splits * 512 > self.chunk:      # 512 keys at least
                 splits //= 2

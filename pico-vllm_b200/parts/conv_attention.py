@@ -22,7 +22,7 @@ from typing import List, Optional
 import torch
 
 from .. import ops
-from .attention import AttentionPlan, _linear, decode_splits
+from .attention import AttentionPlan, _linear, adds_in_cluster, decode_splits
 from .base import FixedState, PagedKV, Param, Part, Piece, StepShape
 from .registry import register
 
@@ -66,7 +66,7 @@ class ConvRopeAttention(Part):
         return ("conv_rope_attention", self.n_heads, self.n_kv_heads, self.row, self.window)
 
     def plan(self, shape: StepShape) -> AttentionPlan:
-        splits = decode_splits(shape, self.n_kv_heads)
+        splits = decode_splits(shape, self.n_kv_heads, cluster=adds_in_cluster(shape, self.n_heads, self.n_kv_heads, self.row))
         scratch = ops.attention_scratch_floats(shape.num_tokens, self.n_heads, self.row, splits)
         return AttentionPlan(key=(splits, 0), scratch_floats=scratch, splits=splits, pair_min_keys=0)
 

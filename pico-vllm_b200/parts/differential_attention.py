@@ -76,7 +76,7 @@ class DifferentialAttention(Part):
         return ("differential_attention", self.n_heads, self.n_kv_heads, self.row)
 
     def plan(self, shape: StepShape) -> AttentionPlan:
-        splits = decode_splits(shape, self.n_kv_heads)
+        splits = decode_splits(shape, self.n_kv_heads, cluster=False)
         scratch = ops.attention_scratch_floats(shape.num_tokens, MAPS * self.n_heads, self.row, splits)
         return AttentionPlan(key=(splits, 0), scratch_floats=scratch, splits=splits, pair_min_keys=0)
 

@@ -145,7 +145,7 @@ class LatentAttention(Part):
         return ("latent_attention", self.heads, self.row, self.window)
 
     def plan(self, shape: StepShape) -> AttentionPlan:
-        splits = decode_splits(shape, 1, self.window)
+        splits = decode_splits(shape, 1, self.window, cluster=False)
         scratch = ops.attention_scratch_floats(shape.num_tokens, self.heads, self.row, splits)
         return AttentionPlan(key=(splits, 0), scratch_floats=scratch, splits=splits, pair_min_keys=0)
 
