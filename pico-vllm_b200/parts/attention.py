@@ -51,13 +51,15 @@ def decode_splits(shape: StepShape, n_kv_heads: int, window: Optional[int] = Non
     projections, 512 keys each: batch 4 in 8 parts 22 / 36 us, in 2 or 4 24 / 38; 200 keys, batch 8 / 16: 24 / 42 us whole, 24 / 42
     or more in two parts).  Contexts of all ages, the longest DECODE_RAGGED_KEYS and more: four parts also where that
     makes more than a wave, since unsplit the longest sets the time (up to 8,000 keys, 4 kv heads: batch 40 / 64 / 48 in 139 / 158 /
-    145 us, now 108 / 133 / 119; up to 4,096, batch 40 / 64: 88 / 100, now 80 / 96; at 3,000 some gain and some lose).  Of
+    145 us, now 108 / 133 / 119; up to 4,096, batch 40 / 64: 88 / 100, now 80 / 96; at 3,000 some gain and some lose), but in no more
+    than seven blocks a multiprocessor: the kernel alone, one of 8,000 / 4,096 keys beside 63 of 300 / 1,000, 4 kv heads 95 / 56 us, 29 / 41
+    in four parts; beside 127 97 / 63, 58 / 77; beside 255 105 / 88, 112 / 144; beside 511 of 8 kv heads 117 / 301, 367 / 498.  Of
     one length they stay whole (8,000 keys, batch 40: 150 us, 156 in four parts)."""
     groups = max(1, shape.num_tokens * n_kv_heads)
     keys = shape.max_kv if window is None else min(shape.max_kv, window)
     want = 16 if groups * 16 <= shape.num_sms else min(2 * shape.num_sms // groups, 8)
     short = cluster and getattr(shape.engine, "dtype", "") == "bfloat16"
-    if short and want < 4 and keys >= DECODE_RAGGED_KEYS:
+    if short and want < 4 and keys >= DECODE_RAGGED_KEYS and 4 * groups <= 7 * shape.num_sms:
         seen = [min(st + 1, keys) for n, st in zip(shape.q_lens, shape.starts) if n == 1]
         portions = sum(n for n in shape.q_lens if n > 1)
         counted = portions == 0 or shape.num_tokens < len(seen) + portions      # (scratch is for all tokens: not beside portions

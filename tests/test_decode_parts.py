@@ -52,3 +52,8 @@ def test_short_parts_only_where_a_cluster_adds_them_up(part, clustered):
                       engine=EngineConfig(dtype="bfloat16", page_size=16))
     assert part().plan(shape).splits == (8 if clustered else 4)
     assert part().plan(replace(shape, engine=EngineConfig(dtype="bfloat16", page_size=24))).splits == 4
+
+
+@pytest.mark.parametrize("batch,kv_heads,parts", [(64, 4, 4), (65, 4, 1), (128, 2, 4), (130, 2, 1), (512, 8, 1)])
+def test_ragged_batches_of_many_requests_stay_whole(batch, kv_heads, parts):
+    assert _splits([8000] + [300] * (batch - 1), kv_heads) == parts
