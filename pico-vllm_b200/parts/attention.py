@@ -47,9 +47,12 @@ def decode_splits(shape: StepShape, n_kv_heads: int, window: Optional[int] = Non
     least two tiles of 64 keys of the context, or of the ``window`` a token sees of it.
 
     bfloat16, in the kernel that adds a token's parts up in a ``cluster`` (in the others a second launch does, and a part costs more: 16
-    tokens of 2 kv heads with 512 keys in 1 / 2 / 4 parts 29 / 19 / 14 us, here 8.9 / 8.0 / 6.6): up to eight parts of one tile, but no two parts of fewer than 512 keys (attention of the 1.5B / 7B shape with its
-    projections, 512 keys each: batch 4 in 8 parts 22 / 36 us, in 2 or 4 24 / 38; 200 keys, batch 8 / 16: 24 / 42 us whole, 24 / 42
-    or more in two parts).  Contexts of all ages, the longest DECODE_RAGGED_KEYS and more: four parts also where that
+    tokens of 2 kv heads with 512 keys in 1 / 2 / 4 parts 29 / 19 / 14 us, here 8.9 / 8.0 / 6.6): eight or four parts of one tile and more,
+    eight while that is at most one block per SM, four up to seven blocks per four (us of the kernel, heads of 128, in 1 / 2 / 4 / 8
+    parts: 16 blocks unsplit, 512 and 800 keys 8.8 / 8.0 / 6.4 / 6.1 and 12.3 / 10.0 / 7.6 / 6.8; 32 blocks 8.9 / 8.0 / 6.7 / 7.4 and 12.3 / 10.1 / 8.0 /
+    8.1; 64 blocks, 300 and 504 keys 7.2 / 8.0 / 7.4 / 13 and 9.3 / 9.0 / 8.0 / 14; 74 blocks 6.9 / 7.2 / 12 / 18 and 8.9 / 8.3 / 13 / 18: clusters of
+    four no longer run all at once); no two parts under 512 keys (64 tokens, 2 kv heads, in 1 / 2 parts: 400 keys 8.5 / 9.3, 504 9.5 / 9.3,
+    616 10.8 / 10.0, 1,000 15.4 / 12.5).  Contexts of all ages, the longest DECODE_RAGGED_KEYS and more: four parts also where that
     makes more than a wave, since unsplit the longest sets the time (up to 8,000 keys, 4 kv heads: batch 40 / 64 / 48 in 139 / 158 /
     145 us, now 108 / 133 / 119; up to 4,096, batch 40 / 64: 88 / 100, now 80 / 96; at 3,000 some gain and some lose), but in no more
     than seven blocks a multiprocessor: the kernel alone, one of 8,000 / 4,096 keys beside 63 of 300 / 1,000, 4 kv heads 95 / 56 us, 29 / 41
@@ -65,11 +68,17 @@ def decode_splits(shape: StepShape, n_kv_heads: int, window: Optional[int] = Non
         counted = portions == 0 or shape.num_tokens < len(seen) + portions      # (scratch is for all tokens: not beside portions
         if counted and seen and 4 * sum(seen) <= 3 * keys * len(seen):          # that the mixer has not taken off)
             want = 4
-    want = min(want, max(keys // 128, min(keys // 64, 8) if short else 0))
+    want = min(want, keys // 128)
     splits = 1
     while splits * 2 <= want:
         splits *= 2
-    return 1 if short and splits == 2 and keys < 1024 else splits
+    if short:
+        for parts, blocks in ((8, shape.num_sms), (4, 7 * shape.num_sms // 4)):
+            if splits < parts <= keys // 64 and parts * groups <= blocks:
+                return parts
+        if splits == 2 and keys < 512:
+            return 1
+    return splits
 
 
 @register("mixer", "gqa_attention")

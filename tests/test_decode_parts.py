@@ -19,7 +19,9 @@ def _splits(contexts, kv_heads, dtype="bfloat16", window=None, cluster=True):
 
 @pytest.mark.parametrize("contexts,kv_heads,parts,before", [
     ([200], 2, 1, 1), ([255], 2, 1, 1), ([256], 2, 4, 2), ([512], 2, 8, 4), ([1500], 2, 8, 8), ([2048], 2, 16, 16),
-    ([500] * 32, 4, 1, 2), ([1023] * 32, 4, 1, 2), ([1024] * 32, 4, 2, 2),                                      # two parts at most
+    ([500] * 32, 4, 1, 2), ([511] * 32, 4, 1, 2), ([512] * 32, 4, 2, 2), ([1024] * 32, 4, 2, 2),                # two parts at most
+    ([512] * 18, 1, 8, 4), ([512] * 19, 1, 4, 4), ([512] * 32, 1, 4, 4), ([1024] * 32, 1, 8, 8),                # eight: a block per SM
+    ([300] * 32, 2, 4, 2), ([300] * 64, 1, 4, 2), ([300] * 65, 1, 1, 2), ([504] * 37, 2, 1, 2), ([511] * 37, 2, 1, 2), ([512] * 37, 2, 4, 4),
     ([8000] * 40, 4, 1, 1), ([8000] + [3000] * 39, 4, 4, 1), ([4095] + [1000] * 39, 4, 1, 1), ([4096] + [1000] * 39, 4, 4, 1),
 ])
 def test_parts(contexts, kv_heads, parts, before):
