@@ -30,6 +30,9 @@ class AttentionPlan(MixerPlan):
 MAX_MIXED_SCRATCH = 32 << 20       # float32 numbers (128 MB) that splitting the single tokens of a mixed step may ask for
 
 
+MIXED_MIN_KEYS = 1024              # longest context of the single tokens of a mixed step from which they are counted alone
+
+
 DECODE_RAGGED_KEYS = 4096          # longest context from which the parts of a ragged batch need not all run at once
 
 
@@ -120,10 +123,13 @@ class GQAAttention(Part):
         return AttentionPlan(key=(splits, pair), scratch_floats=scratch, splits=splits, pair_min_keys=pair)
 
     def _splits(self, shape: StepShape) -> int:
-        """As :func:`decode_splits`, but where single tokens run in a kernel of their own beside the portions only they are
+        """As :func:`decode_splits`, but where single tokens run in a kernel of their own beside the portions and the longest sees
+        MIXED_MIN_KEYS and more, only they are
         counted: 37 of them with 3,001 tokens at most beside two portions (2,013 tokens, 28 / 4 heads) make 148 blocks unsplit,
         and the longest sets the time (68 us; 58 in two parts).  A layer with its projections, a portion of 500
-        beside 20 tokens of up to 2,500 keys, 1.5B / 7B shape: 68 / 94 us, now 51 / 82; beside one of 3,000 66 / 86, now 45 / 68.  Scratch is laid out for every token of the step: no more parts than
+        beside 20 tokens of up to 2,500 keys, 1.5B / 7B shape: 68 / 94 us, now 51 / 82; beside one of 3,000 66 / 86, now 45 / 68.  With
+        short ones the kernel gains no more than what the parts cost the host (27 tokens of 504 keys, 16 / 2 heads: 8.8 us whole,
+        7.5 in four parts, but the layer 57 and 60).  Scratch is laid out for every token of the step: no more parts than
         MAX_MIXED_SCRATCH holds."""
         portions = sum(n for n in shape.q_lens if n > 1)
         dtype = getattr(torch, getattr(shape.engine, "dtype", "") or "float32")
@@ -133,6 +139,8 @@ class GQAAttention(Part):
         if portions == shape.num_tokens:
             return 1
         longest = max([st + n for n, st in zip(shape.q_lens, shape.starts) if n == 1], default=1)
+        if longest < MIXED_MIN_KEYS:
+            return decode_splits(shape, self.n_kv_heads, cluster=cluster)
         splits = decode_splits(replace(shape, num_tokens=shape.num_tokens - portions, max_kv=longest), self.n_kv_heads, cluster=cluster)
         while splits > 1 and ops.attention_scratch_floats(shape.num_tokens, self.n_heads, self.head_dim, splits) > MAX_MIXED_SCRATCH:
             splits //= 2

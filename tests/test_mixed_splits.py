@@ -23,6 +23,13 @@ def test_only_single_tokens_are_counted_beside_portions():
     assert _plan([500], [3000], pad=1).splits == 1                   # a padding row holds no keys
 
 
+def test_short_contexts_beside_portions_stay_whole():
+    assert _plan([419, 406] + [1] * 27, [0] + [504] * 28, heads=16, kv=2).splits == 1
+    assert _plan([500] + [1] * 8, [0] + [1022] * 8).splits == 1
+    assert _plan([500] + [1] * 8, [0] + [1023] * 8).splits == _plan([1] * 8, [1023] * 8).splits == 8
+    assert _plan([6] + [1] * 8, [0] + [600] * 8).splits == _plan([1] * 14, [600] * 14).splits == 4     # few tokens: as if all were single
+
+
 def test_scratch_for_every_token_bounds_the_parts():
     plan = _plan([1] * 8 + [2040], [3000] * 8 + [0])
     assert plan.splits == 2 or plan.scratch_floats <= attention.MAX_MIXED_SCRATCH
