@@ -594,7 +594,7 @@ PICO_API int pico_gemm_tcgen05_pair(const void* x, int ldx, const void* w, void*
 // longest tile needs, and there are as many as fit (at most TG_STAGES).
 // (2,048 tokens, four of 16 experts of 1,536 x 2,240 each: 201 us both products where tiles are 256 or 512 rows of x, 190 here; of 32
 // experts of 2,048 x 2,752: 423 / 361.  With a copy per 16 rows of w and per 32 rows of x from one lane 220, with a lane each 207.)
-#define TG_MAX_GROUPS 512
+#define TG_MAX_GROUPS 1024     // (what a block keeps of the groups lies beside its stages: 8 KB of shared memory, 12 in the form for short groups)
 #define TG_STAGES 8
 #define TG_RING (200 * 1024)
 #define TG_THREADS 320

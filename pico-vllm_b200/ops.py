@@ -1297,7 +1297,7 @@ def gated_rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor], gate_logits:
 # experts, top 4, width 1,536, in us: 256 pairs 97 here and 98 there, 512 98 and 198, 8,192 208 and 763; 32 experts, width
 # 2,048: 256 pairs 255 and 231, 512 265 and 266, 800 269 and 360)
 MOE_TC_MIN_ROWS = 16
-MOE_TC_MAX_EXPERTS = 512
+MOE_TC_MAX_EXPERTS = 1024
 
 
 def moe_tc_takes(h: torch.Tensor, gate_up_weight: torch.Tensor, down_weight: torch.Tensor, n: int) -> bool:

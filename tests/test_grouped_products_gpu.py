@@ -59,3 +59,24 @@ def test_a_short_last_tile_of_a_dense_product(M):
         ops.tc_linear_residual(x, w, res, rows=rows)
         assert torch.allclose(res, y + 1, atol=1e-3, rtol=1e-3)
     assert ops.tc_status() == 0
+
+
+@pytest.mark.parametrize("E", [513, 1024])
+@pytest.mark.parametrize("epi,N", [(0, 72), (2, 96)])
+@pytest.mark.parametrize("rows", [0, -1, 64])
+def test_hundreds_of_groups(E, epi, N, rows):
+    from pico_vllm_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(E + N)
+    counts = [(7 * e) % 5 for e in range(E)]
+    counts[1], counts[-1] = 300, 70
+    n, K = sum(counts), 136
+    x = torch.randn(n, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(E, N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    expert = torch.repeat_interleave(torch.arange(E), torch.tensor(counts)).to(DEV)
+    offsets = torch.tensor([0] + counts, device=DEV).cumsum(0).to(torch.int32)
+    out = torch.empty(n, N if epi == 0 else N // 2, dtype=torch.bfloat16, device=DEV)
+    assert ops.library().pico_gemm_tcgen05_grouped(x.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), n, E, N, K, epi, rows,
+                                                   0.0, ops._stream()) == 0
+    y = torch.bmm(w.float()[expert], x.float()[:, :, None])[:, :, 0]
+    assert torch.allclose(out.float(), y if epi == 0 else _silu_mul(y, 0.0), atol=2e-2, rtol=1e-2)
+    assert ops.tc_status() == 0
