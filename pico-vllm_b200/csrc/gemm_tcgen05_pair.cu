@@ -911,7 +911,7 @@ static int tg_launch(const void* x, const void* w, const TgArgs& a, cudaStream_t
 PICO_API int pico_gemm_tcgen05_grouped(const void* x, const void* w, void* out, const int* offsets, int n, int E, int N, int K, int epi,
                                        int rows, float limit, cudaStream_t stream) {
     if (n <= 0) return 0;
-    if (E < 1 || E > TG_MAX_GROUPS || N < 16 || K < 64 || K % 8 != 0 || rows > 512 || (rows > 0 && rows % 64 != 0)) return PICO_ERR_SIZE;
+    if (E < 1 || E > TG_MAX_GROUPS || N < 16 || K < 16 || K % 8 != 0 || rows > 512 || (rows > 0 && rows % 64 != 0)) return PICO_ERR_SIZE;
     if (epi == TP_STORE ? N % 8 != 0 : (N % 2 != 0 || (N / 2) % 8 != 0)) return PICO_ERR_SIZE;
     if (epi == TP_CAPPED && !(limit > 0.f)) return PICO_ERR_SIZE;
     if (rows < 0 || (rows == 0 && n < (long long)TG_MIN_ROWS * E)) {

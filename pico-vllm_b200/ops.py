@@ -1304,7 +1304,8 @@ def moe_tc_takes(h: torch.Tensor, gate_up_weight: torch.Tensor, down_weight: tor
     """Whether the experts' products run on the tcgen05 tensor cores (bfloat16, many rows, row sizes that are multiples of 16
     bytes) instead of the grouped kernels that need no rows in order."""
     (E, _, D), ff = gate_up_weight.shape, down_weight.shape[2]
-    return (h.dtype == torch.bfloat16 and n > MOE_TC_MIN_ROWS * E and E <= MOE_TC_MAX_EXPERTS and D % 8 == 0 and ff % 8 == 0 and D >= 64 and ff >= 64
+    return (h.dtype == torch.bfloat16 and n > MOE_TC_MIN_ROWS * E and E <= MOE_TC_MAX_EXPERTS and D % 8 == 0 and ff % 8 == 0
+            and D >= 16 and ff >= 16                              # (narrower than a k-block: its copies end with zeros)
             and (h.data_ptr() | gate_up_weight.data_ptr() | down_weight.data_ptr()) % 16 == 0)
 
 

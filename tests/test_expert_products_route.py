@@ -14,3 +14,8 @@ def _takes(E, pairs, D=64, ff=64, gated=True, dtype=torch.bfloat16):
 def test_experts(E, pairs, take):
     assert _takes(E, pairs) == take
     assert not _takes(E, pairs, dtype=torch.float32)
+
+
+@pytest.mark.parametrize("D,ff,take", [(16, 16, True), (48, 24, True), (1024, 48, True), (64, 8, False), (8, 64, False), (64, 20, False), (36, 64, False)])
+def test_widths(D, ff, take):
+    assert _takes(4, 65, D, ff) == take and _takes(4, 65, D, ff, gated=False) == take
