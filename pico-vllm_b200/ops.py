@@ -1298,6 +1298,10 @@ def gated_rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor], gate_logits:
 # 2,048: 256 pairs 255 and 231, 512 265 and 266, 800 269 and 360)
 MOE_TC_MIN_ROWS = 16
 MOE_TC_MAX_EXPERTS = 1024
+# widths under 64, a part of a k-block: only where there is something to multiply (32 experts of 1,024 x 48, in us: 544 pairs 27, 38 there, 8,192
+# 44 and 67; of 48 x 512 35 and 59; but of 40 x 24 544 pairs 18 and 15, 8,192 27 and 23)
+MOE_TC_NARROW_PAIRS = 1024
+MOE_TC_NARROW_SIZE = 16384
 
 
 def moe_tc_takes(h: torch.Tensor, gate_up_weight: torch.Tensor, down_weight: torch.Tensor, n: int) -> bool:
@@ -1305,7 +1309,7 @@ def moe_tc_takes(h: torch.Tensor, gate_up_weight: torch.Tensor, down_weight: tor
     bytes) instead of the grouped kernels that need no rows in order."""
     (E, _, D), ff = gate_up_weight.shape, down_weight.shape[2]
     return (h.dtype == torch.bfloat16 and n > MOE_TC_MIN_ROWS * E and E <= MOE_TC_MAX_EXPERTS and D % 8 == 0 and ff % 8 == 0
-            and D >= 16 and ff >= 16                              # (narrower than a k-block: its copies end with zeros)
+            and (min(D, ff) >= 64 or min(D, ff) >= 16 and D * ff >= MOE_TC_NARROW_SIZE and n >= MOE_TC_NARROW_PAIRS)
             and (h.data_ptr() | gate_up_weight.data_ptr() | down_weight.data_ptr()) % 16 == 0)
 
 

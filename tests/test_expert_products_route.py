@@ -16,6 +16,11 @@ def test_experts(E, pairs, take):
     assert not _takes(E, pairs, dtype=torch.float32)
 
 
-@pytest.mark.parametrize("D,ff,take", [(16, 16, True), (48, 24, True), (1024, 48, True), (64, 8, False), (8, 64, False), (64, 20, False), (36, 64, False)])
+def test_narrow_experts_need_many_rows():
+    assert not _takes(4, 1023, 1024, 48) and _takes(4, 1024, 1024, 48)
+    assert not _takes(4, 1024, 48, 336) and _takes(4, 1024, 48, 344)
+
+
+@pytest.mark.parametrize("D,ff,take", [(16, 1024, True), (48, 24, False), (1024, 48, True), (2048, 8, False), (8, 2048, False), (1024, 20, False), (36, 1024, False)])
 def test_widths(D, ff, take):
-    assert _takes(4, 65, D, ff) == take and _takes(4, 65, D, ff, gated=False) == take
+    assert _takes(4, 1024, D, ff) == take and _takes(4, 1024, D, ff, gated=False) == take
