@@ -29,6 +29,7 @@
 #define TP_BM 128              // rows of x per block (256 per pair)
 #define TP_BK 64
 #define TP_THREADS 192
+#define TP_BOX 32              // rows of x in a copy of the grouped form
 #define TP_WAIT_LIMIT (1 << 14)      // polls of a barrier (some microseconds each) before a thread gives up
 
 enum { TP_STORE = 0, TP_RESIDUAL = 1, TP_SWIGLU = 2, TP_CAPPED = 3, TP_GELU = 4 };
@@ -170,7 +171,10 @@ __device__ __forceinline__ uint32_t tp_pack(float a, float b) {
 // tile of no more than 256 rows leaves out the second one's copies and products (2,111 rows are five tall tiles, the last with
 // 63 rows: gate_up and down of 3,584 x 18,944 took 713 us with them, 690 without).
 // GROUPED: one product per group of neighbouring rows, each with a matrix of its own (the experts of a routed feed-forward); a
-// tile lies inside one group.  The form for short groups, where the weights are a stream: see pico_gemm_tcgen05_grouped.
+// tile lies inside one group.  The form for short groups, where the weights are a stream: see pico_gemm_tcgen05_grouped.  A tile there
+// has few of its 256 rows, and one lane that copies 128 rows of x and of w a k-block gets the weights at 4.2 TB/s; with a lane for w and
+// one for each box of rows that is there, a layer with 24 rows an expert takes 521 us (555; 256 experts of 2,048 x 768), 208 (221; 128 of
+// 1,536 x 768), one with 35 rows 241 (267; 32 of 2,048 x 2,752).  One lane that leaves out the boxes that are not there: 564, 225, 267.
 template <int BN, int EPI, int STAGES, int MB, bool GROUPED>
 __global__ void __launch_bounds__(64 + 128 * MB)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const TpArgs p,
@@ -274,7 +278,35 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
     auto accumulators = [&](const Place& at) { return MB == 2 && at.m_end - at.m0 <= 2 * TP_BM ? 1 : MB; };
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (GROUPED) {
+            // lane 0 copies the rows of w, lanes 1 .. 4 a box of rows of x each, and only boxes that the tile has rows for (what is left in
+            // the stage reaches rows that are not stored)
+            int step = 0;
+            bool stop = false;                    // the same in all lanes
+            for (int t = pair; t < total_tiles && !stop; t += n_pairs) {
+                const Place at = place(t);
+                const int m = min(at.m_end - at.m0, 2 * TP_BM), n0 = at.nt * COLS;
+                const int boxes0 = (min(m, TP_BM) + TP_BOX - 1) / TP_BOX, boxes1 = (max(m - TP_BM, 0) + TP_BOX - 1) / TP_BOX;
+                const int row = at.m0 + (int)rank * TP_BM + (lane - 1) * TP_BOX, boxes = rank ? boxes1 : boxes0;
+                const int w_row = at.w0 + (tp_is_glu(EPI) ? (rank ? p.N / 2 + n0 : n0) : n0 + (int)rank * (BN / 2));
+                for (int kb = 0; kb < nkb; ++kb, ++step) {
+                    const int s = step % STAGES;
+                    if (step >= STAGES && !tp_wait(empty + s, ((step / STAGES) - 1) & 1)) {
+                        g_tp_status = 1;
+                        *abort_s = 1;
+                    }
+                    stop = __any_sync(0xffffffffu, *abort_s != 0);
+                    if (stop) break;
+                    unsigned char* a = smem + s * STAGE_BYTES;
+                    if (lane == 0) {
+                        if (rank == 0) tp_expect_tx(full + s, (boxes0 + boxes1) * TP_BOX * TP_BK * 2 + 2 * B_BYTES);
+                        tp_tma_2d(a + A_BYTES, &w_map, kb * TP_BK, w_row, full + s);
+                    } else if (lane <= boxes) {
+                        tp_tma_2d(a + (lane - 1) * TP_BOX * TP_BK * 2, &x_map, kb * TP_BK, row, full + s);
+                    }
+                }
+            }
+        } else if (lane == 0) {
             int step = 0;
             for (int t = pair; t < total_tiles && !*abort_s; t += n_pairs) {
                 const Place at = place(t);
@@ -504,7 +536,7 @@ static int tp_launch(const void* x, int ldx, const void* w, const TpArgs& a, cud
     constexpr int STAGE_BYTES = (MB * TP_BM + BN / 2) * TP_BK * 2;
     constexpr int STAGES = (200 * 1024) / STAGE_BYTES > 8 ? 8 : (200 * 1024) / STAGE_BYTES;
     CUtensorMap xm, wm;
-    int rc = tp_make_map(&xm, x, a.M, a.K, ldx, TP_BM);
+    int rc = tp_make_map(&xm, x, a.M, a.K, ldx, GROUPED ? TP_BOX : TP_BM);
     if (rc) return rc;
     rc = tp_make_map(&wm, w, GROUPED ? (long long)a.E * a.N : a.N, a.K, a.K, BN / 2);
     if (rc) return rc;

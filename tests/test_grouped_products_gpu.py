@@ -61,6 +61,26 @@ def test_a_short_last_tile_of_a_dense_product(M):
     assert ops.tc_status() == 0
 
 
+@pytest.mark.parametrize("counts", [[1, 0, 32, 33], [300, 0, 64, 65, 513, 2], [31, 64, 250] * 30])
+@pytest.mark.parametrize("N", [352, 4480])           # gate halves of 176 and 2,240: multiples of 16 that end inside a tile of 128
+@pytest.mark.parametrize("epi", [0, 2])
+@pytest.mark.parametrize("rows", [0, -1, 512])
+def test_long_rows_go_around_the_stages(counts, N, epi, rows):
+    """16 blocks of K: every stage is filled again and again, by short tiles after long ones and the other way round."""
+    from pico_vllm_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(sum(counts) + N)
+    n, E, K = sum(counts), len(counts), 1000
+    x = torch.randn(n, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(E, N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    offsets = torch.tensor([0] + counts, device=DEV).cumsum(0).to(torch.int32)
+    out = torch.empty(n, N if epi == 0 else N // 2, dtype=torch.bfloat16, device=DEV)
+    assert ops.library().pico_gemm_tcgen05_grouped(x.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), n, E, N, K, epi, rows,
+                                                   0.0, ops._stream()) == 0
+    y = torch.cat([a.float() @ w[e].float().t() for e, a in enumerate(x.split(counts))])
+    assert torch.allclose(out.float(), y if epi == 0 else _silu_mul(y, 0.0), atol=2e-2, rtol=1e-2)
+    assert ops.tc_status() == 0
+
+
 @pytest.mark.parametrize("N,K", [(16, 16), (48, 24), (352, 48), (272, 56)])
 @pytest.mark.parametrize("epi", [0, 2])
 @pytest.mark.parametrize("rows", [0, -1, 64])
