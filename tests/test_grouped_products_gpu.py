@@ -119,3 +119,52 @@ def test_hundreds_of_groups(E, epi, N, rows):
     y = torch.bmm(w.float()[expert], x.float()[:, :, None])[:, :, 0]
     assert torch.allclose(out.float(), y if epi == 0 else _silu_mul(y, 0.0), atol=2e-2, rtol=1e-2)
     assert ops.tc_status() == 0
+
+
+FORMS = {"gated": dict(), "capped": dict(act="capped", limit=0.9), "weight in": dict(gated=False, act="relu2", weight_on_input=True),
+         "weight out": dict(gated=False, act="silu")}
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("T", [35, 640])             # on either side of 240 rows an expert on average, with five experts of which one gets nothing
+@pytest.mark.parametrize("D,ff", [(64, 64), (72, 104), (136, 112)])
+@pytest.mark.parametrize("identity,base", [(0, False), (2, True)])
+def test_experts_through_the_tensor_cores(form, T, D, ff, identity, base):
+    """Listing, gathering, both products with what lies between them and the placed sum, against the sum in float64."""
+    from pico_vllm_b200 import ops
+    how = dict(FORMS[form])
+    if identity and how.get("weight_on_input"):
+        pytest.skip("experts that pass their input on take their weight on the output")
+    how["act"] = {"capped": ops.MOE_ACT_CAPPED, "relu2": ops.MOE_ACT_RELU2}.get(how.get("act"), ops.MOE_ACT_SILU)
+    gated, limit = how.get("gated", True), how.get("limit", 0.0)
+    E, top = 5, 3
+    g = torch.Generator(device=DEV).manual_seed(T + D + ff)
+    h = torch.randn(T, D, generator=g, device=DEV).bfloat16()
+    up = (torch.randn(E, (2 if gated else 1) * ff, D, generator=g, device=DEV) * D ** -0.5).bfloat16()
+    down = (torch.randn(E, D, ff, generator=g, device=DEV) * ff ** -0.5).bfloat16()
+    keys = torch.rand(T, E + identity, generator=g, device=DEV)
+    keys[:, 3] = -1.0                                                # nobody asks for expert 3
+    idx = keys.topk(top, -1).indices.to(torch.int32).contiguous()
+    wgt = torch.softmax(torch.randn(T, top, generator=g, device=DEV), -1)
+    add = torch.randn(T, D, generator=g, device=DEV).bfloat16() if base else None
+    assert ops.moe_tc_takes(h, up, down, T * top)
+    y = ops.moe_experts(h, idx, wgt, up, down, base=add, identity=identity, **how).double()
+    want = add.double().clone() if base else torch.zeros(T, D, dtype=torch.float64, device=DEV)
+    x = h.double()
+    for e in range(E + identity):
+        w = (wgt.double() * (idx == e)).sum(-1, keepdim=True)
+        if e >= E:
+            want += w * x
+            continue
+        z = x @ up[e].double().t()
+        if gated:
+            a = _silu_mul(z, limit)
+        else:
+            z = z * w if how.get("weight_on_input") else z
+            a = z.clamp(min=0) ** 2 if how["act"] == ops.MOE_ACT_RELU2 else z * torch.sigmoid(z)
+        o = a @ down[e].double().t()
+        want += o * (idx == e).any(-1, keepdim=True) if how.get("weight_on_input") else o * w
+    # bfloat16 keeps 2^-9 of a number: once between the products (and once before the activation where there is no gate), once after the
+    # second, once for the sum
+    assert float((y - want).abs().max()) <= 2 ** -7 * float(want.abs().max())
+    assert ops.tc_status() == 0

@@ -375,9 +375,8 @@ def test_router_kernel(experts, top, T, D):
                                                 (1100, 72, 24, 3, 1)])
 def test_routed_experts_kernels(dtype, T, D, ff, experts, top):
     """Listing per expert, both grouped products and the weighted sum; widths that are no multiple of 8 take the
-    general kernel also in bfloat16.  One expert gets most tokens (more than one tile), another none.  The last
-    cases have enough rows for the library's grouped product in bfloat16 (one with an inner size of 8, one with one expert
-    per token)."""
+    general kernel also in bfloat16.  One expert gets most tokens (more than one tile), another none.  (Experts large enough for
+    the tcgen05 products: test_grouped_products_gpu.py.)"""
     from pico_vllm_b200 import ops
     g = torch.Generator().manual_seed(T + D)
     h = torch.randn(T, D, generator=g).to(dtype)
