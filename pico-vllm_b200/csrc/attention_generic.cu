@@ -75,8 +75,8 @@ __global__ void __launch_bounds__(128) paged_attention_tiled_kernel(const T* __r
     constexpr int KT = tile_keys(NJ, RT), KL = KT / 8, VEC = 16 / (int)sizeof(T);
     constexpr bool SHARED = RT == 32;                      // the four warps share the key tiles
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t0 = a.T - 1 - (int)blockIdx.x;              // the tokens late in a prompt, which see the most keys, first
-    const int kh = blockIdx.y / a.row_chunks, rc = blockIdx.y % a.row_chunks, sp = blockIdx.z;
+    const int t0 = a.T - 1 - (int)(blockIdx.x / a.row_chunks);       // the tokens late in a prompt, which see the most keys, first
+    const int kh = blockIdx.y, rc = blockIdx.x % a.row_chunks, sp = blockIdx.z;
     const int g = a.nh / a.nkv, hd = a.hd, ld = hd + 4;
     const int seg = a.tok_seg[t0], pos0 = a.positions[t0];
     const int in_group = t0 % a.bq;
@@ -335,7 +335,7 @@ static void tile_launch(const T* q, const T* k, const T* v, T* out, TileArgs a, 
     const size_t merge = (size_t)(RT == 32 ? 1 : 4) * RT * (ld + 2) * sizeof(float);
     const size_t smem = fixed + (ring > merge ? ring : merge);
     cudaFuncSetAttribute(paged_attention_tiled_kernel<T, NJ, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    pico_launch((paged_attention_tiled_kernel<T, NJ, RT>), dim3(a.T, a.nkv * a.row_chunks, a.n_splits), dim3(128), smem, stream, q, k, v,
+    pico_launch((paged_attention_tiled_kernel<T, NJ, RT>), dim3((unsigned)a.T * a.row_chunks, a.nkv, a.n_splits), dim3(128), smem, stream, q, k, v,
                 out, a);
 }
 

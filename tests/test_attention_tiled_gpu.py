@@ -86,6 +86,20 @@ def test_a_value_that_is_no_number_stays_with_the_rows_that_see_it(T):
     assert finite[:bad].all() and not finite[bad:].any()
 
 
+def test_as_many_key_heads_as_a_grid_has_rows():
+    """33,000 key heads of 33 query heads each: two tiles of rows a token, more blocks than a grid has in its second dimension."""
+    from pico_vllm_b200 import ops
+    G, n, hd = 33000, 33, 16
+    g = torch.Generator(device=DEV).manual_seed(1)
+    q, k, v = (torch.randn(*s, generator=g, device=DEV) for s in ((1, G * n * hd), (1, G, 4, hd), (1, G, 4, hd)))
+    at = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    out = torch.zeros_like(q)
+    ops.paged_attention(q, k, v, out, at([0]), at([2]), at([[0]]), G * n, G, hd, 4, None, 0.25)
+    p = torch.softmax(torch.einsum("gnd,gkd->gnk", q.view(G, n, hd).double(), k[0, :, :3].double()) * 0.25, -1)
+    want = torch.einsum("gnk,gkd->gnd", p, v[0, :, :3].double())
+    assert float((out.view(G, n, hd) - want).abs().max()) <= 2e-5        # float32 sums of 16 products and of three values
+
+
 @pytest.mark.parametrize("what", ["query", "key"])
 @pytest.mark.parametrize("T,start,splits", [(1, 48, 1), (1, 48, 2), (1, 200, 1), (40, 0, 1), (40, 0, 3), (320, 0, 1)])
 def test_a_score_that_is_no_number_makes_its_row_none(what, T, start, splits):

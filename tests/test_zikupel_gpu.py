@@ -401,7 +401,7 @@ def test_router_with_sigmoid_scores(experts, top):
 @pytest.mark.parametrize("on_input", [True, False])
 def test_ungated_experts_kernels(dtype, T, D, ff, experts, top, on_input):
     """Experts without a gate, relu squared, the weight on the input or on the output, a shared expert's output added:
-    lists longer than a tile, an expert without tokens, widths that are no multiple of 8, enough rows for the library."""
+    lists longer than a tile, an expert without tokens, widths that are no multiple of 8."""
     from pico_vllm_b200 import ops
     g = torch.Generator().manual_seed(T + D)
     h = torch.randn(T, D, generator=g).to(dtype)
