@@ -32,8 +32,9 @@ def test_short_contexts_beside_portions_stay_whole():
 
 def test_scratch_for_every_token_bounds_the_parts():
     plan = _plan([1] * 8 + [2040], [3000] * 8 + [0])
-    assert plan.splits == 2 or plan.scratch_floats <= attention.MAX_MIXED_SCRATCH
-    assert 1 < plan.splits < 8 and plan.scratch_floats == 2048 * 28 * plan.splits * 130
+    assert plan.splits == 4 and plan.scratch_floats == 2048 * 28 * 4 * 130 <= attention.MAX_MIXED_SCRATCH < 2048 * 28 * 8 * 130
+    plan = _plan([1] * 8 + [5000], [3000] * 8 + [0])
+    assert plan.splits == 1 and plan.scratch_floats == 0 and 5008 * 28 * 2 * 130 > attention.MAX_MIXED_SCRATCH
 
 
 def test_the_32_bit_path_still_counts_every_token():
