@@ -90,7 +90,7 @@ delta_prepare_kernel(const float* __restrict__ xc, int xc_stride, int q_off, int
             }
             if (lane == 0) {
                 float* dots = out + 2 * G * d + 4 * H + 8 * g;
-                dots[0] = s[2] * iq * ik;
+                dots[0] = iq == 0.f || ik == 0.f ? 0.f : s[2] * iq * ik;       // (rows whose squares overflow are nought, not inf * 0)
                 if (back) {
 #pragma unroll
                     for (int j = 0; j < 3; ++j) {

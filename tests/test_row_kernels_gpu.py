@@ -82,6 +82,17 @@ def test_delta_inputs(H, G, d, longest):
     _close(got, want, 2e-6, "delta_prepare")
 
 
+def test_delta_inputs_whose_squares_overflow():
+    """A query and a key of 1e20, whose sums of squares are infinite: both come out as nought, and so does their dot product."""
+    from pico_vllm_b200 import ops
+    H, G, d, T = 2, 2, 128, 3
+    xc, proj, zero = torch.ones(T, 2 * G * d, device=DEV), torch.zeros(T, 2 * H, device=DEV), torch.zeros(H, device=DEV)
+    xc[1] = 1e20
+    got = ops.delta_prepare(xc, 0, G * d, proj, 0, proj[:, H:], zero, zero, H, G, d, per_head=True)
+    assert not got[1, :2 * G * d].any() and not got[1, 2 * G * d + 4 * H::8].any()
+    assert got[[0, 2], 2 * G * d + 4 * H].gt(0).all()
+
+
 @pytest.mark.parametrize("T,E,top", [(1, 1, 1), (5, 16, 4), (33, 3, 2), (2050, 16, 4), (700, 130, 32), (64, 4096, 8)])
 def test_lists_of_tokens_per_expert(T, E, top):
     from pico_vllm_b200 import ops
