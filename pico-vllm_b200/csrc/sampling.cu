@@ -11,6 +11,7 @@
 //
 // A row (600 KB for a vocabulary of 150 k entries) belongs to one cluster of eight blocks: each reads an eighth of it once, keeps
 // it in shared memory through all the passes, and what the blocks have to tell one another goes through distributed shared memory.
+// Short rows belong to one block, rows of more than 155,648 entries to sixteen (see sample_shape).
 // Masses are summed as 32.32 fixed-point integers (weight = exp((x - max) / T) <= 1), so that sums do not depend on the order in
 // which blocks and threads add: the choice is reproducible.
 //   1. maximum and its first index (greedy rows end here);
@@ -21,14 +22,16 @@
 //      are kept or dropped together);
 //   3. kept mass per block, the block and then the token at which the running sum passes the target.
 // A pass that is a kernel of its own, over the row in L2, with the blocks' results in device memory, costs 10 to 25 us at 64 rows
-// of 152,064 whatever it computes; the whole choice with top-p took 200 us as five of them (162 without top-p) and 80 (34) as this one; 37 rows run at a time.
-// Longer rows than shared memory holds (155,648 entries) are read again in every pass.
+// of 152,064 whatever it computes; the whole choice with top-p took 214 us as five of them (175 without top-p) and 75 (30) as this one; 37 rows run
+// at a time.  1, 8, 32 rows: 35, 71, 132 us, now 28, 30, 45.
+// Sixteen blocks keep rows of up to 778,240 entries; longer ones are read again in every pass (1,000,000 entries with top-p, 1 / 8 / 32
+// rows: 97 / 131 / 319 us; as five kernels with up to 64 parts a row 75 / 187 / 679: single rows of such a length are slower).
 #include "common.cuh"
 
 #define SAMPLE_THREADS 512
-#define SAMPLE_BLOCKS 8          // of a row
 #define SAMPLE_BINS 2048
 #define SAMPLE_FLUSH 65532       // elements whose masses' halves fit into 32-bit sums
+#define SAMPLE_KEEP_ALONE 48640  // ... with a multiprocessor to itself
 #define SAMPLE_KEEP 19456        // elements of a block's part that shared memory keeps (two blocks on a multiprocessor)
 
 typedef unsigned long long u64;
@@ -99,9 +102,9 @@ __device__ __forceinline__ u64 sample_get(const u64* mine, int block) {
     return v;
 }
 
-// Grid (8, rows) in clusters of 8.  Block b takes elements [b * per, (b + 1) * per) of the row, per a multiple of 4.  KEEP: they stay in
+// Grid (BLOCKS, rows) in clusters of BLOCKS.  Block b takes elements [b * per, (b + 1) * per) of the row, per a multiple of 4.  KEEP: they stay in
 // shared memory (as weights from pass 2 on); vec: the row starts on 16 bytes and V is a multiple of 4.
-template <bool KEEP>
+template <bool KEEP, int BLOCKS>
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_row_kernel(const float* __restrict__ logits, int row_stride, int V, const float* __restrict__ temperature,
                   const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out, int per, bool vec) {
@@ -114,7 +117,7 @@ sample_row_kernel(const float* __restrict__ logits, int row_stride, int V, const
     __shared__ float scratch[33];
     __shared__ int iscratch[33];
     __shared__ u64 scratch64[33];
-    __shared__ u64 told[SAMPLE_BLOCKS], told_kept[SAMPLE_BLOCKS];     // what the blocks say: maximum and index; kept mass
+    __shared__ u64 told[BLOCKS], told_kept[BLOCKS];     // what the blocks say: maximum and index; kept mass
     __shared__ u64 s_above;
     const int r = blockIdx.y, rank = blockIdx.x, tid = threadIdx.x;
     sample_cluster_sync();              // every block of the cluster runs before another writes to it
@@ -126,6 +129,23 @@ sample_row_kernel(const float* __restrict__ logits, int row_stride, int V, const
     // ---- 1: the maximum and its first index; the elements into shared memory
     float best = -INFINITY;
     int best_i = 0x7fffffff;
+    // f(element, place) over a, a + step, .. below b; a row that is read again: eight loads under way
+    auto walk = [&](int a, int b, int step, auto f) {
+        if (KEEP) {
+#pragma unroll 4
+            for (int i = a; i < b; i += step) f(kept[i], i);
+        } else {
+            for (int i = a; i < b; i += 8 * step) {
+                float v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (i + u * step < b) v[u] = x[i + u * step];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (i + u * step < b) f(v[u], i + u * step);
+            }
+        }
+    };
     auto see = [&](float v, int i) {
         if (v > best) { best = v; best_i = i; }
     };
@@ -159,13 +179,13 @@ sample_row_kernel(const float* __restrict__ logits, int row_stride, int V, const
     {
         const float pm = block_max(best, scratch);
         const int pc = block_min_int(best == pm ? best_i : 0x7fffffff, iscratch);
-        if (tid < SAMPLE_BLOCKS) sample_put(told + rank, tid, ((u64)__float_as_uint(pm) << 32) | (unsigned)pc);
+        if (tid < BLOCKS) sample_put(told + rank, tid, ((u64)__float_as_uint(pm) << 32) | (unsigned)pc);
     }
     sample_cluster_sync();
     float mx = -INFINITY;
     int arg = 0x7fffffff;
 #pragma unroll
-    for (int b = 0; b < SAMPLE_BLOCKS; ++b) {                         // in the row's order: the first index of the maximum stays the first
+    for (int b = 0; b < BLOCKS; ++b) {                         // in the row's order: the first index of the maximum stays the first
         const float m = __uint_as_float((unsigned)(told[b] >> 32));
         const int i = (int)(unsigned)told[b];
         if (m > mx || (m == mx && i < arg)) { mx = m; arg = i; }
@@ -189,22 +209,20 @@ sample_row_kernel(const float* __restrict__ logits, int row_stride, int V, const
                 for (int b = tid; b < 2 * SAMPLE_BINS; b += SAMPLE_THREADS) halves[b] = 0u;
                 __syncthreads();
                 const int f1 = min(n, f0 + SAMPLE_FLUSH);
-#pragma unroll 4
-                for (int i = f0 + tid; i < f1; i += SAMPLE_THREADS) {
-                    float w;
-                    if (KEEP && level > 0) w = kept[i];
-                    else {
-                        w = sample_weight(KEEP ? kept[i] : x[i], mx, inv_t);
+                walk(f0 + tid, f1, SAMPLE_THREADS, [&](float v, int i) {
+                    float w = v;
+                    if (!KEEP || level == 0) {
+                        w = sample_weight(v, mx, inv_t);
                         if (KEEP) kept[i] = w;
                     }
                     const unsigned pat = __float_as_uint(w);
                     const u64 fx = sample_fixed(w);
-                    if (fx == 0ull || (level == 1 && (pat >> 21) != prefix) || (level == 2 && (pat >> 10) != prefix)) continue;
+                    if (fx == 0ull || (level == 1 && (pat >> 21) != prefix) || (level == 2 && (pat >> 10) != prefix)) return;
                     const unsigned bin = level == 0 ? pat >> 21 : level == 1 ? (pat >> 10) & 0x7ffu : pat & 0x3ffu;
                     // (32-bit adds: 64-bit ones in shared memory are loops)
                     atomicAdd(halves + bin, (unsigned)fx & 0xffffu);
                     atomicAdd(halves + SAMPLE_BINS + bin, (unsigned)(fx >> 16));
-                }
+                });
                 __syncthreads();
                 for (int b = tid; b < SAMPLE_BINS; b += SAMPLE_THREADS) {
                     const u64 m = (u64)halves[b] + ((u64)halves[SAMPLE_BINS + b] << 16);
@@ -214,13 +232,13 @@ sample_row_kernel(const float* __restrict__ logits, int row_stride, int V, const
             }
             weights = KEEP;
             sample_cluster_sync();                                    // every block's masses are there, every block's `halves` free
-            if (tid < SAMPLE_BINS / SAMPLE_BLOCKS) {                  // a block adds up its share of the bins and tells all
-                const int b = rank * (SAMPLE_BINS / SAMPLE_BLOCKS) + tid;
+            for (int i = tid; i < SAMPLE_BINS / BLOCKS; i += SAMPLE_THREADS) {      // a block adds up its share of the bins and tells all
+                const int b = rank * (SAMPLE_BINS / BLOCKS) + i;
                 u64 sum = 0ull;
 #pragma unroll
-                for (int o = 0; o < SAMPLE_BLOCKS; ++o) sum += sample_get(hist + b, o);
+                for (int o = 0; o < BLOCKS; ++o) sum += sample_get(hist + b, o);
 #pragma unroll
-                for (int o = 0; o < SAMPLE_BLOCKS; ++o) sample_put(all + b, o, sum);
+                for (int o = 0; o < BLOCKS; ++o) sample_put(all + b, o, sum);
             }
             sample_cluster_sync();
             // the lowest bin whose mass above (in higher bins, and above the bits found before) is below the limit: thread t has
@@ -258,21 +276,22 @@ sample_row_kernel(const float* __restrict__ logits, int row_stride, int V, const
         }
     }
 
-    // ---- 3: kept mass, a run of neighbours a thread (an odd number: distinct banks), so that the scan is in the row's order
+    // ---- 3: kept mass.  Of a row in shared memory a thread takes a run of neighbours (an odd number: distinct banks), so that the scan is in the
+    // row's order; of others the whole block reads side by side
     const int run = ((n + SAMPLE_THREADS - 1) / SAMPLE_THREADS) | 1;
-    const int c0 = min(n, tid * run), c1 = min(n, c0 + run);
-    auto weight = [&](int i) { return weights ? kept[i] : sample_weight(KEEP ? kept[i] : x[i], mx, inv_t); };
+    const int c0 = KEEP ? min(n, tid * run) : tid, c1 = KEEP ? min(n, c0 + run) : n, step = KEEP ? 1 : SAMPLE_THREADS;
+    auto kept_mass = [&](float v) {
+        const float w = weights ? v : sample_weight(v, mx, inv_t);
+        return __float_as_uint(w) >= thresh ? sample_fixed(w) : 0ull;
+    };
     u64 mine = 0ull, part;
-    for (int i = c0; i < c1; ++i) {
-        const float w = weight(i);
-        if (__float_as_uint(w) >= thresh) mine += sample_fixed(w);
-    }
+    walk(c0, c1, step, [&](float v, int) { mine += kept_mass(v); });
     u64 before = block_excl_scan_u64(mine, scratch64, &part);
-    if (tid < SAMPLE_BLOCKS) sample_put(told_kept + rank, tid, part);
+    if (tid < BLOCKS) sample_put(told_kept + rank, tid, part);
     sample_cluster_sync();
     u64 mass = 0ull, start = 0ull;
 #pragma unroll
-    for (int b = 0; b < SAMPLE_BLOCKS; ++b) {
+    for (int b = 0; b < BLOCKS; ++b) {
         if (b < rank) start += told_kept[b];
         mass += told_kept[b];
     }
@@ -280,7 +299,7 @@ sample_row_kernel(const float* __restrict__ logits, int row_stride, int V, const
     int winner = -1;                    // the last block that is not empty and starts at or below the target
     u64 at = 0ull;
 #pragma unroll
-    for (int b = 0; b < SAMPLE_BLOCKS; ++b) {
+    for (int b = 0; b < BLOCKS; ++b) {
         if (told_kept[b] > 0ull && at <= target) winner = b;
         at += told_kept[b];
     }
@@ -289,22 +308,95 @@ sample_row_kernel(const float* __restrict__ logits, int row_stride, int V, const
         return;
     }
     if (rank != winner) return;
-    before += start;
-    const int who = -block_min_int((mine > 0ull && before <= target) ? -tid : 1, iscratch);
-    if (tid == who) {
-        int pick = -1, last = -1;
-        for (int i = c0; i < c1; ++i) {
-            const float w = weight(i);
-            if (__float_as_uint(w) >= thresh) {
-                const u64 fx = sample_fixed(w);
+    if (KEEP) {
+        before += start;
+        const int who = -block_min_int((mine > 0ull && before <= target) ? -tid : 1, iscratch);
+        if (tid == who) {
+            int pick = -1, last = -1;
+            for (int i = c0; i < c1; ++i) {
+                const u64 fx = kept_mass(kept[i]);
                 if (fx == 0ull) continue;
                 before += fx;
                 last = p0 + i;
                 if (before > target) { pick = p0 + i; break; }
             }
+            out[r] = pick >= 0 ? pick : (last >= 0 ? last : arg);
         }
-        out[r] = pick >= 0 ? pick : (last >= 0 ? last : arg);
+    } else {
+        // the part that is not empty and starts at or below the target, the last such one: a sixteenth for each warp, then a sixteenth of
+        // that, until an element is left for each thread
+        constexpr int WARPS = SAMPLE_THREADS / 32;
+        const int lane = tid & 31, warp = tid >> 5;
+        int lo = 0, hi = n;
+        u64 upto = start;                                             // mass before lo
+        while (hi - lo > SAMPLE_THREADS) {
+            const int each = (hi - lo + WARPS - 1) / WARPS, w0 = min(hi, lo + warp * each), w1 = min(hi, w0 + each);
+            u64 sum = 0ull;
+            walk(w0 + lane, w1, 32, [&](float v, int) { sum += kept_mass(v); });
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (lane == 0) scratch64[warp] = sum;
+            __syncthreads();
+            u64 at = upto;
+            int who = 0;
+            for (int w = 0; w < WARPS; ++w) {
+                if (scratch64[w] > 0ull && at <= target) {
+                    who = w;
+                    upto = at;
+                }
+                at += scratch64[w];
+            }
+            lo = min(hi, lo + who * each);
+            hi = min(hi, lo + each);
+            __syncthreads();                                          // the sums have been read
+        }
+        mine = lo + tid < hi ? kept_mass(x[lo + tid]) : 0ull;
+        before = upto + block_excl_scan_u64(mine, scratch64, &part);
+        const int who = -block_min_int((mine > 0ull && before <= target) ? -tid : 1, iscratch);
+        if (tid == 0) out[r] = who >= 0 ? p0 + lo + who : arg;
     }
+}
+
+static size_t sample_bytes(int per) { return 2 * SAMPLE_BINS * sizeof(u64) + (size_t)per * sizeof(float); }
+
+// Can clusters of sixteen run here with that much shared memory?
+template <bool KEEP>
+static bool sample_sixteen(size_t smem) {
+    if (cudaFuncSetAttribute(sample_row_kernel<KEEP, 16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(sample_row_kernel<KEEP, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(SAMPLE_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 16;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, sample_row_kernel<KEEP, 16>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return n > 0;
+}
+
+struct SampleShape { int blocks; bool keep; };      // blocks of a row, and whether they keep it
+// One block for rows of up to 4,096 entries, and while more rows wait than run at once also for those that one block keeps: what the
+// passes cost beside the entries, clearing and adding up 2,048 bins and the clusters' barriers, is per block (us with top-p, in 1 / 8 blocks:
+// rows of 2,000: 1 row 11 / 15, 64 rows 11 / 44, 256 18 / 132; of 16,384: 1 row 21 / 16, 64 21 / 46).  Eight up to what eight of them keep, two on a multiprocessor.  Beyond, sixteen
+// where the device runs such clusters, which keep what they can with a multiprocessor to each (262,144 entries, 1 / 64 rows: 29 / 165 us, in eight that keep nothing
+// 72 / 185).  Greedy rows are read once: nothing is kept there.
+static SampleShape sample_shape(int R, int V, bool drawn) {
+    if (V <= 4096 || (R > pico_num_sms() / 4 && V <= SAMPLE_KEEP)) return {1, true};
+    if (V <= 8 * SAMPLE_KEEP) return {8, true};
+    static const bool sixteen_keep = sample_sixteen<true>(sample_bytes(SAMPLE_KEEP_ALONE)), sixteen = sample_sixteen<false>(sample_bytes(0));
+    if (V <= 16 * SAMPLE_KEEP_ALONE) return drawn && sixteen_keep ? SampleShape{16, true} : SampleShape{8, false};
+    return {sixteen ? 16 : 8, false};
 }
 
 // logits: [R, row_stride] float32, the first V columns are used.  temperature, top_p, uniform:
@@ -314,21 +406,25 @@ PICO_API int pico_sample(const float* logits, int row_stride, int R, int V, cons
     if (R <= 0) return 0;
     if (V <= 0) return PICO_ERR_SIZE;
     if (temperature && !uniform) return PICO_ERR_SIZE;
-    const int per = ((V + SAMPLE_BLOCKS - 1) / SAMPLE_BLOCKS + 3) / 4 * 4;
-    const bool keep = per <= SAMPLE_KEEP;
-    const size_t smem = 2 * SAMPLE_BINS * sizeof(u64) + (keep ? (size_t)per * sizeof(float) : 0);
+    const SampleShape shape = sample_shape(R, V, temperature != nullptr);
+    const int per = ((V + shape.blocks - 1) / shape.blocks + 3) / 4 * 4;
+    const size_t smem = sample_bytes(shape.keep ? per : 0);
     const bool vec = V % 4 == 0 && row_stride % 4 == 0 && ((uintptr_t)logits & 15) == 0;
     for (int r0 = 0; r0 < R; r0 += 65535) {
         const int rows = R - r0 < 65535 ? R - r0 : 65535;
         const float* lg = logits + (size_t)r0 * row_stride;
         const float *t = temperature ? temperature + r0 : nullptr, *tp = top_p ? top_p + r0 : nullptr, *u = uniform ? uniform + r0 : nullptr;
-#define SAMPLE_LAUNCH(K)                                                                                                         \
+#define SAMPLE_LAUNCH(K, B)                                                                                                      \
     do {                                                                                                                         \
-        cudaFuncSetAttribute(sample_row_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                      \
-        pico_launch_cluster((sample_row_kernel<K>), dim3(SAMPLE_BLOCKS, rows), dim3(SAMPLE_THREADS), smem, stream, SAMPLE_BLOCKS, \
-                            lg, row_stride, V, t, tp, u, out + r0, per, vec);                                                    \
+        cudaFuncSetAttribute(sample_row_kernel<K, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                   \
+        pico_launch_cluster((sample_row_kernel<K, B>), dim3(B, rows), dim3(SAMPLE_THREADS), smem, stream, B, lg, row_stride, V, t, tp, u, \
+                            out + r0, per, vec);                                                                                 \
     } while (0)
-        if (keep) SAMPLE_LAUNCH(true); else SAMPLE_LAUNCH(false);
+        if (shape.blocks == 1) SAMPLE_LAUNCH(true, 1);
+        else if (shape.blocks == 8 && shape.keep) SAMPLE_LAUNCH(true, 8);
+        else if (shape.blocks == 8) SAMPLE_LAUNCH(false, 8);
+        else if (shape.keep) SAMPLE_LAUNCH(true, 16);
+        else SAMPLE_LAUNCH(false, 16);
 #undef SAMPLE_LAUNCH
     }
     return pico_launch_status();
