@@ -932,11 +932,11 @@ static int tg_launch(const void* x, const void* w, const TgArgs& a, cudaStream_t
 }
 
 // Rows a group from which its rows are the instruction's N; below, tiles of 256 rows of x stand beside 256 of w (gemm_tcgen05_pair_kernel,
-// GROUPED): shorter groups leave a tile partly empty either way, what counts is the stream of weights, and there two blocks that
-// copy 128 rows of each operand a k-block do better.  The two products of a gated feed-forward, that form / this, us: 16 experts of
-// 1,536 x 2,240, 100 rows a group 55 + 36 / 63 + 44, 175 55 + 38 / 67 + 46, 256 91 + 53 / 71 + 48, 512 135 + 73 / 128 + 71; 32 of
-// 2,048 x 2,752, 128 rows 175 + 92 / 195 + 102, 231 185 + 101 / 228 + 119, 256 276 + 147 / 238 + 121, 288 344 + 180 / 250 + 128.
-#define TG_MIN_ROWS 240
+// GROUPED): shorter groups leave a tile partly empty either way, what counts is the stream of weights, and there blocks that copy the boxes
+// of x that are there beside 128 rows of w a k-block do better.  The two products of a gated feed-forward, that form / this, us: 16 experts of
+// 1,536 x 2,240, 100 rows a group 53 + 37 / 63 + 44, 175 55 + 38 / 66 + 45, 240 65 + 38 / 69 + 47, 256 82 + 42 / 71 + 48, 400 103 + 58 / 86 + 54;
+// 32 of 2,048 x 2,752, 128 rows 176 + 92 / 195 + 102, 225 189 + 104 / (231) 228 + 119, 256 284 + 155 / 238 + 121, 288 351 + 204 / 250 + 128.
+#define TG_MIN_ROWS 245
 
 // x [n, K] and w [E, N, K] contiguous; epi 0 (out [n, N]), 2 or 3 (out [n, N / 2]) as above.  rows: 0 = chosen here, < 0: the form for
 // short groups, else of x in a tile at most (a multiple of 64 to 512).

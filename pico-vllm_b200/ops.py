@@ -1293,9 +1293,9 @@ def gated_rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor], gate_logits:
 
 
 # the experts' products run on the tcgen05 tensor cores, over rows in expert order, from this many (token, expert) pairs per expert on
-# (below, the experts' lists fit into tiles of 16 rows of the grouped mma.sync kernels, a stream of the weights; a layer of 16
-# experts, top 4, width 1,536, in us: 256 pairs 97 here and 98 there, 512 98 and 198, 8,192 208 and 763; 32 experts, width
-# 2,048: 256 pairs 255 and 231, 512 265 and 266, 800 269 and 360)
+# (below, the experts' lists fit into tiles of 16 rows of the grouped mma.sync kernels, a stream of the weights; a layer with 12, 16, 20 pairs
+# an expert, in us here / there: 16 experts of 1,536 x 2,240 88 / 75, 89 / 91, 89 / 193; 32 of 2,048 x 2,752 240 / 213, 242 / 247, 244 / 333;
+# 128 of 2,048 x 768 272 / 247, 273 / 283, 274 / 393)
 MOE_TC_MIN_ROWS = 16
 MOE_TC_MAX_EXPERTS = 1024
 # widths under 64, a part of a k-block: only where there is something to multiply (32 experts of 1,024 x 48, in us: 544 pairs 27, 38 there, 8,192

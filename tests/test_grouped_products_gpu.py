@@ -126,7 +126,7 @@ FORMS = {"gated": dict(), "capped": dict(act="capped", limit=0.9), "weight in": 
 
 
 @pytest.mark.parametrize("form", list(FORMS))
-@pytest.mark.parametrize("T", [35, 640])             # on either side of 240 rows an expert on average, with five experts of which one gets nothing
+@pytest.mark.parametrize("T", [35, 640])             # on either side of 245 rows an expert on average, with five experts of which one gets nothing
 @pytest.mark.parametrize("D,ff", [(64, 64), (72, 104), (136, 112)])
 @pytest.mark.parametrize("identity,base", [(0, False), (2, True)])
 def test_experts_through_the_tensor_cores(form, T, D, ff, identity, base):
