@@ -1672,13 +1672,13 @@ def _chunk_scratch(floats: int, device: torch.device) -> Optional[torch.Tensor]:
 
 def gated_delta_rule(prep: torch.Tensor, v: torch.Tensor, state: torch.Tensor, seg_slots: torch.Tensor, cu_q: torch.Tensor,
                      positions: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int, per_head: bool = False,
-                     max_q_len: int = 1) -> torch.Tensor:
+                     max_q_len: int = 1, min_q_len: int = 1) -> torch.Tensor:
     """Per head h, token by token in the order of each segment, from and into ``state`` float32 [slots, heads, vdim, dim] (S
     transposed; row ``seg_slots[s]``):  S <- diag(a) S;  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q.  ``prep``: the rows
     :func:`delta_prepare` made with the same ``per_head`` and ``max_q_len`` (with a decay
     per head and segments of DELTA_BLOCK_MIN_TOKENS and more, four tokens share one pass over the memory; head h reads query and key head h // (heads / kv_heads)); ``v`` float32 rows with head h's values
-    at h * vdim (a column slice is fine).  A segment whose first position is negative is padding.  Returns o float32
-    [T, heads * vdim]."""
+    at h * vdim (a column slice is fine).  A segment whose first position is negative is padding.  ``min_q_len``: no segment that is
+    not padding has fewer tokens.  Returns o float32 [T, heads * vdim]."""
     _cuda(prep, v, state, seg_slots, cu_q, positions)
     _f32_rows(v, "gated_delta_rule: v")
     T, S = prep.shape[0], seg_slots.shape[0]
@@ -1702,8 +1702,7 @@ def gated_delta_rule(prep: torch.Tensor, v: torch.Tensor, state: torch.Tensor, s
         scratch = _chunk_scratch(library().pico_gated_delta_chunk_floats(T, S, H, vdim), prep.device)
     if scratch is not None:
         lib = library()
-        if S > 1:      # (also where no segment is short: without this launch before them the chunks' kernels took longer, 2,048 tokens of 12 heads
-                       # in two segments 303 us with their layer and not 273, in three 268 and not 262)
+        if S > 1 and min_q_len < DELTA_CHUNK_LEAST:
             _check(lib.pico_gated_delta_rule(_ptr(prep), _ptr(v), v.stride(0), _ptr(state), _ptr(seg_slots), _ptr(cu_q), _ptr(positions),
                                              _ptr(out), out.stride(0), S, H, G, d, vdim, 1, 1, DELTA_CHUNK_LEAST, _stream()),
                    f"gated_delta_rule (dim {d})")

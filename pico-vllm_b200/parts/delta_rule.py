@@ -127,8 +127,9 @@ class GatedDeltaRule(Part):
             alone = batch.seg_slots.shape[0] == 1 and ops.delta_chunks_take(xc[:, 2 * G * d:], memory.state, d, dv, batch.max_prefill_q, 1)
             prep = ops.delta_prepare(xc, 0, G * d, proj, b0, proj[:, a0:a0 + H], self.dt_bias, self.a_log, H, G, d, per_head=True,
                                      max_q_len=1 if alone else batch.max_prefill_q)
+            shortest = min(batch.q_lens) if batch.max_prefill_q >= ops.DELTA_CHUNK_MIN_TOKENS else 1       # (of use in chunks only)
             o = ops.gated_delta_rule(prep, xc[:, 2 * G * d:], memory.state, batch.seg_slots, batch.cu_q, batch.positions,
-                                     H, G, d, dv, per_head=True, max_q_len=batch.max_prefill_q)
+                                     H, G, d, dv, per_head=True, max_q_len=batch.max_prefill_q, min_q_len=shortest)
             y = ops.group_rms_norm(o, H, dv, dv, self.out_norm, self.eps, h.dtype, post_gate=proj[:, g0:g0 + H * dv],
                                    post_act=self.gate_act)
             return _linear(y, self.o_weight)

@@ -82,6 +82,17 @@ def test_which_steps_go_in_chunks(lens, d, take):
     assert not ops.delta_chunks_take(v[:, 1:], state, d, 128, max(lens), S)
 
 
+@pytest.mark.parametrize("lens,launches", [([512], 3), ([600, 64], 3), ([600, 63], 4)])
+def test_no_launch_for_short_segments_that_are_not_there(lens, launches):
+    from pico_vllm_b200 import ops
+    H, d, T, S = 2, 68, sum(lens), len(lens)
+    cu, pos, slots = (t.to(DEV) for t in _segments(lens))
+    prep, v, state = torch.zeros(T, 2 * H * d + 12 * H, device=DEV), torch.ones(T, H * 4, device=DEV), torch.zeros(S, H, 4, d, device=DEV)
+    before = ops.launches
+    out = ops.gated_delta_rule(prep, v, state, slots, cu, pos, H, H, d, 4, per_head=True, max_q_len=max(lens), min_q_len=min(lens))
+    assert ops.launches - before == launches and not out.any()
+
+
 @pytest.mark.parametrize("lens", [[520], [600, 70, 3]])
 def test_without_room_for_its_scratch_a_step_goes_without_chunks(lens, monkeypatch):
     """The same outputs and memory, from the allocator's own error on; one segment's rows come without the dot products of neighbours."""
