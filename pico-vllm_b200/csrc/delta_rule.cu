@@ -637,7 +637,8 @@ __global__ void __launch_bounds__(256)
 delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* __restrict__ v, int v_stride, const int* __restrict__ cu_q,
                            const int* __restrict__ positions, int S, float* __restrict__ coef, float* __restrict__ u0, int H, int G,
                            int d, int dv, bool keep_v) {
-    pdl_launch_dependents();
+    // (the chain's blocks, released here, would settle where the first of these end, two long segments on one multiprocessor and none on others:
+    // they are released at the end; a layer of 2,048 tokens in three segments, 12 / 16 heads: 257 / 333 us, 269 / 346 the other way)
     pdl_wait();
     int t0, n;
     if (!dc_find(cu_q, positions, S, blockIdx.x, t0, n)) return;
