@@ -591,10 +591,13 @@ gated_delta_block_kernel(const float* __restrict__ prep, int P, const float* __r
 // the chain from chunk to chunk, two products, which leaves U and every chunk's S behind; O for all chunks side by side.  All
 // float32; decays are products of decays (none is above one, nothing is divided), the inverse comes from forward substitution.
 // Tokens beyond a segment's end are blanks (k = q = v = 0, beta = 0, g = 1).
-// The chain is bound by what a block reads from shared memory (K, M diag(G) K and S once a chunk for every four columns), over
-// len / 32 dependent steps of the longest segment: hence the two products only (with all four in the chain 170 us for the
-// tokens below), four warps a block (eight, with half the columns each: 225) and 16 columns.
-// 2,048 tokens of twelve heads with d = dv = 128 in segments of 341, 682 and 1,025: 195 us, of which the chain 118 (four tokens at a time: 248).
+// The chain is bound by the instructions that its warps issue one after the other, over len / 32 dependent steps of the longest segment:
+// hence the two products only (with all four in the chain 170 us for the tokens below), 16 columns a block, and four more warps that
+// fetch (the loads' addresses were a quarter of the instructions).
+// A layer with projections, twelve heads with d = dv = 128, 2,048 tokens in segments of 341, 682 and 1,025 / of 682 and 1,366 / 1,361 in
+// one: 236 / 275 / 176 us (the chain of the first 87); with both products on the CUDA cores, S and all operands from shared memory, 256 / 303 /
+// 201 (107); eight warps that multiply 257 / 276 / 181 (one block a multiprocessor); both products on the tensor cores 238 / 251 / 165, but
+// S is then off by 1.1e-7 of float64 where decays are strong, 0.7e-7 now and before.
 #define DC_C 32
 #define DC_D 128                               // rows of S, keys padded with zeros
 #define DC_LD (DC_D + 4)                       // rows that lanes read side by side, 16 bytes each
@@ -810,21 +813,77 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* _
     }
 }
 
-// The chain.  Grid (column tiles, H, segments), four warps.  S is kept by the threads (lane: rows 4 lane .. + 3, warp: columns 4 warp ..
-// + 3) and, by columns, in shared memory for the product with it.  u: M V on the way in, U on the way out; s0 float32 [chunks, H,
-// dv rounded up to 4, 128]: S before each chunk, by columns.
-__global__ void __launch_bounds__(128)
+// A float32 number as two of tf32's eleven digits each: what is left over is below half a unit of its last place.
+__device__ __forceinline__ void dc_split(float x, uint32_t& hi, uint32_t& lo) {
+    // Dekker's splitting, each operation rounded by itself (the conversion instruction is a sixteenth of the rate)
+    const float c = __fmul_rn(8193.f, x), h = __fsub_rn(c, __fsub_rn(c, x));
+    hi = __float_as_uint(h);
+    lo = __float_as_uint(__fsub_rn(x, h));
+}
+__device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// c += a b with both in two parts (the product of the two small parts is below what float32 keeps).  The tensor cores
+// cut sums off where float32 rounds them: the large parts' products leave them after eight terms.  The small parts' sums are kept apart,
+// as an instruction that adds into the registers of the one before waits 126 clocks for it.
+__device__ __forceinline__ void dc_mma3(float (&c)[3][4], const uint32_t (&ah)[4], const uint32_t (&al)[4], float b0, float b1) {
+    uint32_t h0, l0, h1, l1;
+    dc_split(b0, h0, l0);
+    dc_split(b1, h1, l1);
+    float big[4] = {};
+    dc_mma(big, ah, h0, h1);
+    dc_mma(c[1], al, h0, h1);
+    dc_mma(c[2], ah, l0, l1);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[0][e] += big[e];
+}
+__device__ __forceinline__ void dc_sum3(float (&c)[4], const float (&p)[3][4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[e] = p[0][e] + (p[1][e] + p[2][e]);
+}
+// The numbers that a lane holds of a product's result, rows r and r + 8 at places 2 j and 2 j + 1, as the rows' operand of a product over
+// those places (dealt to the lanes in the order 0, 2, 4, 6, 1, 3, 5, 7, which the other operand follows).
+__device__ __forceinline__ void dc_rows(const float (&c)[4], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+    dc_split(c[0], hi[0], lo[0]);
+    dc_split(c[2], hi[1], lo[1]);
+    dc_split(c[1], hi[2], lo[2]);
+    dc_split(c[3], hi[3], lo[3]);
+}
+__device__ __forceinline__ bool dc_no_number(const float (&c)[4][4]) {
+    bool no = false;
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) no |= c[t][e] != c[t][e];
+    return __any_sync(0xffffffffu, no);
+}
+
+// The chain.  Grid (column tiles, H, segments), four warps and four that fetch.  A warp keeps 32 rows of the block's 16 columns of S in
+// registers, as the tensor cores take an operand: with columns as the 16 rows of an instruction, (M diag(G) K) S is over the warp's own rows
+// of S, which never goes through shared memory.  The warps' four parts are added through shared memory, each warp makes U for eight tokens,
+// and all of them their own rows of S', in float32 on the CUDA cores.  u: M V on the way in, U on the way out; s0 float32 [chunks, H, dv
+// rounded up to 4, 128]: S before each chunk, by columns.
+// The product with S is three tf32 products, eight terms at a time.  Where a result is no number, plain float32 products decide what it
+// is (the parts of an infinity are no infinity's parts).
+#define DC_LDM (DC_D + 8)                      // rows of M diag(G) K: eight read side by side, 8 bytes a lane
+#define DC_LDT (DC_D + 4)                      // rows of K: pairs of rows, 4 bytes a lane
+#define DC_LDU (DC_NC + 4)
+#define DC_WARPS 4                             // warps that multiply; four more fetch
+#define DC_ROWS (DC_D / DC_WARPS)              // rows of S a warp
+__global__ void __launch_bounds__(32 * (DC_WARPS + 4), 2)
 delta_chunk_kernel(const float* __restrict__ prep, int P, float* __restrict__ state, const int* __restrict__ seg_slots,
                    const int* __restrict__ cu_q, const int* __restrict__ positions, const float* __restrict__ coef, float* __restrict__ u,
                    float* __restrict__ s0, int H, int G, int d, int dv) {
     pdl_wait();                         // the kernel that follows is released at the end (see above)
     extern __shared__ __align__(16) float dsm[];
-    constexpr int MG = DC_C * DC_LDK, BUF = 2 * MG + 2 * DC_C + DC_C * DC_NC;      // a chunk: K, M diag(G) K, G, D_Cj, M V [C][NC]
+    constexpr int MG = DC_C * DC_LDT, GD = MG + DC_C * DC_LDM, UV = GD + 2 * DC_C, BUF = UV + DC_C * DC_LDU;   // a chunk: K, M diag(G) K, G, D_Cj, M V
     const int seg = blockIdx.z, h = blockIdx.y, col_base = blockIdx.x * DC_NC;
     const int t_begin = cu_q[seg], t_end = cu_q[seg + 1];
     if (t_end - t_begin < DC_LEAST || positions[t_begin] < 0) return;      // a short or a padding segment
-    float* s_s = dsm + 2 * BUF;                // S by columns [NC][LDK]
-    float* w_s = s_s + DC_NC * DC_LDK;         // diag(D_Cj) U [C][NC], every number twice (the pairs that two rows at a time want)
+    float* parts = dsm + 2 * BUF;              // [warp][4 tiles of tokens][lane][4]
+    float* w_s = parts + DC_WARPS * 512;                 // diag(D_Cj) U [C][8][4]: columns c, c, c + 8, c + 8 (the pairs that two rows at a time want)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hq = h / (H / G);
     int chunk = 0;
     for (int s = lane; s < seg; s += 32) chunk += dc_chunks_of(cu_q, seg, s);
@@ -834,145 +893,154 @@ delta_chunk_kernel(const float* __restrict__ prep, int P, float* __restrict__ st
         const int n = min(DC_C, t_end - t0);
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
         const float* cf = coef + ((size_t)ch * H + h) * DC_COEF;
-        for (int idx = threadIdx.x; idx < DC_C * (DC_D / 4); idx += 128) {
+        const int tid = threadIdx.x - 32 * DC_WARPS;
+#pragma unroll
+        for (int idx = tid; idx < DC_C * (DC_D / 4); idx += 128) {
             const int i = idx / (DC_D / 4), c = idx % (DC_D / 4) * 4;
-            float* dst = buf + i * DC_LDK + c;
+            float* dst = buf + i * DC_LDT + c;
             if (i < n && c < d) dr_cp16(dst, prep + (size_t)(t0 + i) * P + G * d + hq * d + c);
             else *reinterpret_cast<float4*>(dst) = zero;
-            dr_cp16(dst + MG, cf + i * DC_D + c);
+            dr_cp16(buf + MG + i * DC_LDM + c, cf + i * DC_D + c);
         }
-        if (threadIdx.x < 2 * DC_C / 4) dr_cp16(buf + 2 * MG + 4 * threadIdx.x, cf + DC_C * DC_D + DC_C * DC_C + 4 * threadIdx.x);
+        if (tid < 2 * DC_C / 4) dr_cp16(buf + GD + 4 * tid, cf + DC_C * DC_D + DC_C * DC_C + 4 * tid);
         {
-            const int i = threadIdx.x / (DC_NC / 4), c = threadIdx.x % (DC_NC / 4) * 4;
-            float* dst = buf + 2 * MG + 2 * DC_C + i * DC_NC + c;
+            const int i = tid / (DC_NC / 4), c = tid % (DC_NC / 4) * 4;
+            float* dst = buf + UV + i * DC_LDU + c;
             if (i < n && col_base + c < dv) dr_cp16(dst, u + (size_t)(t0 + i) * H * dv + (size_t)h * dv + col_base + c);
             else *reinterpret_cast<float4*>(dst) = zero;
         }
         dr_commit();
     };
-    fetch(t_begin, chunk, dsm);
-    float* st = state + ((size_t)seg_slots[seg] * H + h) * (size_t)dv * d;
-    f32x2 S[4][2];                             // [column][row pair]
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const int col = col_base + 4 * warp + c;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (col < dv && 4 * lane < d) x = *reinterpret_cast<const float4*>(st + (size_t)col * d + 4 * lane);
-        S[c][0] = db_pair(x.x, x.y);
-        S[c][1] = db_pair(x.z, x.w);
-        *reinterpret_cast<float4*>(s_s + (4 * warp + c) * DC_LDK + 4 * lane) = x;
+    if (warp >= DC_WARPS) {
+        // the warps that fetch: a chunk ahead of the others
+        int turn = 0;
+        fetch(t_begin, chunk, dsm);
+        for (int t0 = t_begin; t0 < t_end; t0 += DC_C, turn ^= 1, ++chunk) {
+            dr_wait_all();
+            __syncthreads();                   // the chunk is in, everyone is done with the other buffer
+            if (t0 + DC_C < t_end) fetch(t0 + DC_C, chunk + 1, dsm + (turn ? 0 : BUF));
+        }
+        return;
     }
-    // the product with S: a lane has rows rt, rt + 8, .. of M diag(G) K, columns 4 warp .. + 3, and of the sums over the rows of S
-    // every fourth four (kg)
-    const int kg = lane & 3, rt = lane >> 2;
+    float* st = state + ((size_t)seg_slots[seg] * H + h) * (size_t)dv * d;
+    const int r = lane >> 2, j = lane & 3, row0 = DC_ROWS * warp + 2 * j;       // this lane: columns r and r + 8, rows row0 + 8 nt and the next
+    float S[DC_ROWS / 8][4];
+#pragma unroll
+    for (int nt = 0; nt < DC_ROWS / 8; ++nt)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int col = col_base + r + 8 * c;
+            float2 x = make_float2(0.f, 0.f);
+            if (col < dv && row0 + 8 * nt < d) x = *reinterpret_cast<const float2*>(st + (size_t)col * d + row0 + 8 * nt);
+            S[nt][2 * c] = x.x;
+            S[nt][2 * c + 1] = x.y;
+        }
     int turn = 0;
     for (int t0 = t_begin; t0 < t_end; t0 += DC_C, turn ^= 1, ++chunk) {
-        dr_wait_all();
-        __syncthreads();                       // the chunk is in, S is written, everyone is done with the other buffer
-        if (t0 + DC_C < t_end) fetch(t0 + DC_C, chunk + 1, dsm + (turn ? 0 : BUF));
+        __syncthreads();                       // the chunk is in, everyone is done with the other buffer
         const float* buf = dsm + (turn ? BUF : 0);
-        const float *k_s = buf, *Gd = buf + 2 * MG, *Wd = Gd + DC_C, *u_s = Wd + DC_C;
-        {
-            f32x2 acc[4][4];
+        const float *k_s = buf + row0, *m_s = buf + MG + row0, *Gd = buf + GD, *Wd = Gd + DC_C, *u_s = buf + UV;
+        // S before this chunk, for the outputs
+        float* s_out = s0 + (((size_t)chunk * H + h) * ((dv + 3) / 4 * 4) + col_base + r) * DC_D + row0;
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
+        for (int nt = 0; nt < DC_ROWS / 8; ++nt)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) acc[r][e] = db_pair(0.f, 0.f);
-            const float* row = buf + MG + rt * DC_LDK + 4 * kg;
-            const float* c0 = s_s + 4 * warp * DC_LDK + 4 * kg;
-#pragma unroll 4
-            for (int c = 0; c < DC_D; c += 16) {
-                ulonglong2 b[4];
+            for (int c = 0; c < 2; ++c)
+                if (col_base + r + 8 * c < dv) *reinterpret_cast<float2*>(s_out + c * 8 * DC_D + 8 * nt) = make_float2(S[nt][2 * c], S[nt][2 * c + 1]);
+        float x[4][4], x3[4][3][4] = {};       // [tile of tokens]: columns r, r + 8, tokens 8 tt + 2 j and the next
 #pragma unroll
-                for (int e = 0; e < 4; ++e) b[e] = *reinterpret_cast<const ulonglong2*>(c0 + e * DC_LDK + c);
+        for (int nt = 0; nt < DC_ROWS / 8; ++nt) {
+            uint32_t ah[4], al[4];
+            dc_rows(S[nt], ah, al);
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(row + r * 8 * DC_LDK + c);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[r][e] = db_fma2(a.y, b[e].y, db_fma2(a.x, b[e].x, acc[r][e]));
-                }
-            }
-            // S before this chunk, for the outputs
-            float* s_out = s0 + (((size_t)chunk * H + h) * ((dv + 3) / 4 * 4) + col_base + 4 * warp) * DC_D + 4 * lane;
-            if (col_base + 4 * warp < dv) {
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const float2 a = db_split(S[c][0]), b = db_split(S[c][1]);
-                    *reinterpret_cast<float4*>(s_out + c * DC_D) = make_float4(a.x, a.y, b.x, b.y);
-                }
-            }
-            // the four lanes' sums: each lane ends with one row
-            float s[4][4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float2 f = db_split(acc[r][e]);
-                    s[r][e] = f.x + f.y;
-                }
-            const bool hi = kg & 1, second = kg & 2;
-#pragma unroll
-            for (int r = 0; r < 2; ++r)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float send = hi ? s[r][e] : s[r + 2][e], keep = hi ? s[r + 2][e] : s[r][e];
-                    s[r][e] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
-                }
-            float x[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float send = second ? s[0][e] : s[1][e], keep = second ? s[1][e] : s[0][e];
-                x[e] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-            }
-            const int i = rt + 8 * ((hi ? 2 : 0) + (second ? 1 : 0));
-            const float4 mv = *reinterpret_cast<const float4*>(u_s + i * DC_NC + 4 * warp);
-            const float4 uu = make_float4(mv.x - x[0], mv.y - x[1], mv.z - x[2], mv.w - x[3]);
-            const float wj = Wd[i];
-            const float4 w4 = make_float4(wj * uu.x, wj * uu.y, wj * uu.z, wj * uu.w);
-            *reinterpret_cast<float4*>(w_s + 2 * (i * DC_NC + 4 * warp)) = make_float4(w4.x, w4.x, w4.y, w4.y);
-            *reinterpret_cast<float4*>(w_s + 2 * (i * DC_NC + 4 * warp) + 4) = make_float4(w4.z, w4.z, w4.w, w4.w);
-            if (t0 + i < t_end && col_base + 4 * warp < dv)
-                *reinterpret_cast<float4*>(u + (size_t)(t0 + i) * H * dv + (size_t)h * dv + col_base + 4 * warp) = uu;
-        }
-        __syncthreads();                       // everyone has read S
-        {
-            const float gc = Gd[DC_C - 1];
-            const f32x2 g2 = db_pair(gc, gc);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                S[c][0] = db_mul2(S[c][0], g2);
-                S[c][1] = db_mul2(S[c][1], g2);
-            }
-#pragma unroll 8
-            for (int j = 0; j < DC_C; ++j) {
-                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(k_s + j * DC_LDK + 4 * lane);
-                const ulonglong2 wa = *reinterpret_cast<const ulonglong2*>(w_s + 2 * (j * DC_NC + 4 * warp));
-                const ulonglong2 wb = *reinterpret_cast<const ulonglong2*>(w_s + 2 * (j * DC_NC + 4 * warp) + 4);
-                S[0][0] = db_fma2(k.x, wa.x, S[0][0]);
-                S[0][1] = db_fma2(k.y, wa.x, S[0][1]);
-                S[1][0] = db_fma2(k.x, wa.y, S[1][0]);
-                S[1][1] = db_fma2(k.y, wa.y, S[1][1]);
-                S[2][0] = db_fma2(k.x, wb.x, S[2][0]);
-                S[2][1] = db_fma2(k.y, wb.x, S[2][1]);
-                S[3][0] = db_fma2(k.x, wb.y, S[3][0]);
-                S[3][1] = db_fma2(k.y, wb.y, S[3][1]);
-            }
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                ulonglong2 x;
-                x.x = S[c][0];
-                x.y = S[c][1];
-                *reinterpret_cast<ulonglong2*>(s_s + (4 * warp + c) * DC_LDK + 4 * lane) = x;
+            for (int tt = 0; tt < 4; ++tt) {
+                const float2 b = *reinterpret_cast<const float2*>(m_s + (8 * tt + r) * DC_LDM + 8 * nt);
+                dc_mma3(x3[tt], ah, al, b.x, b.y);
             }
         }
+#pragma unroll
+        for (int tt = 0; tt < 4; ++tt) dc_sum3(x[tt], x3[tt]);
+        if (dc_no_number(x)) {
+#pragma unroll
+            for (int t = 0; t < DC_C; ++t) {
+                float p0 = 0.f, p1 = 0.f;
+#pragma unroll
+                for (int nt = 0; nt < DC_ROWS / 8; ++nt) {
+                    const float2 b = *reinterpret_cast<const float2*>(m_s + t * DC_LDM + 8 * nt);
+                    p0 = fmaf(S[nt][1], b.y, fmaf(S[nt][0], b.x, p0));
+                    p1 = fmaf(S[nt][3], b.y, fmaf(S[nt][2], b.x, p1));
+                }
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) {
+                    p0 += __shfl_xor_sync(0xffffffffu, p0, o);
+                    p1 += __shfl_xor_sync(0xffffffffu, p1, o);
+                }
+                if (j == (t & 7) >> 1) {
+                    if (x[t >> 3][t & 1] != x[t >> 3][t & 1]) x[t >> 3][t & 1] = p0;
+                    if (x[t >> 3][2 + (t & 1)] != x[t >> 3][2 + (t & 1)]) x[t >> 3][2 + (t & 1)] = p1;
+                }
+            }
+        }
+        float* mine = parts + lane * 4;
+#pragma unroll
+        for (int tt = 0; tt < 4; ++tt) *reinterpret_cast<float4*>(mine + (warp * 4 + tt) * 128) = make_float4(x[tt][0], x[tt][1], x[tt][2], x[tt][3]);
+        asm volatile("bar.sync 1, %0;\n" ::"n"(32 * DC_WARPS) : "memory");
+        if (warp < DC_C / 8) {                 // U and diag(D_Cj) U of eight tokens
+            float4 a[DC_WARPS];
+#pragma unroll
+            for (int p = 0; p < DC_WARPS; ++p) a[p] = *reinterpret_cast<const float4*>(mine + (p * 4 + warp) * 128);
+#pragma unroll
+            for (int o = DC_WARPS / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int p = 0; p < o; ++p) a[p] = make_float4(a[p].x + a[p + o].x, a[p].y + a[p + o].y, a[p].z + a[p + o].z, a[p].w + a[p + o].w);
+            const float* mv = u_s + (8 * warp + 2 * j) * DC_LDU + r;
+            const float2 wj = *reinterpret_cast<const float2*>(Wd + 8 * warp + 2 * j);
+            const float u0 = mv[0] - a[0].x, u1 = mv[DC_LDU] - a[0].y, u2 = mv[8] - a[0].z, u3 = mv[DC_LDU + 8] - a[0].w;
+            float* wo = w_s + ((8 * warp + 2 * j) * 8 + r) * 4;
+            *reinterpret_cast<float4*>(wo) = make_float4(wj.x * u0, wj.x * u0, wj.x * u2, wj.x * u2);
+            *reinterpret_cast<float4*>(wo + 32) = make_float4(wj.y * u1, wj.y * u1, wj.y * u3, wj.y * u3);
+            const int i = t0 + 8 * warp + 2 * j;
+            float* uo = u + (size_t)i * H * dv + (size_t)h * dv + col_base + r;
+            const bool c0 = col_base + r < dv, c1 = col_base + r + 8 < dv;
+            if (i < t_end && c0) uo[0] = u0;
+            if (i + 1 < t_end && c0) uo[(size_t)H * dv] = u1;
+            if (i < t_end && c1) uo[8] = u2;
+            if (i + 1 < t_end && c1) uo[(size_t)H * dv + 8] = u3;
+        }
+        asm volatile("bar.sync 1, %0;\n" ::"n"(32 * DC_WARPS) : "memory");
+        const float gc = Gd[DC_C - 1];
+        const f32x2 g2 = db_pair(gc, gc);
+        f32x2 s2[DC_ROWS / 8][2];
+#pragma unroll
+        for (int nt = 0; nt < DC_ROWS / 8; ++nt)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) s2[nt][c] = db_mul2(db_pair(S[nt][2 * c], S[nt][2 * c + 1]), g2);
+#pragma unroll
+        for (int t = 0; t < DC_C; ++t) {
+            const ulonglong2 w2 = *reinterpret_cast<const ulonglong2*>(w_s + (t * 8 + r) * 4);
+#pragma unroll
+            for (int nt = 0; nt < DC_ROWS / 8; ++nt) {
+                const f32x2 k = *reinterpret_cast<const f32x2*>(k_s + t * DC_LDT + 8 * nt);
+                s2[nt][0] = db_fma2(k, w2.x, s2[nt][0]);
+                s2[nt][1] = db_fma2(k, w2.y, s2[nt][1]);
+            }
+        }
+#pragma unroll
+        for (int nt = 0; nt < DC_ROWS / 8; ++nt)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float2 f = db_split(s2[nt][c]);
+                S[nt][2 * c] = f.x;
+                S[nt][2 * c + 1] = f.y;
+            }
     }
     pdl_launch_dependents();
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const int col = col_base + 4 * warp + c;
-        const float2 a = db_split(S[c][0]), b = db_split(S[c][1]);
-        if (col < dv && 4 * lane < d) *reinterpret_cast<float4*>(st + (size_t)col * d + 4 * lane) = make_float4(a.x, a.y, b.x, b.y);
-    }
+    for (int nt = 0; nt < DC_ROWS / 8; ++nt)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            if (col_base + r + 8 * c < dv && row0 + 8 * nt < d)
+                *reinterpret_cast<float2*>(st + (size_t)(col_base + r + 8 * c) * d + row0 + 8 * nt) = make_float2(S[nt][2 * c], S[nt][2 * c + 1]);
 }
 
 // The outputs.  Grid (chunks at most, H, tiles of 128 columns): O = diag(G) Q S + E U; a thread has tokens 8 ty .. + 7 and columns tx, tx +
@@ -1099,11 +1167,11 @@ PICO_API int pico_gated_delta_chunks(const float* prep, const float* v, int v_st
     cudaFuncSetAttribute(delta_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
     pico_launch(delta_chunk_prepare_kernel, dim3(chunks, G), dim3(256), sm1, stream, prep, P, v, v_stride, cu_q, positions, S, coef, u, H, G, d, dv, keep_v);
     const dim3 grid((dv + DC_NC - 1) / DC_NC, H, S);
-    size_t sm2 = (size_t)(2 * (2 * DC_C * DC_LDK + 2 * DC_C + DC_C * DC_NC) + DC_NC * DC_LDK + 2 * DC_C * DC_NC) * sizeof(float);
+    size_t sm2 = (size_t)(2 * (DC_C * DC_LDT + DC_C * DC_LDM + 2 * DC_C + DC_C * DC_LDU) + DC_WARPS * 512 + DC_C * 32) * sizeof(float);
     // (one block a multiprocessor where there are enough of them: see pico_gated_delta_rule)
     if ((long long)grid.x * grid.y * grid.z <= pico_num_sms() && sm2 < 116 * 1024) sm2 = 116 * 1024;
     cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);
-    pico_launch(delta_chunk_kernel, grid, dim3(128), sm2, stream, prep, P, state, seg_slots, cu_q, positions, (const float*)coef, u, s0, H, G, d, dv);
+    pico_launch(delta_chunk_kernel, grid, dim3(32 * (DC_WARPS + 4)), sm2, stream, prep, P, state, seg_slots, cu_q, positions, (const float*)coef, u, s0, H, G, d, dv);
     const size_t sm3 = (size_t)(DC_OC * DC_LD + DC_C * DC_LD + DC_C * DC_OC + DC_C * DC_C + DC_C) * sizeof(float);
     cudaFuncSetAttribute(delta_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3);
     pico_launch(delta_chunk_out_kernel, dim3(chunks, H, (dv + DC_OC - 1) / DC_OC), dim3(128), sm3, stream, prep, P, cu_q, positions, S,

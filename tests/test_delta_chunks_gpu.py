@@ -150,3 +150,33 @@ def test_what_is_no_number_does_not_reach_the_tokens_before_it(where, bad, monke
     assert not got[bad][reached].isfinite().any()
     if where == "q":
         assert torch.equal(got[bad + 1:], clean[bad + 1:])
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), 3e38])
+@pytest.mark.parametrize("d,row,col", [(128, 0, 0), (128, 127, 15), (68, 66, 9)])
+def test_an_infinity_in_the_memory_stays_in_its_column(value, d, row, col, monkeypatch):
+    """A column of the memory that holds an infinity (or a number whose parts for the tensor cores are none): the column's outputs are
+    what float32 arithmetic makes of it, and the other columns stay what they are, bit for bit."""
+    from pico_vllm_b200 import ops
+    monkeypatch.setattr(ops, "delta_chunks_take", lambda *a: True)
+    T, dv = 70, 20
+    g = torch.Generator().manual_seed(d + row)
+    cu, pos, slots = (t.to(DEV) for t in _segments([T]))
+    q, k = (torch.nn.functional.normalize(torch.randn(T, 1, d, generator=g), dim=-1) for _ in range(2))
+    v, ab, state = torch.randn(T, dv, generator=g).to(DEV), torch.rand(T, 1, 4, generator=g), torch.randn(1, 1, dv, d, generator=g) * 0.3
+    prep = torch.cat([q.reshape(T, -1), k.reshape(T, -1), ab.reshape(T, -1), torch.zeros(T, 8)], 1).to(DEV)
+    runs = []
+    for spoil in (False, True):
+        if spoil:
+            state[0, 0, col, row] = value
+        after = state.to(DEV)
+        runs.append((ops.gated_delta_rule(prep, v, after, slots, cu, pos, 1, 1, d, dv, per_head=True, max_q_len=T), after[0, 0]))
+    others = [c for c in range(dv) if c != col]
+    (clean, clean_s), (got, got_s) = runs
+    assert torch.equal(got[:, others], clean[:, others]) and torch.equal(got_s[others], clean_s[others])
+    if value == 3e38:      # the memory fades: finite, and of the size that the recurrence gives in float64
+        want = _oracle(q, k, v.cpu().view(T, 1, dv), ab[:, :, 0], ab[:, :, 1], state, slots.cpu(), cu.cpu(), pos.cpu())
+        for a, b in ((got[:, col].cpu(), want[0][:, 0, col]), (got_s[col].cpu(), want[1][0, 0, col])):
+            assert a.isfinite().all() and (a.double() - b).abs().max() <= 2e-5 * b.abs().max()
+    else:
+        assert not got[:, col].isfinite().any() and not got_s[col].isfinite().any()
