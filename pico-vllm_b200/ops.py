@@ -5,8 +5,8 @@ take with a :class:`KernelError`, and launches on torch's current CUDA stream.  
 loaded (and, if needed, compiled) at the first call.  There is no CPU path: tensors on another
 device are refused.
 
-Matrix products go to the library (``torch.mm``, cuBLAS), as in the reference, whose
-projections are ``nn.Linear`` (pico_vllm/model.py:147-152, 309-312); everything else on the
+Matrix products that no kernel of ``csrc/`` does faster go to the library (``torch.mm``, cuBLAS), as in
+the reference, whose projections are ``nn.Linear`` (pico_vllm/model.py:147-152, 309-312); everything else on the
 forward path is a kernel of ``csrc/``.
 """
 from __future__ import annotations
@@ -80,6 +80,9 @@ def library():
         "pico_map_rope_store": [vp, i32, i32, i32, i32, vp, vp, i32, f32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp],
         "pico_map_difference": [vp, vp, i32, f32, f32, f32, vp, i32, i32, i32, i32, i32, vp],
         "pico_tp_status": [vp],
+        "pico_gemm_f32": [vp, i64, vp, vp, vp, i32, i32, i32, vp],
+        "pico_gemm_f32_parts": [i32, i32, i32],
+        "pico_tf_status": [vp],
         "pico_sample": [vp, i32, i32, i32, vp, vp, vp, vp, vp],
         "pico_post_add_norm": [vp, vp, vp, i32, f32, vp, i32, f32, vp, vp, i32, i32, i32, i32, i32, vp],
         "pico_scale_softcap": [vp, i32, i32, i32, f32, f32, vp],
@@ -808,8 +811,49 @@ def linear_bias(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, bias_
     raise KernelError(f"linear_bias: activations {x.dtype} with weights {weight.dtype} is not supported")
 
 
+# float32 products on the tensor cores (csrc/gemm_f32_tcgen05.cu) where they are faster than the library's; us here / there:
+# 17 tokens 1,536 x 1,536 15 / 25, 1,024 x 1,024 13.3 / 13.2, 1,024 x 512 12.1 / 9.1; 17 and 33 x 32,000 x 1,024 (250 tiles of w, almost two rounds of
+# the multiprocessors) 69 / 56 and 69 / 86; 340 x 128 and 512 x 1,024 16 / 14.7 and 17 / 21; 340 x 2,048 x 1,536 29 / 64; 2,048 x 17,920 x 1,536
+# 868 / 1,834; 128 x 1,536 x 8,960 39 / 166.  Root mean square of the error against float64, from 17 tokens and 256 columns on over 330 shapes:
+# 2.0e-7 to 2.9e-7, the library's 2.1e-7 to 1.7e-6, never less; for fewer tokens the library's can be smaller (1.2e-7), so they stay there.
+F32_MIN_TOKENS, F32_MIN_OUT, F32_MIN_IN, F32_FEW_TOKENS = 17, 512, 1024, 32
+
+
+def f32_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    (M, K), N = x.shape, weight.shape[0]
+    if not (M >= F32_MIN_TOKENS and N >= F32_MIN_OUT and K >= F32_MIN_IN and x.dtype == weight.dtype == torch.float32 and x.is_cuda):
+        return False
+    if M <= F32_FEW_TOKENS and -(-N // 128) > torch.cuda.get_device_properties(x.device).multi_processor_count:
+        return False
+    return (K % 4 == 0 and N % 4 == 0 and x.stride(1) == 1 and x.stride(0) >= K and x.stride(0) % 4 == 0 and weight.is_contiguous()
+            and (x.data_ptr() | weight.data_ptr()) % 16 == 0 and M <= 65535 * 128)
+
+
+def linear_f32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """x [T, K] times weight[N, K] transposed, float32, each product as three tf32 products of its factors' parts: no further from
+    float64 than float32 multiply-adds."""
+    _cuda(x, weight)
+    (M, K), N = x.shape, weight.shape[0]
+    if x.dtype != torch.float32 or weight.dtype != torch.float32 or weight.shape[1] != K or not weight.is_contiguous() or x.stride(1) != 1:
+        raise KernelError("linear_f32: float32 rows and contiguous float32 weights")
+    parts = library().pico_gemm_f32_parts(M, N, K)
+    out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    scratch = torch.empty(parts * M * N, dtype=torch.float32, device=x.device) if parts > 1 else None
+    _check(library().pico_gemm_f32(_ptr(x), x.stride(0), _ptr(weight), _ptr(out), _ptr(scratch), M, N, K, _stream()), "linear_f32")
+    _count(2 if parts > 1 else 1)
+    return out
+
+
+def tf_status() -> int:
+    """0, or 1 when the float32 product kernel gave up waiting on a barrier since the library was loaded."""
+    out = ctypes.c_int(0)
+    library().pico_tf_status(ctypes.addressof(out))
+    return out.value
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """x [T, K] times weight[N, K] transposed, a library matrix product (cuBLAS through torch).
+    """x [T, K] times weight[N, K] transposed: a library matrix product (cuBLAS through torch), or for float32
+    :func:`linear_f32` where it takes the sizes.
 
     A weight kept in float32 beside bfloat16 activations is multiplied in float32 and the result
     rounded to bfloat16.  float32 products never use a reduced-precision (TF32) mode.
@@ -817,6 +861,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
     _cuda(x, weight)
     if x.dtype == weight.dtype:
         if out is None:
+            if f32_takes(x, weight):
+                return linear_f32(x, weight)
             return torch.mm(x, weight.t())
         return torch.mm(x, weight.t(), out=out)
     if weight.dtype == torch.float32 and x.dtype == torch.bfloat16:
