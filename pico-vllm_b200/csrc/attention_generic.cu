@@ -15,6 +15,7 @@
 #include <type_traits>
 
 #define ATT_MAX_HD 640         // widest head
+#define ATT_WHOLE (-1.0f)      // as a part's denominator: the row is finished
 #define ATT_NOALLOC_MAX_HD 256 // ... that the entry point without allocation takes
 
 // One key/value head's tile: what a block works on.  A tile is up to RT rows, a row being (token, query head of the
@@ -58,7 +59,7 @@ __device__ __forceinline__ void fma2(float2& d, float2 a, float2 b) {
 __device__ __forceinline__ float part_factor(float m, float l, float M) { return m == -INFINITY ? l : expf(m - M); }
 
 struct TileArgs {
-    int q_row_stride, table_stride, T, nh, nkv, hd, page_size, window, n_splits, chunk, bq, row_chunks;
+    int q_row_stride, table_stride, T, nh, nkv, hd, page_size, window, n_splits, chunk, bq, row_chunks, part_keys;
     float scale, softcap;
     const int *tok_seg, *positions, *block_table;
     const float *slopes, *sinks, *rates;
@@ -75,8 +76,9 @@ __global__ void __launch_bounds__(128) paged_attention_tiled_kernel(const T* __r
     constexpr int KT = tile_keys(NJ, RT), KL = KT / 8, VEC = 16 / (int)sizeof(T);
     constexpr bool SHARED = RT == 32;                      // the four warps share the key tiles
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t0 = a.T - 1 - (int)(blockIdx.x / a.row_chunks);       // the tokens late in a prompt, which see the most keys, first
-    const int kh = blockIdx.y, rc = blockIdx.x % a.row_chunks, sp = blockIdx.z;
+    // the tokens late in a prompt, which see the most keys, first; the parts of a run side by side
+    const int sp = (int)(blockIdx.x % a.n_splits), chunk_at = (int)(blockIdx.x / a.n_splits);
+    const int t0 = a.T - 1 - chunk_at / a.row_chunks, kh = blockIdx.y, rc = chunk_at % a.row_chunks;
     const int g = a.nh / a.nkv, hd = a.hd, ld = hd + 4;
     const int seg = a.tok_seg[t0], pos0 = a.positions[t0];
     const int in_group = t0 % a.bq;
@@ -104,7 +106,11 @@ __global__ void __launch_bounds__(128) paged_attention_tiled_kernel(const T* __r
     };
     // the run's keys [lo, hi), and this split's part of them in whole tiles counted from lo
     const int lo = sees(0).x, hi = sees(nrows - 1).y;
-    const int tiles = (hi - lo + KT - 1) / KT, per = (tiles + a.n_splits - 1) / a.n_splits;
+    // a run with few keys is cut into fewer parts than n_splits, and one that stays whole is finished here
+    const int parts = a.part_keys > 0 ? max(1, min(a.n_splits, (hi - lo) / a.part_keys)) : a.n_splits;
+    if (sp >= parts) return;
+    const bool whole = parts == 1;
+    const int tiles = (hi - lo + KT - 1) / KT, per = (tiles + parts - 1) / parts;
     const int begin = lo + sp * per * KT, end = min(begin + per * KT, hi);
     const int step = SHARED ? KT : 4 * KT, first = SHARED ? begin : begin + warp * KT;
     const int* table = a.block_table + (size_t)seg * a.table_stride;
@@ -299,7 +305,7 @@ __global__ void __launch_bounds__(128) paged_attention_tiled_kernel(const T* __r
 #pragma unroll
         for (int w = 0; w < PARTS; ++w) M = fmaxf(M, ml_s[w * RT + r].x);
         // one more key of score sinks[h] with no value: it only adds to the denominator
-        const bool sink = a.sinks && a.n_splits == 1;
+        const bool sink = a.sinks && whole;
         if (sink) M = fmaxf(M, a.sinks[h]);
         float f[PARTS], L = sink ? expf(a.sinks[h] - M) : 0.f;
 #pragma unroll
@@ -308,18 +314,19 @@ __global__ void __launch_bounds__(128) paged_attention_tiled_kernel(const T* __r
             f[w] = part_factor(ml.x, ml.y, M);
             L += ml.y * f[w];
         }
-        const float inv = a.n_splits == 1 ? (L == 0.f ? 0.f : 1.0f / L) : 1.0f;
+        const float inv = whole ? (L == 0.f ? 0.f : 1.0f / L) : 1.0f;
         const size_t slot = ((size_t)tok * a.nh + h) * a.n_splits + sp;
         for (int d = lane; d < hd; d += 32) {
             float v = 0.f;
 #pragma unroll
             for (int w = 0; w < PARTS; ++w) v = fmaf(po_s[(size_t)(w * RT + r) * ld + d], f[w], v);
-            if (a.n_splits == 1) out[((size_t)tok * a.nh + h) * hd + d] = from_f32<T>(v * inv);
+            if (whole) out[((size_t)tok * a.nh + h) * hd + d] = from_f32<T>(v * inv);
             else a.part_o[slot * hd + d] = v;
         }
-        if (a.n_splits > 1 && lane == 0) {
-            a.part_ml[slot * 2] = M;
-            a.part_ml[slot * 2 + 1] = L;
+        if (a.n_splits > 1) {          // the row's first part also says what parts there are not 
+            if (lane == 0) *reinterpret_cast<float2*>(a.part_ml + slot * 2) = whole ? make_float2(0.f, ATT_WHOLE) : make_float2(M, L);
+            if (sp == 0)
+                for (int i = max(parts, 1) + lane; i < a.n_splits; i += 32) *reinterpret_cast<float2*>(a.part_ml + (slot + i) * 2) = make_float2(-INFINITY, 0.f);
         }
     }
 }
@@ -335,7 +342,7 @@ static void tile_launch(const T* q, const T* k, const T* v, T* out, TileArgs a, 
     const size_t merge = (size_t)(RT == 32 ? 1 : 4) * RT * (ld + 2) * sizeof(float);
     const size_t smem = fixed + (ring > merge ? ring : merge);
     cudaFuncSetAttribute(paged_attention_tiled_kernel<T, NJ, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    pico_launch((paged_attention_tiled_kernel<T, NJ, RT>), dim3((unsigned)a.T * a.row_chunks, a.nkv, a.n_splits), dim3(128), smem, stream, q, k, v,
+    pico_launch((paged_attention_tiled_kernel<T, NJ, RT>), dim3((unsigned)a.T * a.row_chunks * a.n_splits, a.nkv), dim3(128), smem, stream, q, k, v,
                 out, a);
 }
 
@@ -345,7 +352,7 @@ static void tile_dispatch(const T* q, const T* k, const T* v, T* out, const Tile
     // side by side over the keys, below.  At the line (1,000 tokens of 12 / 2 heads of 128: 400 blocks of 32 rows) 270 us with
     // 32 rows; 8 rows take 148 us for 700 tokens, which grows to about 300 for 1,000.
     const int g = a.nh / a.nkv, bq = 32 / g > 1 ? 32 / g : 1;
-    const bool tall = (long long)(a.T / bq) * a.nkv * a.n_splits >= 2 * pico_num_sms();
+    const bool tall = (long long)(a.T / bq) * a.nkv * (a.part_keys > 0 ? 1 : a.n_splits) >= 2 * pico_num_sms();
     if (a.hd <= 128) {
         if (tall) tile_launch<T, 1, 32>(q, k, v, out, a, stream); else tile_launch<T, 1, 8>(q, k, v, out, a, stream);
     } else if (a.hd <= 256) {
@@ -364,6 +371,7 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_o, const
     pdl_wait();
     const size_t th = blockIdx.x;  // t * nh + h
     const float* ml = part_ml + th * n_splits * 2;
+    if (ml[1] == ATT_WHOLE) return;
     float M = sinks ? sinks[th % nh] : -INFINITY;
     for (int i = 0; i < n_splits; ++i) M = fmaxf(M, ml[2 * i]);
     float L = sinks ? expf(sinks[th % nh] - M) : 0.f;
@@ -371,27 +379,31 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_o, const
     const float inv = L == 0.f ? 0.f : 1.0f / L;
     for (int d = threadIdx.x; d < hd; d += blockDim.x) {
         float acc = 0.f;
-        for (int i = 0; i < n_splits; ++i) acc += part_o[(th * n_splits + i) * hd + d] * part_factor(ml[2 * i], ml[2 * i + 1], M);
+        for (int i = 0; i < n_splits; ++i) {
+            if (ml[2 * i] == -INFINITY && ml[2 * i + 1] == 0.f) continue;      // no keys, or no such part
+            acc += part_o[(th * n_splits + i) * hd + d] * part_factor(ml[2 * i], ml[2 * i + 1], M);
+        }
         out[th * hd + d] = from_f32<T>(acc * inv);
     }
 }
 
 // q: rows of q_row_stride elements, head h at column h*hd.  out: [T, nh*hd].
 // part_o: [T*nh*n_splits*hd] floats and part_ml: [T*nh*n_splits*2] floats of scratch, needed
-// only when n_splits > 1.  block_table: [segments, table_stride] page numbers.
+// only when n_splits > 1.  part_keys > 0: a run of rows is cut into so many parts only that each has that many keys.  block_table: [segments, table_stride] page numbers.
 PICO_API int pico_paged_attention_generic(const void* q, int q_row_stride, const void* k_pages,
                                           const void* v_pages, void* out, float* part_o, float* part_ml,
                                           const int* tok_seg, const int* positions, const int* block_table,
                                           int table_stride, int T, int nh, int nkv, int hd, int page_size,
                                           int window, float scale, int n_splits, float softcap, int act_dtype,
-                                          const float* slopes, int chunk, const float* sinks, const float* rates,
+                                          const float* slopes, int chunk, const float* sinks, const float* rates, int part_keys,
                                           cudaStream_t stream) {
     if (T <= 0) return 0;
     if (hd % 16 != 0 || hd < 16 || hd > ATT_MAX_HD || (rates && !slopes)) return PICO_ERR_SIZE;
     if (nkv <= 0 || nh % nkv != 0 || n_splits < 1 || n_splits > 65535 || nkv > 65535) return PICO_ERR_SIZE;
     if (n_splits > 1 && (!part_o || !part_ml)) return PICO_ERR_SIZE;
-    if (chunk < 0) return PICO_ERR_SIZE;
-    const TileArgs a = {q_row_stride, table_stride, T, nh, nkv, hd, page_size, window, n_splits, chunk, 1, 1, scale, softcap,
+    // (blocks along x: a row's chunks of 8 rows at most, times the parts)
+    if (chunk < 0 || part_keys < 0 || (long long)T * ((nh / nkv + 7) / 8 + 1) * n_splits > 0x7fffffffLL) return PICO_ERR_SIZE;
+    const TileArgs a = {q_row_stride, table_stride, T, nh, nkv, hd, page_size, window, n_splits, chunk, 1, 1, part_keys, scale, softcap,
                         tok_seg, positions, block_table, slopes, sinks, rates, part_o, part_ml};
     if (act_dtype == PICO_F32) {
         if ((q_row_stride % 4) != 0) return PICO_ERR_ALIGN;
@@ -467,7 +479,7 @@ PICO_API int pico_paged_attention_noalloc(const void* q, int q_row_stride, const
     float* part_ml = part_o + (size_t)T * nh * n_splits * hd;
     const int rc = pico_paged_attention_generic(q, q_row_stride, k_pages, v_pages, out, part_o, part_ml, tok_seg,
                                                 positions, block_table, table_stride, T, nh, nkv, hd, page_size,
-                                                window, scale, n_splits, 0.f, act_dtype, nullptr, 0, nullptr, nullptr, stream);
+                                                window, scale, n_splits, 0.f, act_dtype, nullptr, 0, nullptr, nullptr, 0, stream);
     if (rc == PICO_ERR_SIZE) return noalloc_fail(rc, err, err_len, "a size the attention kernels do not take");
     if (rc == PICO_ERR_DTYPE) return noalloc_fail(rc, err, err_len, "act_dtype must be 0 (float32) or 1 (bfloat16)");
     if (rc == PICO_ERR_ALIGN) return noalloc_fail(rc, err, err_len, "q_row_stride must be a multiple of 4 for float32");

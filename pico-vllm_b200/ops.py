@@ -53,7 +53,7 @@ def library():
         "pico_swiglu": [vp, vp, i32, i32, i32, vp],
         "pico_rope_store": [vp, i32, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp],
         "pico_paged_attention_generic": [vp, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32,
-                                         i32, i32, f32, i32, f32, i32, vp, i32, vp, vp, vp],
+                                         i32, i32, f32, i32, f32, i32, vp, i32, vp, vp, i32, vp],
         "pico_paged_prefill_mma": [vp, i32, vp, vp, vp, vp, i32, vp, i32, vp, vp, i32, i32, i32, i32, i32, i32, f32, f32, vp, i32,
                                    vp, vp, vp],
         "pico_paged_decode_mma": [vp, i32, vp, vp, vp, vp, vp, vp, i32, vp, vp, vp, i32, i32, i32, i32, i32, i32,
@@ -279,7 +279,7 @@ def paged_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
                     n_heads: int, n_kv_heads: int, head_dim: int, page_size: int, window: Optional[int],
                     scale: float, n_splits: int = 1, scratch: Optional[torch.Tensor] = None,
                     softcap: Optional[float] = None, slopes: Optional[torch.Tensor] = None, chunk: Optional[int] = None,
-                    sinks: Optional[torch.Tensor] = None, rates: Optional[torch.Tensor] = None) -> torch.Tensor:
+                    sinks: Optional[torch.Tensor] = None, rates: Optional[torch.Tensor] = None, part_keys: int = 0) -> torch.Tensor:
     """Causal attention of every token of the batch over its request's cache pages.
     ``softcap`` c: the scaled score s becomes c * tanh(s / c) before the softmax.
     ``slopes`` float32 [n_heads]: slopes[h] * (query position - key position) is taken off head h's scores; with ``rates``
@@ -291,7 +291,7 @@ def paged_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
     tok_seg int32 [T]: row of block_table for each token; positions int32 [T]; block_table int32
     [segments, width].  The token at position p sees keys max(0, p+1-window) .. p.  n_splits > 1
     cuts each token's key range into parts that run in parallel and needs ``scratch`` (float32,
-    attention_scratch_floats elements).
+    attention_scratch_floats elements); with ``part_keys`` in no more parts than have that many keys each.
     """
     _cuda(q, k_pages, v_pages, out, tok_seg, positions, block_table, scratch)
     T = q.shape[0]
@@ -322,7 +322,7 @@ def paged_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
         _ptr(q), q.stride(0), _ptr(k_pages), _ptr(v_pages), _ptr(out), part_o, part_ml, _ptr(tok_seg),
         _ptr(positions), _ptr(block_table), block_table.stride(0), T, n_heads, n_kv_heads, head_dim, page_size,
         int(window) if window else 0, float(scale), n_splits, float(softcap) if softcap else 0.0, _dtype_code(q),
-        _ptr(slopes), int(chunk) if chunk else 0, _ptr(sinks), _ptr(rates), _stream()),
+        _ptr(slopes), int(chunk) if chunk else 0, _ptr(sinks), _ptr(rates), int(part_keys), _stream()),
         f"paged_attention (head_dim {head_dim})")
     _count(2 if n_splits > 1 else 1)
     return out

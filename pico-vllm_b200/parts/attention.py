@@ -25,12 +25,17 @@ class AttentionPlan(MixerPlan):
     splits: int = 1            # parts each single token's key range is cut into
     pair_min_keys: int = 0     # > 0: prompt attention gives every query tile two blocks, which share a tile
                                # that sees at least this many keys (two partial results per token and head in scratch)
+    run_parts: int = 0         # > 0: instead of `splits`, parts of every run of rows, portions included (the general kernel)
+    part_keys: int = 0         # > 0: but no more than have this many keys each
 
 
 MAX_MIXED_SCRATCH = 32 << 20       # float32 numbers (128 MB) that splitting the single tokens of a mixed step may ask for
 
 
 MIXED_MIN_KEYS = 1024              # longest context of the single tokens of a mixed step from which they are counted alone
+
+
+RUN_MIN_KEYS, RUN_FEW_ROWS = 640, 400      # see GQAAttention._run_parts
 
 
 DECODE_RAGGED_KEYS = 4096          # longest context from which the parts of a ragged batch need not all run at once
@@ -117,10 +122,33 @@ class GQAAttention(Part):
 
     def plan(self, shape: StepShape) -> AttentionPlan:
         splits = self._splits(shape)
+        run_parts, part_keys = self._run_parts(shape, splits)
         pair = self._pair_min_keys(shape)
-        parts = max(splits, 2) if pair > 0 else splits
+        parts = max(splits, 2) if pair > 0 else max(splits, run_parts)
         scratch = ops.attention_scratch_floats(shape.num_tokens, self.n_heads, self.head_dim, parts)
-        return AttentionPlan(key=(splits, pair), scratch_floats=scratch, splits=splits, pair_min_keys=pair)
+        return AttentionPlan(key=(splits, pair, run_parts, part_keys), scratch_floats=scratch, splits=splits, pair_min_keys=pair, run_parts=run_parts,
+                             part_keys=part_keys)
+
+    def _run_parts(self, shape: StepShape, splits: int):
+        """(parts, least keys of a part) of a float32 step with portions in which some token sees RUN_MIN_KEYS and more: there the
+        longest run of rows sets the time, a portion's rows as well as single ones.  (0, 0): as in other steps.
+        Few rows: blocks of 8 rows in up to four parts of 128 keys and more (us of the kernel, whole / in parts: 12 / 2 heads of 128, 150 tokens beside 8 of
+        700 keys 69 / 33, 100 tokens after 900 102 / 69; 4 / 1 of 256, 40 after 1,000 124 / 47; 8 / 8 of 64, 17 after 600 53 / 27).  Many: all in four
+        parts, which makes blocks of 32 rows, as long as those are no more than four a multiprocessor (12 / 2 heads: 333 after
+        400 124 / 97, 1,000 alone 270 / 199, a layer with 333 beside 7 of 777 136 / 117; 28 / 4: 500 after 1,500 833 / 658; 4 / 1 of 256: 2,048 alone
+        836 / 369; above that line 12 / 2 heads, 2,048 alone 576 / 652, 28 / 4, 1,000 alone 455 / 459).  Fewer than four query heads a key
+        head make single tokens poor rows of 32 (8 / 8: 300 tokens beside 30 of 1,000 keys 113 / 171), and shorter contexts gain nothing
+        (16 / 2 of 64: 333 beside 7 of 500 53 / 56; 4 / 1 of 256: 200 after 400 78 / 86)."""
+        portions = sum(n for n in shape.q_lens if n > 1)
+        if getattr(shape.engine, "dtype", "") != "float32" or not portions or shape.max_kv < RUN_MIN_KEYS or self.window is not None:
+            return 0, 0
+        if 4 * shape.num_tokens * self.n_heads * (self.head_dim + 2) > MAX_MIXED_SCRATCH or splits >= 4:
+            return 0, 0
+        if portions * self.n_kv_heads < RUN_FEW_ROWS:
+            return 4, 128
+        g = self.n_heads // self.n_kv_heads
+        tall = shape.num_tokens // max(1, 32 // g) * self.n_kv_heads
+        return (4, 0) if g >= 4 and 2 * shape.num_sms <= 4 * tall and tall < 4 * shape.num_sms else (0, 0)
 
     def _splits(self, shape: StepShape) -> int:
         """As :func:`decode_splits`, but where single tokens run in a kernel of their own beside the portions and the longest sees
@@ -202,7 +230,8 @@ class GQAAttention(Part):
         else:       # float32, or sizes the tensor-core kernels do not take
             ops.paged_attention(qkv, cache.k, cache.v, out, batch.tok_seg, batch.positions, gb.block_table,
                                 self.n_heads, self.n_kv_heads, self.head_dim, cache.page_size, self.window,
-                                self.scale, splits, batch.scratch)
+                                self.scale, max(splits, plan.run_parts) if plan is not None else 1, batch.scratch,
+                                part_keys=plan.part_keys if plan is not None else 0)
         if residual is not None and ops.skinny_takes(out, self.o_weight):
             ops.skinny_linear_residual(out, self.o_weight, residual)
             return None

@@ -1,4 +1,7 @@
 """Parts of the key range in steps that hold portions of prompts beside single tokens."""
+import pytest
+
+from pico_vllm_b200 import ops
 from pico_vllm_b200.config import EngineConfig
 from pico_vllm_b200.parts import GQAAttention, Rotary
 from pico_vllm_b200.parts import attention
@@ -39,3 +42,18 @@ def test_scratch_for_every_token_bounds_the_parts():
 
 def test_the_32_bit_path_still_counts_every_token():
     assert _plan([1] * 8 + [500], [3000] * 8 + [0], dtype="float32").splits == 1
+
+
+@pytest.mark.parametrize("H,G,hd,q_lens,starts,want", [
+    (12, 2, 128, [333] + [1] * 7, [0] + [777] * 7, (4, 0)), (12, 2, 128, [333], [0], (0, 0)), (12, 2, 128, [333], [306], (0, 0)),
+    (12, 2, 128, [333], [307], (4, 0)), (12, 2, 128, [199] + [1] * 8, [0] + [700] * 8, (4, 128)), (12, 2, 128, [200] + [1] * 8, [0] + [700] * 8, (4, 0)),
+    (12, 2, 128, [1479], [0], (4, 0)), (12, 2, 128, [1480], [0], (0, 0)), (8, 8, 64, [333] + [1] * 7, [0] + [777] * 7, (0, 0)),
+    (8, 8, 64, [40], [1000], (4, 128)), (4, 1, 256, [500], [500], (0, 0)), (4, 1, 256, [600], [500], (4, 0)), (12, 2, 128, [2, 1], [3000, 3000], (0, 0)),
+    (2000, 500, 128, [40], [1000], (0, 0))])
+def test_parts_of_float32_steps_with_portions(H, G, hd, q_lens, starts, want):
+    part = GQAAttention(H * hd, H, G, hd, position=Rotary(hd, 1e6))
+    shape = StepShape(num_tokens=sum(q_lens), num_segments=len(q_lens), q_lens=q_lens, starts=starts, max_kv=max(a + b for a, b in zip(q_lens, starts)),
+                      decode_only=False, num_sms=148, engine=EngineConfig(dtype="float32"))
+    plan = part.plan(shape)
+    assert (plan.run_parts, plan.part_keys) == want and plan.key == (plan.splits, 0) + want
+    assert plan.scratch_floats == ops.attention_scratch_floats(shape.num_tokens, H, hd, max(plan.splits, want[0]))
