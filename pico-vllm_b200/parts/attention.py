@@ -228,10 +228,10 @@ class GQAAttention(Part):
                                     batch.scratch, cache.k_map, cache.v_map, cache.k_map2d, cache.v_map2d,
                                     pair_min_keys)
         else:       # float32, or sizes the tensor-core kernels do not take
+            parts = {"part_keys": plan.part_keys} if plan is not None and plan.run_parts else {}
             ops.paged_attention(qkv, cache.k, cache.v, out, batch.tok_seg, batch.positions, gb.block_table,
                                 self.n_heads, self.n_kv_heads, self.head_dim, cache.page_size, self.window,
-                                self.scale, max(splits, plan.run_parts) if plan is not None else 1, batch.scratch,
-                                part_keys=plan.part_keys if plan is not None else 0)
+                                self.scale, max(splits, plan.run_parts) if plan is not None else 1, batch.scratch, **parts)
         if residual is not None and ops.skinny_takes(out, self.o_weight):
             ops.skinny_linear_residual(out, self.o_weight, residual)
             return None
