@@ -595,9 +595,10 @@ gated_delta_block_kernel(const float* __restrict__ prep, int P, const float* __r
 // hence the two products only (with all four in the chain 170 us for the tokens below), 16 columns a block, and four more warps that
 // fetch (the loads' addresses were a quarter of the instructions).
 // A layer with projections, twelve heads with d = dv = 128, 2,048 tokens in segments of 341, 682 and 1,025 / of 682 and 1,366 / 1,361 in
-// one: 236 / 275 / 176 us (the chain of the first 87); with both products on the CUDA cores, S and all operands from shared memory, 256 / 303 /
-// 201 (107); eight warps that multiply 257 / 276 / 181 (one block a multiprocessor); both products on the tensor cores 238 / 251 / 165, but
-// S is then off by 1.1e-7 of float64 where decays are strong, 0.7e-7 now and before.
+// one: 223 / 263 / 176 us (the chain of the first 87).  Before the kernel that prepares had three blocks a multiprocessor 236 / 275 / 176; then
+// with both products on the CUDA cores, S and all operands from shared memory, 256 / 303 / 201 (107).
+// Eight warps that multiply (one block a multiprocessor) took 257 / 276 / 181; both products on the tensor cores 238 / 251 / 165, but S is
+// then off by 1.1e-7 of float64 where decays are strong, 0.7e-7 now and before.
 #define DC_C 32
 #define DC_D 128                               // rows of S, keys padded with zeros
 #define DC_LD (DC_D + 4)                       // rows that lanes read side by side, 16 bytes each
@@ -636,7 +637,8 @@ __device__ __forceinline__ bool dc_find(const int* __restrict__ cu_q, const int*
 }
 
 // Grid (chunks at most, G): block (c, g) takes the heads of query/key head g.  u0 float32 [T, H * dv]: M V.
-__global__ void __launch_bounds__(256)
+template <bool THREE>
+__global__ void __launch_bounds__(256, THREE ? 3 : 2)
 delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* __restrict__ v, int v_stride, const int* __restrict__ cu_q,
                            const int* __restrict__ positions, int S, float* __restrict__ coef, float* __restrict__ u0, int H, int G,
                            int d, int dv, bool keep_v) {
@@ -648,21 +650,23 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* _
     extern __shared__ __align__(16) float dsm[];
     float* k_s = dsm;                          // [C][LD]
     float* q_s = k_s + DC_C * DC_LD;
-    float* kk = q_s + DC_C * DC_LD;            // [C][C + 1]: k_i . k_j
+    const int heads = H / G, slots = min(heads, 8), vw = heads * dv;
+    const int v_floats = keep_v ? DC_C * vw : 0;                              // the heads' values [C][heads * dv]
+    float* kk = q_s + (THREE ? max(DC_C * DC_LD, v_floats) : DC_C * DC_LD);   // [C][C + 1]: k_i . k_j
     float* qk = kk + DC_C * (DC_C + 1);        // q_i . k_j
-    const int heads = H / G, slots = min(heads, 8);
     float* l_s = qk + DC_C * (DC_C + 1);       // a head's L [C][C], then M by columns; one for each of the warps that take heads
     float* g_s = l_s + slots * DC_C * DC_C;    // [slots][C]: G
-    float* v_s = g_s + slots * DC_C;           // keep_v: [C][heads * dv]
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = blockIdx.y, vw = heads * dv;
-    if (keep_v) {                              // the heads' values, side by side in a row, on their way while M is made
+    float* v_s = THREE ? q_s : g_s + slots * DC_C;         // THREE: in the place of the queries, once they are done with
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = blockIdx.y;
+    auto fetch_v = [&]() {                     // the heads' values, side by side in a row, on their way while M is made
         for (int idx = threadIdx.x; idx < DC_C * (vw / 4); idx += 256) {
             const int j = idx / (vw / 4), c = idx % (vw / 4) * 4;
             if (j < n) dr_cp16(v_s + j * vw + c, v + (size_t)(t0 + j) * v_stride + (size_t)g * vw + c);
             else *reinterpret_cast<float4*>(v_s + j * vw + c) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         dr_commit();
-    }
+    };
+    if (!THREE && keep_v) fetch_v();
     for (int idx = threadIdx.x; idx < DC_C * (DC_D / 4); idx += 256) {
         const int i = idx / (DC_D / 4), c = idx % (DC_D / 4) * 4;
         float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), q4 = k4;
@@ -698,6 +702,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* _
         }
     }
     __syncthreads();
+    if (THREE && keep_v) fetch_v();
     for (int h0 = 0; h0 < heads; h0 += 8) {    // eight heads at a time, a warp each
         if (h0 + warp < heads) {
             const int h = g * heads + h0 + warp;
@@ -1161,11 +1166,19 @@ PICO_API int pico_gated_delta_chunks(const float* prep, const float* v, int v_st
     float* s0 = coef + (size_t)chunks * H * DC_COEF;
     float* u = s0 + (size_t)chunks * H * ((dv + 3) / 4 * 4) * DC_D;
     const int slots = H / G < 8 ? H / G : 8;
-    size_t sm1 = (size_t)(2 * DC_C * DC_LD + 2 * DC_C * (DC_C + 1) + slots * (DC_C * DC_C + DC_C)) * sizeof(float);
     const bool keep_v = (size_t)DC_C * (H / G) * dv * sizeof(float) <= 32 * 1024;
-    if (keep_v) sm1 += (size_t)DC_C * (H / G) * dv * sizeof(float);
-    cudaFuncSetAttribute(delta_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
-    pico_launch(delta_chunk_prepare_kernel, dim3(chunks, G), dim3(256), sm1, stream, prep, P, v, v_stride, cu_q, positions, S, coef, u, H, G, d, dv, keep_v);
+    // Two blocks a multiprocessor; three, with fewer registers and the values in the place of the queries, where that saves a round of them
+    // (us of the kernel / of the layer, 2,048 tokens in three segments: 6 key heads, 408 blocks, two a multiprocessor 45 / 236, three 32 / 224;
+    // 8 key heads, 544 blocks, two rounds either way, the layer 303 and 308; 1,361 tokens, 270 blocks, one round, 176 and 183).
+    const long long blocks = (long long)chunks * G, two = 2LL * pico_num_sms(), three = 3LL * pico_num_sms();
+    const long long v_floats = keep_v ? (long long)DC_C * (H / G) * dv : 0, q_floats = DC_C * DC_LD;
+    const long long other = DC_C * DC_LD + 2 * DC_C * (DC_C + 1) + slots * (DC_C * DC_C + DC_C), shared = other + (v_floats > q_floats ? v_floats : q_floats);
+    const bool crowded = keep_v && 3 * (shared * (long long)sizeof(float) + 1024) <= 228 * 1024 &&
+                         (blocks + three - 1) / three < (blocks + two - 1) / two;
+    const size_t sm1 = (size_t)(crowded ? shared : other + q_floats + v_floats) * sizeof(float);
+    auto prepare = crowded ? delta_chunk_prepare_kernel<true> : delta_chunk_prepare_kernel<false>;
+    cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
+    pico_launch(prepare, dim3(chunks, G), dim3(256), sm1, stream, prep, P, v, v_stride, cu_q, positions, S, coef, u, H, G, d, dv, keep_v);
     const dim3 grid((dv + DC_NC - 1) / DC_NC, H, S);
     size_t sm2 = (size_t)(2 * (DC_C * DC_LDT + DC_C * DC_LDM + 2 * DC_C + DC_C * DC_LDU) + DC_WARPS * 512 + DC_C * 32) * sizeof(float);
     // (one block a multiprocessor where there are enough of them: see pico_gated_delta_rule)
