@@ -400,13 +400,13 @@ def tma_status() -> int:
 def check_kernel_status() -> None:
     """Raises KernelError when a kernel gave up a bounded wait (on a TMA copy or a tensor-core barrier)
     since the library was loaded: such a block leaves its part of the result unwritten, so the
-    tokens computed since are not to be trusted.  Reads three status words from the device (a few
+    tokens computed since are not to be trusted.  Reads four status words from the device (a few
     synchronous 4-byte copies); does nothing before the library was first used."""
     if _lib is None:
         return
     bad = [name for name, word in (("paged_decode_tma (decode attention)", tma_status()),
                                    ("paged_prefill_tcgen05 (prompt attention)", tca_status()),
-                                   ("gemm_tcgen05_pair (feed-forward product)", tc_status())) if word]
+                                   ("gemm_tcgen05_pair or gemm_f32_tcgen05 (products)", tc_status())) if word]
     if bad:
         raise KernelError("a bounded wait ran out in: " + ", ".join(bad) + "; results since then are invalid")
 
@@ -689,10 +689,10 @@ def tc_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
 
 
 def tc_status() -> int:
-    """0, or 1 when the tcgen05 product kernel gave up waiting on a barrier since the library was loaded."""
+    """0, or 1 when a tcgen05 product kernel (bfloat16 or float32) gave up waiting on a barrier since the library was loaded."""
     out = ctypes.c_int(0)
     library().pico_tp_status(ctypes.addressof(out))
-    return out.value
+    return out.value or tf_status()
 
 
 TC_PAIR_MIN_TOKENS = 200      # from here on the tcgen05 path pays
@@ -824,6 +824,8 @@ def f32_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
     if not (M >= F32_MIN_TOKENS and N >= F32_MIN_OUT and K >= F32_MIN_IN and x.dtype == weight.dtype == torch.float32 and x.is_cuda):
         return False
     if M <= F32_FEW_TOKENS and -(-N // 128) > torch.cuda.get_device_properties(x.device).multi_processor_count:
+        return False
+    if x.requires_grad or weight.requires_grad:        # the library's product has a gradient
         return False
     return (K % 4 == 0 and N % 4 == 0 and x.stride(1) == 1 and x.stride(0) >= K and x.stride(0) % 4 == 0 and weight.is_contiguous()
             and (x.data_ptr() | weight.data_ptr()) % 16 == 0 and M <= 65535 * 128)

@@ -58,3 +58,13 @@ def test_which_products_go_there(M, N, K, off, takes):
     assert (ops.launches > before) == takes
     if M == 17 and takes:
         assert not ops.f32_takes(torch.ones(1, K, device=DEV).expand(M, K), w) and not ops.f32_takes(x, torch.ones(K, N, device=DEV).t())
+
+
+def test_a_product_with_a_gradient_is_the_library_s_and_a_wait_that_ran_out_is_seen(monkeypatch):
+    from pico_vllm_b200 import ops
+    x, w = torch.ones(32, 1024, device=DEV, requires_grad=True), torch.ones(512, 1024, device=DEV)
+    ops.linear(x, w).sum().backward()
+    assert bool((x.grad == 512).all())
+    assert ops.tc_status() == 0
+    monkeypatch.setattr(ops, "tf_status", lambda: 1)
+    assert ops.tc_status() == 1
