@@ -26,6 +26,8 @@
 //   RT = 32: four warps of 8 rows each share the tiles of KT keys (long prompts: a key is read once for 32 rows);
 //   RT =  8: four warps share the 8 rows and take every fourth tile of keys, their sums are added at the end (single
 //            tokens and short prompts, where blocks are few and a row's chain of keys sets the time).
+// With part_keys > 0 every run, a portion's too, goes in parts of at least so many keys, up to n_splits; a run that stays whole is written by
+// its own block and left alone by the combining kernel.  The parts of a run are neighbours in the grid: side by side and in L2 together.
 // Keys and values come in by cp.async into buffers of their own (values land while the scores are computed, the next keys
 // while the values are multiplied); scores: a lane has 2 rows x KT / 8 keys; output: a lane has 8 rows x 4 NJ dimensions,
 // probabilities pass through shared memory.  All arithmetic is float32 on the CUDA cores: with enough rows those bound it
@@ -323,7 +325,7 @@ __global__ void __launch_bounds__(128) paged_attention_tiled_kernel(const T* __r
             if (whole) out[((size_t)tok * a.nh + h) * hd + d] = from_f32<T>(v * inv);
             else a.part_o[slot * hd + d] = v;
         }
-        if (a.n_splits > 1) {          // the row's first part also says what parts there are not 
+        if (a.n_splits > 1) {          // the row's first part also says what parts there are not
             if (lane == 0) *reinterpret_cast<float2*>(a.part_ml + slot * 2) = whole ? make_float2(0.f, ATT_WHOLE) : make_float2(M, L);
             if (sp == 0)
                 for (int i = max(parts, 1) + lane; i < a.n_splits; i += 32) *reinterpret_cast<float2*>(a.part_ml + (slot + i) * 2) = make_float2(-INFINITY, 0.f);

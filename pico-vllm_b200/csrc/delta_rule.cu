@@ -599,6 +599,8 @@ gated_delta_block_kernel(const float* __restrict__ prep, int P, const float* __r
 // with both products on the CUDA cores, S and all operands from shared memory, 256 / 303 / 201 (107).
 // Eight warps that multiply (one block a multiprocessor) took 257 / 276 / 181; both products on the tensor cores 238 / 251 / 165, but S is
 // then off by 1.1e-7 of float64 where decays are strong, 0.7e-7 now and before.
+// The outputs (39 us of the first) in the chain's fetching warps, without a kernel of their own: the chain 130 instead of 87, 228 / 289 / 186;
+// with Q S on the tensor cores in their kernel 218 / 257 / 177, but one segment and 1,000 tokens 1 % slower.
 #define DC_C 32
 #define DC_D 128                               // rows of S, keys padded with zeros
 #define DC_LD (DC_D + 4)                       // rows that lanes read side by side, 16 bytes each
