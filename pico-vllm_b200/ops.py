@@ -862,11 +862,11 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
     """
     _cuda(x, weight)
     if x.dtype == weight.dtype:
-        if out is None:
-            if f32_takes(x, weight):
-                return linear_f32(x, weight)
-            return torch.mm(x, weight.t())
-        return torch.mm(x, weight.t(), out=out)
+        if out is not None:
+            return torch.mm(x, weight.t(), out=out)
+        if x.dtype == torch.float32 and f32_takes(x, weight):
+            return linear_f32(x, weight)
+        return torch.mm(x, weight.t())
     if weight.dtype == torch.float32 and x.dtype == torch.bfloat16:
         y = torch.mm(x.float(), weight.t()).to(torch.bfloat16)
         if out is not None:

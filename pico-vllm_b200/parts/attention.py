@@ -139,8 +139,10 @@ class GQAAttention(Part):
         836 / 369; above that line 12 / 2 heads, 2,048 alone 576 / 652, 28 / 4, 1,000 alone 455 / 459).  Fewer than four query heads a key
         head make single tokens poor rows of 32 (8 / 8: 300 tokens beside 30 of 1,000 keys 113 / 171), and shorter contexts gain nothing
         (16 / 2 of 64: 333 beside 7 of 500 53 / 56; 4 / 1 of 256: 200 after 400 78 / 86)."""
+        if getattr(shape.engine, "dtype", "") != "float32" or shape.max_kv < RUN_MIN_KEYS or self.window is not None:
+            return 0, 0
         portions = sum(n for n in shape.q_lens if n > 1)
-        if getattr(shape.engine, "dtype", "") != "float32" or not portions or shape.max_kv < RUN_MIN_KEYS or self.window is not None:
+        if not portions:
             return 0, 0
         if 4 * shape.num_tokens * self.n_heads * (self.head_dim + 2) > MAX_MIXED_SCRATCH or splits >= 4:
             return 0, 0
