@@ -115,12 +115,12 @@ class ModelRunner:
             self._stage = _Staging(max(n, 4096), self.device)
         return self._stage
 
-    def _plan(self, q_lens: List[int], starts: List[int], T: int, S: int):
+    def _plan(self, q_lens: List[int], starts: List[int], T: int, S: int, spare: bool = True):
         """Asks every planner for its plan of this step.  Returns (plans by plan key, a hashable key of
-        all of them, float32 elements of scratch the largest of them needs)."""
+        all of them, float32 elements of scratch the largest of them needs).  ``spare``: as in StepShape."""
         shape = StepShape(num_tokens=T, num_segments=S, q_lens=q_lens, starts=starts,
                           max_kv=max(st + n for st, n in zip(starts, q_lens)),
-                          decode_only=all(n == 1 for n in q_lens), num_sms=self._num_sms, engine=self.cfg)
+                          decode_only=all(n == 1 for n in q_lens), num_sms=self._num_sms, engine=self.cfg, spare=spare)
         plans, need = {}, 0
         for key, mixer in self._planners.items():
             plan = mixer.plan(shape)
@@ -129,12 +129,15 @@ class ModelRunner:
                 need = max(need, int(plan.scratch_floats))
         return plans, tuple((repr(k), p.key) for k, p in plans.items()), need
 
+    def _new_scratch(self, need: int) -> Optional[torch.Tensor]:
+        return torch.empty(need, dtype=torch.float32, device=self.device) if need > 0 else None
+
     def _scratch_for(self, need: int) -> Optional[torch.Tensor]:
         """The step function's float32 scratch, grown when a plan asks for more."""
         if need <= 0:
             return None
         if self._scratch is None or self._scratch.numel() < need:
-            self._scratch = torch.empty(need, dtype=torch.float32, device=self.device)
+            self._scratch = self._new_scratch(need)
         return self._scratch
 
     # ------------------------------------------------------------------ the step
@@ -298,7 +301,11 @@ class ModelRunner:
                   for gi in range(len(cache.groups))}
         if plans is None:
             plans, _, need = self._plan(q_lens, starts, T, S)
-            scratch = self._scratch_for(need)
+            try:
+                scratch = self._scratch_for(need)
+            except torch.OutOfMemoryError:     # the pages leave no room: as a step goes that asks for less
+                plans, _, need = self._plan(q_lens, starts, T, S, spare=False)
+                scratch = self._scratch_for(need)
         return Batch(num_tokens=T, num_segments=S, token_ids=d(lay.token_ids, T), positions=d(lay.positions, T),
                      tok_seg=d(lay.tok_seg, T), seg_slots=d(lay.seg_slots, S), cu_q=d(lay.cu_q, S + 1),
                      logit_rows=d(lay.logit_rows, R), num_logit_rows=R, groups=groups, q_lens=q_lens,
@@ -326,7 +333,7 @@ class ModelRunner:
         key = ("decode", B, plan_key, greedy)
         entry = self._graphs.get(key)
         if entry is None:
-            logits = self._record(key, full, starts, B, B, plans, need, greedy)
+            logits = self._record(key, full, starts, B, B, plans, self._new_scratch(need), greedy)
         else:
             self._build(full, starts, pad_to=B, buffers=entry["buffers"], scratch=entry["scratch"], plans=entry["plans"],
                         greedy=greedy)
@@ -350,7 +357,15 @@ class ModelRunner:
         key = ("prefill", T, R, plan_key, greedy)
         entry = self._graphs.get(key)
         if entry is None:
-            logits = self._record(key, items, starts, 1, R, plans, need, greedy)
+            try:
+                scratch = self._new_scratch(need)
+            except torch.OutOfMemoryError:     # the pages leave no room: as a step goes that asks for less
+                plans, plan_key, need = self._plan([T], starts, T, 1, spare=False)
+                key = ("prefill", T, R, plan_key, greedy)
+                entry = self._graphs.get(key)
+                scratch = self._new_scratch(need) if entry is None else None
+        if entry is None:
+            logits = self._record(key, items, starts, 1, R, plans, scratch, greedy)
         else:
             self._build(items, starts, pad_to=1, buffers=entry["buffers"], scratch=entry["scratch"], rows=R,
                         plans=entry["plans"], greedy=greedy)
@@ -360,14 +375,13 @@ class ModelRunner:
         self.graph_replays += 1
         return logits
 
-    def _record(self, key, items: Sequence[StepItem], starts: List[int], S: int, R: int, plans, need: int,
+    def _record(self, key, items: Sequence[StepItem], starts: List[int], S: int, R: int, plans, scratch,
                 greedy: bool = False) -> Optional[torch.Tensor]:
         """First step of a shape: a graph keeps the addresses it was recorded with, so the shape owns its
         staging buffer and its scratch."""
         T = sum(len(it.tokens) for it in items) + (S - len(items))
         lay = _Layout(T, S, R, len(self.cache.groups), self.cache.max_blocks)
         buffers = _Staging(lay.total, self.device)
-        scratch = torch.empty(need, dtype=torch.float32, device=self.device) if need > 0 else None
         batch = self._build(items, starts, pad_to=S, buffers=buffers, scratch=scratch, rows=R, plans=plans, greedy=greedy)
         return self._run_and_record(key, batch, {"buffers": buffers, "scratch": scratch, "plans": plans})
 

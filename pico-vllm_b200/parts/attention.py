@@ -144,7 +144,7 @@ class GQAAttention(Part):
         portions = sum(n for n in shape.q_lens if n > 1)
         if not portions:
             return 0, 0
-        if 4 * shape.num_tokens * self.n_heads * (self.head_dim + 2) > MAX_MIXED_SCRATCH or splits >= 4:
+        if 4 * shape.num_tokens * self.n_heads * (self.head_dim + 2) > MAX_MIXED_SCRATCH or splits >= 4 or not shape.spare:
             return 0, 0
         if portions * self.n_kv_heads < RUN_FEW_ROWS:
             return 4, 128

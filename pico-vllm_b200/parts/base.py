@@ -129,6 +129,7 @@ class StepShape:
     decode_only: bool
     num_sms: int                     # multiprocessors of the device (1 off the GPU)
     engine: object = None            # the EngineConfig (dtype, knobs a mixer may read by name)
+    spare: bool = True               # False: the device had no room for the scratch of the plan made first
 
 
 @dataclass(frozen=True)

@@ -1,5 +1,6 @@
 """Parts of the key range in steps that hold portions of prompts beside single tokens."""
 import pytest
+import torch
 
 from pico_vllm_b200 import ops
 from pico_vllm_b200.config import EngineConfig
@@ -57,3 +58,32 @@ def test_parts_of_float32_steps_with_portions(H, G, hd, q_lens, starts, want):
     plan = part.plan(shape)
     assert (plan.run_parts, plan.part_keys) == want and plan.key == (plan.splits, 0) + want
     assert plan.scratch_floats == ops.attention_scratch_floats(shape.num_tokens, H, hd, max(plan.splits, want[0]))
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_a_float32_step_without_room_for_its_parts_goes_without_them(graph, monkeypatch):
+    """The device's pages leave no room: the allocator's own error leads to the plan that needs no scratch, and a full portion is recorded with it."""
+    import helpers
+    from pico_vllm_b200.engine import StepItem
+    import fake_ops
+    fake_ops.install(monkeypatch)
+    runner, _ = helpers.make_runner_from_tensors("a", "float32", "cpu", 2048)
+    monkeypatch.setattr(GQAAttention, "_run_parts", lambda self, shape, splits: (4, 128) if shape.spare else (0, 0))
+    slot = runner.cache.acquire("x")
+    item, plans = StepItem(slot, helpers.random_ids(700, 256, 5), (699,)), []
+    if graph:
+        monkeypatch.setattr(runner, "on_gpu", True)
+        monkeypatch.setattr(runner.cfg, "use_cuda_graph", True)
+        runner._graph_prefill_tokens = 700
+        monkeypatch.setattr(runner, "_run_and_record", lambda key, batch, entry: (runner._graphs.setdefault(key, entry), plans.append((batch.plans, batch.scratch))))
+    else:
+        forward = runner.model.forward
+        monkeypatch.setattr(runner.model, "forward", lambda batch, views: (plans.append((batch.plans, batch.scratch)), forward(batch, views))[1])
+
+    def full(need):
+        if need > 0:
+            raise torch.OutOfMemoryError("no room")
+    monkeypatch.setattr(runner, "_new_scratch", full)
+    runner.step([item])
+    (plan,), scratch = plans[0][0].values(), plans[0][1]
+    assert plan.run_parts == 0 and plan.scratch_floats == 0 and scratch is None
