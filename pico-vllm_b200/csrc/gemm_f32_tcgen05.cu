@@ -108,7 +108,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_
     pdl_launch_dependents();
     extern __shared__ unsigned char tf_dyn[];
     unsigned char* smem = tf_dyn + ((1024u - (tf_u32(tf_dyn) & 1023u)) & 1023u);
-    __shared__ uint64_t full[TF_STAGES], split[TF_STAGES], empty[TF_STAGES], sum_full[2], sum_empty[2];
+    __shared__ uint64_t full[TF_STAGES], split[TF_STAGES], empty[TF_STAGES], sum_full[2], sum_empty[2], done;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_s;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -124,6 +124,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_
             tf_init(sum_full + i, 1);
             tf_init(sum_empty + i, TF_WORKERS);
         }
+        tf_init(&done, 1);
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -144,18 +145,16 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_
             for (; kb < nk; ++kb) {
                 const int s = kb % TF_STAGES;
                 if (kb >= TF_STAGES && !tf_wait(empty + s, ((kb / TF_STAGES) - 1) & 1, &abort_s)) break;
-                if (abort_s) break;
                 unsigned char* dst = smem + s * 2 * TF_HALF;
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(tf_u32(full + s)), "r"(bytes) : "memory");
                 tf_load(dst, &w_map, (kb0 + kb) * TF_BK, n0, full + s);
                 tf_load(dst + TF_BM * TF_BK * 4, &x_map, (kb0 + kb) * TF_BK, t0, full + s);
             }
-            // copies that nobody waits for any more, after an error, still land before the block leaves
-            if (abort_s)
-                for (int i = kb > TF_STAGES ? kb - TF_STAGES : 0; i < kb; ++i) {
-                    volatile int never = 0;
-                    tf_wait(full + i % TF_STAGES, (i / TF_STAGES) & 1, &never);
-                }
+            // the last copies land before the block leaves, also where an error comes after the last of them was asked for
+            for (int i = kb > TF_STAGES ? kb - TF_STAGES : 0; i < kb; ++i) {
+                volatile int never = 0;
+                tf_wait(full + i % TF_STAGES, (i / TF_STAGES) & 1, &never);
+            }
         }
     } else if (warp == 1) {
         if (lane == 0) {
@@ -176,6 +175,10 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_
                 tf_commit(empty + s);
                 if (within == TF_GROUP - 1 || kb == nk - 1) tf_commit(sum_full + buf);
             }
+            // products that nobody waits for any more, after an error, end before the tensor memory is given back
+            volatile int never = 0;
+            tf_commit(&done);
+            tf_wait(&done, 0, &never);
         }
     } else {
         // a worker drains tensor-memory lanes 32 (warp % 4) .. (rows of w) at half of the tokens
