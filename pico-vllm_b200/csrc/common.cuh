@@ -65,6 +65,19 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
     return scratch[32];
 }
 
+// A float32 number as the sum of three bfloat16 numbers of eight digits each, nothing left over: a is x without its low 16 bits, b what that
+// leaves without its low 16 bits, c the rest; both subtractions are exact (below 2^-110 the last bits may be smaller than any bfloat16 number,
+// 2^-133, and are lost; an infinity's parts are no numbers).  For two numbers, their parts side by side as the tensor cores read them.
+__device__ __forceinline__ void pico_split3(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
+    const uint32_t xa = __float_as_uint(x) & 0xffff0000u, ya = __float_as_uint(y) & 0xffff0000u;
+    const float xr = __fsub_rn(x, __uint_as_float(xa)), yr = __fsub_rn(y, __uint_as_float(ya));
+    const uint32_t xb = __float_as_uint(xr) & 0xffff0000u, yb = __float_as_uint(yr) & 0xffff0000u;
+    const float xc = __fsub_rn(xr, __uint_as_float(xb)), yc = __fsub_rn(yr, __uint_as_float(yb));
+    a = __byte_perm(xa, ya, 0x7632);
+    b = __byte_perm(xb, yb, 0x7632);
+    c = __byte_perm(__float_as_uint(xc), __float_as_uint(yc), 0x7632);
+}
+
 // An attention score in log2 units (the softmax uses exp2): raw * scale_log2, or, with a soft cap c on the scaled score,
 // c * tanh(raw * scale / c) in the same units.  cap_log2 = c * log2(e) (0: no cap); cap_2x = 2 * scale / c.
 // tanh(x) = 1 - 2 / (e^(2x) + 1): exact at both ends, absolute error ~1e-7 near 0.

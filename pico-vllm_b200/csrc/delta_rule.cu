@@ -594,13 +594,13 @@ gated_delta_block_kernel(const float* __restrict__ prep, int P, const float* __r
 // The chain is bound by the instructions that its warps issue one after the other, over len / 32 dependent steps of the longest segment:
 // hence the two products only (with all four in the chain 170 us for the tokens below), 16 columns a block, and four more warps that
 // fetch (the loads' addresses were a quarter of the instructions).
-// A layer with projections, twelve heads with d = dv = 128, 2,048 tokens in segments of 341, 682 and 1,025 / of 682 and 1,366 / 1,361 in
-// one: 223 / 263 / 176 us (the chain of the first 87).  Before the kernel that prepares had three blocks a multiprocessor 236 / 275 / 176; then
-// with both products on the CUDA cores, S and all operands from shared memory, 256 / 303 / 201 (107).
-// Eight warps that multiply (one block a multiprocessor) took 257 / 276 / 181; both products on the tensor cores 238 / 251 / 165, but S is
-// then off by 1.1e-7 of float64 where decays are strong, 0.7e-7 now and before.
-// The outputs (39 us of the first) in the chain's fetching warps, without a kernel of their own: the chain 130 instead of 87, 228 / 289 / 186;
-// with Q S on the tensor cores in their kernel 218 / 257 / 177, but one segment and 1,000 tokens 1 % slower.
+// A layer with projections, twelve heads with d = dv = 128, 2,048 tokens in segments of 341, 682 and 1,025 / of 682 and 1,366 / in one / 1,361 in
+// one: 235 / 273 / 267 / 193 us; with both products on the CUDA cores, S and all operands from shared memory, 265 / 311 / 307 / 215.
+// With two tf32 numbers for a factor, which leave out a unit of its last place, 234 / 273 / 261 / 191; root mean square of S's error against
+// float64, relative, without decay 3.60e-7, now 3.54e-7, on the CUDA cores 3.57e-7 (keys of one place 1.135e-7 / 1.129e-7 / 1.129e-7).
+// Eight warps that multiply (one block a multiprocessor) were 5 to 20 us slower; both products on the tensor cores left S
+// off by 1.1e-7 instead of 0.7e-7 where decays are strong.  The outputs in the chain's fetching warps, without a kernel of their own, lengthened
+// the chain by half.
 #define DC_C 32
 #define DC_D 128                               // rows of S, keys padded with zeros
 #define DC_LD (DC_D + 4)                       // rows that lanes read side by side, 16 bytes each
@@ -820,29 +820,28 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const float* _
     }
 }
 
-// A float32 number as two of tf32's eleven digits each: what is left over is below half a unit of its last place.
-__device__ __forceinline__ void dc_split(float x, uint32_t& hi, uint32_t& lo) {
-    // Dekker's splitting, each operation rounded by itself (the conversion instruction is a sixteenth of the rate)
-    const float c = __fmul_rn(8193.f, x), h = __fsub_rn(c, __fsub_rn(c, x));
-    hi = __float_as_uint(h);
-    lo = __float_as_uint(__fsub_rn(x, h));
-}
-__device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+__device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// c += a b with both in two parts (the product of the two small parts is below what float32 keeps).  The tensor cores
-// cut sums off where float32 rounds them: the large parts' products leave them after eight terms.  The small parts' sums are kept apart,
-// as an instruction that adds into the registers of the one before waits 23 clocks for it (one can be issued every 8).
-__device__ __forceinline__ void dc_mma3(float (&c)[3][4], const uint32_t (&ah)[4], const uint32_t (&al)[4], float b0, float b1) {
-    uint32_t h0, l0, h1, l1;
-    dc_split(b0, h0, l0);
-    dc_split(b1, h1, l1);
+// c += a b over sixteen places with both in their three parts (pico_split3), in eight products of the nine: the one of the two smallest parts is
+// below 2^-30 of a b.  The tensor cores cut sums off where float32 rounds them: the large parts' products leave them after one instruction.
+// The others' sums, below 2^-6 of those, are kept in two, as an instruction that adds into the registers of the one before waits 23 clocks for it
+// (one can be issued every 8).
+__device__ __forceinline__ void dc_mma8(float (&c)[3][4], const uint32_t (&a)[3][4], const float2& b0, const float2& b1) {
+    uint32_t b[3][2];
+    pico_split3(b0.x, b0.y, b[0][0], b[1][0], b[2][0]);
+    pico_split3(b1.x, b1.y, b[0][1], b[1][1], b[2][1]);
     float big[4] = {};
-    dc_mma(big, ah, h0, h1);
-    dc_mma(c[1], al, h0, h1);
-    dc_mma(c[2], ah, l0, l1);
+    dc_mma(big, a[0], b[0]);
+    dc_mma(c[1], a[1], b[2]);
+    dc_mma(c[2], a[2], b[1]);
+    dc_mma(c[1], a[0], b[2]);
+    dc_mma(c[2], a[2], b[0]);
+    dc_mma(c[1], a[1], b[1]);
+    dc_mma(c[2], a[1], b[0]);
+    dc_mma(c[1], a[0], b[1]);
 #pragma unroll
     for (int e = 0; e < 4; ++e) c[0][e] += big[e];
 }
@@ -850,13 +849,13 @@ __device__ __forceinline__ void dc_sum3(float (&c)[4], const float (&p)[3][4]) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) c[e] = p[0][e] + (p[1][e] + p[2][e]);
 }
-// The numbers that a lane holds of a product's result, rows r and r + 8 at places 2 j and 2 j + 1, as the rows' operand of a product over
-// those places (dealt to the lanes in the order 0, 2, 4, 6, 1, 3, 5, 7, which the other operand follows).
-__device__ __forceinline__ void dc_rows(const float (&c)[4], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
-    dc_split(c[0], hi[0], lo[0]);
-    dc_split(c[2], hi[1], lo[1]);
-    dc_split(c[1], hi[2], lo[2]);
-    dc_split(c[3], hi[3], lo[3]);
+// The numbers that a lane holds of two neighbouring results of products, rows r and r + 8 at places 2 j and 2 j + 1 of each, as the rows' operand of a
+// product over those sixteen places.
+__device__ __forceinline__ void dc_rows(const float (&c)[4], const float (&d)[4], uint32_t (&a)[3][4]) {
+    pico_split3(c[0], c[1], a[0][0], a[1][0], a[2][0]);
+    pico_split3(c[2], c[3], a[0][1], a[1][1], a[2][1]);
+    pico_split3(d[0], d[1], a[0][2], a[1][2], a[2][2]);
+    pico_split3(d[2], d[3], a[0][3], a[1][3], a[2][3]);
 }
 __device__ __forceinline__ bool dc_no_number(const float (&c)[4][4]) {
     bool no = false;
@@ -872,8 +871,8 @@ __device__ __forceinline__ bool dc_no_number(const float (&c)[4][4]) {
 // of S, which never goes through shared memory.  The warps' four parts are added through shared memory, each warp makes U for eight tokens,
 // and all of them their own rows of S', in float32 on the CUDA cores.  u: M V on the way in, U on the way out; s0 float32 [chunks, H, dv
 // rounded up to 4, 128]: S before each chunk, by columns.
-// The product with S is three tf32 products, eight terms at a time.  Where a result is no number, plain float32 products decide what it
-// is (the parts of an infinity are no infinity's parts).
+// The product with S is eight products of bfloat16 parts that leave nothing of a factor out, sixteen terms at a time.  Where a result is no number,
+// plain float32 products decide what it is (the parts of an infinity are no infinity's parts).
 #define DC_LDM (DC_D + 8)                      // rows of M diag(G) K: eight read side by side, 8 bytes a lane
 #define DC_LDT (DC_D + 4)                      // rows of K: pairs of rows, 4 bytes a lane
 #define DC_LDU (DC_NC + 4)
@@ -956,13 +955,13 @@ delta_chunk_kernel(const float* __restrict__ prep, int P, float* __restrict__ st
                 if (col_base + r + 8 * c < dv) *reinterpret_cast<float2*>(s_out + c * 8 * DC_D + 8 * nt) = make_float2(S[nt][2 * c], S[nt][2 * c + 1]);
         float x[4][4], x3[4][3][4] = {};       // [tile of tokens]: columns r, r + 8, tokens 8 tt + 2 j and the next
 #pragma unroll
-        for (int nt = 0; nt < DC_ROWS / 8; ++nt) {
-            uint32_t ah[4], al[4];
-            dc_rows(S[nt], ah, al);
+        for (int nt = 0; nt < DC_ROWS / 8; nt += 2) {
+            uint32_t a[3][4];
+            dc_rows(S[nt], S[nt + 1], a);
 #pragma unroll
             for (int tt = 0; tt < 4; ++tt) {
-                const float2 b = *reinterpret_cast<const float2*>(m_s + (8 * tt + r) * DC_LDM + 8 * nt);
-                dc_mma3(x3[tt], ah, al, b.x, b.y);
+                const float* b = m_s + (8 * tt + r) * DC_LDM + 8 * nt;
+                dc_mma8(x3[tt], a, *reinterpret_cast<const float2*>(b), *reinterpret_cast<const float2*>(b + 8));
             }
         }
 #pragma unroll

@@ -180,3 +180,23 @@ def test_an_infinity_in_the_memory_stays_in_its_column(value, d, row, col, monke
             assert a.isfinite().all() and (a.double() - b).abs().max() <= 2e-5 * b.abs().max()
     else:
         assert not got[:, col].isfinite().any() and not got_s[col].isfinite().any()
+
+
+@pytest.mark.parametrize("d,dv,T", [(128, 128, 128), (68, 20, 65)])
+def test_what_is_held_under_a_key_is_taken_off_to_the_last_bit(d, dv, T, monkeypatch):
+    """Keys that are one place each, all different, without decay, written with nought at full strength: every product with the memory selects a
+    row of it, which is nought afterwards, and the rows of no key stay what they are."""
+    from pico_vllm_b200 import ops
+    monkeypatch.setattr(ops, "delta_chunks_take", lambda *a: True)
+    g = torch.Generator().manual_seed(T)
+    cu, pos, slots = (t.to(DEV) for t in _segments([T]))
+    at = torch.randperm(d, generator=g)[:T]
+    k = torch.nn.functional.one_hot(at, d).float()
+    state = torch.randn(1, 2, dv, d, generator=g)
+    ab = torch.ones(T, 2, 4)
+    prep = torch.cat([torch.randn(T, d, generator=g), k, ab.reshape(T, -1), torch.zeros(T, 8)], 1).to(DEV)
+    after = state.to(DEV)
+    ops.gated_delta_rule(prep, torch.zeros(T, 2 * dv, device=DEV), after, slots, cu, pos, 2, 1, d, dv, per_head=True, max_q_len=T)
+    want = state.clone()
+    want[..., at] = 0
+    assert torch.equal(after.cpu(), want)
