@@ -24,7 +24,7 @@ def canonical_dtype(name: str) -> str:
 
 @dataclass
 class EngineConfig:
-    dtype: str = "bfloat16"            # "bfloat16": serving kernels; "float32": everything in true 32-bit
+    dtype: str = "bfloat16"            # "bfloat16": serving kernels; "float32": 32-bit numbers throughout, whole in every product
     page_size: int = 16                # tokens per cache page (pico_vllm/model.py:33)
     num_pages: Optional[int] = None    # pages per layer group; None = sized from max_cache_tokens
     max_cache_tokens: Optional[int] = None  # tokens the pool must hold when num_pages is None

@@ -21,7 +21,7 @@ TORCH_DTYPES = {"bfloat16": torch.bfloat16, "float32": torch.float32}
 
 
 def _prepare_precision(dtype: str) -> None:
-    # float32 matrix products must be true float32: no TF32, no reduced-precision reductions
+    # float32 matrix products take all digits of their factors: the library no TF32 and no reduced-precision reductions (ops.linear_f32: all parts)
     torch.backends.cuda.matmul.allow_tf32 = False
     torch.backends.cudnn.allow_tf32 = False
     torch.set_float32_matmul_precision("highest")

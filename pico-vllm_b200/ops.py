@@ -814,8 +814,9 @@ def linear_bias(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, bias_
 # float32 products on the tensor cores (csrc/gemm_f32_tcgen05.cu) where they are faster than the library's; us here / there:
 # 17 tokens 1,536 x 1,536 15 / 25, 1,024 x 1,024 13.3 / 13.2, 1,024 x 512 12.1 / 9.1; 17 and 33 x 32,000 x 1,024 (250 tiles of w, almost two rounds of
 # the multiprocessors) 69 / 56 and 69 / 86; 340 x 128 and 512 x 1,024 16 / 14.7 and 17 / 21; 340 x 2,048 x 1,536 29 / 64; 2,048 x 17,920 x 1,536
-# 868 / 1,834; 128 x 1,536 x 8,960 39 / 166.  Root mean square of the error against float64, from 17 tokens and 256 columns on over 330 shapes:
-# 2.0e-7 to 2.9e-7, the library's 2.1e-7 to 1.7e-6, never less; for fewer tokens the library's can be smaller (1.2e-7), so they stay there.
+# 868 / 1,834; 128 x 1,536 x 8,960 39 / 166.  Root mean square of the error against float64, relative, 17 to 2,048 tokens and 1,024 to 8,960 columns, here /
+# there: normal numbers 1.0e-7 to 1.2e-7 / 2.7e-7 to 1.7e-6, all of one sign 0.9e-7 to 1.5e-7 / 1.1e-7 to 1.3e-6, four terms a row 2.7e-8 / 4.3e-8 to
+# 4.7e-8, one 2.5e-8 / 2.5e-8; for fewer tokens the library's can be smaller, so they stay there.
 F32_MIN_TOKENS, F32_MIN_OUT, F32_MIN_IN, F32_FEW_TOKENS = 17, 512, 1024, 32
 
 
@@ -832,15 +833,15 @@ def f32_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
 
 
 def linear_f32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """x [T, K] times weight[N, K] transposed, float32, each product as three tf32 products of its factors' parts: no further from
-    float64 than float32 multiply-adds."""
+    """x [T, K] times weight[N, K] transposed, float32, on the tensor cores: every factor whole, as three bfloat16 parts
+    (csrc/gemm_f32_tcgen05.cu), sums in float32."""
     _cuda(x, weight)
     (M, K), N = x.shape, weight.shape[0]
     if x.dtype != torch.float32 or weight.dtype != torch.float32 or weight.shape[1] != K or not weight.is_contiguous() or x.stride(1) != 1:
         raise KernelError("linear_f32: float32 rows and contiguous float32 weights")
     parts = library().pico_gemm_f32_parts(M, N, K)
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    scratch = torch.empty(parts * M * N, dtype=torch.float32, device=x.device) if parts > 1 else None
+    scratch = torch.empty(2 * parts * M * N, dtype=torch.float32, device=x.device) if parts > 1 else None
     _check(library().pico_gemm_f32(_ptr(x), x.stride(0), _ptr(weight), _ptr(out), _ptr(scratch), M, N, K, _stream()), "linear_f32")
     _count(2 if parts > 1 else 1)
     return out
@@ -858,7 +859,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
     :func:`linear_f32` where it takes the sizes.
 
     A weight kept in float32 beside bfloat16 activations is multiplied in float32 and the result
-    rounded to bfloat16.  float32 products never use a reduced-precision (TF32) mode.
+    rounded to bfloat16.  float32 products take all digits of their factors, here and in the library (TF32 is off).
     """
     _cuda(x, weight)
     if x.dtype == weight.dtype:

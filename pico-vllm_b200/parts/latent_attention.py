@@ -52,7 +52,7 @@ def _round_up(n: int, m: int) -> int:
 
 
 def _linear(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """A handful of tokens: the weight-streaming kernel; more: the library product."""
+    """A handful of tokens: the weight-streaming kernel; more: :func:`ops.linear`."""
     if ops.skinny_takes(x, weight):
         return ops.skinny_linear(x, weight)
     return ops.linear(x, weight)
