@@ -325,10 +325,16 @@ __global__ void __launch_bounds__(128) paged_attention_tiled_kernel(const T* __r
             if (whole) out[((size_t)tok * a.nh + h) * hd + d] = from_f32<T>(v * inv);
             else a.part_o[slot * hd + d] = v;
         }
-        if (a.n_splits > 1) {          // the row's first part also says what parts there are not
-            if (lane == 0) *reinterpret_cast<float2*>(a.part_ml + slot * 2) = whole ? make_float2(0.f, ATT_WHOLE) : make_float2(M, L);
+        if (a.n_splits > 1) {          // the row's first part also says what parts there are not (the scratch may begin at any float)
+            if (lane == 0) {
+                a.part_ml[slot * 2] = whole ? 0.f : M;
+                a.part_ml[slot * 2 + 1] = whole ? ATT_WHOLE : L;
+            }
             if (sp == 0)
-                for (int i = max(parts, 1) + lane; i < a.n_splits; i += 32) *reinterpret_cast<float2*>(a.part_ml + (slot + i) * 2) = make_float2(-INFINITY, 0.f);
+                for (int i = parts + lane; i < a.n_splits; i += 32) {
+                    a.part_ml[(slot + i) * 2] = -INFINITY;
+                    a.part_ml[(slot + i) * 2 + 1] = 0.f;
+                }
         }
     }
 }

@@ -26,7 +26,7 @@ def _batch(seed, lens, starts, G, hd, ps, dtype, pad=0):
     return g, k, v, seg, pos, table
 
 
-def _check(dtype, H, G, hd, ps, lens, starts, splits=1, pad=0, window=None, seed=0, part_keys=0, **extra):
+def _check(dtype, H, G, hd, ps, lens, starts, splits=1, pad=0, window=None, seed=0, part_keys=0, off=0, **extra):
     from pico_vllm_b200 import ops
     g, k, v, seg, pos, table = _batch(seed, lens, starts, G, hd, ps, dtype, pad)
     T = seg.shape[0]
@@ -39,7 +39,7 @@ def _check(dtype, H, G, hd, ps, lens, starts, splits=1, pad=0, window=None, seed
     fake_ops.paged_attention(q.float(), k.float(), v.float(), want, seg, pos, table, H, G, hd, ps, window, scale, **extra)
     d = lambda t: t.to(DEV) if torch.is_tensor(t) else t
     out = torch.full((T, H * hd), float("nan"), dtype=dtype, device=DEV)
-    scratch = torch.full((max(1, ops.attention_scratch_floats(T, H, hd, splits)),), float("nan"), device=DEV)
+    scratch = torch.full((max(1, ops.attention_scratch_floats(T, H, hd, splits)) + off,), float("nan"), device=DEV)[off:]
     ops.paged_attention(d(q), d(k), d(v), out, d(seg), d(pos), d(table), H, G, hd, ps, window, scale, splits, scratch, part_keys=part_keys,
                         **{n: d(t) for n, t in extra.items()})
     # float32: sums of up to some hundreds of terms of order 1; bfloat16: the result's own rounding, 2^-9, of values up to 4
@@ -63,6 +63,12 @@ def test_options_over_portions_and_single_tokens(i, splits):
 def test_runs_in_as_many_parts_as_they_have_keys_for(splits, part_keys, i):
     # whole runs beside runs in parts; parts that the tiles of keys leave without any; a padding row
     _check(torch.float32, 12, 2, 48, 4, [1, 33, 1, 1, 2, 17], [70, 0, 0, 129, 31, 8], splits, pad=1, seed=i, part_keys=part_keys, **OPTIONS[i])
+
+
+@pytest.mark.parametrize("splits,part_keys", [(3, 0), (4, 40)])
+@pytest.mark.parametrize("lens,starts", [([1, 1], [70, 129]), ([1, 33, 2], [70, 0, 31])])
+def test_scratch_may_begin_at_any_float(lens, starts, splits, part_keys):
+    _check(torch.float32, 12, 2, 48, 4, lens, starts, splits, part_keys=part_keys, off=1)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
