@@ -27,7 +27,7 @@
 //   RT =  8: four warps share the 8 rows and take every fourth tile of keys, their sums are added at the end (single
 //            tokens and short prompts, where blocks are few and a row's chain of keys sets the time).
 // With part_keys > 0 every run, a portion's too, goes in parts of at least so many keys, up to n_splits; a run that stays whole is written by
-// its own block and left alone by the combining kernel.  The parts of a run are neighbours in the grid: side by side and in L2 together.
+// its own block and left alone by the combining kernel.
 // Keys and values come in by cp.async into buffers of their own (values land while the scores are computed, the next keys
 // while the values are multiplied); scores: a lane has 2 rows x KT / 8 keys; output: a lane has 8 rows x 4 NJ dimensions,
 // probabilities pass through shared memory.  All arithmetic is float32 on the CUDA cores: with enough rows those bound it
@@ -70,6 +70,10 @@ struct TileArgs {
 
 __host__ __device__ constexpr int tile_keys(int nj, int rt) { return rt == 8 ? (nj == 5 ? 8 : 16) : (nj == 1 ? 32 : nj == 2 ? 16 : 8); }
 
+// Whether the parts of a run are neighbours in the grid, at work and in L2 together, or all first parts come before the second ones: single
+// tokens in parts lose by the former (64 of 12 / 2 heads of 96, 777 keys in two parts 84.7 us, side by side 86.7; of 128, 300 keys 28.6 / 29.5).
+__host__ __device__ constexpr bool tile_side_by_side(int rt, int part_keys) { return rt == 32 || part_keys > 0; }
+
 template <typename T, int NJ, int RT>
 __global__ void __launch_bounds__(128) paged_attention_tiled_kernel(const T* __restrict__ q, const T* __restrict__ k_pages,
                                                                     const T* __restrict__ v_pages, T* __restrict__ out, const TileArgs a) {
@@ -78,8 +82,9 @@ __global__ void __launch_bounds__(128) paged_attention_tiled_kernel(const T* __r
     constexpr int KT = tile_keys(NJ, RT), KL = KT / 8, VEC = 16 / (int)sizeof(T);
     constexpr bool SHARED = RT == 32;                      // the four warps share the key tiles
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // the tokens late in a prompt, which see the most keys, first; the parts of a run side by side
-    const int sp = (int)(blockIdx.x % a.n_splits), chunk_at = (int)(blockIdx.x / a.n_splits);
+    // the tokens late in a prompt, which see the most keys, first
+    const bool side = tile_side_by_side(RT, a.part_keys);
+    const int sp = side ? (int)(blockIdx.x % a.n_splits) : blockIdx.z, chunk_at = side ? (int)(blockIdx.x / a.n_splits) : blockIdx.x;
     const int t0 = a.T - 1 - chunk_at / a.row_chunks, kh = blockIdx.y, rc = chunk_at % a.row_chunks;
     const int g = a.nh / a.nkv, hd = a.hd, ld = hd + 4;
     const int seg = a.tok_seg[t0], pos0 = a.positions[t0];
@@ -350,7 +355,8 @@ static void tile_launch(const T* q, const T* k, const T* v, T* out, TileArgs a, 
     const size_t merge = (size_t)(RT == 32 ? 1 : 4) * RT * (ld + 2) * sizeof(float);
     const size_t smem = fixed + (ring > merge ? ring : merge);
     cudaFuncSetAttribute(paged_attention_tiled_kernel<T, NJ, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    pico_launch((paged_attention_tiled_kernel<T, NJ, RT>), dim3((unsigned)a.T * a.row_chunks * a.n_splits, a.nkv), dim3(128), smem, stream, q, k, v,
+    const bool side = tile_side_by_side(RT, a.part_keys);
+    pico_launch((paged_attention_tiled_kernel<T, NJ, RT>), dim3((unsigned)a.T * a.row_chunks * (side ? a.n_splits : 1), a.nkv, side ? 1 : a.n_splits), dim3(128), smem, stream, q, k, v,
                 out, a);
 }
 
@@ -370,8 +376,10 @@ static void tile_dispatch(const T* q, const T* k, const T* v, T* out, const Tile
     }
 }
 
-// out[t, h, :] = sum_i o_i exp(m_i - M) / sum_i l_i exp(m_i - M) over the splits i.
-template <typename T>
+// out[t, h, :] = sum_i o_i exp(m_i - M) / sum_i l_i exp(m_i - M) over the splits i.  RUNS: a row may be finished already, or have fewer parts than
+// n_splits, whose places hold anything; asked for each part in front of its loads that costs every call (attention and this kernel, one token of 12 / 2 heads of
+// 128 after 2,000 keys in eight parts: 32.4 us, 29.2 without).
+template <typename T, bool RUNS>
 __global__ void attention_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                          T* __restrict__ out, int hd, int n_splits, const float* __restrict__ sinks,
                                          int nh) {
@@ -379,7 +387,7 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_o, const
     pdl_wait();
     const size_t th = blockIdx.x;  // t * nh + h
     const float* ml = part_ml + th * n_splits * 2;
-    if (ml[1] == ATT_WHOLE) return;
+    if (RUNS && ml[1] == ATT_WHOLE) return;
     float M = sinks ? sinks[th % nh] : -INFINITY;
     for (int i = 0; i < n_splits; ++i) M = fmaxf(M, ml[2 * i]);
     float L = sinks ? expf(sinks[th % nh] - M) : 0.f;
@@ -388,8 +396,8 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_o, const
     for (int d = threadIdx.x; d < hd; d += blockDim.x) {
         float acc = 0.f;
         for (int i = 0; i < n_splits; ++i) {
-            if (ml[2 * i] == -INFINITY && ml[2 * i + 1] == 0.f) continue;      // no keys, or no such part
-            acc += part_o[(th * n_splits + i) * hd + d] * part_factor(ml[2 * i], ml[2 * i + 1], M);
+            const float o = part_o[(th * n_splits + i) * hd + d], m = ml[2 * i], l = ml[2 * i + 1];
+            acc += (RUNS && m == -INFINITY && l == 0.f ? 0.f : o) * part_factor(m, l, M);
         }
         out[th * hd + d] = from_f32<T>(acc * inv);
     }
@@ -410,18 +418,18 @@ PICO_API int pico_paged_attention_generic(const void* q, int q_row_stride, const
     if (nkv <= 0 || nh % nkv != 0 || n_splits < 1 || n_splits > 65535 || nkv > 65535) return PICO_ERR_SIZE;
     if (n_splits > 1 && (!part_o || !part_ml)) return PICO_ERR_SIZE;
     // (blocks along x: a row's chunks of 8 rows at most, times the parts)
-    if (chunk < 0 || part_keys < 0 || (long long)T * ((nh / nkv + 7) / 8 + 1) * n_splits > 0x7fffffffLL) return PICO_ERR_SIZE;
+    if (chunk < 0 || part_keys < 0 || (long long)T * ((nh / nkv + 7) / 8) * n_splits > 0x7fffffffLL) return PICO_ERR_SIZE;
     const TileArgs a = {q_row_stride, table_stride, T, nh, nkv, hd, page_size, window, n_splits, chunk, 1, 1, part_keys, scale, softcap,
                         tok_seg, positions, block_table, slopes, sinks, rates, part_o, part_ml};
     if (act_dtype == PICO_F32) {
         if ((q_row_stride % 4) != 0) return PICO_ERR_ALIGN;
         tile_dispatch<float>((const float*)q, (const float*)k_pages, (const float*)v_pages, (float*)out, a, stream);
         if (n_splits > 1)
-            pico_launch((attention_combine_kernel<float>), dim3(T * nh), dim3(64), 0, stream, part_o, part_ml, (float*)out, hd, n_splits, sinks, nh);
+            pico_launch((part_keys > 0 ? attention_combine_kernel<float, true> : attention_combine_kernel<float, false>), dim3(T * nh), dim3(64), 0, stream, part_o, part_ml, (float*)out, hd, n_splits, sinks, nh);
     } else if (act_dtype == PICO_BF16) {
         tile_dispatch<bf16>((const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, (bf16*)out, a, stream);
         if (n_splits > 1)
-            pico_launch((attention_combine_kernel<bf16>), dim3(T * nh), dim3(64), 0, stream, part_o, part_ml, (bf16*)out, hd, n_splits, sinks, nh);
+            pico_launch((part_keys > 0 ? attention_combine_kernel<bf16, true> : attention_combine_kernel<bf16, false>), dim3(T * nh), dim3(64), 0, stream, part_o, part_ml, (bf16*)out, hd, n_splits, sinks, nh);
     } else
         return PICO_ERR_DTYPE;
     return pico_launch_status();
