@@ -12,9 +12,11 @@ forward path is a kernel of ``csrc/``.
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional
 
 import torch
+from torch.autograd import forward_ad
 
 from .errors import KernelError
 
@@ -820,16 +822,41 @@ def linear_bias(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, bias_
 F32_MIN_TOKENS, F32_MIN_OUT, F32_MIN_IN, F32_FEW_TOKENS = 17, 512, 1024, 32
 
 
+def _nothing_follows() -> bool:
+    """No compilation, trace, ``torch.func`` transform, dispatch mode or autocast is at work that would have to see a product as the library's."""
+    return not (torch.compiler.is_compiling() or torch._C._is_tracing() or torch._C._len_torch_dispatch_stack()
+                or torch._C._is_any_autocast_enabled() or torch._C._functorch.peek_interpreter_stack() is not None)
+
+
+def _plain(t: torch.Tensor) -> bool:
+    """A tensor that is nothing but its numbers in memory, of no other class (fake tensors), not sparse, lazily negated or with a
+    tangent (forward-mode differentiation); the library's product takes those too."""
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and t.layout is torch.strided and not t.is_neg()
+            and (forward_ad._current_level < 0 or forward_ad.unpack_dual(t).tangent is None))
+
+
 def f32_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    (M, K), N = x.shape, weight.shape[0]
-    if not (M >= F32_MIN_TOKENS and N >= F32_MIN_OUT and K >= F32_MIN_IN and x.dtype == weight.dtype == torch.float32 and x.is_cuda):
+    if not (x.dim() == weight.dim() == 2 and x.shape[0] >= F32_MIN_TOKENS and x.dtype == weight.dtype == torch.float32 and x.is_cuda):
         return False
-    if M <= F32_FEW_TOKENS and -(-N // 128) > torch.cuda.get_device_properties(x.device).multi_processor_count:
+    (M, K), (N, width) = x.shape, weight.shape
+    if not (N >= F32_MIN_OUT and K >= F32_MIN_IN and width == K):
         return False
-    if x.requires_grad or weight.requires_grad:        # the library's product has a gradient
+    # what is followed or recorded, and what is not simply memory, is the library's; so are tensors of a device that is not the current one
+    if x.requires_grad or weight.requires_grad or not (_nothing_follows() and _plain(x) and _plain(weight)):
         return False
-    return (K % 4 == 0 and N % 4 == 0 and x.stride(1) == 1 and x.stride(0) >= K and x.stride(0) % 4 == 0 and weight.is_contiguous()
+    device = x.get_device()
+    if weight.get_device() != device or torch.cuda.current_device() != device:
+        return False
+    if M <= F32_FEW_TOKENS and -(-N // 128) > _multiprocessors(device):
+        return False
+    apart, step = x.stride()
+    return (K % 4 == 0 and N % 4 == 0 and step == 1 and apart >= K and apart % 4 == 0 and weight.is_contiguous()
             and (x.data_ptr() | weight.data_ptr()) % 16 == 0 and M <= 65535 * 128)
+
+
+@functools.lru_cache(maxsize=None)
+def _multiprocessors(device: int) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
 
 
 def linear_f32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
@@ -839,10 +866,22 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     (M, K), N = x.shape, weight.shape[0]
     if x.dtype != torch.float32 or weight.dtype != torch.float32 or weight.shape[1] != K or not weight.is_contiguous() or x.stride(1) != 1:
         raise KernelError("linear_f32: float32 rows and contiguous float32 weights")
-    parts = library().pico_gemm_f32_parts(M, N, K)
-    out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    scratch = torch.empty(2 * parts * M * N, dtype=torch.float32, device=x.device) if parts > 1 else None
-    _check(library().pico_gemm_f32(_ptr(x), x.stride(0), _ptr(weight), _ptr(out), _ptr(scratch), M, N, K, _stream()), "linear_f32")
+    if weight.get_device() != x.get_device() or x.get_device() != torch.cuda.current_device():
+        raise KernelError("linear_f32: rows and weights must be on the current device")
+    return _f32_product(x, weight)
+
+
+@functools.lru_cache(maxsize=256)
+def _f32_parts(M: int, N: int, K: int, device: int) -> int:
+    return library().pico_gemm_f32_parts(M, N, K)
+
+
+def _f32_product(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    (M, K), N = x.shape, weight.shape[0]
+    parts = _f32_parts(M, N, K, x.get_device())
+    out = x.new_empty((M, N))
+    scratch = x.new_empty(2 * parts * M * N) if parts > 1 else None
+    _check(library().pico_gemm_f32(x.data_ptr(), x.stride(0), weight.data_ptr(), out.data_ptr(), _ptr(scratch), M, N, K, _stream()), "linear_f32")
     _count(2 if parts > 1 else 1)
     return out
 
@@ -861,12 +900,13 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
     A weight kept in float32 beside bfloat16 activations is multiplied in float32 and the result
     rounded to bfloat16.  float32 products take all digits of their factors, here and in the library (TF32 is off).
     """
-    _cuda(x, weight)
+    if not (x.is_cuda and weight.is_cuda):
+        _cuda(x, weight)
     if x.dtype == weight.dtype:
         if out is not None:
             return torch.mm(x, weight.t(), out=out)
-        if x.dtype == torch.float32 and f32_takes(x, weight):
-            return linear_f32(x, weight)
+        if x.dtype is torch.float32 and f32_takes(x, weight):
+            return _f32_product(x, weight)
         return torch.mm(x, weight.t())
     if weight.dtype == torch.float32 and x.dtype == torch.bfloat16:
         y = torch.mm(x.float(), weight.t()).to(torch.bfloat16)

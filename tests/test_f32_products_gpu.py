@@ -133,3 +133,30 @@ def test_a_product_with_a_gradient_is_the_library_s_and_a_wait_that_ran_out_is_s
     assert ops.tc_status() == 0
     monkeypatch.setattr(ops, "tf_status", lambda: 1)
     assert ops.tc_status() == 1
+
+
+def test_what_is_more_than_numbers_in_memory_is_the_library_s():
+    from torch.autograd import forward_ad
+    from torch.utils.flop_counter import FlopCounterMode
+    from pico_vllm_b200 import ops
+    x, w = torch.ones(32, 1024, device=DEV), torch.ones(512, 1024, device=DEV)
+    with forward_ad.dual_level():
+        out = forward_ad.unpack_dual(ops.linear(forward_ad.make_dual(x, x), w))
+        assert bool((out.primal == 1024).all()) and bool((out.tangent == 1024).all())
+    assert bool((torch.func.vmap(lambda a: ops.linear(a, w))(x.expand(2, 32, 1024)) == 1024).all())
+    assert bool((torch.func.grad(lambda a: ops.linear(a, w).sum())(x) == 512).all())
+    assert bool((ops.linear(torch._neg_view(x), w) == -1024).all())
+    with FlopCounterMode(display=False) as flops:
+        ops.linear(x, w)
+    assert flops.get_total_flops() == 2 * 32 * 512 * 1024
+    assert ops.f32_takes(x, w) and ops.f32_takes(x, torch.nn.Parameter(w, requires_grad=False))
+    with pytest.raises(RuntimeError):
+        ops.linear(x, torch.ones(512, 1028, device=DEV))
+
+
+def test_under_autocast_a_product_is_what_it_was():
+    from pico_vllm_b200 import ops
+    x, w = torch.randn(32, 1024, device=DEV), torch.randn(512, 1024, device=DEV)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        got, plain = ops.linear(x, w), torch.mm(x, w.t())
+    assert got.dtype == plain.dtype and torch.equal(got, plain)
