@@ -880,7 +880,12 @@ def _f32_product(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     (M, K), N = x.shape, weight.shape[0]
     parts = _f32_parts(M, N, K, x.get_device())
     out = x.new_empty((M, N))
-    scratch = x.new_empty(2 * parts * M * N) if parts > 1 else None
+    scratch = None
+    if parts > 1:
+        try:
+            scratch = x.new_empty(2 * parts * M * N)
+        except torch.OutOfMemoryError:         # no room for the parts' sums
+            return torch.mm(x, weight.t(), out=out)
     _check(library().pico_gemm_f32(x.data_ptr(), x.stride(0), weight.data_ptr(), out.data_ptr(), _ptr(scratch), M, N, K, _stream()), "linear_f32")
     _count(2 if parts > 1 else 1)
     return out

@@ -160,3 +160,19 @@ def test_under_autocast_a_product_is_what_it_was():
     with torch.autocast("cuda", dtype=torch.bfloat16):
         got, plain = ops.linear(x, w), torch.mm(x, w.t())
     assert got.dtype == plain.dtype and torch.equal(got, plain)
+
+
+def test_without_room_for_its_parts_a_product_is_the_library_s(monkeypatch):
+    from pico_vllm_b200 import ops
+    x, w = torch.randn(40, 2048, device=DEV), torch.randn(512, 2048, device=DEV)
+    assert ops.library().pico_gemm_f32_parts(40, 512, 2048) > 1
+    real, asked = torch.Tensor.new_empty, []
+
+    def new_empty(self, size, *rest):
+        if isinstance(size, int):
+            asked.append(size)
+            raise torch.OutOfMemoryError("no room")
+        return real(self, size, *rest)
+    monkeypatch.setattr(torch.Tensor, "new_empty", new_empty)
+    got = ops.linear(x, w)
+    assert len(asked) == 1 and torch.equal(got, torch.mm(x, w.t()))
