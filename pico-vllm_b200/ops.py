@@ -312,7 +312,8 @@ def paged_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
     for t in (tok_seg, positions, block_table):
         if t.dtype != torch.int32:
             raise KernelError("paged_attention: index tensors must be int32")
-    _check_bias(slopes, sinks, rates, n_heads, "paged_attention")
+    if slopes is not None or sinks is not None or rates is not None:
+        _check_bias(slopes, sinks, rates, n_heads, "paged_attention")
     part_o = part_ml = None
     if n_splits > 1:
         need = attention_scratch_floats(T, n_heads, head_dim, n_splits)
@@ -910,7 +911,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
     if x.dtype == weight.dtype:
         if out is not None:
             return torch.mm(x, weight.t(), out=out)
-        if x.dtype is torch.float32 and f32_takes(x, weight):
+        if x.dtype is torch.float32 and x.numel() >= F32_MIN_TOKENS * F32_MIN_IN and f32_takes(x, weight):
             return _f32_product(x, weight)
         return torch.mm(x, weight.t())
     if weight.dtype == torch.float32 and x.dtype == torch.bfloat16:
