@@ -35,7 +35,7 @@ MAX_MIXED_SCRATCH = 32 << 20       # float32 numbers (128 MB) that splitting the
 MIXED_MIN_KEYS = 1024              # longest context of the single tokens of a mixed step from which they are counted alone
 
 
-RUN_MIN_KEYS, RUN_FEW_ROWS = 640, 400      # see GQAAttention._run_parts
+RUN_MIN_KEYS, RUN_SHARED = 384, 228 << 10      # see GQAAttention._run_parts; bytes of shared memory of a multiprocessor
 
 
 DECODE_RAGGED_KEYS = 4096          # longest context from which the parts of a ragged batch need not all run at once
@@ -130,15 +130,17 @@ class GQAAttention(Part):
                              part_keys=part_keys)
 
     def _run_parts(self, shape: StepShape, splits: int):
-        """(parts, least keys of a part) of a float32 step with portions in which some token sees RUN_MIN_KEYS and more: there the
-        longest run of rows sets the time, a portion's rows as well as single ones.  (0, 0): as in other steps.
-        Few rows: blocks of 8 rows in up to four parts of 128 keys and more (us of the kernel, whole / in parts: 12 / 2 heads of 128, 150 tokens beside 8 of
-        700 keys 69 / 33, 100 tokens after 900 102 / 69; 4 / 1 of 256, 40 after 1,000 124 / 47; 8 / 8 of 64, 17 after 600 53 / 27).  Many: all in four
-        parts, which makes blocks of 32 rows, as long as those are no more than four a multiprocessor (12 / 2 heads: 333 after
-        400 124 / 97, 1,000 alone 270 / 199, a layer with 333 beside 7 of 777 136 / 117; 28 / 4: 500 after 1,500 833 / 658; 4 / 1 of 256: 2,048 alone
-        836 / 369; above that line 12 / 2 heads, 2,048 alone 576 / 652, 28 / 4, 1,000 alone 455 / 459).  Fewer than four query heads a key
-        head make single tokens poor rows of 32 (8 / 8: 300 tokens beside 30 of 1,000 keys 113 / 171), and shorter contexts gain nothing
-        (16 / 2 of 64: 333 beside 7 of 500 53 / 56; 4 / 1 of 256: 200 after 400 78 / 86)."""
+        """(parts, least keys of a part) of a float32 step with portions whose time its longest run of rows sets, a portion's rows or a single
+        one; (0, 0): as in other steps.  What the runs are held against is the load: the keys that all blocks of 8 rows see over the
+        blocks that the device holds at once, as many steps of keys as every place of it would take if all were dealt evenly.
+        In up to four parts of 128 keys and more: where the longest run has 256 keys more than 1.3 loads (in two or three parts already, half or a
+        third of them and 192), while blocks of 32 rows would not fill the device.  All in four, which makes blocks of 32 rows: portions
+        that take more than one round of blocks of 8, of four query heads a key head or more and not beside many single tokens (poor rows of 32),
+        as long as blocks of 32 are no more than four a multiprocessor; of both, the former from two loads on.
+        2,700 random steps of seven head sizes, up to 1,400 tokens and 200 single ones, 50 to 2,500 keys, us of the kernel whole / in parts: 683 are cut, 1.6
+        times as fast in the geometric mean, five of them slower, by 8 % at most (12 / 2 heads of 128, 145 tokens beside 16 of up to 1,242 keys 127 / 46, 70
+        after 530 in two parts 45 / 50 in four, left; 16 / 2, 184 beside 16 of 1,350 116 / 46; 4 / 1 of 256, 884 after 1,100 beside 8 528 / 269; 16 / 2, 2 beside 200
+        of 694 84 / 109, left; 32 / 8, 63 beside 64 of 1,832 232 / 344, left)."""
         if getattr(shape.engine, "dtype", "") != "float32" or shape.max_kv < RUN_MIN_KEYS or self.window is not None:
             return 0, 0
         portions = sum(n for n in shape.q_lens if n > 1)
@@ -146,11 +148,22 @@ class GQAAttention(Part):
             return 0, 0
         if 4 * shape.num_tokens * self.n_heads * (self.head_dim + 2) > MAX_MIXED_SCRATCH or splits >= 4 or not shape.spare:
             return 0, 0
-        if portions * self.n_kv_heads < RUN_FEW_ROWS:
-            return 4, 128
         g = self.n_heads // self.n_kv_heads
-        tall = shape.num_tokens // max(1, 32 // g) * self.n_kv_heads
-        return (4, 0) if g >= 4 and 2 * shape.num_sms <= 4 * tall and tall < 4 * shape.num_sms else (0, 0)
+        rows, tall = max(1, 8 // g), max(1, 32 // g)                   # tokens a block of 8 or 32 rows
+        held = shape.num_sms * max(1, min(4, RUN_SHARED // (544 * (self.head_dim + 4) + 3264)))
+        blocks = keys = 0
+        for n, start in zip(shape.q_lens, shape.starts):
+            b = -(-n // rows) * -(-rows * g // 8) * self.n_kv_heads
+            blocks += b
+            keys += b * (start + (n + 1) / 2)
+        talls, singles = shape.num_tokens // tall * self.n_kv_heads, sum(1 for n in shape.q_lens if n == 1)
+        many = (splits == 1 and g >= 4 and shape.max_kv * min(self.head_dim, 128) >= 640 * 128 and shape.num_sms <= 2 * talls
+                and talls < 4 * shape.num_sms and 10 * blocks >= 11 * held and portions >= 2 * singles * tall)
+        if talls < 2 * shape.num_sms and (splits == 1 or shape.max_kv >= 512):
+            over = shape.max_kv / splits - (256 if splits == 1 else 192)
+            if over * held >= (2 if many else 1.3) * keys:
+                return 4, 128
+        return (4, 0) if many else (0, 0)
 
     def _splits(self, shape: StepShape) -> int:
         """As :func:`decode_splits`, but where single tokens run in a kernel of their own beside the portions and the longest sees

@@ -47,10 +47,18 @@ def test_the_32_bit_path_still_counts_every_token():
 
 @pytest.mark.parametrize("H,G,hd,q_lens,starts,want", [
     (12, 2, 128, [333] + [1] * 7, [0] + [777] * 7, (4, 0)), (12, 2, 128, [333], [0], (0, 0)), (12, 2, 128, [333], [306], (0, 0)),
-    (12, 2, 128, [333], [307], (4, 0)), (12, 2, 128, [199] + [1] * 8, [0] + [700] * 8, (4, 128)), (12, 2, 128, [200] + [1] * 8, [0] + [700] * 8, (4, 0)),
-    (12, 2, 128, [1479], [0], (4, 0)), (12, 2, 128, [1480], [0], (0, 0)), (8, 8, 64, [333] + [1] * 7, [0] + [777] * 7, (0, 0)),
+    (12, 2, 128, [333], [307], (4, 0)), (12, 2, 128, [199] + [1] * 8, [0] + [700] * 8, (4, 128)), (12, 2, 128, [200] + [1] * 8, [0] + [700] * 8, (4, 128)),
+    (12, 2, 128, [1479], [0], (4, 0)), (12, 2, 128, [1480], [0], (0, 0)), (8, 8, 64, [333] + [1] * 7, [0] + [777] * 7, (4, 128)),
     (8, 8, 64, [40], [1000], (4, 128)), (4, 1, 256, [500], [500], (0, 0)), (4, 1, 256, [600], [500], (4, 0)), (12, 2, 128, [2, 1], [3000, 3000], (0, 0)),
-    (2000, 500, 128, [40], [1000], (0, 0))])
+    (2000, 500, 128, [40], [1000], (0, 0)),
+    # many single tokens already fill the device; a few do not
+    (12, 2, 128, [2] + [1] * 200, [700] * 201, (0, 0)), (12, 2, 128, [2] + [1] * 64, [850] * 65, (0, 0)), (32, 8, 128, [63] + [1] * 64, [1700] * 65, (0, 0)),
+    (12, 2, 128, [17] + [1] * 64, [0] + [100] * 63 + [1000], (4, 128)),
+    # portions that fit at once, of a quarter of a round more
+    (28, 4, 128, [110, 1], [1250, 1000], (0, 0)), (28, 4, 128, [140, 1], [1250, 1000], (4, 0)),
+    # short contexts
+    (12, 2, 128, [17] * 3 + [1], [0] * 3 + [382], (0, 0)), (12, 2, 128, [60], [500], (0, 0)), (12, 2, 128, [40] + [1] * 8, [0] + [510] * 8, (0, 0)),
+    (12, 2, 128, [40] + [1] * 8, [0] + [511] * 8, (4, 128))])
 def test_parts_of_float32_steps_with_portions(H, G, hd, q_lens, starts, want):
     part = GQAAttention(H * hd, H, G, hd, position=Rotary(hd, 1e6))
     shape = StepShape(num_tokens=sum(q_lens), num_segments=len(q_lens), q_lens=q_lens, starts=starts, max_kv=max(a + b for a, b in zip(q_lens, starts)),
