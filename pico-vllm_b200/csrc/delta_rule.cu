@@ -1168,10 +1168,13 @@ PICO_API int pico_gated_delta_chunks(const float* prep, const float* v, int v_st
     float* u = s0 + (size_t)chunks * H * ((dv + 3) / 4 * 4) * DC_D;
     const int slots = H / G < 8 ? H / G : 8;
     const bool keep_v = (size_t)DC_C * (H / G) * dv * sizeof(float) <= 32 * 1024;
-    // Two blocks a multiprocessor; three, with fewer registers and the values in the place of the queries, where that saves a round of them
-    // (us of the kernel / of the layer, 2,048 tokens in three segments: 6 key heads, 408 blocks, two a multiprocessor 45 / 236, three 32 / 224;
-    // 8 key heads, 544 blocks, two rounds either way, the layer 303 and 308; 1,361 tokens, 270 blocks, one round, 176 and 183).
-    const long long blocks = (long long)chunks * G, two = 2LL * pico_num_sms(), three = 3LL * pico_num_sms();
+    // Two blocks a multiprocessor; three, with fewer registers (80 a thread, 44 bytes of them stored and 56 loaded again) and the values in the place of the
+    // queries, where that saves a round of them.  The blocks that have a chunk are counted as if every segment's last chunk were half full; the grid
+    // has up to one a segment more, which leave at once: 2 % more blocks were enough for a round that there was not (8 key heads, 1,100 tokens in three
+    // segments, 288 at work and 304 in the grid: a layer 189 us, three a multiprocessor 197).  us of a layer, two / three, by the grid: 6 key heads, 324
+    // blocks 209 / 202, 408 247 / 236, 432 252 / 242, 624 357 / 349, 870 549 / 542; 8 key heads, 368 243 / 231, 672 404 / 395, 912 539 / 529.
+    const long long two = 2LL * pico_num_sms(), three = 3LL * pico_num_sms();
+    const long long blocks = (long long)G * (2 * (T / DC_C) + (S < T / DC_LEAST ? S : T / DC_LEAST)) / 2;
     const long long v_floats = keep_v ? (long long)DC_C * (H / G) * dv : 0, q_floats = DC_C * DC_LD;
     const long long other = DC_C * DC_LD + 2 * DC_C * (DC_C + 1) + slots * (DC_C * DC_C + DC_C), shared = other + (v_floats > q_floats ? v_floats : q_floats);
     const bool crowded = keep_v && 3 * (shared * (long long)sizeof(float) + 1024) <= 228 * 1024 &&

@@ -39,6 +39,21 @@ def _oracle(q, k, v, a, beta, state, slots, cu, pos):
 @pytest.mark.parametrize("lens,pad_at", [([64], None), ([1, 31, 32, 33, 70, 1], None), ([97, 5, 2, 64], 1), ([0, 128, 0, 65], None)])
 @pytest.mark.parametrize("decays,off", [("middling", 0), ("nought and one", 0), ("middling", 1)])
 def test_chunks(H, G, d, dv, lens, pad_at, decays, off, monkeypatch):
+    _check(H, G, d, dv, lens, pad_at, decays, off, monkeypatch)
+
+
+@pytest.mark.parametrize("H,G,d,dv,lens,blocks", [
+    (28, 28, 68, 20, [320], 294), (29, 29, 68, 20, [320], 304), (58, 29, 128, 128, [320], 304), (52, 26, 100, 128, [31, 65, 224], 299),
+    (42, 42, 100, 36, [320], 441), (84, 42, 128, 128, [320], 441), (43, 43, 128, 4, [320], 451), (56, 56, 68, 20, [320], 588),
+    (57, 57, 100, 36, [320], 598), (168, 84, 72, 128, [320], 882), (85, 85, 68, 8, [320], 892)])
+def test_three_blocks_a_multiprocessor_prepare(H, G, d, dv, lens, blocks, monkeypatch):
+    """Chunks times key heads at both ends of the ranges in which three blocks a multiprocessor save a round (297 to 444 and 593 to 888 of
+    148 multiprocessors) and outside them, values narrower and wider than the queries whose place they take."""
+    assert (2 * (sum(lens) // 32) + min(len(lens), sum(lens) // 64)) * G // 2 == blocks
+    _check(H, G, d, dv, lens, None, "middling", 0, monkeypatch)
+
+
+def _check(H, G, d, dv, lens, pad_at, decays, off, monkeypatch):
     from pico_vllm_b200 import ops
     monkeypatch.setattr(ops, "delta_chunks_take", lambda *a: True)
     g = torch.Generator().manual_seed(d + dv + len(lens))
