@@ -814,13 +814,21 @@ def linear_bias(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, bias_
     raise KernelError(f"linear_bias: activations {x.dtype} with weights {weight.dtype} is not supported")
 
 
-# float32 products on the tensor cores (csrc/gemm_f32_tcgen05.cu) where they are faster than the library's; us here / there:
-# 17 tokens 1,536 x 1,536 15 / 25, 1,024 x 1,024 13.3 / 13.2, 1,024 x 512 12.1 / 9.1; 17 and 33 x 32,000 x 1,024 (250 tiles of w, almost two rounds of
-# the multiprocessors) 69 / 56 and 69 / 86; 340 x 128 and 512 x 1,024 16 / 14.7 and 17 / 21; 340 x 2,048 x 1,536 29 / 64; 2,048 x 17,920 x 1,536
-# 868 / 1,834; 128 x 1,536 x 8,960 39 / 166.  Root mean square of the error against float64, relative, 17 to 2,048 tokens and 1,024 to 8,960 columns, here /
-# there: normal numbers 1.0e-7 to 1.2e-7 / 2.7e-7 to 1.7e-6, all of one sign 0.9e-7 to 1.5e-7 / 1.1e-7 to 1.3e-6, four terms a row 2.7e-8 / 4.3e-8 to
-# 4.7e-8, one 2.5e-8 / 2.5e-8; for fewer tokens the library's can be smaller, so they stay there.
-F32_MIN_TOKENS, F32_MIN_OUT, F32_MIN_IN, F32_FEW_TOKENS = 17, 512, 1024, 32
+# float32 products on the tensor cores (csrc/gemm_f32_tcgen05.cu) where they are faster than the library's; us here / there: 340 x 2,048 x 1,536 32 / 65, 64
+# of them 20 / 37, 17 18 / 39; 100 x 1,536 x 8,960 43 / 215; 2,048 x 17,920 x 1,536 981 / 1,835.  Root mean square of the error against float64,
+# relative, 17 to 2,048 tokens and 1,024 to 8,960 columns: normal numbers 1.0e-7 to 1.2e-7 / 2.7e-7 to 1.7e-6, all of one sign 0.9e-7 to 1.5e-7 / 1.1e-7
+# to 1.3e-6, four terms a row 2.7e-8 / 4.3e-8 to 4.7e-8, one 2.5e-8 / 2.5e-8; for fewer tokens the library's can be smaller, so they stay there.
+F32_MIN_TOKENS, F32_MIN_OUT, F32_MIN_IN = 17, 512, 1024
+
+
+def _f32_pays(M: int, N: int, K: int, device: int) -> bool:
+    """The lines between the two, us here / there.  Short columns: 17 x 512 x 1,024 14.0 / 13.3 and x 1,152 13.9 / 17.5; 17 x 1,536 x 1,024 14.4 / 14.0, x 2,048 15.0
+    / 25.6; 64 x 768 16.0 / 15.3, x 1,024 15.9 / 19.2; 96 x 512 16.0 / 15.3, x 640 16.1 / 19.1; 128 x 512 16.6 / 19.1.  Few tokens and so many tiles of w that K
+    is left in one part: 17 x 8,192 x 1,024 25.8 / 26.5, x 12,288 38.4 / 34.4, x 18,944 39.1 / 35.9, x 14,336 x 1,536 52.7 / 51.1; x 18,944 x 3,584 112 / 119, but x 22,016 x
+    2,048 (two rounds of tiles) 133 / 98; 33 x 12,288 x 1,024 39.0 / 45.5, x 32,000 77 / 86."""
+    if M < F32_MIN_TOKENS or K < F32_MIN_IN or N < (F32_MIN_OUT if K >= 1152 or M > 96 else 640 if M > 64 else 1024 if M > 32 else 2048):
+        return False
+    return M > 32 or N <= 8192 or (K >= 3584 and -(-N // 128) <= _multiprocessors(device))
 
 
 def _nothing_follows() -> bool:
@@ -840,15 +848,13 @@ def f32_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
     if not (x.dim() == weight.dim() == 2 and x.shape[0] >= F32_MIN_TOKENS and x.dtype == weight.dtype == torch.float32 and x.is_cuda):
         return False
     (M, K), (N, width) = x.shape, weight.shape
-    if not (N >= F32_MIN_OUT and K >= F32_MIN_IN and width == K):
+    device = x.get_device()
+    if width != K or not _f32_pays(M, N, K, device):
         return False
     # what is followed or recorded, and what is not simply memory, is the library's; so are tensors of a device that is not the current one
     if x.requires_grad or weight.requires_grad or not (_nothing_follows() and _plain(x) and _plain(weight)):
         return False
-    device = x.get_device()
     if weight.get_device() != device or torch.cuda.current_device() != device:
-        return False
-    if M <= F32_FEW_TOKENS and -(-N // 128) > _multiprocessors(device):
         return False
     apart, step = x.stride()
     return (K % 4 == 0 and N % 4 == 0 and step == 1 and apart >= K and apart % 4 == 0 and weight.is_contiguous()

@@ -112,8 +112,11 @@ def test_sums_that_are_no_number_are_what_float32_gives(M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K,off,takes", [(16, 2048, 1536, 0, False), (17, 2048, 1536, 0, True), (17, 508, 1536, 0, False), (17, 512, 1020, 0, False),
-                                             (17, 512, 1026, 0, False), (17, 514, 1024, 0, False), (17, 512, 1024, 1, False), (17, 512, 1024, 4, True),
-                                             (32, 32000, 1024, 0, False), (33, 32000, 1024, 0, True)])
+                                             (17, 512, 1154, 0, False), (17, 514, 1152, 0, False), (17, 512, 1152, 1, False), (17, 512, 1152, 4, True),
+                                             (17, 512, 1148, 0, False), (17, 2044, 1024, 0, False), (17, 2048, 1024, 0, True), (33, 1020, 1024, 0, False),
+                                             (33, 1024, 1024, 0, True), (65, 636, 1024, 0, False), (65, 640, 1024, 0, True), (97, 512, 1024, 0, True),
+                                             (32, 8192, 1024, 0, True), (32, 8196, 1024, 0, False), (32, 18944, 3584, 0, True), (32, 18948, 3584, 0, False),
+                                             (32, 18944, 3580, 0, False), (33, 32000, 1024, 0, True)])
 def test_which_products_go_there(M, N, K, off, takes):
     from pico_vllm_b200 import ops
     x, w = torch.ones(M, K + off, device=DEV)[:, off:], torch.ones(N, K, device=DEV)
@@ -127,7 +130,7 @@ def test_which_products_go_there(M, N, K, off, takes):
 
 def test_a_product_with_a_gradient_is_the_library_s_and_a_wait_that_ran_out_is_seen(monkeypatch):
     from pico_vllm_b200 import ops
-    x, w = torch.ones(32, 1024, device=DEV, requires_grad=True), torch.ones(512, 1024, device=DEV)
+    x, w = torch.ones(32, 1152, device=DEV, requires_grad=True), torch.ones(512, 1152, device=DEV)
     ops.linear(x, w).sum().backward()
     assert bool((x.grad == 512).all())
     assert ops.tc_status() == 0
@@ -139,24 +142,24 @@ def test_what_is_more_than_numbers_in_memory_is_the_library_s():
     from torch.autograd import forward_ad
     from torch.utils.flop_counter import FlopCounterMode
     from pico_vllm_b200 import ops
-    x, w = torch.ones(32, 1024, device=DEV), torch.ones(512, 1024, device=DEV)
+    x, w = torch.ones(32, 1152, device=DEV), torch.ones(512, 1152, device=DEV)
     with forward_ad.dual_level():
         out = forward_ad.unpack_dual(ops.linear(forward_ad.make_dual(x, x), w))
-        assert bool((out.primal == 1024).all()) and bool((out.tangent == 1024).all())
-    assert bool((torch.func.vmap(lambda a: ops.linear(a, w))(x.expand(2, 32, 1024)) == 1024).all())
+        assert bool((out.primal == 1152).all()) and bool((out.tangent == 1152).all())
+    assert bool((torch.func.vmap(lambda a: ops.linear(a, w))(x.expand(2, 32, 1152)) == 1152).all())
     assert bool((torch.func.grad(lambda a: ops.linear(a, w).sum())(x) == 512).all())
-    assert bool((ops.linear(torch._neg_view(x), w) == -1024).all())
+    assert bool((ops.linear(torch._neg_view(x), w) == -1152).all())
     with FlopCounterMode(display=False) as flops:
         ops.linear(x, w)
-    assert flops.get_total_flops() == 2 * 32 * 512 * 1024
+    assert flops.get_total_flops() == 2 * 32 * 512 * 1152
     assert ops.f32_takes(x, w) and ops.f32_takes(x, torch.nn.Parameter(w, requires_grad=False))
     with pytest.raises(RuntimeError):
-        ops.linear(x, torch.ones(512, 1028, device=DEV))
+        ops.linear(x, torch.ones(512, 1156, device=DEV))
 
 
 def test_under_autocast_a_product_is_what_it_was():
     from pico_vllm_b200 import ops
-    x, w = torch.randn(32, 1024, device=DEV), torch.randn(512, 1024, device=DEV)
+    x, w = torch.randn(32, 1152, device=DEV), torch.randn(512, 1152, device=DEV)
     with torch.autocast("cuda", dtype=torch.bfloat16):
         got, plain = ops.linear(x, w), torch.mm(x, w.t())
     assert got.dtype == plain.dtype and torch.equal(got, plain)

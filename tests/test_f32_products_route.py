@@ -22,7 +22,7 @@ def test_tensors_that_are_only_numbers_in_memory():
 def test_fake_tensors_and_devices_without_kernels_are_the_library_s():
     from torch._subclasses import FakeTensorMode
     with FakeTensorMode():
-        x, w = torch.empty(32, 1024, device="cuda"), torch.empty(512, 1024, device="cuda")
+        x, w = torch.empty(32, 1152, device="cuda"), torch.empty(512, 1152, device="cuda")
         assert not ops._plain(x) and not ops.f32_takes(x, w) and ops.linear(x, w).shape == (32, 512)
-    x, w = torch.ones(32, 1024), torch.ones(512, 1024)
+    x, w = torch.ones(32, 1152), torch.ones(512, 1152)
     assert ops._plain(x) and not ops.f32_takes(x, w)
