@@ -604,7 +604,6 @@ gated_delta_block_kernel(const float* __restrict__ prep, int P, const float* __r
 #define DC_C 32
 #define DC_D 128                               // rows of S, keys padded with zeros
 #define DC_LD (DC_D + 4)                       // rows that lanes read side by side, 16 bytes each
-#define DC_LDK (DC_D + 16)                     // rows that four lanes read 64 bytes of
 #define DC_NC 16                               // columns of S a block of the chain
 #define DC_OC 128                              // columns of O a block
 #define DC_COEF (DC_C * DC_D + DC_C * DC_C + 2 * DC_C)      // floats a chunk and head: M diag(G) K, E by columns, G, D_Cj
@@ -991,7 +990,8 @@ delta_chunk_kernel(const float* __restrict__ prep, int P, float* __restrict__ st
 #pragma unroll
         for (int tt = 0; tt < 4; ++tt) *reinterpret_cast<float4*>(mine + (warp * 4 + tt) * 128) = make_float4(x[tt][0], x[tt][1], x[tt][2], x[tt][3]);
         asm volatile("bar.sync 1, %0;\n" ::"n"(32 * DC_WARPS) : "memory");
-        if (warp < DC_C / 8) {                 // U and diag(D_Cj) U of eight tokens
+        static_assert(DC_WARPS == DC_C / 8, "a warp makes U and diag(D_Cj) U of eight tokens");
+        {
             float4 a[DC_WARPS];
 #pragma unroll
             for (int p = 0; p < DC_WARPS; ++p) a[p] = *reinterpret_cast<const float4*>(mine + (p * 4 + warp) * 128);
