@@ -826,8 +826,7 @@ __device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], co
 }
 // c += a b over sixteen places with both in their three parts (pico_split3), in eight products of the nine: the one of the two smallest parts is
 // below 2^-30 of a b.  The tensor cores cut sums off where float32 rounds them: the large parts' products leave them after one instruction.
-// The others' sums, below 2^-6 of those, are kept in two, as an instruction that adds into the registers of the one before waits 23 clocks for it
-// (one can be issued every 8).
+// The others' sums, below 2^-6 of those, are kept in two, as an instruction that adds into the registers of the one before waits 20 clocks for it.
 __device__ __forceinline__ void dc_mma8(float (&c)[3][4], const uint32_t (&a)[3][4], const float2& b0, const float2& b1) {
     uint32_t b[3][2];
     pico_split3(b0.x, b0.y, b[0][0], b[1][0], b[2][0]);
