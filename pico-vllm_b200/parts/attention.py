@@ -136,7 +136,9 @@ class GQAAttention(Part):
         In up to four parts of 128 keys and more: where the longest run has 256 keys more than 1.3 loads (in two or three parts already, half or a
         third of them and 192), while blocks of 32 rows would not fill the device.  All in four, which makes blocks of 32 rows: portions
         that take more than one round of blocks of 8, of four query heads a key head or more and not beside many single tokens (poor rows of 32),
-        as long as blocks of 32 are no more than four a multiprocessor; of both, the former from two loads on.
+        as long as blocks of 32 are no more than four a multiprocessor; of both, the former from two loads on, more where a head's queries leave rows of the 8
+        empty (12 / 2 heads of 128, a layer, all in four / in parts of 128 keys: 150 and 137 tokens beside 8 single ones, 2.1 loads, 121 / 129; 260 beside 8,
+        3 loads, 122 / 109).
         2,700 random steps of seven head sizes, up to 1,400 tokens and 200 single ones, 50 to 2,500 keys, us of the kernel whole / in parts: 683 are cut, 1.6
         times as fast in the geometric mean, five of them slower, by 8 % at most (12 / 2 heads of 128, 145 tokens beside 16 of up to 1,242 keys 127 / 46, 70
         after 530 in two parts 45 / 50 in four, left; 16 / 2, 184 beside 16 of 1,350 116 / 46; 4 / 1 of 256, 884 after 1,100 beside 8 528 / 269; 16 / 2, 2 beside 200
@@ -161,7 +163,7 @@ class GQAAttention(Part):
                 and talls < 4 * shape.num_sms and 10 * blocks >= 11 * held and portions >= 2 * singles * tall)
         if talls < 2 * shape.num_sms and (splits == 1 or shape.max_kv >= 512):
             over = shape.max_kv / splits - (256 if splits == 1 else 192)
-            if over * held >= (2 if many else 1.3) * keys:
+            if over * held >= (2 * (8 / (min(rows * g, 8))) ** 0.5 if many else 1.3) * keys:
                 return 4, 128
         return (4, 0) if many else (0, 0)
 

@@ -56,6 +56,9 @@ def test_the_32_bit_path_still_counts_every_token():
     (12, 2, 128, [17] + [1] * 64, [0] + [100] * 63 + [1000], (4, 128)),
     # portions that fit at once, of a quarter of a round more
     (28, 4, 128, [110, 1], [1250, 1000], (0, 0)), (28, 4, 128, [140, 1], [1250, 1000], (4, 0)),
+    # of both: by the load, and by the rows of a block of 8 that a head's queries leave empty
+    (12, 2, 128, [150, 137] + [1] * 8, [0, 185, 401, 282, 242, 714, 197, 294, 426, 201], (4, 0)),
+    (16, 2, 128, [150, 137] + [1] * 8, [0, 185, 401, 282, 242, 714, 197, 294, 426, 201], (4, 128)),
     # short contexts
     (12, 2, 128, [17] * 3 + [1], [0] * 3 + [382], (0, 0)), (12, 2, 128, [60], [500], (0, 0)), (12, 2, 128, [40] + [1] * 8, [0] + [510] * 8, (0, 0)),
     (12, 2, 128, [40] + [1] * 8, [0] + [511] * 8, (4, 128))])
